@@ -1298,10 +1298,10 @@ tpe_ctx* tpe_create(int32_t device, int32_t* status) {
         return nullptr;
     }
     cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
-    // the concurrent gradient's share: the factorization and the gradient end
-    // together at V = 8192 (a sweep of 49, 53, 57, 61 SMs: 15.55, 15.08, 14.82,
-    // 14.84 ms per step), and smaller curves factor relatively faster still
-    ctx->grad_sms = ctx->num_sms * 2 / 5;
+    // the concurrent gradient's share: a quarter of the SMs ends it well within the
+    // factorization at V = 8192 (a sweep of 12, 20, 28, 36, 44, 59, 74 SMs: 12.3, 10.9,
+    // 10.9, 10.8, 11.1, 10.9, 11.1 ms per step)
+    ctx->grad_sms = ctx->num_sms / 4;
     if (const char* g = getenv("TPE_GRAD_SMS")) {
         const int n = atoi(g);
         if (n >= 0) ctx->grad_sms = n;  // 0: an ordinary grid over all SMs
@@ -1337,7 +1337,7 @@ void tpe_destroy(tpe_ctx* ctx) {
                       &ctx->mx_Zd, &ctx->mx_Wd, &ctx->grad_ctr, &ctx->mx_ctr, &ctx->mat_Ainv,
                       &ctx->inv_X, &ctx->inv_W, &ctx->inv_T, &ctx->sch_nz, &ctx->sch_S,
                       &ctx->sch_L, &ctx->sch_Linv, &ctx->sch_Sinv, &ctx->sch_vec,
-                      &ctx->ref_r, &ctx->ref_x, &ctx->ycomb_part};
+                      &ctx->ref_r, &ctx->ref_x, &ctx->ycomb_part, &ctx->ev_lists, &ctx->ev_vert};
     for (DevBuf* b : bufs)
         if (b->ptr) cudaFree(b->ptr);
     for (auto& p : ctx->prof_pending) {
@@ -1393,6 +1393,7 @@ int32_t tpe_set_topology(tpe_ctx* ctx, const int32_t* edges, int32_t E, int32_t 
         TPE_TRY(upload(ctx, ctx->d_inc, ctx->h_inc.data(), sizeof(int32_t) * 2 * (size_t)(E > 0 ? E : 1)));
         TPE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
         ctx->has_topology = true;
+        ctx->ev_state = 0;
         ctx->op.valid = false;
         return TPE_OK;
     });

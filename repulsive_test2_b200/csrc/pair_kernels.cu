@@ -5,7 +5,9 @@
 // never materialised: the J edges stream through shared memory in tiles and
 // disjointness is tested from endpoint indices.
 //
-// The context's energy and gradient use the symmetric tile-pair form: each
+// The context's energy and gradient take the (edge, vertex) form of pair_ev.cu;
+// the symmetric tile-pair form here serves topologies with a hub of very high
+// degree, where most pairs share a neighbour. In it each
 // unordered pair is evaluated once for both orders (I, J) and (J, I), which
 // share |d|, d_hat and (|d|+eps)^b. The adjoint gradient recomputes the pair
 // terms (nothing of size E^2 is stored) and uses no atomics: every
@@ -16,6 +18,7 @@
 
 #include <algorithm>
 
+#include "pair_math.cuh"
 #include "tpe_internal.h"
 
 namespace tpe {
@@ -43,32 +46,8 @@ __device__ __forceinline__ double pow_b(double x, double b) {
     return pow(x, b);
 }
 
-// s = sqrt(x), inv_s = 1/s (0 below 1e-14) and inv_se = 1/(s + eps) for x >= 0,
-// from one reciprocal square root r: s = x r and 1/(s + eps) = r / (1 + t) with
-// t = eps r, summed as r (1 - t + t^2) when t < 2^-20 (the first term left out
-// is below 2^-60 relative). Distances within about 1e6 eps of zero (and
-// non-finite input) take the square root and the divisions themselves.
-__device__ __forceinline__ void dist_terms(double x, double eps, double& s, double& inv_s,
-                                           double& inv_se) {
-    const double r = rsqrt(x);
-    const double t = eps * r;
-    if (t < 9.5367431640625e-07) {
-        s = x * r;
-        inv_s = r;
-        inv_se = fma(-r, t * (1.0 - t), r);
-    } else {
-        s = sqrt(x);
-        inv_s = s < 1e-14 ? 0.0 : 1.0 / s;
-        inv_se = 1.0 / (s + eps);
-    }
-}
-
 // sqrt(x) for x >= 0 from a reciprocal square root (0 at x = 0).
 __device__ __forceinline__ double sqrt_r(double x) { return x > 0.0 ? x * rsqrt(x) : sqrt(x); }
-
-__device__ __forceinline__ bool disjoint(int2 a, int2 b) {
-    return a.x != b.x && a.x != b.y && a.y != b.x && a.y != b.y;
-}
 
 // Per-edge records: a = (p1, |e|+eps), b = (p2, (|e|+eps)^(1-alpha)).
 __global__ void edge_prep_kernel(const double* __restrict__ pos, const int2* __restrict__ edges,
@@ -639,6 +618,9 @@ int32_t edge_prep(tpe_ctx* ctx, const double* d_pos, int32_t ncurves, double eps
     const int32_t E = ctx->E;
     TPE_TRY(ensure(ctx, ctx->edge_a, sizeof(double4) * (size_t)E * ncurves));
     TPE_TRY(ensure(ctx, ctx->edge_b, sizeof(double4) * (size_t)E * ncurves));
+    bool ev = false;
+    TPE_TRY(ev_topology(ctx, &ev));
+    if (ev) return ev_prep(ctx, d_pos, ncurves, eps, alpha);
     const int64_t n = (int64_t)E * ncurves;
     KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
     edge_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(
@@ -650,6 +632,17 @@ int32_t edge_prep(tpe_ctx* ctx, const double* d_pos, int32_t ncurves, double eps
 
 int32_t energy_fp64(tpe_ctx* ctx, int32_t ncurves, double alpha, double beta, double eps,
                     double* d_energy) {
+    bool ev = false;
+    TPE_TRY(ev_topology(ctx, &ev));
+    if (ev) {
+        KernelScope ks(ctx, TPE_KGROUP_ENERGY, 2);
+        int32_t nparts = 0;
+        TPE_TRY(ev_energy(ctx, ncurves, alpha, beta, eps, &nparts));
+        reduce_partials<<<ncurves, 256, 0, ctx->stream>>>(ctx->partial.as<double>(), nparts, 0.125,
+                                                          d_energy);
+        TPE_CUDA_TRY(cudaGetLastError());
+        return TPE_OK;
+    }
     const int32_t E = ctx->E;
     const int32_t T = (E + kTile - 1) / kTile;
     const int32_t ntiles = T * (T + 1) / 2;
@@ -709,6 +702,16 @@ int32_t energy_fp64_scratch(cudaStream_t stream, const double* d_pos, const int2
 
 int32_t energy_grad_fp64(tpe_ctx* ctx, double alpha, double beta, double eps, double* d_energy,
                          double* d_grad, int32_t max_blocks) {
+    bool ev = false;
+    TPE_TRY(ev_topology(ctx, &ev));
+    if (ev) {
+        KernelScope ks(ctx, TPE_KGROUP_GRADIENT, 2 + (d_grad ? 1 : 0) + (d_energy ? 1 : 0));
+        TPE_TRY(ev_gradient(ctx, alpha, beta, eps, d_grad, max_blocks));
+        if (d_energy)
+            reduce_partials<<<1, 256, 0, ctx->stream>>>(ctx->partial.as<double>(), ctx->E, 0.125, d_energy);
+        TPE_CUDA_TRY(cudaGetLastError());
+        return TPE_OK;
+    }
     const int32_t E = ctx->E, V = ctx->V;
     const int32_t T = (E + kTile - 1) / kTile;
     const int32_t ntiles = T * (T + 1) / 2;

@@ -143,6 +143,11 @@ struct tpe_ctx {
     std::vector<int32_t> h_inc_off;   // V+1
     std::vector<int32_t> h_inc;       // 2E entries: edge*2 + slot, ascending edge order per vertex
     tpe::DevBuf d_edges, d_inc_off, d_inc;
+    // lists of the (edge, vertex) pair kernels (pair_ev.cu), built on first use:
+    // ev_state 0 not built, 1 in ev_lists, 2 not used for this topology
+    int32_t ev_state = 0, ev_VA = 0;
+    int64_t ev_at[6] = {};
+    tpe::DevBuf ev_lists, ev_vert;
 
     // per-evaluation buffers
     tpe::DevBuf pos, pos2, pos3, edge_a, edge_b, grad, edge_acc, partial, scalars, flat0, flat1,
@@ -265,6 +270,16 @@ int32_t energy_fp64_scratch(cudaStream_t stream, const double* d_pos, const int2
 // bounds the SMs the pair kernel occupies (one block per SM).
 int32_t energy_grad_fp64(tpe_ctx* ctx, double alpha, double beta, double eps, double* d_energy,
                          double* d_grad, int32_t max_blocks = 0);
+
+// ---- (edge, vertex) pair kernels (pair_ev.cu) ---------------------------------
+// The topology's lists, built on first use; *ok = false when the edge-pair
+// kernels serve this topology.
+int32_t ev_topology(tpe_ctx* ctx, bool* ok);
+int32_t ev_prep(tpe_ctx* ctx, const double* d_pos, int32_t ncurves, double eps, double alpha);
+int32_t ev_energy(tpe_ctx* ctx, int32_t ncurves, double alpha, double beta, double eps,
+                  int32_t* nparts);
+int32_t ev_gradient(tpe_ctx* ctx, double alpha, double beta, double eps, double* d_grad,
+                    int32_t max_blocks);
 
 // Barnes-Hut energy (bh.cu) of this context's curve: h_xyz (host) builds the
 // tree, d_xyz (device, the same positions) is traversed. stats (nullable):

@@ -358,7 +358,7 @@ int32_t launch_gradient(tpe_ctx* ctx) {
     {
         StreamSwap sw(ctx, ctx->stream3);
         TPE_TRY(energy_grad_fp64(ctx, ctx->grad_params[0], ctx->grad_params[1], ctx->grad_params[2],
-                                 nullptr, ctx->grad_dE, ctx->grad_sms));
+                                 nullptr, ctx->grad_dE, ctx->grad_first ? 0 : ctx->grad_sms));
     }
     TPE_CUDA_TRY(cudaEventRecord(ctx->ev_grad, ctx->stream3));
     return TPE_OK;
@@ -458,6 +458,7 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
         return TPE_OK;
     };
     const int32_t nrhs = 3 * rows;
+    bool flags_unread = false;  // the FP64 factorization's {singular, timed out}
     if (o && o->precision == TPE_PRECISION_MIXED && nrhs <= kMixedMaxRhs) {
         // FP32 tensor-core factor as the preconditioner of an FP64 CG; the FP64
         // factorization below is the fallback (breakdown or no convergence).
@@ -486,14 +487,6 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
         op.int8 = o && o->precision == TPE_PRECISION_MIXED && k > kLargeSchur &&
                   o->projection_mode == TPE_PROJECTION_FROZEN;
         op.chol_tol = tol;
-        if (!op.int8) {
-            int32_t bad = 0;
-            TPE_TRY(cholesky_fp64(ctx, op.L, op.Linv, V, tol, &bad));
-            if (bad) {
-                *singular = true;
-                return TPE_OK;
-            }
-        }
         if (k > kLargeSchur) {
             // explicit inverses, Y by gathers, the Schur complement on the device
             op.large = true;
@@ -505,11 +498,18 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
                 return TPE_OK;
             }
         } else {
+            // the right-hand sides' forward solves ride along with the factorization
             TPE_TRY(load_rhs());
-            for (int32_t r0 = 0; r0 < nrhs; r0 += 64) {
-                const int32_t nr = (nrhs - r0) < 64 ? (nrhs - r0) : 64;
-                TPE_TRY(chol_solve_fp64(ctx, op.L, op.Linv, V, op.Y + (size_t)r0 * V, nr));
-            }
+            CholDag f;
+            f.L = op.L;
+            f.Linv = op.Linv;
+            f.n = V;
+            f.tol = tol;
+            f.B = op.Y;
+            f.nr = nrhs;
+            TPE_TRY(chol_dag(ctx, f, nullptr));
+            TPE_TRY(chol_solve(ctx, op.L, op.Linv, V, op.Y, nrhs, false));
+            flags_unread = true;
         }
     }
     if (k > 0) {
@@ -522,8 +522,20 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
         row_stats_kernel<<<k, 256, 0, ctx->stream>>>(op.C, V, dR); }
         TPE_CUDA_TRY(cudaGetLastError());
         std::vector<double> rs((size_t)4 * k);
-        if (!op.large) TPE_TRY(download(ctx, op.Scc.data(), dS, sizeof(double) * (size_t)k * k));
-        TPE_TRY(download(ctx, rs.data(), dR, sizeof(double) * 4 * (size_t)k));
+        int32_t late = 0;  // a triangular solve's wait ran out
+        int32_t ff[2] = {0, 0};
+        const HostCopy cp[4] = {
+            {op.Scc.data(), dS, op.large ? 0 : sizeof(double) * (size_t)k * k},
+            {rs.data(), dR, sizeof(double) * 4 * (size_t)k},
+            {&late, ctx->dag_err.ptr, ctx->dag_err.ptr ? sizeof(int32_t) : 0},
+            {ff, ctx->dag_flags.ptr, flags_unread ? sizeof(ff) : 0}};
+        TPE_TRY(download_many(ctx, ctx->stream, cp, 4));
+        TPE_TRY(chol_dag_status(ctx, ff));
+        if (late) return chol_timeout(ctx);
+        if (ff[0]) {
+            *singular = true;
+            return TPE_OK;
+        }
         // symmetrise the Gram matrix (two sides of one dot product)
         if (!op.large)
             for (int32_t i = 0; i < k; i++)
@@ -581,6 +593,15 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
                 *singular = true;
                 return TPE_OK;
             }
+        }
+    }
+    if (k == 0 && flags_unread) {
+        int32_t ff[2] = {0, 0};
+        TPE_TRY(download(ctx, ff, ctx->dag_flags.ptr, sizeof(ff)));
+        TPE_TRY(chol_dag_status(ctx, ff));
+        if (ff[0]) {
+            *singular = true;
+            return TPE_OK;
         }
     }
     op.valid = true;
@@ -720,7 +741,10 @@ int32_t op_solve_once(tpe_ctx* ctx, const double* b_flat, const double* d, doubl
             } else if (op.large) {
                 TPE_TRY(mrhs_fp64(ctx, op.Ainv, V, b_flat, V, 3, w));
             } else {
-                TPE_TRY(chol_solve_fp64(ctx, op.L, op.Linv, V, w, 3));
+                TPE_TRY(chol_solve(ctx, op.L, op.Linv, V, w, 3, true));
+                int32_t out = 0;
+                TPE_TRY(download(ctx, &out, ctx->dag_err.ptr, sizeof(int32_t)));
+                if (out) return chol_timeout(ctx);
             }
         }
         if (k > 0) {
@@ -1337,7 +1361,8 @@ void tpe_destroy(tpe_ctx* ctx) {
                       &ctx->mx_Zd, &ctx->mx_Wd, &ctx->grad_ctr, &ctx->mx_ctr, &ctx->mat_Ainv,
                       &ctx->inv_X, &ctx->inv_W, &ctx->inv_T, &ctx->sch_nz, &ctx->sch_S,
                       &ctx->sch_L, &ctx->sch_Linv, &ctx->sch_Sinv, &ctx->sch_vec,
-                      &ctx->ref_r, &ctx->ref_x, &ctx->ycomb_part, &ctx->ev_lists, &ctx->ev_vert};
+                      &ctx->ref_r, &ctx->ref_x, &ctx->ycomb_part, &ctx->ev_lists, &ctx->ev_vert,
+                      &ctx->dag_flags, &ctx->dag_solve, &ctx->dag_err};
     for (DevBuf* b : bufs)
         if (b->ptr) cudaFree(b->ptr);
     for (auto& p : ctx->prof_pending) {
@@ -1723,7 +1748,7 @@ int32_t step_impl(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, cons
         // and factors A_rho (a latency-bound chain); the solve joins it.
         // op_build launches it right after the assembly (launch_gradient), so it
         // overlaps the factorization and not the (equally compute-bound) Gram
-        // assembly.
+        // assembly; but see grad_first.
         TPE_TRY(edge_prep(ctx, P, 1, o->epsilon, o->alpha));
         ctx->grad_unlaunched = true;
         ctx->grad_params[0] = o->alpha;
@@ -1734,6 +1759,11 @@ int32_t step_impl(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, cons
         ctx->grad_dE = dE;
         ctx->grad_flat = ctx->flat2.as<double>();
         ctx->grad_pen = pen ? &o->penalties : nullptr;
+        // The FP64 factorization of a small constraint set takes the right-hand
+        // sides along (their forward solves), so there the gradient runs beside
+        // the assembly, on all SMs.
+        ctx->grad_first = o->precision != TPE_PRECISION_MIXED && S.k <= kLargeSchur;
+        if (ctx->grad_first) TPE_TRY(launch_gradient(ctx));
     } else {
         // sequential (finite differences, or the per-phase timing ledger)
         {

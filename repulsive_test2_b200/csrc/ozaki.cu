@@ -538,7 +538,7 @@ struct InvCtx {
     double* X;  // L^{-1}, lower
     double* W;  // X^T, upper
     double* Tt;
-    double* base;  // kBase^2 (block) + 64 kBase (diagonal inverses) + 2 kBase^2 (X, W) + T
+    double* base;  // kBase^2 (block) + 64 kBase (diagonal inverses) + 2 kBase^2 (X, W)
     int32_t n;
     double tol;
     int32_t nbase;
@@ -572,16 +572,24 @@ int32_t inv_base(InvCtx& c, int32_t o, int32_t m) {
     double* Binv = Bm + (size_t)kBase * kBase;
     double* Xb = Binv + (size_t)kBase * kNB;  // (kBase / 64) diagonal 64 x 64 inverses
     double* Wb = Xb + (size_t)kBase * kBase;
-    double* Tb = Wb + (size_t)kBase * kBase;
     TPE_CUDA_TRY(cudaMemcpy2DAsync(Bm, sizeof(double) * m, c.M + o * n + o, sizeof(double) * n,
                                    sizeof(double) * m, m, cudaMemcpyDeviceToDevice, st));
+    // (the products' triangular K ranges start at 128-column tiles: zeros beside the tiles)
+    TPE_CUDA_TRY(cudaMemsetAsync(Xb, 0, sizeof(double) * (size_t)m * m, st));
+    TPE_CUDA_TRY(cudaMemsetAsync(Wb, 0, sizeof(double) * (size_t)m * m, st));
+    CholDag f;
+    f.L = Bm;
+    f.Linv = Binv;
+    f.n = m;
+    f.tol = c.tol;
+    f.W = Wb;
+    f.X = Xb;
     int32_t bad = 0;
-    TPE_TRY(cholesky_fp64(ctx, Bm, Binv, m, c.tol, &bad));
+    TPE_TRY(chol_dag(ctx, f, &bad));
     if (bad) {
         c.singular = true;
         return TPE_OK;
     }
-    TPE_TRY(lower_inverse_fp64(ctx, Bm, Binv, m, Xb, Wb, Tb));
     TPE_CUDA_TRY(cudaMemcpy2DAsync(c.X + o * n + o, sizeof(double) * n, Xb, sizeof(double) * m,
                                    sizeof(double) * m, m, cudaMemcpyDeviceToDevice, st));
     TPE_CUDA_TRY(cudaMemcpy2DAsync(c.W + o * n + o, sizeof(double) * n, Wb, sizeof(double) * m,
@@ -625,8 +633,7 @@ int32_t spd_inverse_int8(tpe_ctx* ctx, double* Mat, int32_t n, double piv_tol, d
     *singular = false;
     if (n <= 0) return TPE_OK;
     TPE_TRY(ozaki_reserve(ctx, ozaki_scratch_bytes(n, 0, n)));
-    const size_t base_doubles = (size_t)kBase * kBase * 3 + (size_t)kBase * kNB +
-                                (size_t)(kBase / 2 + kNB) * (kBase / 2 + kNB);
+    const size_t base_doubles = (size_t)kBase * kBase * 3 + (size_t)kBase * kNB;
     TPE_TRY(ensure(ctx, ctx->oz_base, sizeof(double) * base_doubles));
     TPE_CUDA_TRY(cudaMemsetAsync(X, 0, sizeof(double) * (size_t)n * n, ctx->stream));
     TPE_CUDA_TRY(cudaMemsetAsync(W, 0, sizeof(double) * (size_t)n * n, ctx->stream));

@@ -7,8 +7,8 @@
 // Schur complement S = C A3^{-1} C^T (A3 = A_rho per coordinate block), which the
 // small-k path forms from k x 3 solves and factors on the host. For large k that
 // is k^3 host work and 3k solves; here instead:
-//   Ainv = A_rho^{-1} explicitly (FP64: Cholesky, recursive triangular
-//   inverse, X^T X), then Y = A3^{-1} C^T row by row as a gather of at most
+//   Ainv = A_rho^{-1} explicitly (FP64: factor, L^-T and W W^T in one kernel,
+//   chol_dag.cu), then Y = A3^{-1} C^T row by row as a gather of at most
 //   kNZ rows of Ainv per coordinate block (an edge-length row has two nonzeros
 //   per block); rows with more nonzeros (barycenter) go through one multi-RHS
 //   product with Ainv;
@@ -186,12 +186,14 @@ int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool
     const size_t nn = (size_t)nmax * nmax;
     const size_t half = (size_t)(nmax / 2 + kNB) * (nmax / 2 + kNB);
     TPE_TRY(ensure(ctx, ctx->mat_Ainv, sizeof(double) * (size_t)V * V));
-    TPE_TRY(ensure(ctx, ctx->inv_X, sizeof(double) * nn));
     TPE_TRY(ensure(ctx, ctx->inv_W, sizeof(double) * nn));
-    TPE_TRY(ensure(ctx, ctx->inv_T, sizeof(double) * half));
-    double* Ainv = ctx->mat_Ainv.as<double>();
     if (op.int8) {
-        // op.L holds A_rho unfactored; it is overwritten
+        TPE_TRY(ensure(ctx, ctx->inv_X, sizeof(double) * nn));
+        TPE_TRY(ensure(ctx, ctx->inv_T, sizeof(double) * half));
+    }
+    double* Ainv = ctx->mat_Ainv.as<double>();
+    // op.L holds A_rho unfactored; it is overwritten
+    if (op.int8) {
         bool sing = false;
         TPE_TRY(spd_inverse_int8(ctx, op.L, V, op.chol_tol, ctx->inv_X.as<double>(),
                                  ctx->inv_W.as<double>(), ctx->inv_T.as<double>(), Ainv, &sing));
@@ -200,8 +202,19 @@ int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool
             return TPE_OK;
         }
     } else {
-        TPE_TRY(spd_inverse_fp64(ctx, op.L, op.Linv, V, ctx->inv_X.as<double>(),
-                                 ctx->inv_W.as<double>(), ctx->inv_T.as<double>(), Ainv));
+        CholDag f;  // factor, L^-T and inverse in one kernel
+        f.L = op.L;
+        f.Linv = op.Linv;
+        f.n = V;
+        f.tol = op.chol_tol;
+        f.W = ctx->inv_W.as<double>();
+        f.Ainv = Ainv;
+        int32_t bad = 0;
+        TPE_TRY(chol_dag(ctx, f, &bad));
+        if (bad) {
+            *singular = true;
+            return TPE_OK;
+        }
     }
     op.Ainv = Ainv;
     // sparse structure of C
@@ -265,15 +278,19 @@ int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool
             return TPE_OK;
         }
     } else {
+        CholDag f;
+        f.L = Ls;
+        f.Linv = ctx->sch_Linv.as<double>();
+        f.n = k;
+        f.tol = 0.0;
+        f.W = ctx->inv_W.as<double>();
+        f.Ainv = ctx->sch_Sinv.as<double>();
         int32_t bad = 0;
-        TPE_TRY(cholesky_fp64(ctx, Ls, ctx->sch_Linv.as<double>(), k, 0.0, &bad));
+        TPE_TRY(chol_dag(ctx, f, &bad));
         if (bad) {
             *singular = true;
             return TPE_OK;
         }
-        TPE_TRY(spd_inverse_fp64(ctx, Ls, ctx->sch_Linv.as<double>(), k, ctx->inv_X.as<double>(),
-                                 ctx->inv_W.as<double>(), ctx->inv_T.as<double>(),
-                                 ctx->sch_Sinv.as<double>()));
     }
     op.Sinv = ctx->sch_Sinv.as<double>();
     return TPE_OK;

@@ -118,6 +118,7 @@ struct tpe_ctx {
     // a gradient launched on stream3 and not yet joined (step_impl / finish_gradient)
     bool grad_pending = false;
     bool grad_unlaunched = false;
+    bool grad_first = false;  // before the assembly, on all SMs: the factorization needs it (step_impl)
     double grad_params[3] = {0, 0, 0};  // alpha, beta, eps
     const double* grad_pos = nullptr;
     double* grad_dE = nullptr;
@@ -159,6 +160,8 @@ struct tpe_ctx {
     tpe::DevBuf oz_planes, oz_err;  // digit planes and timeout flag of ozaki_gemm_nt
     tpe::DevBuf oz_base;            // the FP64 base blocks of spd_inverse_int8
     tpe::DevBuf bh_buf;             // Barnes-Hut tree, permutation and per-edge sums (bh.cu)
+    tpe::DevBuf dag_solve, dag_err;  // the same of the triangular solves, and their error flag
+    tpe::DevBuf dag_flags;     // flags and counters of the data-flow factorization (chol_dag.cu)
     tpe::DevBuf ycomb_part;    // split-over-rows partial sums of Y^T coef
     tpe::DevBuf mx_ctr;    // tile counters of the persistent trailing updates
     tpe::DevBuf pairM;                      // E x E double2 (Mb, M0) pair matrix
@@ -308,13 +311,32 @@ int32_t assemble_fp64(tpe_ctx* ctx, double alpha, double beta, double eps, doubl
                       double* d_B, double* d_B0);
 
 // ---- dense linear algebra (dense.cu) --------------------------------------
-// In-place lower Cholesky of the V x V row-major matrix (lower triangle read);
-// also writes the inverses of the 64x64 diagonal blocks. Sets *singular.
-int32_t cholesky_fp64(tpe_ctx* ctx, double* d_L, double* d_Linv, int32_t n, double piv_tol,
-                      int32_t* singular);
-// Solves (L L^T) X = B in place for nrhs right-hand sides stored as B[nrhs][n].
-int32_t chol_solve_fp64(tpe_ctx* ctx, const double* d_L, const double* d_Linv, int32_t n,
-                        double* d_B, int32_t nrhs);
+// Lower Cholesky of an n x n row-major matrix as one data-flow kernel
+// (chol_dag.cu), optionally with rows of right-hand sides (B <- B L^-T, the
+// forward solves), W = L^-T (upper tiles; X = L^-1, lower tiles) and the symmetric
+// inverse Ainv = W W^T. A pivot at or below tol sets *singular.
+struct CholDag {
+    double* L = nullptr;     // lower triangle read; L on return
+    double* Linv = nullptr;  // nb x 64 x 64: inverses of L's diagonal blocks
+    int32_t n = 0;
+    double tol = 0.0;
+    double* B = nullptr;  // nr x n
+    int32_t nr = 0;
+    double* W = nullptr;  // n x n or null; X and Ainv need it
+    double* X = nullptr;
+    double* Ainv = nullptr;
+};
+// With singular = null nothing is read back: the caller reads the two ints at
+// ctx->dag_flags ({singular, timed out}) with its next copy and passes them to
+// chol_dag_status before it uses the result.
+int32_t chol_dag(tpe_ctx* ctx, const CholDag& c, int32_t* singular);
+int32_t chol_dag_status(tpe_ctx* ctx, const int32_t flags[2]);
+// Solves (L L^T) X = B in place for nr right-hand sides stored as B[nr][n]
+// (down = false: only L^T X = B). A wait that runs out leaves NaN in B and sets
+// ctx->dag_err, for which the caller returns chol_timeout once it has read it.
+int32_t chol_solve(tpe_ctx* ctx, const double* d_L, const double* d_Linv, int32_t n, double* d_B,
+                   int32_t nr, bool down);
+int32_t chol_timeout(tpe_ctx* ctx);
 // out[i*ncols + j] = dot(X[i], Y[j]) over len (rows of length len): FP64, deterministic.
 int32_t gram_dots(tpe_ctx* ctx, const double* X, int32_t nx, const double* Y, int32_t ny,
                   int64_t len, double* d_out);
@@ -348,15 +370,6 @@ int32_t ozaki_reserve(tpe_ctx* ctx, size_t bytes);
 int32_t ozaki_gemm_nt(tpe_ctx* ctx, const DGemmArgs& g, cudaStream_t stream,
                       int group = TPE_KGROUP_TRSV);
 int32_t ozaki_status(tpe_ctx* ctx, cudaStream_t stream);
-// out = (L L^T)^{-1}, n x n symmetric, from the Cholesky factor and its 64x64
-// diagonal-block inverses (cholesky_fp64); X, W (n x n) and Tt ((n/2 + 64)^2)
-// are scratch. X = L^{-1} by recursive halving, then out = X^T X.
-int32_t spd_inverse_fp64(tpe_ctx* ctx, const double* d_L, const double* d_Linv, int32_t n,
-                         double* X, double* W, double* Tt, double* out);
-// X = L^{-1} (lower) and W = X^T (upper), n x n, from the Cholesky factor and its
-// 64x64 diagonal-block inverses (the first half of spd_inverse_fp64).
-int32_t lower_inverse_fp64(tpe_ctx* ctx, const double* d_L, const double* d_Linv, int32_t n,
-                           double* X, double* W, double* Tt);
 // M[j][i] = M[i][j] for j > i (n x n, row-major).
 int32_t mirror_lower(tpe_ctx* ctx, double* M, int32_t n);
 // dst[j][i] = src[i][j] for an m x c block (row strides lds, ldd).
@@ -365,8 +378,7 @@ int32_t transpose_fp64(tpe_ctx* ctx, const double* src, int64_t lds, int32_t m, 
 // out = A^{-1} for the SPD n x n matrix in Mat (lower triangle read; Mat is
 // overwritten) with the heavy products on the integer tensor cores
 // (ozaki_gemm_nt): recursive Cholesky and triangular inverse in halves down to
-// blocks of at most 1024 (cholesky_fp64 + lower_inverse_fp64 there), then
-// out = X^T X. X, W (n x n) and Tt ((n/2 + 64)^2) are scratch. A pivot at or
+// blocks of at most 1024 (chol_dag there), then out = X^T X. X, W (n x n) and Tt ((n/2 + 64)^2) are scratch. A pivot at or
 // below piv_tol sets *singular.
 int32_t spd_inverse_int8(tpe_ctx* ctx, double* Mat, int32_t n, double piv_tol, double* X,
                          double* W, double* Tt, double* out, bool* singular);
@@ -400,7 +412,7 @@ constexpr int32_t kLargeRefineMax = 4;
 // same or stall far above this (rows whose entries span many orders of
 // magnitude lose digits under a per-row scale).
 constexpr double kInt8ResidualGate = 1e-12;
-// From the FP64 factor op.L: op.Ainv, op.Y (k x 3V), op.W = A3^{-1} b when b is
+// From A_rho in op.L (overwritten): op.Ainv, op.Y (k x 3V), op.W = A3^{-1} b when b is
 // given, and op.Sinv; *singular when the Schur complement is not SPD.
 int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool* singular);
 // out[c] = Sinv rc[c] for nr host vectors of length k (host in and out).

@@ -22,7 +22,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <array>
 #include <chrono>
 #include <vector>
 
@@ -439,11 +438,14 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
     // Y = Abar_rho^{-1} C^T (3k right-hand sides of length V) and, when given,
     // w = Abar_rho^{-1} b (3 more), solved together.
     const int32_t rows = k + (b_flat ? 1 : 0);
-    TPE_TRY(ensure(ctx, ctx->con_Y, sizeof(double) * (size_t)(rows > 0 ? rows : 1) * 3 * V));
-    op.Y = ctx->con_Y.as<double>();
-    if (b_flat) {
-        op.W = op.Y + (size_t)k * 3 * V;
-        op.w_src = b_flat;
+    // (large sets: large_schur_build, for the dense rows only)
+    if (k <= kLargeSchur) {
+        TPE_TRY(ensure(ctx, ctx->con_Y, sizeof(double) * (size_t)(rows > 0 ? rows : 1) * 3 * V));
+        op.Y = ctx->con_Y.as<double>();
+        if (b_flat) {
+            op.W = op.Y + (size_t)k * 3 * V;
+            op.w_src = b_flat;
+        }
     }
     // the right-hand sides, loaded right before the solves (b may still be in
     // the making on another stream: finish_gradient joins it)
@@ -517,10 +519,12 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
                                                          4 * (size_t)k + 16)));
         double* dS = ctx->tmp.as<double>();
         if (!op.large) TPE_TRY(gram_dots(ctx, op.C, k, op.Y, k, 3 * (int64_t)V, dS));
-        double* dR = dS + (op.large ? 0 : (size_t)k * k);
-        { KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
-        row_stats_kernel<<<k, 256, 0, ctx->stream>>>(op.C, V, dR); }
-        TPE_CUDA_TRY(cudaGetLastError());
+        double* dR = op.large ? op.sp.stats : dS + (size_t)k * k;
+        if (!op.large) {
+            KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+            row_stats_kernel<<<k, 256, 0, ctx->stream>>>(op.C, V, dR);
+            TPE_CUDA_TRY(cudaGetLastError());
+        }
         std::vector<double> rs((size_t)4 * k);
         int32_t late = 0;  // a triangular solve's wait ran out
         int32_t ff[2] = {0, 0};
@@ -569,7 +573,7 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
                 std::vector<double> su3((size_t)3 * k), z3((size_t)3 * k);
                 for (int c = 0; c < 3; c++)
                     for (int32_t r = 0; r < k; r++) su3[(size_t)c * k + r] = op.Scu[(size_t)r * 3 + c];
-                TPE_TRY(large_schur_apply(ctx, op, su3.data(), 3, z3.data()));
+                TPE_TRY(large_sinv(ctx, op, su3.data(), 3, z3.data()));
                 for (int c = 0; c < 3; c++)
                     Z[c].assign(z3.begin() + (size_t)c * k, z3.begin() + (size_t)(c + 1) * k);
             } else {
@@ -593,6 +597,7 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
                 *singular = true;
                 return TPE_OK;
             }
+            if (op.large) TPE_TRY(large_set_mu(ctx, op, op.Scu.data(), op.M.data()));
         }
     }
     if (k == 0 && flags_unread) {
@@ -632,23 +637,15 @@ int32_t op_build(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int32_t k, 
 }
 
 // Multipliers of the bordered Schur system for the reduced right-hand side
-// rc = C w - d (k) and ru = U^T w (3): lam (k) and mu (3).
-int32_t schur_multipliers(tpe_ctx* ctx, const SaddleOp& op, const std::vector<double>& rc,
-                          const double* ru, std::vector<double>& lam, double mu[3]) {
+// rc = C w - d (k) and ru = U^T w (3): lam (k) and mu (3). (Large sets: large_multipliers.)
+void schur_multipliers(const SaddleOp& op, const std::vector<double>& rc, const double* ru,
+                       std::vector<double>& lam, double mu[3]) {
     const int32_t k = op.k;
     lam.assign((size_t)k, 0.0);
     mu[0] = mu[1] = mu[2] = 0.0;
-    if (k == 0) return TPE_OK;
-    auto scc_solve = [&](std::vector<double>& b) -> int32_t {
-        if (op.large) {
-            std::vector<double> in = b;
-            return large_schur_apply(ctx, op, in.data(), 1, b.data());
-        }
-        host_chol_solve(op.Scc, k, b);
-        return TPE_OK;
-    };
+    if (k == 0) return;
     std::vector<double> t = rc;
-    TPE_TRY(scc_solve(t));
+    host_chol_solve(op.Scc, k, t);
     if (op.trans_constrained) {
         std::vector<double> rhs(3);
         for (int c = 0; c < 3; c++) {
@@ -661,55 +658,11 @@ int32_t schur_multipliers(tpe_ctx* ctx, const SaddleOp& op, const std::vector<do
         std::vector<double> r2 = rc;
         for (int32_t r = 0; r < k; r++)
             for (int c = 0; c < 3; c++) r2[r] -= op.Scu[(size_t)r * 3 + c] * mu[c];
-        TPE_TRY(scc_solve(r2));
+        host_chol_solve(op.Scc, k, r2);
         lam = r2;
     } else {
         lam = t;
     }
-    return TPE_OK;
-}
-
-// schur_multipliers for several reduced right-hand sides at once (the trials
-// of a batched projection): with a large constraint set the Sinv products of
-// all of them share one pass over Sinv; otherwise one host solve each.
-int32_t schur_multipliers_multi(tpe_ctx* ctx, const SaddleOp& op,
-                                const std::vector<std::vector<double>>& rcs, const double* ru,
-                                std::vector<std::vector<double>>& lams,
-                                std::vector<std::array<double, 3>>& mus) {
-    const int32_t k = op.k, n = (int32_t)rcs.size();
-    lams.assign((size_t)n, std::vector<double>((size_t)k, 0.0));
-    mus.assign((size_t)n, {0.0, 0.0, 0.0});
-    if (n == 0 || k == 0) return TPE_OK;
-    if (!op.large) {
-        for (int32_t q = 0; q < n; q++) TPE_TRY(schur_multipliers(ctx, op, rcs[q], ru, lams[q], mus[q].data()));
-        return TPE_OK;
-    }
-    std::vector<double> in((size_t)n * k), t((size_t)n * k);
-    for (int32_t q = 0; q < n; q++) std::copy(rcs[q].begin(), rcs[q].end(), in.begin() + (size_t)q * k);
-    TPE_TRY(large_schur_apply(ctx, op, in.data(), n, t.data()));
-    if (!op.trans_constrained) {
-        for (int32_t q = 0; q < n; q++)
-            std::copy(t.begin() + (size_t)q * k, t.begin() + (size_t)(q + 1) * k, lams[q].begin());
-        return TPE_OK;
-    }
-    for (int32_t q = 0; q < n; q++) {
-        const double* tq = t.data() + (size_t)q * k;
-        std::vector<double> rhs(3);
-        for (int c = 0; c < 3; c++) {
-            double s = 0;
-            for (int32_t r = 0; r < k; r++) s += op.Scu[(size_t)r * 3 + c] * tq[r];
-            rhs[c] = s - ru[c];
-        }
-        host_chol_solve(op.M, 3, rhs);
-        for (int c = 0; c < 3; c++) mus[q][c] = rhs[c];
-        double* r2 = in.data() + (size_t)q * k;
-        for (int32_t r = 0; r < k; r++)
-            for (int c = 0; c < 3; c++) r2[r] -= op.Scu[(size_t)r * 3 + c] * mus[q][c];
-    }
-    TPE_TRY(large_schur_apply(ctx, op, in.data(), n, t.data()));
-    for (int32_t q = 0; q < n; q++)
-        std::copy(t.begin() + (size_t)q * k, t.begin() + (size_t)(q + 1) * k, lams[q].begin());
-    return TPE_OK;
 }
 
 // One solve with the current operator: b_flat (device, 3V, or null = 0), d
@@ -749,7 +702,10 @@ int32_t op_solve_once(tpe_ctx* ctx, const double* b_flat, const double* d, doubl
         }
         if (k > 0) {
             TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double) * ((size_t)k + 16)));
-            TPE_TRY(gram_dots(ctx, op.C, k, w, 1, m, ctx->tmp.as<double>()));
+            if (op.large)
+                TPE_TRY(large_cx(ctx, op, w, ctx->tmp.as<double>()));
+            else
+                TPE_TRY(gram_dots(ctx, op.C, k, w, 1, m, ctx->tmp.as<double>()));
             TPE_TRY(download(ctx, rc.data(), ctx->tmp.as<double>(), sizeof(double) * k));
         }
         if (op.trans_constrained) {
@@ -763,8 +719,18 @@ int32_t op_solve_once(tpe_ctx* ctx, const double* b_flat, const double* d, doubl
     }
     if (d)
         for (int32_t r = 0; r < k; r++) rc[r] -= d[r];
+    if (op.large && k > 0) {
+        TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double) * ((size_t)k + 16)));
+        TPE_CUDA_TRY(cudaMemcpyAsync(ctx->tmp.ptr, rc.data(), sizeof(double) * (size_t)k, cudaMemcpyHostToDevice,
+                                     ctx->stream));
+        double* coef = nullptr;
+        TPE_TRY(large_multipliers(ctx, op, ctx->tmp.as<double>(), k, nullptr, 1, ru.data(), &coef));
+        TPE_TRY(large_solution(ctx, op, coef, b_flat ? w : nullptr, x_flat));
+        lam.assign((size_t)k, 0.0);
+        return download(ctx, lam.data(), coef, sizeof(double) * (size_t)k);
+    }
     double mu[3] = {0, 0, 0};
-    TPE_TRY(schur_multipliers(ctx, op, rc, ru.data(), lam, mu));
+    schur_multipliers(op, rc, ru.data(), lam, mu);
     TPE_TRY(combine_solution(ctx, b_flat ? w : nullptr, op.Y, k, lam.data(), mu, op.rho, V,
                              x_flat));
     return TPE_OK;
@@ -793,7 +759,7 @@ int32_t op_solve(tpe_ctx* ctx, const double* b_flat, const double* d, double* x_
         for (int32_t it = 0;; it++) {
             double r0 = 0.0;
             TPE_TRY(saddle_residual(ctx, op.A, V, op.C, k, x_flat, lam.data(), b_flat, bottom.data(),
-                                    &r0, rt, rb.data()));
+                                    &r0, rt, rb.data(), &op));
             const bool done = it > 0 && (!(r0 > kRefineStop) || !(r0 < 0.5 * prev) ||
                                          it >= kLargeRefineMax);
             if (done) {
@@ -817,7 +783,7 @@ int32_t op_solve(tpe_ctx* ctx, const double* b_flat, const double* d, double* x_
         if (d)
             for (int32_t r = 0; r < k; r++) bottom[r] = d[r];
         TPE_TRY(saddle_residual(ctx, op.A, V, op.C, k, x_flat, lam.data(), top, bottom.data(),
-                                residual));
+                                residual, nullptr, nullptr, op.large ? &op : nullptr));
     }
     return TPE_OK;
 }
@@ -984,9 +950,9 @@ int32_t project_batch_dev(tpe_ctx* ctx, const double* d_start, int32_t ntrial, c
         iters[a] = o->proj_max_iter;
         phi_norm[a] = INFINITY;
     }
-    TPE_TRY(ensure(ctx, ctx->status, sizeof(int32_t) * (4 + 2 * (size_t)ntrial)));
+    TPE_TRY(ensure(ctx, ctx->status, sizeof(int32_t) * (4 + 3 * (size_t)ntrial)));
     int32_t* d_bad = ctx->status.as<int32_t>() + 4;
-    int32_t* d_idx = d_bad + ntrial;
+    int32_t* d_idx = d_bad + ntrial;  // and the positions of the corrected ones in it
     TPE_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int32_t) * ntrial, ctx->stream));
     TPE_TRY(ensure(ctx, ctx->con_red, sizeof(double) * (size_t)ntrial * ((size_t)k + 2 * nb + k + 3)));
     double* d_phi = ctx->con_red.as<double>();
@@ -995,9 +961,9 @@ int32_t project_batch_dev(tpe_ctx* ctx, const double* d_start, int32_t ntrial, c
     std::vector<double> phi((size_t)ntrial * k), ns((size_t)ntrial * 2 * nb);
     std::vector<int32_t> hbad(ntrial, 0);
     std::vector<double> coef;
-    std::vector<std::vector<double>> rcs, lams;
-    std::vector<std::array<double, 3>> mus;
-    std::vector<int32_t> upd;
+    std::vector<std::vector<double>> rcs;
+    std::vector<double> lam;
+    std::vector<int32_t> upd, pos;
     const double ru[3] = {0.0, 0.0, 0.0};
     for (int32_t it = 0; it <= o->proj_max_iter && !active.empty(); it++) {
         const int32_t na = (int32_t)active.size();
@@ -1012,6 +978,7 @@ int32_t project_batch_dev(tpe_ctx* ctx, const double* d_start, int32_t ntrial, c
         }
         std::vector<int32_t> next;
         upd.clear();
+        pos.clear();
         coef.clear();
         rcs.clear();
         for (int32_t q = 0; q < na; q++) {
@@ -1044,20 +1011,35 @@ int32_t project_batch_dev(tpe_ctx* ctx, const double* d_start, int32_t ntrial, c
                 iters[a] = it;
                 continue;
             }
-            std::vector<double> rc((size_t)k);
-            for (int32_t r = 0; r < k; r++) rc[r] = 0.0 - (-ph[r]);
-            rcs.push_back(std::move(rc));
+            if (op.large) {
+                pos.push_back(q);  // its Phi is the reduced right-hand side, on the device
+            } else {
+                std::vector<double> rc((size_t)k);
+                for (int32_t r = 0; r < k; r++) rc[r] = 0.0 - (-ph[r]);
+                rcs.push_back(std::move(rc));
+            }
             upd.push_back(a);
             next.push_back(a);
         }
         active = next;
         if (upd.empty()) break;
-        // the Newton multipliers of every trial corrected this iteration, together
-        TPE_TRY(schur_multipliers_multi(ctx, op, rcs, ru, lams, mus));
+        if (op.large) {
+            Timer t(ctx, timings, TPE_PHASE_SADDLE);
+            const int32_t nu = (int32_t)upd.size();
+            upd.insert(upd.end(), pos.begin(), pos.end());
+            TPE_CUDA_TRY(cudaMemcpyAsync(d_idx, upd.data(), sizeof(int32_t) * 2 * nu, cudaMemcpyHostToDevice,
+                                         ctx->stream));
+            double* d_c = nullptr;
+            TPE_TRY(large_multipliers(ctx, op, d_phi, k, d_idx + nu, nu, ru, &d_c));
+            TPE_TRY(large_update(ctx, op, d_c, nu, d_idx, d_cur, m, d_bad));
+            continue;
+        }
         const double su = 1.0 / (op.rho * sqrt((double)V));
         for (size_t q = 0; q < upd.size(); q++) {
-            for (int32_t r = 0; r < k; r++) coef.push_back(lams[q][r]);
-            for (int c = 0; c < 3; c++) coef.push_back(mus[q][c] * su);
+            double mu[3];
+            schur_multipliers(op, rcs[q], ru, lam, mu);
+            coef.insert(coef.end(), lam.begin(), lam.end());
+            for (int c = 0; c < 3; c++) coef.push_back(mu[c] * su);
         }
         {
             Timer t(ctx, timings, TPE_PHASE_SADDLE);
@@ -1359,10 +1341,11 @@ void tpe_destroy(tpe_ctx* ctx) {
                       &ctx->mx_Lhi, &ctx->mx_Llo, &ctx->mx_Zhi, &ctx->mx_Zlo, &ctx->mx_Whi,
                       &ctx->mx_Wlo, &ctx->mx_Thi, &ctx->mx_Tlo, &ctx->mx_T2hi, &ctx->mx_T2lo, &ctx->mx_vec, &ctx->mx_part,
                       &ctx->mx_Zd, &ctx->mx_Wd, &ctx->grad_ctr, &ctx->mx_ctr, &ctx->mat_Ainv,
-                      &ctx->inv_X, &ctx->inv_W, &ctx->inv_T, &ctx->sch_nz, &ctx->sch_S,
-                      &ctx->sch_L, &ctx->sch_Linv, &ctx->sch_Sinv, &ctx->sch_vec,
+                      &ctx->inv_X, &ctx->inv_W, &ctx->inv_T, &ctx->sch_nz, &ctx->sch_G, &ctx->sch_S,
+                      &ctx->sch_Linv, &ctx->sch_Sinv, &ctx->sch_vec,
                       &ctx->ref_r, &ctx->ref_x, &ctx->ycomb_part, &ctx->ev_lists, &ctx->ev_vert,
-                      &ctx->dag_flags, &ctx->dag_solve, &ctx->dag_err};
+                      &ctx->dag_flags, &ctx->dag_solve, &ctx->dag_err,
+                      &ctx->mrhs_xt};
     for (DevBuf* b : bufs)
         if (b->ptr) cudaFree(b->ptr);
     for (auto& p : ctx->prof_pending) {

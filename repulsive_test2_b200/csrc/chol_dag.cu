@@ -54,13 +54,14 @@ constexpr int kTile = NB * kTP;
 constexpr int64_t kSpin = 1 << 22;  // polls before a wait gives up (seconds)
 
 struct Dag {
-    double* L;     // n x n: A on entry (lower), L on return
+    double* L;     // n x n (rows ld apart): A on entry (lower), L on return
     double* Linv;  // nb x 64 x 64: inverses of the diagonal blocks
     double* B;     // nr rows of n: right-hand sides on entry, B L^-T on return
-    double* W;     // n x n, upper: L^-T (its diagonal tiles whole), or null
-    double* X;     // n x n, lower: L^-1, or null
+    double* W;     // n x n (ld), upper: L^-T (its diagonal tiles whole), or null
+    double* X;     // n x n (ld), lower: L^-1, or null
     double* Ainv;  // n x n, or null
     int32_t n, nb, nr, nrb;  // nrb row blocks of right-hand sides
+    int64_t ld;              // row length of L, W and X (n or more); B and Ainv have n
     double tol;
     int32_t* flag;  // [(nb + nrb + nb) x nb] tiles done, then diag, preA, preD [nb each]
     int32_t* ctl;   // [0] a pivot failed, [1] a wait ran out, [2] role ticket, [3] tile counter
@@ -461,9 +462,10 @@ __device__ __forceinline__ int64_t column_count(const Dag& g, int32_t c) {
 template <bool kAl>
 __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, int32_t x) {
     const int32_t nb = g.nb, n = g.n;
+    const int64_t ld = g.ld;
     int32_t* diag = g.flag + (int64_t)(2 * nb + g.nrb) * nb;
     const int32_t s = min(NB, n - j * NB);  // columns of this tile
-    const Rows Lj{g.L + (int64_t)j * NB * n, n, s};
+    const Rows Lj{g.L + (int64_t)j * NB * ld, ld, s};
     const int32_t* fj = g.flag + (int64_t)j * nb;
     const int32_t below = nb - j - 1;  // rows under the diagonal block
     double* O = dyn_tile();  // the tile as it is in memory, fetched ahead of the sum
@@ -472,15 +474,15 @@ __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, i
         // sums of the chain's next tile (x = 0) and next diagonal block (x = 1)
         if (j == 0) return true;
         const int32_t i = j + 1, rows = min(NB, n - i * NB);
-        const Rows Li{g.L + (int64_t)i * NB * n, n, rows};
+        const Rows Li{g.L + (int64_t)i * NB * ld, ld, rows};
         const int32_t* fi = g.flag + (int64_t)i * nb;
-        double* out = g.L + (int64_t)i * NB * n + (int64_t)(x == 0 ? j : i) * NB;
+        double* out = g.L + (int64_t)i * NB * ld + (int64_t)(x == 0 ? j : i) * NB;
         load_tile<kAl>(O, Li, (x == 0 ? j : i) * NB, n);
         cp_commit();
         acc.zero();
         if (!sum_tiles<kAl>(g, sm, acc, Li, fi, x == 0 ? Lj : Li, x == 0 ? fj : fi, 0, j)) return false;
         each(acc, [&](int r, int c, double v) {
-            if (r < rows && (x == 0 || c <= r)) out[(int64_t)r * n + c] = O[r * kTP + c] - v;
+            if (r < rows && (x == 0 || c <= r)) out[r * ld + c] = O[r * kTP + c] - v;
         });
         raise(diag + nb + (x == 0 ? 0 : nb) + j);
         return true;
@@ -494,8 +496,8 @@ __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, i
     if (x < below - 1) {
         const int32_t i = j + 2 + x;
         gid = i;
-        out = g.L + (int64_t)i * NB * n;
-        A = Rows{out, n, min(NB, n - i * NB)};
+        out = g.L + (int64_t)i * NB * ld;
+        A = Rows{out, ld, min(NB, n - i * NB)};
     } else if ((x -= std::max(0, below - 1)) < g.nrb) {
         gid = nb + x;
         out = g.B + (int64_t)x * NB * n;
@@ -503,8 +505,8 @@ __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, i
     } else {
         const int32_t c = x - g.nrb;
         gid = nb + g.nrb + c;
-        out = g.W + (int64_t)c * NB * n;
-        A = Rows{out, n, min(NB, n - c * NB)};
+        out = g.W + (int64_t)c * NB * ld;
+        A = Rows{out, ld, min(NB, n - c * NB)};
         k0 = c;
         isw = true;
     }
@@ -522,8 +524,8 @@ __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, i
         for (int e = threadIdx.x; e < NB * NB; e += kThr) {
             const int r = e >> 6, c = e & 63;
             if (r < s && c < s) {
-                out[(int64_t)r * n + c] = Z[c * kTP + r];
-                if (g.X) g.X[(int64_t)(j * NB + r) * n + j * NB + c] = Z[r * kTP + c];
+                out[r * ld + c] = Z[c * kTP + r];
+                if (g.X) g.X[(int64_t)(j * NB + r) * ld + j * NB + c] = Z[r * kTP + c];
             }
         }
         raise(fg + j);
@@ -546,7 +548,7 @@ __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, i
     RowAcc y;
     mma_lower(y, T, Z);
     each_row(y, [&](int r, int c, double v) {
-        if (r < A.rows && c < s) out[(int64_t)r * n + c] = v;
+        if (r < A.rows && c < s) out[r * A.ld + c] = v;
     });
     if (isw && g.X) {
         __syncthreads();
@@ -556,7 +558,7 @@ __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, i
         __syncthreads();
         for (int e = threadIdx.x; e < NB * NB; e += kThr) {
             const int r = e >> 6, c = e & 63;  // X tile (j, c-block): row r of block j
-            if (r < s) g.X[(int64_t)(j * NB + r) * n + k0 * NB + c] = T[c * kTP + r];
+            if (r < s) g.X[(int64_t)(j * NB + r) * ld + k0 * NB + c] = T[c * kTP + r];
         }
     }
     raise(fg + j);
@@ -614,7 +616,7 @@ __device__ __forceinline__ void chain(const Dag& g, Smem& sm) {
     int32_t *preA = diag + g.nb, *preD = preA + g.nb;
     // the lower triangle is what counts; past the matrix's end the identity
     auto fetch_diag = [&](int32_t j) {
-        load_tile<kAl>(a, Rows{g.L + (int64_t)j * NB * g.n, g.n, min(NB, g.n - j * NB)}, j * NB, g.n);
+        load_tile<kAl>(a, Rows{g.L + (int64_t)j * NB * g.ld, g.ld, min(NB, g.n - j * NB)}, j * NB, g.n);
         cp_commit();
     };
     auto pad_diag = [&](int32_t j) {
@@ -643,7 +645,7 @@ __device__ __forceinline__ void chain(const Dag& g, Smem& sm) {
 #pragma unroll 4
         for (int e = threadIdx.x; e < NB * NB; e += kThr) {
             const int r = e >> 6, c = e & 63;
-            if (r < s && c <= r) g.L[(int64_t)(r0 + r) * g.n + r0 + c] = a[r * kTP + c];
+            if (r < s && c <= r) g.L[(int64_t)(r0 + r) * g.ld + r0 + c] = a[r * kTP + c];
         }
         if (j + 1 == g.nb) break;
         const int32_t r1 = r0 + NB, rows = min(NB, g.n - r1);
@@ -652,7 +654,7 @@ __device__ __forceinline__ void chain(const Dag& g, Smem& sm) {
             return;
         __syncthreads();  // L_jj is stored: a may be overwritten
         if (helped[0] || helped[1]) load_tile<true>(z, Rows{g.Linv + (int64_t)j * NB * NB, NB, NB}, 0, NB);
-        load_tile<kAl>(t, Rows{g.L + (int64_t)r1 * g.n, g.n, rows}, r0, g.n);
+        load_tile<kAl>(t, Rows{g.L + (int64_t)r1 * g.ld, g.ld, rows}, r0, g.n);
         cp_commit();
         fetch_diag(j + 1);
         cp_wait<1>();
@@ -662,7 +664,7 @@ __device__ __forceinline__ void chain(const Dag& g, Smem& sm) {
         __syncthreads();
         each_row(acc, [&](int r, int c, double v) {
             t[r * kTP + c] = r < rows ? v : 0.0;
-            if (r < rows) g.L[(int64_t)(r1 + r) * g.n + r0 + c] = v;
+            if (r < rows) g.L[(int64_t)(r1 + r) * g.ld + r0 + c] = v;
         });
         raise(g.flag + (int64_t)(j + 1) * g.nb + j);
         mma_syrk(acc, t);
@@ -684,8 +686,8 @@ __device__ __forceinline__ bool inverse_tile(const Dag& g, Smem& sm, int32_t i, 
     const int32_t* wf = g.flag + (int64_t)(nb + g.nrb) * nb;
     Acc acc;
     acc.zero();
-    if (!sum_tiles<kAl>(g, sm, acc, Rows{g.W + (int64_t)i * NB * n, n, ri}, wf + (int64_t)i * nb,
-                        Rows{g.W + (int64_t)j * NB * n, n, rj}, wf + (int64_t)j * nb, i, nb))
+    if (!sum_tiles<kAl>(g, sm, acc, Rows{g.W + (int64_t)i * NB * g.ld, g.ld, ri}, wf + (int64_t)i * nb,
+                        Rows{g.W + (int64_t)j * NB * g.ld, g.ld, rj}, wf + (int64_t)j * nb, i, nb))
         return false;
     double* T = sm.buf;
     each(acc, [&](int r, int c, double v) { T[r * kTP + c] = v; });
@@ -888,6 +890,7 @@ int32_t chol_dag(tpe_ctx* ctx, const CholDag& c, int32_t* singular) {
     g.X = c.X;
     g.Ainv = c.Ainv;
     g.n = c.n;
+    g.ld = c.ld > 0 ? c.ld : c.n;
     g.nb = (c.n + NB - 1) / NB;
     g.nr = c.nr;
     g.nrb = (c.nr + NB - 1) / NB;
@@ -899,7 +902,7 @@ int32_t chol_dag(tpe_ctx* ctx, const CholDag& c, int32_t* singular) {
     const cudaStream_t st = ctx->stream;
     TPE_CUDA_TRY(cudaMemsetAsync(g.ctl, 0, sizeof(int32_t) * (nflag + 4), st));
     auto even = [](const double* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-    const bool al = (c.n & 1) == 0 && even(c.L) && even(c.B) && even(c.W);
+    const bool al = (c.n & 1) == 0 && (g.ld & 1) == 0 && even(c.L) && even(c.B) && even(c.W);
     auto kern = al ? chol_dag_kernel<true> : chol_dag_kernel<false>;
     const size_t smem = (sizeof(Smem) + 15) / 16 * 16 + sizeof(double) * kTile;
     TPE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

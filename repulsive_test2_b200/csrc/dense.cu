@@ -547,7 +547,7 @@ int32_t project_update(tpe_ctx* ctx, const double* d_Y, int32_t k, int32_t V, co
 int32_t saddle_residual(tpe_ctx* ctx, const double* d_A, int32_t V, const double* d_C, int32_t k,
                         const double* d_x, const double* lam, const double* d_rhs_top,
                         const double* rhs_bottom, double* out, double* d_res_top,
-                        double* res_bottom) {
+                        double* res_bottom, const SaddleOp* large) {
     const int64_t m = 3 * (int64_t)V;
     TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double) * (size_t)(2 * V + 16 + k + m)));
     TPE_TRY(ensure(ctx, ctx->scalars, sizeof(double) * (size_t)(k + 3 + 512)));
@@ -558,9 +558,10 @@ int32_t saddle_residual(tpe_ctx* ctx, const double* d_A, int32_t V, const double
     double* rr = ctx->tmp.as<double>();
     double* rb = rr + V;
     double* ctl = rb + V + 16 + k;
+    if (large && k > 0) TPE_TRY(large_ct(ctx, *large, dl, ctl));
     {
-        KernelScope ks(ctx, TPE_KGROUP_OTHER, k > 0 ? 2 : 1);
-        if (k > 0)
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, k > 0 && !large ? 2 : 1);
+        if (k > 0 && !large)
             ct_lambda_kernel<<<grid_for(m, 256), 256, 0, ctx->stream>>>(d_C, k, m, dl, ctl);
         residual_top_kernel<<<V, 256, 0, ctx->stream>>>(d_A, V, k > 0 ? ctl : nullptr, d_x, d_rhs_top,
                                                         rr, rb, d_res_top);
@@ -573,11 +574,12 @@ int32_t saddle_residual(tpe_ctx* ctx, const double* d_A, int32_t V, const double
     double bot_r = 0.0, bot_b = 0.0;
     if (k > 0) {
         double* cx = ctx->tmp.as<double>() + 2 * V;
-        TPE_TRY(gram_dots(ctx, d_C, k, d_x, 1, 3 * (int64_t)V, cx));
+        if (large)
+            TPE_TRY(large_cx(ctx, *large, d_x, cx));
+        else
+            TPE_TRY(gram_dots(ctx, d_C, k, d_x, 1, 3 * (int64_t)V, cx));
         std::vector<double> h((size_t)k);
-        TPE_CUDA_TRY(cudaMemcpyAsync(h.data(), cx, sizeof(double) * k, cudaMemcpyDeviceToHost,
-                                     ctx->stream));
-        TPE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        TPE_TRY(download_on(ctx, ctx->stream, h.data(), cx, sizeof(double) * k));
         for (int32_t r = 0; r < k; r++) {
             const double b = rhs_bottom ? rhs_bottom[r] : 0.0;
             const double d = h[r] - b;

@@ -557,109 +557,13 @@ __global__ void __launch_bounds__(256) cg_prep_t_kernel(const double* __restrict
     }
 }
 
-// ---- multi-right-hand-side products on the FP64 tensor cores ----------------
-//
-// part[z][c][i] = sum_{j in range z of row block} M[i][j] X[c][j] for c < 16:
-// mma.sync m8n8k4 (FP64), 64 rows per CTA (8 per warp), the row block's column
-// range split into gridDim.y equal parts (split K, summed in a fixed order by
-// mrhs_reduce_kernel). TRI = 0: all columns; 1: j < r0 + 64 (lower-triangular
-// M); 2: j >= r0 (upper). The K order inside a 16-column group is permuted
-// (MMA step s takes columns 4m + s, m = 0..3) so each lane's four consecutive
-// columns of M feed four MMAs without shuffles; X is staged transposed in
-// shared memory with rows padded to 17 doubles (conflict-free fragment loads).
-constexpr int kMvRows = 64;
-constexpr int kMvChunk = 256;
-constexpr int kXs = kMaxRhs + 1;
-
 __device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
 }
 
-template <int TRI, typename MT>
-__global__ void __launch_bounds__(256)
-mrhs_dmma_kernel(const MT* __restrict__ M, int32_t ldm, int32_t n,
-                 const double* __restrict__ X, int32_t ldx, int32_t nr,
-                 double* __restrict__ part) {
-    __shared__ double xs[kMvChunk * kXs];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int32_t r0 = blockIdx.x * kMvRows;
-    int32_t lo = 0, hi = n;
-    if (TRI == 1) hi = min(n, r0 + kMvRows);
-    if (TRI == 2) lo = r0;
-    const int32_t per = (((hi - lo) + (int32_t)gridDim.y - 1) / (int32_t)gridDim.y + 15) / 16 * 16;
-    const int32_t ks = lo + (int32_t)blockIdx.y * per;
-    const int32_t ke = min(hi, ks + per);
-    const int32_t row = r0 + warp * 8 + (lane >> 2);
-    const bool rin = row < n;
-    const MT* mrow = M + (size_t)(rin ? row : 0) * ldm;
-    const int m4 = (lane & 3) * 4;
-    const int gq = lane >> 2;
-    const bool vec = sizeof(MT) == 8 ? (ldm & 1) == 0 : (ldm & 3) == 0;
-    double c0a = 0.0, c0b = 0.0, c1a = 0.0, c1b = 0.0;
-    for (int32_t kc = ks; kc < ke; kc += kMvChunk) {
-        const int32_t kn = min(kMvChunk, ke - kc);
-        __syncthreads();
-        for (int e = threadIdx.x; e < kMaxRhs * kMvChunk; e += 256) {
-            const int c = e / kMvChunk, jj = e % kMvChunk;
-            xs[jj * kXs + c] = (c < nr && jj < kn) ? X[(size_t)c * ldx + kc + jj] : 0.0;
-        }
-        __syncthreads();
-        // kUG 16-column groups per pass (the same bytes in flight per thread for
-        // FP32 and FP64 M): their loads of M are all issued before the first MMA
-        // (the MMA order, and so the sums, are those of one group at a time)
-        constexpr int kUG = sizeof(MT) == 8 ? 4 : 8;
-        for (int g0 = 0; g0 < kn; g0 += 16 * kUG) {
-            MT a[kUG][4];
-#pragma unroll
-            for (int u = 0; u < kUG; u++) {
-                const int32_t col = kc + g0 + 16 * u + m4;
-                if (g0 + 16 * u < kn && rin && vec && col + 3 < ke) {
-                    if constexpr (sizeof(MT) == 8) {
-                        const double2 p0 = *reinterpret_cast<const double2*>(mrow + col);
-                        const double2 p1 = *reinterpret_cast<const double2*>(mrow + col + 2);
-                        a[u][0] = p0.x;
-                        a[u][1] = p0.y;
-                        a[u][2] = p1.x;
-                        a[u][3] = p1.y;
-                    } else {
-                        const float4 p0 = *reinterpret_cast<const float4*>(mrow + col);
-                        a[u][0] = p0.x;
-                        a[u][1] = p0.y;
-                        a[u][2] = p0.z;
-                        a[u][3] = p0.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int t = 0; t < 4; t++)
-                        a[u][t] = (g0 + 16 * u < kn && rin && col + t < ke) ? mrow[col + t] : (MT)0;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kUG; u++) {
-                const int g = g0 + 16 * u;
-                if (g >= kn) break;
-#pragma unroll
-                for (int s4 = 0; s4 < 4; s4++) {
-                    const double* xr = xs + (g + m4 + s4) * kXs;
-                    dmma884(c0a, c0b, (double)a[u][s4], xr[gq]);
-                    dmma884(c1a, c1b, (double)a[u][s4], xr[8 + gq]);
-                }
-            }
-        }
-    }
-    if (rin) {
-        double* P = part + (size_t)blockIdx.y * kMaxRhs * ldx;
-        const int cb = 2 * (lane & 3);
-        P[(size_t)cb * ldx + row] = c0a;
-        P[(size_t)(cb + 1) * ldx + row] = c0b;
-        P[(size_t)(8 + cb) * ldx + row] = c1a;
-        P[(size_t)(9 + cb) * ldx + row] = c1b;
-    }
-}
-
-// ---- the CG's multi-RHS products, right-hand-side-major form ------------------
+// ---- multi-right-hand-side products on the FP64 tensor cores, right-hand-side major --
 //
 // Y = M X for up to 16 right-hand sides with the vectors held right-hand-side
 // major (XT[j][c], 16 doubles per row j): every DMMA B fragment is then eight
@@ -667,10 +571,15 @@ mrhs_dmma_kernel(const MT* __restrict__ M, int32_t ldm, int32_t n,
 // L2, with no shared-memory staging and no block barriers. A warp owns 32 rows
 // (four m8 fragments sharing each B fragment), a CTA 128 rows (one 128-row tile
 // of the FP32 factor copies, whose lower or upper tiles alone are defined), and
-// the columns split into chunks of kKChunk (grid.x) whose partial sums go to
+// the columns split into chunks of kch (grid.x) whose partial sums go to
 // part[chunk][c][row] for a fixed-order reduction.
-constexpr int kKChunk = 512;
 constexpr int kTRows = 128;   // rows per CTA (four warps of 32)
+
+// Columns per chunk: 512 fill the SMs at 8192 columns with few partials; below, the
+// kernel is bound by the loads that a warp waits for in turn and by CTAs, and shorter
+// chunks give more of both. V = 1024 step: 2044 / 2114 / 2276 us with chunks of
+// 128 / 256 / 512; V = 6000: 7575 / 7412 / 7528; V = 8192: 11635 / 11388 / 11187.
+inline int32_t mrhs_chunk(int32_t n) { return n <= 4224 ? 128 : (n <= 7168 ? 256 : 512); }
 
 // XT[j][c] = X[c][j] (j < n, c < nr), 0 elsewhere; nout rows of 16.
 __global__ void rhs_major_kernel(const double* __restrict__ X, int32_t ldx, int32_t nr, int32_t n,
@@ -683,24 +592,25 @@ __global__ void rhs_major_kernel(const double* __restrict__ X, int32_t ldx, int3
 }
 
 // Columns [lo, hi) of chunk ch for the 128-row tile at rb0 (empty when lo >= hi).
-__host__ __device__ __forceinline__ void mrhs_t_range(int tri, int32_t n, int32_t ch, int32_t rb0,
-                                                      int32_t& lo, int32_t& hi) {
-    lo = ch * kKChunk;
-    hi = min(n, lo + kKChunk);
+__device__ __forceinline__ void mrhs_t_range(int tri, int32_t n, int32_t kch, int32_t ch, int32_t rb0,
+                                             int32_t& lo, int32_t& hi) {
+    lo = ch * kch;
+    hi = min(n, lo + kch);
     if (tri == 1) hi = min(hi, rb0 + kTRows);  // lower tiles: k < tile end
     if (tri == 2) lo = max(lo, rb0);           // upper tiles: k >= tile start
 }
 
 // part[ch][c][row] = sum_{k in chunk ch} M[row][k] X[c][k], TRI as in mrhs_t_range.
 // MT float: two 16-column groups per pass (A loads of both issued first).
+// n columns, nrows rows.
 template <int TRI, typename MT>
 __global__ void __launch_bounds__(128, 4)
-mrhs_t_kernel(const MT* __restrict__ M, int32_t ldm, int32_t n, const double* __restrict__ XT,
-              double* __restrict__ part, int32_t ldp) {
+mrhs_t_kernel(const MT* __restrict__ M, int32_t ldm, int32_t n, int32_t nrows, int32_t kch,
+              const double* __restrict__ XT, double* __restrict__ part, int32_t ldp) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int32_t ch = blockIdx.x, rb0 = blockIdx.y * kTRows;
     int32_t lo, hi;
-    mrhs_t_range(TRI, n, ch, rb0, lo, hi);
+    mrhs_t_range(TRI, n, kch, ch, rb0, lo, hi);
     if (lo >= hi) return;  // the reduction skips this chunk for these rows
     const int q = lane & 3, gq = lane >> 2;
     constexpr int kF = 4;                       // m8 fragments per warp
@@ -710,7 +620,7 @@ mrhs_t_kernel(const MT* __restrict__ M, int32_t ldm, int32_t n, const double* __
 #pragma unroll
     for (int f = 0; f < kF; f++) {
         const int32_t row = rb0 + warp * 32 + 8 * f + gq;
-        rin[f] = row < n;
+        rin[f] = row < nrows;
         mrow[f] = M + (size_t)(rin[f] ? row : 0) * ldm;
     }
     const bool vec = sizeof(MT) == 8 ? (ldm & 1) == 0 : (ldm & 3) == 0;
@@ -784,7 +694,7 @@ mrhs_t_kernel(const MT* __restrict__ M, int32_t ldm, int32_t n, const double* __
 // shift sum_z spart[z][c]) for i < n, c < nr (scale, spart optional); also
 // YT[i][c] when YT is given (its columns c >= nr stay as they are: zero).
 __global__ void mrhs_t_reduce_kernel(const double* __restrict__ part, int32_t ldp, int tri,
-                                     int32_t n, int32_t nr, const double* __restrict__ scale,
+                                     int32_t n, int32_t kch, int32_t nr, const double* __restrict__ scale,
                                      double shift, const double* __restrict__ spart, int32_t nz,
                                      double* __restrict__ Y, int32_t ldy, double* __restrict__ YT) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -792,11 +702,12 @@ __global__ void mrhs_t_reduce_kernel(const double* __restrict__ part, int32_t ld
     const int c = (int)(t / n);
     const int32_t i = (int32_t)(t % n);
     const int32_t rb0 = i / kTRows * kTRows;
-    const int32_t nch = (n + kKChunk - 1) / kKChunk;
+    const int32_t nch = (n + kch - 1) / kch;
     double acc = 0.0;
+#pragma unroll 4
     for (int32_t ch = 0; ch < nch; ch++) {
         int32_t lo, hi;
-        mrhs_t_range(tri, n, ch, rb0, lo, hi);
+        mrhs_t_range(tri, n, kch, ch, rb0, lo, hi);
         if (lo < hi) acc += part[((size_t)ch * kMaxRhs + c) * ldp + i];
     }
     if (spart) {
@@ -807,22 +718,6 @@ __global__ void mrhs_t_reduce_kernel(const double* __restrict__ part, int32_t ld
     if (scale) acc *= scale[i];
     if (Y) Y[(size_t)c * ldy + i] = acc;
     if (YT) YT[(size_t)i * kMaxRhs + c] = acc;
-}
-
-// Y[c][i] = scale_i (sum_z part[z][c][i] + shift s[c]) for i < n (scale, s optional).
-__global__ void mrhs_reduce_kernel(const double* __restrict__ part, int32_t nsplit, int32_t n,
-                                   int32_t ldx, int32_t nr, const double* __restrict__ scale,
-                                   double shift, const double* __restrict__ s,
-                                   double* __restrict__ Y) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)nr * n) return;
-    const int c = (int)(t / n);
-    const int32_t i = (int32_t)(t % n);
-    double acc = 0.0;
-    for (int z = 0; z < nsplit; z++) acc += part[((size_t)z * kMaxRhs + c) * ldx + i];
-    if (s) acc += shift * s[c];
-    if (scale) acc *= scale[i];
-    Y[(size_t)c * ldx + i] = acc;
 }
 
 // Plain FP32 copies of the inverse factor (hi + lo is exact in FP32): Zf = Z on
@@ -1341,6 +1236,21 @@ int32_t mixed_factor(tpe_ctx* ctx, const double* d_A, int32_t V, double rho, boo
     return TPE_OK;
 }
 
+// part[ch][c][i] of M X, M rows x cols (row length cols), X right-hand-side major (rows
+// of 16): see mrhs_t_kernel.
+int32_t mrhs_part(tpe_ctx* ctx, const double* M, int32_t rows, int32_t cols, const double* XT,
+                  const double** part, int32_t* nch) {
+    const int32_t kch = mrhs_chunk(cols);
+    *nch = (cols + kch - 1) / kch;
+    TPE_TRY(ensure(ctx, ctx->mx_part, sizeof(double) * (size_t)*nch * kMaxRhs * rows));
+    *part = ctx->mx_part.as<double>();
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    mrhs_t_kernel<0, double><<<dim3((unsigned)*nch, (unsigned)((rows + kTRows - 1) / kTRows)), 128, 0,
+                               ctx->stream>>>(M, cols, cols, rows, kch, XT, ctx->mx_part.as<double>(), rows);
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
+}
+
 int32_t mrhs_fp64(tpe_ctx* ctx, const double* M, int32_t n, const double* X, int32_t ldx,
                   int32_t nr, double* Y) {
     if (nr <= 0 || n <= 0) return TPE_OK;
@@ -1348,14 +1258,20 @@ int32_t mrhs_fp64(tpe_ctx* ctx, const double* M, int32_t n, const double* X, int
         set_error(ctx, TPE_ERR_TOO_LARGE, "mrhs_fp64: at most 16 right-hand sides, ldx >= n");
         return TPE_ERR_TOO_LARGE;
     }
-    constexpr int kSplit = 8;
-    TPE_TRY(ensure(ctx, ctx->mx_part, sizeof(double) * (size_t)kSplit * kMaxRhs * ldx));
-    double* part = ctx->mx_part.as<double>();
-    KernelScope ks(ctx, TPE_KGROUP_OTHER, 2);
-    mrhs_dmma_kernel<0, double><<<dim3((unsigned)((n + kMvRows - 1) / kMvRows), kSplit), 256, 0,
-                                  ctx->stream>>>(M, n, n, X, ldx, nr, part);
-    mrhs_reduce_kernel<<<nblk((int64_t)nr * n, 256), 256, 0, ctx->stream>>>(
-        part, kSplit, n, ldx, nr, nullptr, 0.0, nullptr, Y);
+    const int32_t rows = (n + 15) / 16 * 16;  // the kernel reads whole groups of 16 columns
+    TPE_TRY(ensure(ctx, ctx->mrhs_xt, sizeof(double) * kMaxRhs * (size_t)rows));
+    double* XT = ctx->mrhs_xt.as<double>();
+    {
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+        rhs_major_kernel<<<nblk((int64_t)rows * kMaxRhs, 256), 256, 0, ctx->stream>>>(X, ldx, nr, n, rows, XT);
+        TPE_CUDA_TRY(cudaGetLastError());
+    }
+    const double* part = nullptr;
+    int32_t nch = 0;
+    TPE_TRY(mrhs_part(ctx, M, n, n, XT, &part, &nch));
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    mrhs_t_reduce_kernel<<<nblk((int64_t)nr * n, 256), 256, 0, ctx->stream>>>(
+        part, n, 0, n, mrhs_chunk(n), nr, nullptr, 0.0, nullptr, 0, Y, ldx, nullptr);
     TPE_CUDA_TRY(cudaGetLastError());
     return TPE_OK;
 }
@@ -1381,7 +1297,8 @@ int32_t mixed_solve(tpe_ctx* ctx, const double* d_A, const double* d_B, double* 
                                                        (size_t)nz * kMaxRhs)));
     // split-K partial sums of the right-hand-side-major products: one slot per
     // column chunk
-    const int32_t nch = (Vp + kKChunk - 1) / kKChunk;
+    const int32_t kch = mrhs_chunk(Vp);
+    const int32_t nch = (Vp + kch - 1) / kch;
     TPE_TRY(ensure(ctx, ctx->mx_part, sizeof(double) * (size_t)nch * kMaxRhs * Vp));
     double* X = ctx->mx_vec.as<double>();
     double* R = X + vec;
@@ -1408,7 +1325,7 @@ int32_t mixed_solve(tpe_ctx* ctx, const double* d_A, const double* d_B, double* 
     std::vector<double> hist((size_t)(kRateSpan + 1) * kMaxRhs);
     int32_t max_iters = 0;
     const dim3 grid_p((unsigned)nch, (unsigned)(Vp / kTRows));
-    const dim3 grid_a((unsigned)((V + kKChunk - 1) / kKChunk), (unsigned)((V + kTRows - 1) / kTRows));
+    const dim3 grid_a((unsigned)((V + kch - 1) / kch), (unsigned)((V + kTRows - 1) / kTRows));
     for (int32_t c0 = 0; c0 < nr; c0 += kMaxRhs) {
         const int32_t n = nr - c0 < kMaxRhs ? nr - c0 : kMaxRhs;
         const int64_t tot = (int64_t)n * Vp;
@@ -1419,11 +1336,11 @@ int32_t mixed_solve(tpe_ctx* ctx, const double* d_A, const double* d_B, double* 
         auto precond = [&](const double* in, double* out) -> int32_t {
             KernelScope ks(ctx, TPE_KGROUP_TRSV, 5);
             rhs_major_kernel<<<nblk(vec, 256), 256, 0, st>>>(in, Vp, n, Vp, Vp, XT);
-            mrhs_t_kernel<1, float><<<grid_p, 128, 0, st>>>(Zf, Vp, Vp, XT, part, Vp);
-            mrhs_t_reduce_kernel<<<nblk(tot, 256), 256, 0, st>>>(part, Vp, 1, Vp, n, nullptr, 0.0,
+            mrhs_t_kernel<1, float><<<grid_p, 128, 0, st>>>(Zf, Vp, Vp, Vp, kch, XT, part, Vp);
+            mrhs_t_reduce_kernel<<<nblk(tot, 256), 256, 0, st>>>(part, Vp, 1, Vp, kch, n, nullptr, 0.0,
                                                                   nullptr, 0, nullptr, Vp, UT);
-            mrhs_t_kernel<2, float><<<grid_p, 128, 0, st>>>(Wf, Vp, Vp, UT, part, Vp);
-            mrhs_t_reduce_kernel<<<nblk(tot, 256), 256, 0, st>>>(part, Vp, 2, Vp, n, nullptr, 0.0,
+            mrhs_t_kernel<2, float><<<grid_p, 128, 0, st>>>(Wf, Vp, Vp, Vp, kch, UT, part, Vp);
+            mrhs_t_reduce_kernel<<<nblk(tot, 256), 256, 0, st>>>(part, Vp, 2, Vp, kch, n, nullptr, 0.0,
                                                                   nullptr, 0, out, Vp, nullptr);
             TPE_CUDA_TRY(cudaGetLastError());
             return TPE_OK;
@@ -1432,8 +1349,8 @@ int32_t mixed_solve(tpe_ctx* ctx, const double* d_A, const double* d_B, double* 
         auto matvec = [&](const double* in, double* out) -> int32_t {
             KernelScope ks(ctx, TPE_KGROUP_OTHER, 3);
             cg_prep_t_kernel<<<nz, 256, 0, st>>>(in, d, V, Vp, n, XT, spart);
-            mrhs_t_kernel<0, double><<<grid_a, 128, 0, st>>>(d_A, V, V, XT, part, Vp);
-            mrhs_t_reduce_kernel<<<nblk((int64_t)n * V, 256), 256, 0, st>>>(part, Vp, 0, V, n, d, shift,
+            mrhs_t_kernel<0, double><<<grid_a, 128, 0, st>>>(d_A, V, V, V, kch, XT, part, Vp);
+            mrhs_t_reduce_kernel<<<nblk((int64_t)n * V, 256), 256, 0, st>>>(part, Vp, 0, V, kch, n, d, shift,
                                                                              spart, nz, out, Vp, nullptr);
             TPE_CUDA_TRY(cudaGetLastError());
             return TPE_OK;

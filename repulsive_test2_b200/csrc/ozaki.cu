@@ -521,7 +521,10 @@ int32_t ozaki_status(tpe_ctx* ctx, cudaStream_t stream) {
 
 namespace {
 
-constexpr int32_t kBase = 1024;  // largest block factored and inverted by the FP64 kernels
+// Largest block factored and inverted by the FP64 data-flow kernel (per-edge step
+// with blocks of 512 / 1024 / 2048 / 4096, ms: V = 2500 10.6 / 9.0 / 8.6 / 9.4, 4096
+// 18.7 / 17.5 / 17.8 / 19.1, 8192 62.3 / 60.0 / 61.0 / 64.5).
+constexpr int32_t kBase = 2048;
 
 // The base block size: kBase, or TPE_INT8_BASE (128..kBase) to test the
 // recursion at small orders.
@@ -538,7 +541,7 @@ struct InvCtx {
     double* X;  // L^{-1}, lower
     double* W;  // X^T, upper
     double* Tt;
-    double* base;  // kBase^2 (block) + 64 kBase (diagonal inverses) + 2 kBase^2 (X, W)
+    double* base;  // 64 kBase: inverses of a base block's 64 x 64 diagonal blocks
     int32_t n;
     double tol;
     int32_t nbase;
@@ -565,35 +568,18 @@ DGemmArgs gemm_args(const double* A, int64_t lda, const double* B, int64_t ldb, 
 }
 
 int32_t inv_base(InvCtx& c, int32_t o, int32_t m) {
-    tpe_ctx* ctx = c.ctx;
-    const cudaStream_t st = ctx->stream;
-    const int64_t n = c.n;
-    double* Bm = c.base;
-    double* Binv = Bm + (size_t)kBase * kBase;
-    double* Xb = Binv + (size_t)kBase * kNB;  // (kBase / 64) diagonal 64 x 64 inverses
-    double* Wb = Xb + (size_t)kBase * kBase;
-    TPE_CUDA_TRY(cudaMemcpy2DAsync(Bm, sizeof(double) * m, c.M + o * n + o, sizeof(double) * n,
-                                   sizeof(double) * m, m, cudaMemcpyDeviceToDevice, st));
-    // (the products' triangular K ranges start at 128-column tiles: zeros beside the tiles)
-    TPE_CUDA_TRY(cudaMemsetAsync(Xb, 0, sizeof(double) * (size_t)m * m, st));
-    TPE_CUDA_TRY(cudaMemsetAsync(Wb, 0, sizeof(double) * (size_t)m * m, st));
-    CholDag f;
-    f.L = Bm;
-    f.Linv = Binv;
+    const int64_t at = o * (int64_t)c.n + o;
+    CholDag f;  // in place (X and W are zero outside the tiles it writes)
+    f.L = c.M + at;
+    f.Linv = c.base;
     f.n = m;
+    f.ld = c.n;
     f.tol = c.tol;
-    f.W = Wb;
-    f.X = Xb;
+    f.W = c.W + at;
+    f.X = c.X + at;
     int32_t bad = 0;
-    TPE_TRY(chol_dag(ctx, f, &bad));
-    if (bad) {
-        c.singular = true;
-        return TPE_OK;
-    }
-    TPE_CUDA_TRY(cudaMemcpy2DAsync(c.X + o * n + o, sizeof(double) * n, Xb, sizeof(double) * m,
-                                   sizeof(double) * m, m, cudaMemcpyDeviceToDevice, st));
-    TPE_CUDA_TRY(cudaMemcpy2DAsync(c.W + o * n + o, sizeof(double) * n, Wb, sizeof(double) * m,
-                                   sizeof(double) * m, m, cudaMemcpyDeviceToDevice, st));
+    TPE_TRY(chol_dag(c.ctx, f, &bad));
+    if (bad) c.singular = true;
     return TPE_OK;
 }
 
@@ -633,8 +619,7 @@ int32_t spd_inverse_int8(tpe_ctx* ctx, double* Mat, int32_t n, double piv_tol, d
     *singular = false;
     if (n <= 0) return TPE_OK;
     TPE_TRY(ozaki_reserve(ctx, ozaki_scratch_bytes(n, 0, n)));
-    const size_t base_doubles = (size_t)kBase * kBase * 3 + (size_t)kBase * kNB;
-    TPE_TRY(ensure(ctx, ctx->oz_base, sizeof(double) * base_doubles));
+    TPE_TRY(ensure(ctx, ctx->oz_base, sizeof(double) * (size_t)kBase * kNB));
     TPE_CUDA_TRY(cudaMemsetAsync(X, 0, sizeof(double) * (size_t)n * n, ctx->stream));
     TPE_CUDA_TRY(cudaMemsetAsync(W, 0, sizeof(double) * (size_t)n * n, ctx->stream));
     InvCtx c{ctx, Mat, X, W, Tt, ctx->oz_base.as<double>(), n, piv_tol, base_size(), false};

@@ -8,13 +8,20 @@
 // small-k path forms from k x 3 solves and factors on the host. For large k that
 // is k^3 host work and 3k solves; here instead:
 //   Ainv = A_rho^{-1} explicitly (FP64: factor, L^-T and W W^T in one kernel,
-//   chol_dag.cu), then Y = A3^{-1} C^T row by row as a gather of at most
-//   kNZ rows of Ainv per coordinate block (an edge-length row has two nonzeros
-//   per block); rows with more nonzeros (barycenter) go through one multi-RHS
-//   product with Ainv;
-//   S[r][s] = C_r . Y_s as the same gather (dense rows r: full dot products),
-//   symmetrized, factored and inverted on the device (Sinv), so that every
-//   multiplier solve is one product with Sinv.
+//   chol_dag.cu). An edge-length row is one 3-vector w_s times the difference of two
+//   vertices (a pin: times one), so A3^{-1} C^T on those rows is w_s times one column
+//   of Gt, Gt[v][s] = Ainv[v][a_s] - Ainv[v][b_s], a third of the size; the other
+//   rows (barycenter) go through a multi-RHS product with Ainv. S from differences of
+//   Gt's rows; its inverse Sinv on the device makes every multiplier solve one product.
+// A solution is x = w - Gt (w_s lam_s) - dense rows - mu term: one product with Gt for
+// up to five trial step sizes (15 columns). The multipliers stay on the device: a
+// projection iteration reads back only Phi and the norms that decide it.
+// Measured per call at V = 2500, k = 2503 against the dense forms (us): the combination
+// of eight trials 166 -> 2 x 28, C^T lam 658 -> 6, C x 35 -> 10, Y and S 233 -> Gt and S 43.
+// (x = w - Ainv (C^T lam) needs no Gt, but rounds u |Ainv| |C^T lam| where Gt's
+// differences round u |Gt| |lam|: 1e5 times more error on a loop network.)
+#include <math.h>
+
 #include <algorithm>
 
 #include "tpe_internal.h"
@@ -22,159 +29,347 @@
 namespace tpe {
 namespace {
 
-constexpr int kNZ = 4;  // nonzeros per (row, coordinate block) kept as a sparse row
+constexpr int kRhs = 16;      // columns of the right-hand-side-major products (mrhs_part)
+constexpr int kPerPass = 5;   // trials (three columns each) per product with Ainv
 
-// Per row s and coordinate block c: the nonzero entries in index order when
-// there are at most kNZ, else dense[s] = 1.
+template <int kWarps>
+__device__ __forceinline__ double block_sum(double v, double* red) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double t = 0.0;
+    for (int w = 0; w < kWarps; w++) t += red[w];
+    __syncthreads();
+    return t;  // on every thread
+}
+
+// One pass over the dense rows of C. Row s: its two vertices (or one) and its
+// 3-vector when it has that form, else (-1, -1) and dense[s] = 1; and the row's sums
+// over each coordinate block and of absolute values.
 __global__ void __launch_bounds__(256)
-sparse_rows_kernel(const double* __restrict__ C, int32_t V, int32_t* __restrict__ nz_idx,
-                   double* __restrict__ nz_val, int32_t* __restrict__ nz_cnt,
-                   int32_t* __restrict__ dense) {
+sparse_rows_kernel(const double* __restrict__ C, int32_t V, SparseRows sp, int32_t* __restrict__ dense) {
     const int32_t s = blockIdx.x;
-    __shared__ int cnt[3];
-    __shared__ int idx[3][kNZ];
-    __shared__ double val[3][kNZ];
-    if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
+    __shared__ int cnt;
+    __shared__ int idx[2];
+    __shared__ double val[2][3];
+    __shared__ double red[8];
+    if (threadIdx.x == 0) cnt = 0;
     __syncthreads();
     const double* row = C + (int64_t)s * 3 * V;
-    for (int64_t t = threadIdx.x; t < 3 * (int64_t)V; t += blockDim.x) {
-        const double x = row[t];
-        if (x != 0.0) {
-            const int c = (int)(t / V);
-            const int q = atomicAdd(&cnt[c], 1);
-            if (q < kNZ) {
-                idx[c][q] = (int)(t - (int64_t)c * V);
-                val[c][q] = x;
+    double sum[4] = {0, 0, 0, 0};
+    for (int32_t v = threadIdx.x; v < V; v += 256) {
+        const double x = row[v], y = row[V + v], z = row[2 * (int64_t)V + v];
+        sum[0] += x;
+        sum[1] += y;
+        sum[2] += z;
+        sum[3] += fabs(x) + fabs(y) + fabs(z);
+        if (x != 0.0 || y != 0.0 || z != 0.0) {
+            const int q = atomicAdd(&cnt, 1);
+            if (q < 2) {
+                idx[q] = v;
+                val[q][0] = x;
+                val[q][1] = y;
+                val[q][2] = z;
             }
         }
     }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        sum[q] = block_sum<8>(sum[q], red);
+        if (threadIdx.x == 0) sp.stats[4 * (int64_t)s + q] = sum[q];
+    }
+    if (threadIdx.x != 0) return;
+    const int n = cnt;
+    // vertex order, so that no sum depends on the race above
+    const int f = n == 2 && idx[1] < idx[0] ? 1 : 0;
+    bool ok = n == 1 || n == 2;
+    if (n == 2)
+        for (int d = 0; d < 3; d++) ok = ok && val[1][d] == -val[0][d];
+    dense[s] = ok || n == 0 ? 0 : 1;
+    sp.ab[s] = ok ? make_int2(idx[f], n == 2 ? idx[1 - f] : -1) : make_int2(-1, -1);
+    for (int d = 0; d < 3; d++) sp.w[3 * (int64_t)s + d] = ok ? val[f][d] : 0.0;
+}
+
+// The same entries by vertex: off[v] .. off[v + 1] of ent, in row order (counted,
+// summed, filled in any order, then placed by rank).
+__global__ void col_count_kernel(SparseRows sp, int32_t k, int32_t* __restrict__ count) {
+    const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= k) return;
+    const int2 ab = sp.ab[s];
+    if (ab.x >= 0) atomicAdd(&count[ab.x], 1);
+    if (ab.y >= 0) atomicAdd(&count[ab.y], 1);
+}
+__global__ void __launch_bounds__(1024) col_scan_kernel(SparseRows sp, int32_t V, int32_t* __restrict__ count) {
+    __shared__ int32_t part[1024];
+    const int32_t per = (V + 1023) / 1024, b = min(V, (int32_t)threadIdx.x * per), e = min(V, b + per);
+    int32_t s = 0;
+    for (int32_t v = b; v < e; v++) s += count[v];
+    part[threadIdx.x] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        bool dn = false;
-        for (int c = 0; c < 3; c++) {
-            const int n = cnt[c];
-            if (n > kNZ) {
-                dn = true;
-                continue;
-            }
-            // index order, so the sums below do not depend on the race above
-            for (int a = 1; a < n; a++)
-                for (int b = a; b > 0 && idx[c][b - 1] > idx[c][b]; b--) {
-                    const int ti = idx[c][b];
-                    idx[c][b] = idx[c][b - 1];
-                    idx[c][b - 1] = ti;
-                    const double tv = val[c][b];
-                    val[c][b] = val[c][b - 1];
-                    val[c][b - 1] = tv;
-                }
-            for (int q = 0; q < kNZ; q++) {
-                nz_idx[((int64_t)s * 3 + c) * kNZ + q] = q < n ? idx[c][q] : 0;
-                nz_val[((int64_t)s * 3 + c) * kNZ + q] = q < n ? val[c][q] : 0.0;
-            }
-            nz_cnt[(int64_t)s * 3 + c] = n;
-        }
-        dense[s] = dn ? 1 : 0;
+    for (int o = 1; o < 1024; o <<= 1) {
+        const int32_t t = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
+        __syncthreads();
+        part[threadIdx.x] += t;
+        __syncthreads();
+    }
+    s = threadIdx.x > 0 ? part[threadIdx.x - 1] : 0;
+    for (int32_t v = b; v < e; v++) {
+        const int32_t c = count[v];
+        sp.off[v] = s;
+        count[v] = s;  // the fill's cursor
+        s += c;
+    }
+    if (threadIdx.x == 1023) sp.off[V] = part[1023];
+}
+__global__ void col_fill_kernel(SparseRows sp, int32_t k, int32_t* __restrict__ cursor,
+                                int32_t* __restrict__ raw) {
+    const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= k) return;
+    const int2 ab = sp.ab[s];
+    if (ab.x >= 0) raw[atomicAdd(&cursor[ab.x], 1)] = 2 * s;
+    if (ab.y >= 0) raw[atomicAdd(&cursor[ab.y], 1)] = 2 * s + 1;
+}
+__global__ void col_sort_kernel(SparseRows sp, int32_t V, const int32_t* __restrict__ raw) {
+    const int32_t v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (v >= V) return;
+    const int32_t b = sp.off[v], e = sp.off[v + 1];
+    for (int32_t a = b + lane; a < e; a += 32) {
+        const int32_t x = raw[a];
+        int32_t rank = 0;
+        for (int32_t i = b; i < e; i++) rank += raw[i] < x;
+        sp.ent[b + rank] = x;
     }
 }
 
-// Y[s][c][u] = sum_q val[s][c][q] Ainv[idx[s][c][q]][u] for the sparse rows s
-// (Ainv symmetric: row idx is column idx). Grid (k, 3, V / 256).
+// Gt[v][s] = Ainv[v][a_s] - Ainv[v][b_s] (0 for dense rows). Differences first: they
+// are exact where neighbouring columns are close.
 __global__ void __launch_bounds__(256)
-y_sparse_kernel(const double* __restrict__ Ainv, int32_t V, const int32_t* __restrict__ nz_idx,
-                const double* __restrict__ nz_val, const int32_t* __restrict__ nz_cnt,
-                const int32_t* __restrict__ dense, double* __restrict__ Y) {
-    const int32_t s = blockIdx.x, c = blockIdx.y;
-    if (dense[s]) return;
-    const int32_t u = blockIdx.z * blockDim.x + threadIdx.x;
-    if (u >= V) return;
-    const int64_t rc = (int64_t)s * 3 + c;
-    const int n = nz_cnt[rc];
-    double acc = 0.0;
-    for (int q = 0; q < n; q++)
-        acc += nz_val[rc * kNZ + q] * Ainv[(int64_t)nz_idx[rc * kNZ + q] * V + u];
-    Y[rc * V + u] = acc;
+g_kernel(const double* __restrict__ Ainv, int32_t V, int32_t k, SparseRows sp, double* __restrict__ Gt) {
+    const int32_t s = blockIdx.x * 256 + threadIdx.x;
+    if (s >= k) return;
+    const int2 ab = sp.ab[s];
+    for (int32_t v = blockIdx.y; v < V; v += gridDim.y) {
+        const double* row = Ainv + (int64_t)v * V;
+        const double x = ab.x >= 0 ? row[ab.x] : 0.0;
+        Gt[(int64_t)v * k + s] = ab.y >= 0 ? x - row[ab.y] : x;
+    }
 }
 
-// S[r][s] = sum_c sum_q val[r][c][q] Y[s][c][idx[r][c][q]] for sparse rows r;
-// 32 x 32 tiles (r, s), transposed through shared memory so that the gathers
-// (consecutive r of one s) and the stores (consecutive s of one r) coalesce.
+// S[r][s] = (w_r . w_s) (Gt[a_r][s] - Gt[b_r][s]) for sparse rows: 32 x 32 tiles on or
+// below the diagonal, mirrored. Dense rows are s_dense_kernel's.
 __global__ void __launch_bounds__(256)
-s_sparse_kernel(const double* __restrict__ Y, int32_t V, int32_t k,
-                const int32_t* __restrict__ nz_idx, const double* __restrict__ nz_val,
-                const int32_t* __restrict__ nz_cnt, const int32_t* __restrict__ dense,
-                double* __restrict__ S) {
+s_sparse_kernel(const double* __restrict__ Gt, int32_t k, SparseRows sp, double* __restrict__ S) {
+    if (blockIdx.x > blockIdx.y) return;
     __shared__ double t[32][33];
-    const int32_t r0 = blockIdx.x * 32, s0 = blockIdx.y * 32;
+    const int32_t r0 = blockIdx.y * 32, s0 = blockIdx.x * 32;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    const int32_t r = r0 + tx;
-    const bool rv = r < k && !dense[r];
-    int ix[3][kNZ];
-    double vv[3][kNZ];
-    int nn[3] = {0, 0, 0};
-    if (rv) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const int64_t rc = (int64_t)r * 3 + c;
-            nn[c] = nz_cnt[rc];
-#pragma unroll
-            for (int q = 0; q < kNZ; q++) {
-                ix[c][q] = nz_idx[rc * kNZ + q];
-                vv[c][q] = nz_val[rc * kNZ + q];
-            }
-        }
-    }
+    const int32_t s = s0 + tx;
+    double ws[3] = {0, 0, 0};
+    if (s < k)
+        for (int d = 0; d < 3; d++) ws[d] = sp.w[3 * (int64_t)s + d];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const int sl = ty + 8 * i;
-        const int32_t s = s0 + sl;
-        double acc = 0.0;
-        if (rv && s < k) {
-#pragma unroll
-            for (int c = 0; c < 3; c++) {
-                const double* ys = Y + ((int64_t)s * 3 + c) * V;
-#pragma unroll
-                for (int q = 0; q < kNZ; q++)
-                    if (q < nn[c]) acc += vv[c][q] * ys[ix[c][q]];
-            }
+        const int32_t r = r0 + ty + 8 * i;
+        double x = 0.0;
+        if (r < k && s < k) {
+            const int2 ab = sp.ab[r];
+            const double* wr = sp.w + 3 * (int64_t)r;
+            if (ab.x >= 0) x = Gt[(int64_t)ab.x * k + s];
+            if (ab.y >= 0) x -= Gt[(int64_t)ab.y * k + s];
+            x *= wr[0] * ws[0] + wr[1] * ws[1] + wr[2] * ws[2];
         }
-        t[sl][tx] = acc;
+        t[ty + 8 * i][tx] = x;
     }
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int rl = ty + 8 * i;
-        const int32_t rr = r0 + rl, s = s0 + tx;
-        if (rr < k && s < k && !dense[rr]) S[(int64_t)rr * k + s] = t[tx][rl];
+        const bool dg = r0 == s0;
+        if (r0 + rl < k && s < k) S[(int64_t)(r0 + rl) * k + s] = dg && tx > rl ? t[tx][rl] : t[rl][tx];
+        if (!dg && s0 + rl < k && r0 + tx < k) S[(int64_t)(s0 + rl) * k + r0 + tx] = t[tx][rl];
     }
 }
 
-// S = (S + S^T) / 2, one pair of 32 x 32 tiles per block (bi >= bj).
-__global__ void symmetrize_kernel(double* __restrict__ S, int32_t n) {
-    __shared__ double a[32][33], b[32][33];
-    const int32_t bi = blockIdx.y, bj = blockIdx.x;
-    if (bj > bi) return;
-    const int32_t i0 = bi * 32, j0 = bj * 32;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int32_t i = i0 + r, j = j0 + threadIdx.x;
-        if (i < n && j < n) a[r][threadIdx.x] = S[(int64_t)i * n + j];
-        const int32_t i2 = j0 + r, j2 = i0 + threadIdx.x;
-        if (i2 < n && j2 < n) b[r][threadIdx.x] = S[(int64_t)i2 * n + j2];
+// Dense row a = list[blockIdx.y] against the sparse rows s: both S entries from Y_a.
+__global__ void s_dense_kernel(const double* __restrict__ Y, int32_t V, int32_t k, SparseRows sp,
+                               const int32_t* __restrict__ dense, double* __restrict__ S) {
+    const int32_t s = blockIdx.x * blockDim.x + threadIdx.x, a = sp.list[blockIdx.y];
+    if (s >= k || dense[s]) return;
+    const double* y = Y + (int64_t)blockIdx.y * 3 * V;
+    const int2 ab = sp.ab[s];
+    double acc = 0.0;
+    for (int d = 0; d < 3; d++) {
+        double x = 0.0;
+        if (ab.x >= 0) x = y[(int64_t)d * V + ab.x];
+        if (ab.y >= 0) x -= y[(int64_t)d * V + ab.y];
+        acc += sp.w[3 * (int64_t)s + d] * x;
     }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        const int32_t i = i0 + r, j = j0 + threadIdx.x;
-        // a[r][x] = S[i0 + r][j0 + x], b[x][r] = S[j0 + x][i0 + r]
-        if (i < n && j < n) {
-            const double m = 0.5 * (a[r][threadIdx.x] + b[threadIdx.x][r]);
-            S[(int64_t)i * n + j] = m;
-        }
-        const int32_t i2 = j0 + r, j2 = i0 + threadIdx.x;
-        if (i2 < n && j2 < n && bi != bj) {
-            const double m = 0.5 * (b[r][threadIdx.x] + a[threadIdx.x][r]);
-            S[(int64_t)i2 * n + j2] = m;
-        }
+    S[(int64_t)a * k + s] = acc;
+    S[(int64_t)s * k + a] = acc;
+}
+// Two dense rows a >= b: (C_a . Y_b + C_b . Y_a) / 2.
+__global__ void __launch_bounds__(256)
+s_dense_pair_kernel(const double* __restrict__ C, const double* __restrict__ Y, int64_t m, int32_t k,
+                    SparseRows sp, double* __restrict__ S) {
+    if (blockIdx.y > blockIdx.x) return;
+    __shared__ double red[8];
+    const int32_t a = sp.list[blockIdx.x], b = sp.list[blockIdx.y];
+    double s = 0.0;
+    for (int64_t t = threadIdx.x; t < m; t += 256)
+        s += C[a * m + t] * Y[blockIdx.y * m + t] + C[b * m + t] * Y[blockIdx.x * m + t];
+    s = block_sum<8>(s, red);
+    if (threadIdx.x == 0) S[(int64_t)a * k + b] = S[(int64_t)b * k + a] = 0.5 * s;
+}
+
+// XT[s][3 q + d] = w_s,d coef_q[s], q < n <= kPerPass; zero rows s >= k.
+__global__ void coef_rhs_kernel(SparseRows sp, int32_t k, int32_t rows, const double* __restrict__ coef,
+                                int32_t n, double* __restrict__ XT) {
+    const int32_t s = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y;
+    if (s >= rows || q >= n) return;
+    const double l = s < k ? coef[(int64_t)q * (k + 3) + s] : 0.0;
+    for (int d = 0; d < 3; d++) XT[(int64_t)s * kRhs + 3 * q + d] = s < k ? sp.w[3 * (int64_t)s + d] * l : 0.0;
+}
+// out = C^T lam, coordinate blocks: each vertex's sparse entries in row order, then
+// the dense rows.
+__global__ void ct_block_kernel(const double* __restrict__ C, int32_t V, SparseRows sp,
+                                const double* __restrict__ lam, double* __restrict__ out) {
+    const int32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= V) return;
+    double t[3] = {0, 0, 0};
+    for (int32_t e = sp.off[v]; e < sp.off[v + 1]; e++) {
+        const int32_t x = sp.ent[e], s = x >> 1;
+        const double l = x & 1 ? -lam[s] : lam[s];
+        for (int d = 0; d < 3; d++) t[d] += sp.w[3 * (int64_t)s + d] * l;
+    }
+    for (int32_t a = 0; a < sp.nd; a++) {
+        const double* row = C + (int64_t)sp.list[a] * 3 * V;
+        const double l = lam[sp.list[a]];
+        for (int d = 0; d < 3; d++) t[d] += row[(int64_t)d * V + v] * l;
+    }
+    for (int d = 0; d < 3; d++) out[(int64_t)d * V + v] = t[d];
+}
+// out = C x: one thread per sparse row; the first nd blocks take a dense row each.
+__global__ void __launch_bounds__(256)
+cx_kernel(const double* __restrict__ C, int32_t V, SparseRows sp, const int32_t* __restrict__ dense, int32_t k,
+          const double* __restrict__ x, double* __restrict__ out) {
+    __shared__ double red[8];
+    if ((int32_t)blockIdx.x < sp.nd) {
+        const int32_t a = sp.list[blockIdx.x];
+        const int64_t m = 3 * (int64_t)V;
+        double s = 0.0;
+        for (int64_t t = threadIdx.x; t < m; t += 256) s += C[a * m + t] * x[t];
+        s = block_sum<8>(s, red);
+        if (threadIdx.x == 0) out[a] = s;
+        return;
+    }
+    const int32_t r = (blockIdx.x - sp.nd) * 256 + threadIdx.x;
+    if (r >= k || dense[r]) return;
+    const int2 ab = sp.ab[r];
+    double acc = 0.0;
+    for (int d = 0; d < 3; d++) {
+        double y = 0.0;
+        if (ab.x >= 0) y = x[(int64_t)d * V + ab.x];
+        if (ab.y >= 0) y -= x[(int64_t)d * V + ab.y];
+        acc += sp.w[3 * (int64_t)r + d] * y;
+    }
+    out[r] = acc;
+}
+
+// XT[j][c] = rc[pos[c]][j] (pos null: c) for j < k, 0 for the rows after it; c < n <= 16.
+__global__ void rc_rhs_kernel(const double* __restrict__ rc, int64_t stride, const int32_t* __restrict__ pos,
+                              int32_t k, int32_t rows, int32_t n, double* __restrict__ XT) {
+    const int32_t j = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (j >= rows || c >= n) return;
+    XT[(int64_t)j * kRhs + c] = j < k ? rc[(pos ? pos[c] : c) * stride + j] : 0.0;
+}
+
+// One block per multiplier solve c: t = Sinv rc (its chunk sums), the 3 x 3 system
+// M mu = Scu^T t - ru through M's Cholesky factor, and the second right-hand side
+// rc - Scu mu into XT; mu su to coef[c][k ..]. 1024 threads, four chunks' loads at a
+// time: 43 -> 20 us at k = 2503 against 256 threads and one.
+__global__ void __launch_bounds__(1024)
+mu_kernel(const double* __restrict__ part, int32_t nch, int32_t k, const double* __restrict__ scu,
+          const double* __restrict__ mchol, double3 ru, double su, double* __restrict__ XT,
+          double* __restrict__ coef) {
+    __shared__ double red[32];
+    const int c = blockIdx.x;
+    double s[3] = {0, 0, 0};
+    for (int32_t r = threadIdx.x; r < k; r += 1024) {
+        const double* p = part + (int64_t)c * k + r;
+        double t = 0.0;
+#pragma unroll 4
+        for (int32_t ch = 0; ch < nch; ch++) t += p[(int64_t)ch * kRhs * k];
+        for (int d = 0; d < 3; d++) s[d] += scu[3 * (int64_t)r + d] * t;
+    }
+    for (int d = 0; d < 3; d++) s[d] = block_sum<32>(s[d], red);
+    const double b[3] = {s[0] - ru.x, s[1] - ru.y, s[2] - ru.z};
+    double y[3], mu[3];
+    for (int i = 0; i < 3; i++) {
+        double v = b[i];
+        for (int q = 0; q < i; q++) v -= mchol[3 * i + q] * y[q];
+        y[i] = v / mchol[4 * i];
+    }
+    for (int i = 2; i >= 0; i--) {
+        double v = y[i];
+        for (int q = i + 1; q < 3; q++) v -= mchol[3 * q + i] * mu[q];
+        mu[i] = v / mchol[4 * i];
+    }
+    for (int32_t r = threadIdx.x; r < k; r += 1024) {
+        double v = XT[(int64_t)r * kRhs + c];
+        for (int d = 0; d < 3; d++) v -= scu[3 * (int64_t)r + d] * mu[d];
+        XT[(int64_t)r * kRhs + c] = v;
+    }
+    if (threadIdx.x < 3) coef[(int64_t)c * (k + 3) + k + threadIdx.x] = mu[threadIdx.x] * su;
+}
+// coef[c][r] = the chunk sums; zero_mu: coef[c][k ..] = 0 as well.
+__global__ void lam_kernel(const double* __restrict__ part, int32_t nch, int32_t k, int zero_mu,
+                           double* __restrict__ coef) {
+    const int32_t r = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
+    if (r < k) {
+        double t = 0.0;
+#pragma unroll 4
+        for (int32_t ch = 0; ch < nch; ch++) t += part[((int64_t)ch * kRhs + c) * k + r];
+        coef[(int64_t)c * (k + 3) + r] = t;
+    } else if (r < k + 3 && zero_mu) {
+        coef[(int64_t)c * (k + 3) + r] = 0.0;
     }
 }
+
+// x = w - A3^{-1} C^T coef - mu term at (d, v): the chunk sums of column c (the sparse
+// rows), then the dense rows in order.
+__device__ __forceinline__ double solution_at(const double* __restrict__ part, int32_t nch, int32_t V, int c,
+                                              const double* __restrict__ Y, const SparseRows& sp,
+                                              const double* __restrict__ coef, int32_t k, int d, int32_t v,
+                                              double w) {
+    double s = 0.0;
+    for (int32_t ch = 0; ch < nch; ch++) s += part[((int64_t)ch * kRhs + c) * V + v];
+    for (int32_t a = 0; a < sp.nd; a++) s += Y[((int64_t)a * 3 + d) * V + v] * coef[sp.list[a]];
+    return (w - s) - coef[k + d];
+}
+__global__ void solution_kernel(const double* __restrict__ part, int32_t nch, int32_t V,
+                                const double* __restrict__ Y, SparseRows sp, const double* __restrict__ w,
+                                const double* __restrict__ coef, int32_t k, double* __restrict__ x) {
+    const int32_t v = blockIdx.x * blockDim.x + threadIdx.x, d = blockIdx.y;
+    if (v >= V) return;
+    const int64_t t = (int64_t)d * V + v;
+    x[t] = solution_at(part, nch, V, d, Y, sp, coef, k, d, v, w ? w[t] : 0.0);
+}
+// cur[idx[q]] (interleaved, rows stride apart) += the solution of coef_q, w = 0.
+__global__ void update_kernel(const double* __restrict__ part, int32_t nch, int32_t V,
+                              const double* __restrict__ Y, SparseRows sp, const double* __restrict__ coef,
+                              int32_t k, const int32_t* __restrict__ idx, double* __restrict__ cur,
+                              int64_t stride, int32_t* __restrict__ bad) {
+    const int32_t v = blockIdx.x * blockDim.x + threadIdx.x, q = blockIdx.y / 3, d = blockIdx.y % 3;
+    if (v >= V) return;
+    const int a = idx[q];
+    const double x = solution_at(part, nch, V, 3 * q + d, Y, sp, coef + (int64_t)q * (k + 3), k, d, v, 0.0);
+    if (!isfinite(x)) bad[a] = 1;
+    double* p = cur + (int64_t)a * stride + 3 * (int64_t)v + d;
+    *p = *p + x;
+}
+
+inline unsigned blocks(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
+inline int32_t rows16(int32_t n) { return (n + 15) / 16 * 16; }
 
 }  // namespace
 
@@ -217,58 +412,76 @@ int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool
         }
     }
     op.Ainv = Ainv;
-    // sparse structure of C
-    TPE_TRY(ensure(ctx, ctx->sch_nz, (sizeof(int32_t) + sizeof(double)) * (size_t)k * 3 * kNZ +
-                                         sizeof(int32_t) * (size_t)k * 4));
-    double* nz_val = ctx->sch_nz.as<double>();
-    int32_t* nz_idx = reinterpret_cast<int32_t*>(nz_val + (size_t)k * 3 * kNZ);
-    int32_t* nz_cnt = nz_idx + (size_t)k * 3 * kNZ;
-    int32_t* dense = nz_cnt + (size_t)k * 3;
+    // sparse structure of C, by row and by vertex
+    const int64_t m = 3 * (int64_t)V;
+    const size_t kk = (size_t)k;
+    TPE_TRY(ensure(ctx, ctx->sch_nz, sizeof(double) * 7 * kk + sizeof(int32_t) * (8 * kk + 2 * (size_t)V + 1)));
+    SparseRows& sp = op.sp;
+    sp.w = ctx->sch_nz.as<double>();
+    sp.stats = sp.w + 3 * kk;
+    sp.ab = reinterpret_cast<int2*>(sp.stats + 4 * kk);
+    sp.ent = reinterpret_cast<int32_t*>(sp.ab + kk);
+    int32_t* raw = sp.ent + 2 * kk;
+    int32_t* dense = raw + 2 * kk;
+    sp.list = dense + kk;
+    sp.off = sp.list + kk;
+    int32_t* count = sp.off + V + 1;
+    sp.nd = 0;
+    TPE_CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(int32_t) * (size_t)V, st));
     {
-        KernelScope ks(ctx, TPE_KGROUP_OTHER, 2);
-        sparse_rows_kernel<<<k, 256, 0, st>>>(op.C, V, nz_idx, nz_val, nz_cnt, dense);
-        y_sparse_kernel<<<dim3(k, 3, (V + 255) / 256), 256, 0, st>>>(Ainv, V, nz_idx, nz_val, nz_cnt,
-                                                                     dense, op.Y);
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 5);
+        sparse_rows_kernel<<<k, 256, 0, st>>>(op.C, V, sp, dense);
+        col_count_kernel<<<blocks(k, 256), 256, 0, st>>>(sp, k, count);
+        col_scan_kernel<<<1, 1024, 0, st>>>(sp, V, count);
+        col_fill_kernel<<<blocks(k, 256), 256, 0, st>>>(sp, k, count, raw);
+        col_sort_kernel<<<blocks(V, 8), 256, 0, st>>>(sp, V, raw);
         TPE_CUDA_TRY(cudaGetLastError());
     }
-    std::vector<int32_t> hdense((size_t)k);
-    TPE_CUDA_TRY(cudaMemcpyAsync(hdense.data(), dense, sizeof(int32_t) * k, cudaMemcpyDeviceToHost, st));
-    TPE_CUDA_TRY(cudaStreamSynchronize(st));
-    std::vector<int32_t> drows;
+    std::vector<int32_t> hdense(kk), drows;
+    TPE_TRY(download_on(ctx, st, hdense.data(), dense, sizeof(int32_t) * kk));
     for (int32_t s = 0; s < k; s++)
         if (hdense[s]) drows.push_back(s);
-    // dense rows: Y_s = Ainv C_s per coordinate block (3 right-hand sides each)
-    for (int32_t s : drows)
-        TPE_TRY(mrhs_fp64(ctx, Ainv, V, op.C + (size_t)s * 3 * V, V, 3, op.Y + (size_t)s * 3 * V));
+    sp.nd = (int32_t)drows.size();
+    sp.dense = dense;
+    if (sp.nd > 0)
+        TPE_CUDA_TRY(cudaMemcpyAsync(sp.list, drows.data(), sizeof(int32_t) * drows.size(),
+                                     cudaMemcpyHostToDevice, st));
+    // dense rows: Y_a = Ainv C_s per coordinate block, runs of up to five rows per product
+    TPE_TRY(ensure(ctx, ctx->con_Y, sizeof(double) * ((size_t)sp.nd + 1) * m));
+    op.Y = ctx->con_Y.as<double>();
+    for (size_t a = 0; a < drows.size();) {
+        size_t b = a + 1;
+        while (b < drows.size() && b - a < (size_t)kPerPass && drows[b] == drows[b - 1] + 1) b++;
+        TPE_TRY(mrhs_fp64(ctx, Ainv, V, op.C + (int64_t)drows[a] * m, V, 3 * (int32_t)(b - a), op.Y + a * m));
+        a = b;
+    }
     // the gradient right-hand side: w = A3^{-1} b
     if (b_flat) {
         TPE_TRY(finish_gradient(ctx));
+        op.W = op.Y + (size_t)sp.nd * m;
+        op.w_src = b_flat;
         TPE_TRY(mrhs_fp64(ctx, Ainv, V, b_flat, V, 3, op.W));
     }
-    // S = C Y (k x k)
-    TPE_TRY(ensure(ctx, ctx->sch_S, sizeof(double) * (size_t)k * k));
-    TPE_TRY(ensure(ctx, ctx->sch_L, sizeof(double) * (size_t)k * k));
+    // S = C A3^{-1} C^T (k x k)
+    TPE_TRY(ensure(ctx, ctx->sch_G, sizeof(double) * kk * V));
+    TPE_TRY(ensure(ctx, ctx->sch_S, sizeof(double) * kk * k));
     TPE_TRY(ensure(ctx, ctx->sch_Linv, sizeof(double) * (size_t)((k + kNB - 1) / kNB) * kNB * kNB));
-    TPE_TRY(ensure(ctx, ctx->sch_Sinv, sizeof(double) * (size_t)k * k));
+    TPE_TRY(ensure(ctx, ctx->sch_Sinv, sizeof(double) * kk * k));
+    TPE_TRY(ensure(ctx, ctx->sch_vec, sizeof(double) * (2 * kRhs * (size_t)rows16(k) + kRhs * (kk + 3) + 3 * kk + 16)));
     double* S = ctx->sch_S.as<double>();
+    op.Gt = ctx->sch_G.as<double>();
     {
-        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
-        const unsigned tk = (unsigned)((k + 31) / 32);
-        s_sparse_kernel<<<dim3(tk, tk), dim3(32, 8), 0, st>>>(op.Y, V, k, nz_idx, nz_val, nz_cnt,
-                                                             dense, S);
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, sp.nd > 0 ? 4 : 2);
+        const unsigned tk = blocks(k, 32);
+        g_kernel<<<dim3(blocks(k, 256), (unsigned)std::min(V, 4096)), 256, 0, st>>>(Ainv, V, k, sp, op.Gt);
+        s_sparse_kernel<<<dim3(tk, tk), dim3(32, 8), 0, st>>>(op.Gt, k, sp, S);
+        if (sp.nd > 0) {
+            s_dense_kernel<<<dim3(blocks(k, 256), (unsigned)sp.nd), 256, 0, st>>>(op.Y, V, k, sp, dense, S);
+            s_dense_pair_kernel<<<dim3((unsigned)sp.nd, (unsigned)sp.nd), 256, 0, st>>>(op.C, op.Y, m, k, sp, S);
+        }
         TPE_CUDA_TRY(cudaGetLastError());
     }
-    for (int32_t r : drows)
-        TPE_TRY(gram_dots(ctx, op.C + (size_t)r * 3 * V, 1, op.Y, k, 3 * (int64_t)V,
-                          S + (size_t)r * k));
-    {
-        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
-        const unsigned tk = (unsigned)((k + 31) / 32);
-        symmetrize_kernel<<<dim3(tk, tk), dim3(32, 8), 0, st>>>(S, k);
-        TPE_CUDA_TRY(cudaGetLastError());
-    }
-    double* Ls = ctx->sch_L.as<double>();
-    TPE_CUDA_TRY(cudaMemcpyAsync(Ls, S, sizeof(double) * (size_t)k * k, cudaMemcpyDeviceToDevice, st));
+    double* Ls = S;  // S itself is not needed again
     if (op.int8) {
         bool sing = false;
         TPE_TRY(spd_inverse_int8(ctx, Ls, k, 0.0, ctx->inv_X.as<double>(), ctx->inv_W.as<double>(),
@@ -296,21 +509,114 @@ int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool
     return TPE_OK;
 }
 
-int32_t large_schur_apply(tpe_ctx* ctx, const SaddleOp& op, const double* rc, int32_t nr,
-                          double* out) {
+// sch_vec: XT (two of them), coefficients of up to 16 solves, Scu and M's factor.
+namespace {
+double* vec_xt(tpe_ctx* ctx) { return ctx->sch_vec.as<double>(); }
+double* vec_coef(tpe_ctx* ctx, const SaddleOp& op) {
+    return vec_xt(ctx) + 2 * (size_t)kRhs * rows16(op.k);
+}
+double* vec_scu(tpe_ctx* ctx, const SaddleOp& op) { return vec_coef(ctx, op) + kRhs * ((size_t)op.k + 3); }
+}  // namespace
+
+int32_t large_set_mu(tpe_ctx* ctx, const SaddleOp& op, const double* h_scu, const double* h_mchol) {
+    double* d = vec_scu(ctx, op);
+    TPE_CUDA_TRY(cudaMemcpyAsync(d, h_scu, sizeof(double) * 3 * (size_t)op.k, cudaMemcpyHostToDevice, ctx->stream));
+    TPE_CUDA_TRY(cudaMemcpyAsync(d + 3 * (size_t)op.k, h_mchol, sizeof(double) * 9, cudaMemcpyHostToDevice, ctx->stream));
+    return TPE_OK;
+}
+
+int32_t large_sinv(tpe_ctx* ctx, const SaddleOp& op, const double* h_rc, int32_t nr, double* h_out) {
     const int32_t k = op.k;
-    TPE_TRY(ensure(ctx, ctx->sch_vec, sizeof(double) * 2 * 16 * (size_t)k));
-    double* din = ctx->sch_vec.as<double>();
-    double* dout = din + (size_t)16 * k;
-    for (int32_t c0 = 0; c0 < nr; c0 += 16) {
-        const int32_t n = std::min(16, nr - c0);
-        TPE_CUDA_TRY(cudaMemcpyAsync(din, rc + (size_t)c0 * k, sizeof(double) * (size_t)n * k,
-                                     cudaMemcpyHostToDevice, ctx->stream));
-        TPE_TRY(mrhs_fp64(ctx, op.Sinv, k, din, k, n, dout));
-        TPE_CUDA_TRY(cudaMemcpyAsync(out + (size_t)c0 * k, dout, sizeof(double) * (size_t)n * k,
-                                     cudaMemcpyDeviceToHost, ctx->stream));
-        TPE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    double* din = vec_xt(ctx);  // rows of k, then the products' rows
+    double* dout = din + (size_t)kRhs * rows16(k);
+    TPE_CUDA_TRY(cudaMemcpyAsync(din, h_rc, sizeof(double) * (size_t)nr * k, cudaMemcpyHostToDevice, ctx->stream));
+    TPE_TRY(mrhs_fp64(ctx, op.Sinv, k, din, k, nr, dout));
+    return download_on(ctx, ctx->stream, h_out, dout, sizeof(double) * (size_t)nr * k);
+}
+
+int32_t large_multipliers(tpe_ctx* ctx, const SaddleOp& op, const double* d_rc, int64_t stride,
+                          const int32_t* d_pos, int32_t n, const double ru[3], double** d_coef) {
+    const int32_t k = op.k;
+    const cudaStream_t st = ctx->stream;
+    double *XT = vec_xt(ctx), *coef = vec_coef(ctx, op), *scu = vec_scu(ctx, op);
+    *d_coef = coef;
+    {
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+        rc_rhs_kernel<<<dim3(blocks(rows16(k), 256), (unsigned)n), 256, 0, st>>>(d_rc, stride, d_pos, k, rows16(k),
+                                                                             n, XT);
+        TPE_CUDA_TRY(cudaGetLastError());
     }
+    const double* part = nullptr;
+    int32_t nch = 0;
+    TPE_TRY(mrhs_part(ctx, op.Sinv, k, k, XT, &part, &nch));
+    if (op.trans_constrained) {
+        {
+            KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+            mu_kernel<<<(unsigned)n, 1024, 0, st>>>(part, nch, k, scu, scu + 3 * (size_t)k,
+                                                   make_double3(ru[0], ru[1], ru[2]),
+                                                   1.0 / (op.rho * sqrt((double)op.V)), XT, coef);
+            TPE_CUDA_TRY(cudaGetLastError());
+        }
+        TPE_TRY(mrhs_part(ctx, op.Sinv, k, k, XT, &part, &nch));
+    }
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    lam_kernel<<<dim3(blocks(k + 3, 256), (unsigned)n), 256, 0, st>>>(part, nch, k, op.trans_constrained ? 0 : 1, coef);
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
+}
+
+int32_t large_solution(tpe_ctx* ctx, const SaddleOp& op, const double* d_coef, const double* d_w, double* d_x) {
+    const int32_t V = op.V, k = op.k;
+    double* XT = vec_xt(ctx);
+    {
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+        coef_rhs_kernel<<<dim3(blocks(rows16(k), 256), 1), 256, 0, ctx->stream>>>(op.sp, k, rows16(k), d_coef, 1, XT);
+        TPE_CUDA_TRY(cudaGetLastError());
+    }
+    const double* part = nullptr;
+    int32_t nch = 0;
+    TPE_TRY(mrhs_part(ctx, op.Gt, V, k, XT, &part, &nch));
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    solution_kernel<<<dim3(blocks(V, 128), 3), 128, 0, ctx->stream>>>(part, nch, V, op.Y, op.sp, d_w, d_coef, k, d_x);
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
+}
+
+int32_t large_update(tpe_ctx* ctx, const SaddleOp& op, const double* d_coef, int32_t nu, const int32_t* d_idx,
+                     double* d_cur, int64_t stride, int32_t* d_bad) {
+    const int32_t V = op.V, k = op.k;
+    double* XT = vec_xt(ctx);
+    for (int32_t q0 = 0; q0 < nu; q0 += kPerPass) {
+        const int32_t n = std::min(nu - q0, kPerPass);
+        const double* coef = d_coef + (size_t)q0 * (k + 3);
+        {
+            KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+            coef_rhs_kernel<<<dim3(blocks(rows16(k), 256), (unsigned)n), 256, 0, ctx->stream>>>(op.sp, k, rows16(k),
+                                                                                           coef, n, XT);
+            TPE_CUDA_TRY(cudaGetLastError());
+        }
+        const double* part = nullptr;
+        int32_t nch = 0;
+        TPE_TRY(mrhs_part(ctx, op.Gt, V, k, XT, &part, &nch));
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+        update_kernel<<<dim3(blocks(V, 128), 3 * (unsigned)n), 128, 0, ctx->stream>>>(
+            part, nch, V, op.Y, op.sp, coef, k, d_idx + q0, d_cur, stride, d_bad);
+        TPE_CUDA_TRY(cudaGetLastError());
+    }
+    return TPE_OK;
+}
+
+int32_t large_ct(tpe_ctx* ctx, const SaddleOp& op, const double* d_lam, double* d_out) {
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    ct_block_kernel<<<blocks(op.V, 128), 128, 0, ctx->stream>>>(op.C, op.V, op.sp, d_lam, d_out);
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
+}
+
+int32_t large_cx(tpe_ctx* ctx, const SaddleOp& op, const double* d_x, double* d_out) {
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    cx_kernel<<<op.sp.nd + blocks(op.k, 256), 256, 0, ctx->stream>>>(op.C, op.V, op.sp, op.sp.dense, op.k, d_x, d_out);
+    TPE_CUDA_TRY(cudaGetLastError());
     return TPE_OK;
 }
 

@@ -48,6 +48,21 @@ constexpr int kMixedMaxRhs = 48;
 // Most step sizes one batched line-search launch projects together.
 constexpr int kMaxTrials = 16;
 
+// The rows of a large constraint Jacobian that are one 3-vector w times one vertex
+// (a pin) or times the difference of two (an edge length: w at a, -w at b): row s is
+// w_s (x) (e_a - e_b), b = -1 for one vertex. The same by vertex, and the list of
+// the other (dense) rows. Device pointers (schur.cu).
+struct SparseRows {
+    int2* ab = nullptr;        // k: (a, b); (-1, -1) for a dense row
+    double* w = nullptr;       // k x 3
+    int32_t* off = nullptr;    // V + 1
+    int32_t* ent = nullptr;    // 2 row + (0: at a, 1: at b), by vertex, in row order
+    int32_t* dense = nullptr;  // k: 1 for a row of another form
+    int32_t* list = nullptr;   // nd dense rows
+    double* stats = nullptr;   // k x 4: sums over the coordinate blocks, sum of |.|
+    int32_t nd = 0;
+};
+
 // Everything the structured saddle solve keeps between the factorization and
 // later solves: the frozen operator of optimizer.ts's 'frozen' projection.
 struct SaddleOp {
@@ -65,13 +80,15 @@ struct SaddleOp {
     double* L = nullptr;     // V x V Cholesky factor of A_rho (lower, row-major)
     double* Linv = nullptr;  // nb x 64 x 64 inverses of the diagonal blocks of L
     double* C = nullptr;     // k x 3V dense constraint Jacobian
-    double* Y = nullptr;     // k x 3V: Abar_rho^{-1} C^T (row s = column s of C^T)
+    double* Y = nullptr;     // k x 3V: Abar_rho^{-1} C^T (row s = column s of C^T; large: the nd dense rows)
     double* W = nullptr;     // 3V: Abar_rho^{-1} b for the b given at factor time (row k of Y)
     const double* w_src = nullptr;  // that b (device), or null
     // large constraint sets (schur.cu): explicit inverses on the device
     bool large = false;
     double* Ainv = nullptr;  // V x V: A_rho^{-1}
     double* Sinv = nullptr;  // k x k: (C A3^{-1} C^T)^{-1}
+    SparseRows sp;
+    double* Gt = nullptr;    // V x k: column s = Ainv (e_a - e_b) of sparse row s
     bool int8 = false;       // both inverses with their products on the int8 tensor cores
     double chol_tol = 0.0;   // pivot tolerance of A_rho's Cholesky
     // host: small Schur complement and its factors
@@ -155,13 +172,14 @@ struct tpe_ctx {
         flat2, flat3, dir;
     tpe::DevBuf grad_ctr;  // tile counter of the SM-bounded gradient kernel
     // large constraint sets (schur.cu)
-    tpe::DevBuf mat_Ainv, inv_X, inv_W, inv_T, sch_nz, sch_S, sch_L, sch_Linv, sch_Sinv, sch_vec;
+    tpe::DevBuf mat_Ainv, inv_X, inv_W, inv_T, sch_nz, sch_G, sch_S, sch_Linv, sch_Sinv, sch_vec;
     tpe::DevBuf ref_r, ref_x;  // residual and correction of the refinement step
     tpe::DevBuf oz_planes, oz_err;  // digit planes and timeout flag of ozaki_gemm_nt
-    tpe::DevBuf oz_base;            // the FP64 base blocks of spd_inverse_int8
+    tpe::DevBuf oz_base;            // diagonal-block inverses of spd_inverse_int8's base blocks
     tpe::DevBuf bh_buf;             // Barnes-Hut tree, permutation and per-edge sums (bh.cu)
     tpe::DevBuf dag_solve, dag_err;  // the same of the triangular solves, and their error flag
     tpe::DevBuf dag_flags;     // flags and counters of the data-flow factorization (chol_dag.cu)
+    tpe::DevBuf mrhs_xt;       // right-hand-side-major input of mrhs_fp64
     tpe::DevBuf ycomb_part;    // split-over-rows partial sums of Y^T coef
     tpe::DevBuf mx_ctr;    // tile counters of the persistent trailing updates
     tpe::DevBuf pairM;                      // E x E double2 (Mb, M0) pair matrix
@@ -319,6 +337,7 @@ struct CholDag {
     double* L = nullptr;     // lower triangle read; L on return
     double* Linv = nullptr;  // nb x 64 x 64: inverses of L's diagonal blocks
     int32_t n = 0;
+    int64_t ld = 0;  // row length of L, W and X (0: n)
     double tol = 0.0;
     double* B = nullptr;  // nr x n
     int32_t nr = 0;
@@ -378,7 +397,7 @@ int32_t transpose_fp64(tpe_ctx* ctx, const double* src, int64_t lds, int32_t m, 
 // out = A^{-1} for the SPD n x n matrix in Mat (lower triangle read; Mat is
 // overwritten) with the heavy products on the integer tensor cores
 // (ozaki_gemm_nt): recursive Cholesky and triangular inverse in halves down to
-// blocks of at most 1024 (chol_dag there), then out = X^T X. X, W (n x n) and Tt ((n/2 + 64)^2) are scratch. A pivot at or
+// blocks of at most 2048 (chol_dag there), then out = X^T X. X, W (n x n) and Tt ((n/2 + 64)^2) are scratch. A pivot at or
 // below piv_tol sets *singular.
 int32_t spd_inverse_int8(tpe_ctx* ctx, double* Mat, int32_t n, double piv_tol, double* X,
                          double* W, double* Tt, double* out, bool* singular);
@@ -386,6 +405,11 @@ int32_t spd_inverse_int8(tpe_ctx* ctx, double* Mat, int32_t n, double piv_tol, d
 // X and Y nr rows of stride ldx >= n (mixed.cu: the CG's multi-RHS kernel).
 int32_t mrhs_fp64(tpe_ctx* ctx, const double* M, int32_t n, const double* X, int32_t ldx,
                   int32_t nr, double* Y);
+// The same for a rows x cols matrix M and X right-hand-side major (XT: (cols + 15) / 16
+// * 16 rows of 16, zero rows past cols) without the last sum: part[ch][c][i], ch <
+// *nch, i < rows, to be added in order.
+int32_t mrhs_part(tpe_ctx* ctx, const double* M, int32_t rows, int32_t cols, const double* XT,
+                  const double** part, int32_t* nch);
 int32_t trace(tpe_ctx* ctx, const double* d_A, int32_t n, double* d_out);
 
 // ---- mixed-precision solve (mixed.cu) ------------------------------------
@@ -403,8 +427,9 @@ int32_t mixed_solve(tpe_ctx* ctx, const double* d_A, const double* d_B, double* 
 constexpr int32_t kLargeSchur = 64;
 // Iterative refinement of the large-set gradient solve: stop at this relative
 // saddle residual, or after kLargeRefineMax corrections, or when a correction
-// no longer halves the residual.
-constexpr double kRefineStop = 1e-13;
+// no longer halves the residual. (At 1e-13 the int8 inverses could stop with a
+// residual of 5e-14, which on a loop network left the step's energy 2e-7 off.)
+constexpr double kRefineStop = 1e-14;
 constexpr int32_t kLargeRefineMax = 4;
 // The refined gradient-solve residual the int8-tensor-core inverses must reach;
 // above it the step rebuilds them in FP64. The FP64 inverses reach 1e-14 after
@@ -412,12 +437,25 @@ constexpr int32_t kLargeRefineMax = 4;
 // same or stall far above this (rows whose entries span many orders of
 // magnitude lose digits under a per-row scale).
 constexpr double kInt8ResidualGate = 1e-12;
-// From A_rho in op.L (overwritten): op.Ainv, op.Y (k x 3V), op.W = A3^{-1} b when b is
-// given, and op.Sinv; *singular when the Schur complement is not SPD.
+// From A_rho in op.L (overwritten): op.Ainv, op.sp, op.W = A3^{-1} b when b is given,
+// and op.Sinv; *singular when the Schur complement is not SPD.
 int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool* singular);
-// out[c] = Sinv rc[c] for nr host vectors of length k (host in and out).
-int32_t large_schur_apply(tpe_ctx* ctx, const SaddleOp& op, const double* rc, int32_t nr,
-                          double* out);
+// out[c] = Sinv rc[c] for nr <= 16 host vectors of length k (host in and out).
+int32_t large_sinv(tpe_ctx* ctx, const SaddleOp& op, const double* h_rc, int32_t nr, double* h_out);
+// Scu (k x 3) and the Cholesky factor of M (3 x 3) for large_multipliers.
+int32_t large_set_mu(tpe_ctx* ctx, const SaddleOp& op, const double* h_scu, const double* h_mchol);
+// Multipliers of n <= 16 reduced right-hand sides d_rc + pos[c] * stride (pos null: c):
+// *d_coef (n x (k + 3)): lam, then the scaled mu. ru: U^T w, the same for all.
+int32_t large_multipliers(tpe_ctx* ctx, const SaddleOp& op, const double* d_rc, int64_t stride,
+                          const int32_t* d_pos, int32_t n, const double ru[3], double** d_coef);
+// x = w - A3^{-1} C^T lam - mu term (block layout; w may be null), and the same for nu
+// coefficient vectors added to cur[idx[q]] (project_update's contract).
+int32_t large_solution(tpe_ctx* ctx, const SaddleOp& op, const double* d_coef, const double* d_w, double* d_x);
+int32_t large_update(tpe_ctx* ctx, const SaddleOp& op, const double* d_coef, int32_t nu, const int32_t* d_idx,
+                     double* d_cur, int64_t stride, int32_t* d_bad);
+// C^T lam (3V) and C x (k) from the sparse rows.
+int32_t large_ct(tpe_ctx* ctx, const SaddleOp& op, const double* d_lam, double* d_out);
+int32_t large_cx(tpe_ctx* ctx, const SaddleOp& op, const double* d_x, double* d_out);
 // Joins the gradient running on stream3 (api.cu).
 int32_t finish_gradient(tpe_ctx* ctx);
 
@@ -456,10 +494,10 @@ int32_t project_update(tpe_ctx* ctx, const double* d_Y, int32_t k, int32_t V, co
                        int32_t* d_bad);
 // Structured residual ||K z - rhs|| / max(1, ||rhs||) with A (V x V), C (k x 3V);
 // optionally the residual vector rhs - K z itself: top (device, 3V) and bottom
-// (host, k).
+// (host, k). large: C through its sparse rows.
 int32_t saddle_residual(tpe_ctx* ctx, const double* d_A, int32_t V, const double* d_C, int32_t k,
                         const double* d_x, const double* lam, const double* d_rhs_top,
                         const double* rhs_bottom, double* out, double* d_res_top = nullptr,
-                        double* res_bottom = nullptr);
+                        double* res_bottom = nullptr, const SaddleOp* large = nullptr);
 
 }  // namespace tpe

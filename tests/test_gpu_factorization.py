@@ -74,3 +74,42 @@ def test_repeats_bit_for_bit():
         again = T.solveSaddleFromA(A, 777, C, b, d)
         assert np.array_equal(first["x"], again["x"])
         assert np.array_equal(first["lambda"], again["lambda"])
+
+
+def test_rows_of_every_form():
+    """More than 64 rows of all kinds: one vertex, a difference of two (also along one
+    axis only), two vertices that are no difference, one vertex shared by 40 rows, and
+    two dense rows."""
+    n = 150
+    A, _, b, _ = _system(n, 1, 5)
+    rng = np.random.default_rng(6)
+    C = []
+    for s in range(60):
+        row = np.zeros((3, n))
+        w = rng.standard_normal(3) if s % 3 else np.array([0.0, 1.5, 0.0])
+        p, q = (0, 1 + s) if s < 40 else (2 * s - 20, 2 * s - 19)
+        row[:, p] += w
+        row[:, q] -= w
+        C.append(row)
+    for v in (100, 105):
+        for c in range(3):
+            row = np.zeros((3, n))
+            row[c, v] = 1.0
+            C.append(row)
+    for v in (110, 120, 130):
+        row = np.zeros((3, n))
+        row[:, v], row[:, v + 3] = rng.standard_normal(3), rng.standard_normal(3)
+        C.append(row)
+    C += [rng.standard_normal((3, n)) / n for _ in range(2)]
+    C = np.array(C).reshape(len(C), 3 * n)
+    assert len(C) > 64
+    d = rng.standard_normal(len(C))
+    K = np.zeros((3 * n + len(C),) * 2)
+    for c in range(3):
+        K[c * n:(c + 1) * n, c * n:(c + 1) * n] = A
+    K[3 * n:, :3 * n], K[:3 * n, 3 * n:] = C, C.T
+    ref = np.linalg.solve(K, np.concatenate([b, d]))
+    r = T.solveSaddleFromA(A, n, C, b, d)
+    assert r["residual"] <= 1e-10
+    assert np.linalg.norm(r["x"] - ref[:3 * n]) <= 1e-9 * np.linalg.norm(ref[:3 * n])
+    assert np.linalg.norm(r["lambda"] - ref[3 * n:]) <= 1e-9 * max(1.0, np.linalg.norm(ref[3 * n:]))

@@ -761,7 +761,7 @@ int32_t op_solve(tpe_ctx* ctx, const double* b_flat, const double* d, double* x_
             TPE_TRY(saddle_residual(ctx, op.A, V, op.C, k, x_flat, lam.data(), b_flat, bottom.data(),
                                     &r0, rt, rb.data(), &op));
             const bool done = it > 0 && (!(r0 > kRefineStop) || !(r0 < 0.5 * prev) ||
-                                         it >= kLargeRefineMax);
+                                         it >= (op.int8 ? kInt8RefineMax : kLargeRefineMax));
             if (done) {
                 if (residual) *residual = r0;
                 return TPE_OK;

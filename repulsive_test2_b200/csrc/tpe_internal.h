@@ -431,12 +431,15 @@ constexpr int32_t kLargeSchur = 64;
 // residual of 5e-14, which on a loop network left the step's energy 2e-7 off.)
 constexpr double kRefineStop = 1e-14;
 constexpr int32_t kLargeRefineMax = 4;
-// The refined gradient-solve residual the int8-tensor-core inverses must reach;
-// above it the step rebuilds them in FP64. The FP64 inverses reach 1e-14 after
-// one or two corrections on every measured curve; the int8 ones either do the
-// same or stall far above this (rows whose entries span many orders of
-// magnitude lose digits under a per-row scale).
-constexpr double kInt8ResidualGate = 1e-12;
+// The residual the int8-tensor-core inverses must reach within kInt8RefineMax
+// corrections; else the step rebuilds them in FP64. Good inverses lose four digits or
+// more of it per correction, as the FP64 ones do. Where rows span many orders of
+// magnitude (digits lost under a per-row scale) a correction takes one digit or less,
+// and the projection, which uses the inverses without refinement, is off with them: on
+// a loop network residuals of 3.4e-7, 3.9e-12, 1.2e-12, 2.2e-13, 5.9e-14 left the
+// step's energy 9e-8 off.
+constexpr double kInt8ResidualGate = 1e-13;
+constexpr int32_t kInt8RefineMax = 2;
 // From A_rho in op.L (overwritten): op.Ainv, op.sp, op.W = A3^{-1} b when b is given,
 // and op.Sinv; *singular when the Schur complement is not SPD.
 int32_t large_schur_build(tpe_ctx* ctx, SaddleOp& op, const double* b_flat, bool* singular);

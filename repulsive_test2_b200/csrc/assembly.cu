@@ -19,38 +19,51 @@
 // symmetrisation.
 #include <math.h>
 
+#include "pair_math.cuh"
 #include "tpe_internal.h"
 
 namespace tpe {
 namespace {
 
 
+// x^(-1/3) for x > 0: an FP32 estimate y (exp2 of log2) times the binomial series
+// of (1 - e)^(-1/3), e = 1 - x y^3, through e^2 (the e^3 left out is below 2^-60).
+// Beyond the range where FP32 holds y and y^3, CUDA's own.
+__device__ __forceinline__ double inv_cbrt(double x) {
+    if (!(x > 1e-30 && x < 1e30)) return rcbrt(x);
+    const double y = (double)exp2f(-0.33333334f * __log2f((float)x));
+    const double e = fma(-x * y, y * y, 1.0);
+    return fma(y * e, fma(2.0 / 9.0, e, 1.0 / 3.0), y);
+}
+
 // (|d|+eps)^(-(2 sigma + 1)) from dn = |d|+eps and its reciprocal idn;
 // MODE 1: alpha = 3, beta = 6 -> exponent 7/3.
 template <int MODE>
 __device__ __forceinline__ double inv_dist_pow(double dn, double idn, double distExp) {
-    if (MODE == 1) return rcbrt(dn) * (idn * idn);
+    if (MODE == 1) return inv_cbrt(dn) * (idn * idn);
     return 1.0 / pow(dn, distExp);
 }
 
-// |d| and 1/(|d| + eps) for x = |d|^2 from one reciprocal square root r:
-// 1/(|d| + eps) = r / (1 + t), t = eps r, summed as r (1 - t + t^2) when
-// t < 2^-20 (the first term left out is below 2^-60 relative); otherwise the
-// square root and the division themselves.
-__device__ __forceinline__ void dist_inv(double x, double eps, double& s, double& inv_se) {
-    const double r = rsqrt(x);
-    const double t = eps * r;
-    if (t < 9.5367431640625e-07) {
-        s = x * r;
-        inv_se = fma(-r, t * (1.0 - t), r);
-    } else {
-        s = sqrt(x);
-        inv_se = 1.0 / (s + eps);
-    }
+// Of one endpoint pair at squared distance x: kd = (|d|+eps)^(-(2 sigma + 1)) and
+// kq = kd (|d|+eps)^-4.
+template <int MODE>
+__device__ __forceinline__ void dist_weights(double x, double distExp, double eps, double& kd, double& kq) {
+    double s, inv, idn;
+    dist_terms(x, eps, s, inv, idn);
+    kd = inv_dist_pow<MODE>(s + eps, idn, distExp);
+    const double i2 = idn * idn;
+    kq = kd * (i2 * i2);
 }
 
-// sqrt(x) for x >= 0 from a reciprocal square root (0 at x = 0).
-__device__ __forceinline__ double sqrt_r(double x) { return x > 0.0 ? x * rsqrt(x) : sqrt(x); }
+// (|T x d| + eps)^2 for the two ends d1, d2 of an edge with tangent T seen from one
+// point (T x d is the same for both: the nearer one loses the least).
+__device__ __forceinline__ double area_sq(double Tx, double Ty, double Tz, double dx, double dy, double dz,
+                                          double eps) {
+    const double cx = Ty * dz - Tz * dy, cy = Tz * dx - Tx * dz, cz = Tx * dy - Ty * dx;
+    const double c2 = cx * cx + cy * cy + cz * cz;
+    const double cn = (c2 > 1e-300 && c2 < 1e300 ? c2 * rsqrt_normal(c2) : sqrt(c2)) + eps;
+    return cn * cn;
+}
 
 constexpr int kT = 32;  // pair tile: 32 edges I x 32 edges J
 
@@ -85,36 +98,39 @@ __device__ __forceinline__ void load_edge(const double4* __restrict__ ea,
     }
 }
 
-// Symmetric pair weights of one unordered pair: (w_IJ + w_JI, q_IJ + q_JI).
+// Symmetric pair weights of one unordered pair: (w_IJ + w_JI, q_IJ + q_JI). Four
+// distances and four areas (an edge against a point: the same area for its two ends).
 template <int MODE>
 __device__ __forceinline__ double2 pair_weight(const EdgeRec& a, const EdgeRec& b, double distExp,
                                                double eps) {
-    double sumDist = 0.0, sumLowIJ = 0.0, sumLowJI = 0.0;
+    double d[2][2][3], x[2][2], kq[2][2], sumDist = 0.0;
 #pragma unroll
-    for (int s = 0; s < 4; s++) {
-        const int ai = s >> 1, bj = s & 1;
-        const double dx = (ai ? a.p2.x : a.p1.x) - (bj ? b.p2.x : b.p1.x);
-        const double dy = (ai ? a.p2.y : a.p1.y) - (bj ? b.p2.y : b.p1.y);
-        const double dz = (ai ? a.p2.z : a.p1.z) - (bj ? b.p2.z : b.p1.z);
-        double dlen, idn;
-        dist_inv(dx * dx + dy * dy + dz * dz, eps, dlen, idn);
-        const double dn = dlen + eps;
-        const double kd = inv_dist_pow<MODE>(dn, idn, distExp);
-        sumDist += kd;
-        const double idn2 = idn * idn;
-        const double kq = kd * (idn2 * idn2);
-        double cx = a.T.y * dz - a.T.z * dy, cy = a.T.z * dx - a.T.x * dz,
-               cz = a.T.x * dy - a.T.y * dx;
-        double cn = sqrt_r(cx * cx + cy * cy + cz * cz) + eps;
-        sumLowIJ += cn * cn * kq;
-        cx = b.T.y * dz - b.T.z * dy;
-        cy = b.T.z * dx - b.T.x * dz;
-        cz = b.T.x * dy - b.T.y * dx;
-        cn = sqrt_r(cx * cx + cy * cy + cz * cz) + eps;
-        sumLowJI += cn * cn * kq;
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            d[i][j][0] = (i ? a.p2.x : a.p1.x) - (j ? b.p2.x : b.p1.x);
+            d[i][j][1] = (i ? a.p2.y : a.p1.y) - (j ? b.p2.y : b.p1.y);
+            d[i][j][2] = (i ? a.p2.z : a.p1.z) - (j ? b.p2.z : b.p1.z);
+            x[i][j] = d[i][j][0] * d[i][j][0] + d[i][j][1] * d[i][j][1] + d[i][j][2] * d[i][j][2];
+            double kd;
+            dist_weights<MODE>(x[i][j], distExp, eps, kd, kq[i][j]);
+            sumDist += kd;
+        }
+    double low = 0.0;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {  // edge a against point j of b
+        const int n = x[0][j] <= x[1][j] ? 0 : 1;
+        low += area_sq(a.T.x, a.T.y, a.T.z, n ? d[1][j][0] : d[0][j][0], n ? d[1][j][1] : d[0][j][1],
+                       n ? d[1][j][2] : d[0][j][2], eps) * (kq[0][j] + kq[1][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {  // edge b against point i of a
+        const int n = x[i][0] <= x[i][1] ? 0 : 1;
+        low += area_sq(b.T.x, b.T.y, b.T.z, n ? d[i][1][0] : d[i][0][0], n ? d[i][1][1] : d[i][0][1],
+                       n ? d[i][1][2] : d[i][0][2], eps) * (kq[i][0] + kq[i][1]);
     }
     const double ll = a.p1.w * b.p1.w;
-    return make_double2(0.5 * ll * sumDist, 0.0625 * ll * (sumLowIJ + sumLowJI));
+    return make_double2(0.5 * ll * sumDist, 0.0625 * ll * low);
 }
 
 // One block per upper-triangular 32x32 tile (it <= jt) of the E x E pair
@@ -308,155 +324,231 @@ gather_A_kernel(const double2* __restrict__ M, int32_t E, const int32_t* __restr
 // v is the second vertex of edge v-1 and the first of edge v, so
 //   A[v][u] = sum_{I in {v-1, v}} sum_{J in {u-1, u}} s_vI s_uJ Mb'[I][J] + M0'[I][J]
 // (s = +1 for the first vertex, -1 for the second): a 2 x 2 stencil on the pair
-// matrix. One block per lower-triangular 32 x 32 vertex tile computes the
-// 33 x 33 pair weights of its edges and the one edge before (shared memory) and
-// writes A's tile and its mirror once each; nothing of size E^2 is stored. The
-// pair matrix's diagonal (the row sums) is added to A's cyclic band afterwards
-// (loop_band_kernel), from the same per-tile row sums as the general path.
-constexpr int kLT = 32;       // vertex tile
-constexpr int kLH = kLT + 1;  // edges per side: the tile's own and the one before
+// matrix. A warp takes kStrip columns u of A and marches down R rows v: lane j holds
+// vertex u0 - 1 + j and the edge that begins there. Each row's vertex is taken once
+// against the 32 lane vertices (one distance), the lane's edge against the row's
+// vertex and the row's edge against the lane's vertex (one area each: an area is the
+// same from both ends of the edge); the four distances and areas of an edge pair, and
+// the stencil, are then sums with the neighbour lane (shuffles) and the row before
+// (registers): 1 distance and 2 areas per pair where a pair on its own has 4 and 8.
+// A's lower tile is written along rows, its mirror through shared memory 16 rows at a
+// time; nothing of size E^2 is stored. The pair matrix's diagonal (the row sums of the
+// weights over I > J, by rows and by columns) is added to A's cyclic band afterwards
+// (loop_band_kernel).
+//
+// Bound: FP64 pipe and its latency, about 100 FP64 operations per unordered pair.
+// Measured at V = 8192: 1290 us with each pair on its own; 984 with tables of distances
+// and areas in shared memory (issue-bound: 690 instructions per pair); 525 in this form
+// (350 instructions, FP64 pipe 44 %). The band 103 -> 20.
+constexpr int kStrip = 30;   // columns per warp: 32 vertices, 31 edges
+constexpr int kBatch = 16;   // rows per mirror write
+constexpr int kLoopWarps = 4;
+
+struct LoopSmem {
+    double a[kBatch][33];          // A's rows
+    double w[kBatch][33], q[kBatch][33];  // the weights of own pairs I > J
+    double row[kBatch][8];         // the batch's vertices, tangents and l^eps
+};
 
 template <int MODE>
-__global__ void __launch_bounds__(256)
-assemble_loop_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
-                     const int2* __restrict__ edges, int32_t V, double distExp, double eps,
-                     double* __restrict__ A, double2* __restrict__ rowpart) {
-    __shared__ EdgeRec sI[kLH], sJ[kLH];
-    __shared__ double2 W[kLH][kLH + 1];  // (Mb', M0') of edge pair (k, l)
-    // the symmetric weights w of the same pairs, then (after the row sums) the
-    // A tile staged for its mirror
-    __shared__ double2 wr_raw[kLH * (kLH + 1)];
-    double2(*Wr)[kLH + 1] = reinterpret_cast<double2(*)[kLH + 1]>(wr_raw);
-    double(*ta)[kLT + 1] = reinterpret_cast<double(*)[kLT + 1]>(wr_raw);
-    static_assert(sizeof(double) * kLT * (kLT + 1) <= sizeof(double2) * kLH * (kLH + 1),
-                  "the staged A tile fits in the weights' space");
-    const int32_t t = blockIdx.x;
-    int32_t ti = (int32_t)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
-    while ((int64_t)ti * (ti + 1) / 2 > t) ti--;
-    while ((int64_t)(ti + 1) * (ti + 2) / 2 <= t) ti++;
-    const int32_t tj = t - ti * (ti + 1) / 2;
-    const int32_t v0 = ti * kLT, u0 = tj * kLT;
-    const int tid = threadIdx.x;
-    // edge index of row k: k = 0 is the edge before the tile, k >= 1 edge v0 + k - 1
-    auto edge_of = [&](int32_t w0, int k) -> int32_t {
-        if (k == 0) return w0 == 0 ? V - 1 : w0 - 1;
-        const int32_t I = w0 + k - 1;
-        return I < V ? I : -1;
+__global__ void __launch_bounds__(32 * kLoopWarps)
+assemble_loop_kernel(const double4* __restrict__ ea, int32_t V, int32_t R, double distExp, double eps,
+                     double* __restrict__ A, double2* __restrict__ rowslot, double2* __restrict__ colslot) {
+    extern __shared__ __align__(16) unsigned char loop_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    LoopSmem& sm = reinterpret_cast<LoopSmem*>(loop_smem)[warp];
+    const int32_t rb = blockIdx.y, cs = blockIdx.x * kLoopWarps + warp;
+    const int32_t v0 = rb * R, u0 = cs * kStrip;
+    if (u0 >= V || u0 >= v0 + R) return;  // (no block-wide barrier below)
+    auto wrap = [&](int32_t v) -> int32_t { return v < 0 ? v + V : (v >= V ? 0 : v); };
+    // edge I begins at vertex I: ea[I] = (vertex I, l^eps of edge I)
+    const int32_t J = u0 - 1 + lane;  // this lane's vertex and edge (-1: the last)
+    const double4 me = ea[wrap(J)];
+    const bool lvalid = J < V && lane < 31;
+    const double nx = __shfl_down_sync(0xffffffffu, me.x, 1), ny = __shfl_down_sync(0xffffffffu, me.y, 1),
+                 nz = __shfl_down_sync(0xffffffffu, me.z, 1);
+    double tx = nx - me.x, ty = ny - me.y, tz = nz - me.z;
+    {
+        const double len = sqrt(tx * tx + ty * ty + tz * tz);
+        const double inv = len < 1e-14 ? 0.0 : 1.0 / len;
+        tx *= inv;
+        ty *= inv;
+        tz *= inv;
+    }
+    const int32_t Jw = wrap(J);
+    const bool own = lane >= 1 && lane <= kStrip && J < V;  // J among the strip's own columns
+    double csw = 0.0, csq = 0.0;
+    // the row vertex before, against this lane
+    double pdx = 0, pdy = 0, pdz = 0, px2 = 1.0, pkd = 0, pkq = 0, pr = 0;
+    double gprev = 0.0;
+    // one row vertex: distances, and the lane's edge against it
+    auto vertex = [&](double x, double y, double z, double& dx, double& dy, double& dz, double& x2, double& kd,
+                      double& kq, double& r) {
+        dx = x - me.x;
+        dy = y - me.y;
+        dz = z - me.z;
+        x2 = dx * dx + dy * dy + dz * dz;
+        if (MODE == 1) {
+            const double ir = rsqrt_normal(x2);
+            const double t = eps * ir;
+            const double idn = fma(-ir, t * (1.0 - t), ir);
+            const double dn = fma(x2, ir, eps);
+            const float y0 = exp2f(-0.33333334f * __log2f((float)dn));
+            const double yd = (double)y0;
+            const double e = fma(-dn * yd, yd * yd, 1.0);
+            const double ic = fma(yd * e, fma(2.0 / 9.0, e, 1.0 / 3.0), yd);
+            const double i2 = idn * idn;
+            kd = ic * i2;
+            kq = kd * (i2 * i2);
+            // near zero, or beyond what FP32 holds: the general form
+            if (!(t < 9.5367431640625e-07 && dn > 1e-30 && dn < 1e30)) dist_weights<MODE>(x2, distExp, eps, kd, kq);
+        } else {
+            dist_weights<MODE>(x2, distExp, eps, kd, kq);
+        }
+        const double kqn = __shfl_down_sync(0xffffffffu, kq, 1);
+        const bool mine = kq >= kqn;  // the nearer end of the lane's edge
+        r = area_sq(tx, ty, tz, mine ? dx : x - nx, mine ? dy : y - ny, mine ? dz : z - nz, eps) * (kq + kqn);
     };
-    if (tid < kLH) {
-        const int32_t I = edge_of(v0, tid);
-        load_edge(ea, eb, edges, V, I < 0 ? V : I, sI[tid]);  // I = V: an empty record
-    } else if (tid < 2 * kLH) {
-        const int32_t J = edge_of(u0, tid - kLH);
-        load_edge(ea, eb, edges, V, J < 0 ? V : J, sJ[tid - kLH]);
-    }
-    __syncthreads();
-    for (int e = tid; e < kLH * kLH; e += blockDim.x) {
-        const int k = e / kLH, l = e % kLH;
-        const EdgeRec& a = sI[k];
-        const EdgeRec& b = sJ[l];
-        const int32_t I = edge_of(v0, k), J = edge_of(u0, l);
-        double2 out = make_double2(0.0, 0.0), w = out;
-        const bool ok = I >= 0 && J >= 0 && I != J && a.ij.x != b.ij.x && a.ij.x != b.ij.y &&
-                        a.ij.y != b.ij.x && a.ij.y != b.ij.y;
-        if (ok) {
-            w = pair_weight<MODE>(a, b, distExp, eps);
-            const double dotT = a.T.x * b.T.x + a.T.y * b.T.y + a.T.z * b.T.z;
-            out = make_double2(-w.x * dotT / (a.p1.w * b.p1.w), -w.y);
+    // the row edge that ends at the vertex just taken: W of (k, lane), its stencil terms
+    auto edge = [&](int32_t I, bool kvalid, double Tx, double Ty, double Tz, double ell, double dx, double dy,
+                    double dz, double x2, double kd, double kq, double r, double& wx, double& wy, double& w) {
+        const double s = pkd + kd;
+        const double sumDist = s + __shfl_down_sync(0xffffffffu, s, 1);
+        const bool first = px2 <= x2;
+        const double p = area_sq(Tx, Ty, Tz, first ? pdx : dx, first ? pdy : dy, first ? pdz : dz, eps) * (pkq + kq);
+        const double low = (p + __shfl_down_sync(0xffffffffu, p, 1)) + (pr + r);
+        const double ll = ell * me.w;
+        const double dotT = Tx * tx + Ty * ty + Tz * tz;
+        const int32_t gap = I < Jw ? Jw - I : I - Jw;
+        const bool ok = kvalid && lvalid && gap > 1 && gap < V - 1;
+        wx = ok ? -0.5 * sumDist * dotT : 0.0;
+        wy = ok ? -0.0625 * ll * low : 0.0;
+        w = ok ? 0.5 * ll * sumDist : 0.0;
+    };
+    const int32_t rows = min(R, V - v0);
+    for (int32_t i0 = -1; i0 < rows; i0 += (i0 < 0 ? 1 : kBatch)) {
+        // (the first round takes vertices v0 - 1 and v0 and the edge between them)
+        const int32_t nb = i0 < 0 ? 1 : min(kBatch, rows - i0);
+        if (i0 < 0) {
+            const double4 q = ea[wrap(v0 - 1)];
+            vertex(q.x, q.y, q.z, pdx, pdy, pdz, px2, pkd, pkq, pr);
         }
-        W[k][l] = out;
-        Wr[k][l] = w;
-    }
-    __syncthreads();
-    // row sums of the tile's own edges (k, l >= 1): row I over tile tj's edges,
-    // and (off-diagonal tiles) row J over tile ti's edges
-    if (tid < kLT) {
-        const int32_t I = v0 + tid;
-        if (I < V) {
-            double2 rs = make_double2(0.0, 0.0);
-            for (int l = 1; l < kLH; l++) {
-                rs.x += Wr[tid + 1][l].x;
-                rs.y += Wr[tid + 1][l].y;
+        // the batch's rows: edge I = v0 + i and the vertex it ends at
+        __syncwarp();
+        if (lane < nb) {
+            const int32_t I = wrap(v0 + i0 + lane);
+            const double4 b = ea[I], q = ea[wrap(v0 + i0 + lane + 1)];
+            double ex = q.x - b.x, ey = q.y - b.y, ez = q.z - b.z;
+            const double len = sqrt(ex * ex + ey * ey + ez * ez);
+            const double inv = len < 1e-14 ? 0.0 : 1.0 / len;
+            double* o = sm.row[lane];
+            o[0] = q.x;
+            o[1] = q.y;
+            o[2] = q.z;
+            o[3] = b.w;
+            o[4] = ex * inv;
+            o[5] = ey * inv;
+            o[6] = ez * inv;
+        }
+        __syncwarp();
+        for (int i = 0; i < nb; i++) {
+            const double* o = sm.row[i];
+            const int32_t I = wrap(v0 + i0 + i);
+            double dx, dy, dz, x2, kd, kq, r, wx, wy, w;
+            vertex(o[0], o[1], o[2], dx, dy, dz, x2, kd, kq, r);
+            edge(I, true, o[4], o[5], o[6], o[3], dx, dy, dz, x2, kd, kq, r, wx, wy, w);
+            pdx = dx;
+            pdy = dy;
+            pdz = dz;
+            px2 = x2;
+            pkd = kd;
+            pkq = kq;
+            pr = r;
+            const double z = wx - __shfl_up_sync(0xffffffffu, wx, 1), y = wy + __shfl_up_sync(0xffffffffu, wy, 1);
+            if (i0 >= 0) {
+                const bool count = own && I > J;
+                sm.a[i][lane] = (y + z) + gprev;
+                sm.w[i][lane] = count ? w : 0.0;
+                sm.q[i][lane] = count ? -wy : 0.0;
+                csw += count ? w : 0.0;
+                csq += count ? -wy : 0.0;
             }
-            rowpart[(int64_t)tj * V + I] = rs;
+            gprev = y - z;
         }
-    } else if (tid < 2 * kLT && ti != tj) {
-        const int c = tid - kLT;
-        const int32_t J = u0 + c;
-        if (J < V) {
-            double2 cs = make_double2(0.0, 0.0);
-            for (int k = 1; k < kLH; k++) {
-                cs.x += Wr[k][c + 1].x;
-                cs.y += Wr[k][c + 1].y;
+        if (i0 < 0) continue;
+        __syncwarp();
+        // A[v][u], u <= v, along rows
+        for (int i = 0; i < nb; i++) {
+            const int32_t v = v0 + i0 + i;
+            if (own && J <= v) A[(int64_t)v * V + J] = sm.a[i][lane];
+        }
+        // the mirror A[u][v], u < v: 16 columns v of two rows u at a time
+        for (int c = lane >> 4; c < kStrip; c += 2) {
+            const int i = lane & 15;
+            const int32_t u = u0 + c, v = v0 + i0 + i;
+            if (i < nb && u < V && u < v) A[(int64_t)u * V + v] = sm.a[i][c + 1];
+        }
+        // row sums over the strip: two lanes per row
+        {
+            const int i = lane & 15, c0 = 1 + 15 * (lane >> 4);
+            double sw = 0.0, sq = 0.0;
+#pragma unroll
+            for (int c = 0; c < 15; c++) {
+                sw += sm.w[i][c0 + c];
+                sq += sm.q[i][c0 + c];
             }
-            rowpart[(int64_t)ti * V + J] = cs;
+            sw += __shfl_down_sync(0xffffffffu, sw, 16);
+            sq += __shfl_down_sync(0xffffffffu, sq, 16);
+            if (lane < nb) rowslot[(int64_t)cs * V + v0 + i0 + i] = make_double2(sw, sq);
         }
     }
-    __syncthreads();  // the row sums have read Wr; ta takes its place
-    // A[v][u] for the tile (rows v0 + r, columns u0 + c, u <= v), the incident
-    // edges of each vertex in ascending edge order
-    for (int e = tid; e < kLT * kLT; e += blockDim.x) {
-        const int r = e / kLT, c = e % kLT;
-        const int32_t v = v0 + r, u = u0 + c;
-        double sb = 0.0, s0 = 0.0;
-        if (v < V && u < V && u <= v) {
-            // (row index in W, sign): v's edges v-1 (second vertex, -1) and v (+1)
-            int kp[2], lq[2];
-            double sp[2], sq[2];
-            if (v == 0) { kp[0] = 1; sp[0] = 1.0; kp[1] = 0; sp[1] = -1.0; }
-            else { kp[0] = r; sp[0] = -1.0; kp[1] = r + 1; sp[1] = 1.0; }
-            if (u == 0) { lq[0] = 1; sq[0] = 1.0; lq[1] = 0; sq[1] = -1.0; }
-            else { lq[0] = c; sq[0] = -1.0; lq[1] = c + 1; sq[1] = 1.0; }
-#pragma unroll
-            for (int p = 0; p < 2; p++)
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const double2 m = W[kp[p]][lq[q]];
-                    sb += sp[p] * sq[q] * m.x;
-                    s0 += m.y;
-                }
-        }
-        ta[r][c] = sb + s0;
-    }
-    __syncthreads();
-    for (int e = tid; e < kLT * kLT; e += blockDim.x) {
-        const int r = e / kLT, c = e % kLT;
-        const int32_t v = v0 + r, u = u0 + c;
-        if (v < V && u < V && u <= v) A[(int64_t)v * V + u] = ta[r][c];
-        // mirror: entry (u0 + r, v0 + c) = value (v0 + c, u0 + r)
-        const int32_t mr = u0 + r, mc = v0 + c;
-        if (mc < V && mr < V && mr < mc) A[(int64_t)mr * V + mc] = ta[c][r];
-    }
+    if (own) colslot[(int64_t)rb * V + J] = make_double2(csw, csq);
 }
 
 // The pair matrix's diagonal on A's cyclic band: for each vertex v, the terms
 // with I = J of the stencil: A[v][v] += Mb'_{v-1} + Mb'_v + M0'_{v-1} + M0'_v,
 // A[v][v+1] = A[v+1][v] += -Mb'_v + M0'_v, with (Mb'_I, M0'_I) = (d_I / l_I^2, d0_I)
-// summed from the per-tile row sums in tile order. Each block forms the
-// diagonal entries of its 256 vertices and of the vertex before them once, in
-// shared memory.
-__global__ void __launch_bounds__(256) loop_band_kernel(const double4* __restrict__ ea, int32_t V,
-                                                        int32_t nt, const double2* __restrict__ rowpart,
+// summed from the row slots of the strips before I and the column slots of the row
+// blocks that reach past it, in order within each of eight groups. Each block forms
+// the diagonal entries of its 31 vertices and of the vertex before them once.
+__global__ void __launch_bounds__(256) loop_band_kernel(const double4* __restrict__ ea, int32_t V, int32_t R,
+                                                        const double2* __restrict__ rowslot,
+                                                        const double2* __restrict__ colslot,
                                                         double* __restrict__ A) {
-    __shared__ double2 dg[257];
-    const int32_t b0 = blockIdx.x * 256;
-    auto diag = [&](int32_t I) -> double2 {
-        double sx = 0.0, sy = 0.0;
-#pragma unroll 8
-        for (int32_t s = 0; s < nt; s++) {
-            const double2 p = rowpart[(int64_t)s * V + I];
+    __shared__ double2 part[8][32], dg[32];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int32_t b0 = blockIdx.x * 31, v = b0 - 1 + x;
+    const int32_t I = v < 0 ? V - 1 : v;
+    double sx = 0.0, sy = 0.0;
+    if (I < V) {
+        // strips whose tile (row block of I, strip) exists, and row blocks from that of I on
+        const int32_t nr = min((V + kStrip - 1) / kStrip, (I / R * R + R - 1) / kStrip + 1);
+        const int32_t nrb = (V + R - 1) / R, rb0 = (I / kStrip * kStrip) / R;
+        for (int32_t s = y; s < nr; s += 8) {
+            const double2 p = rowslot[(int64_t)s * V + I];
             sx += p.x;
             sy += p.y;
         }
-        const double ell = ea[I].w;
-        return make_double2(sx / (ell * ell), sy);
-    };
-    const int32_t v = b0 + threadIdx.x;
-    if (v < V) dg[threadIdx.x + 1] = diag(v);
-    if (threadIdx.x == 0) dg[0] = diag(b0 == 0 ? V - 1 : b0 - 1);
+        for (int32_t s = rb0 + y; s < nrb; s += 8) {
+            const double2 p = colslot[(int64_t)s * V + I];
+            sx += p.x;
+            sy += p.y;
+        }
+    }
+    part[y][x] = make_double2(sx, sy);
     __syncthreads();
-    if (v >= V) return;
-    const double2 dv = dg[threadIdx.x + 1], dp = dg[threadIdx.x];
+    if (y > 0) return;
+    if (I < V) {
+        for (int g = 1; g < 8; g++) {
+            sx += part[g][x].x;
+            sy += part[g][x].y;
+        }
+        const double ell = ea[I].w;
+        dg[x] = make_double2(sx / (ell * ell), sy);
+    }
+    __syncwarp();
+    if (x == 0 || v >= V) return;
+    const double2 dv = dg[x], dp = dg[x - 1];
     A[(int64_t)v * V + v] += (dp.x + dv.x) + (dp.y + dv.y);
     const int32_t u = v + 1 == V ? 0 : v + 1;
     const double off = -dv.x + dv.y;
@@ -486,24 +578,26 @@ int32_t assemble_fp64(tpe_ctx* ctx, double alpha, double beta, double eps, doubl
         const int32_t V = ctx->V;
         const double s = (beta - 1.0) / alpha;
         const double distExp = 2.0 * (s - 1.0) + 1.0;
-        const int32_t nt = (V + kLT - 1) / kLT;
-        const int64_t tiles = (int64_t)nt * (nt + 1) / 2;
-        TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double2) * (size_t)nt * V));
+        // rows per warp: short marches where there are few warps, few first rows on large
+        // curves (with the band, us: V = 128 24 / 28 / 35 at 4 / 8 / 16 rows, 777 37 / 31 / 39,
+        // 2048 75 / 70 / 67 / 97 at 8 / 16 / 32 / 64, 8192 599 / 559 / 545 at 16 / 32 / 64)
+        const int32_t R = V >= 3072 ? 64 : (V >= 1400 ? 32 : (V >= 400 ? 8 : 4));
+        const int32_t ncs = (V + kStrip - 1) / kStrip, nrb = (V + R - 1) / R;
+        TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double2) * (size_t)(ncs + nrb) * V));
+        double2* rowslot = ctx->tmp.as<double2>();
+        double2* colslot = rowslot + (size_t)ncs * V;
         {
             KernelScope ks(ctx, TPE_KGROUP_PAIR_WEIGHTS, 1);
-            if (alpha == 3.0 && beta == 6.0)
-                assemble_loop_kernel<1><<<(unsigned)tiles, 256, 0, ctx->stream>>>(
-                    ctx->edge_a.as<double4>(), ctx->edge_b.as<double4>(), ctx->d_edges.as<int2>(), V,
-                    distExp, eps, d_A, ctx->tmp.as<double2>());
-            else
-                assemble_loop_kernel<0><<<(unsigned)tiles, 256, 0, ctx->stream>>>(
-                    ctx->edge_a.as<double4>(), ctx->edge_b.as<double4>(), ctx->d_edges.as<int2>(), V,
-                    distExp, eps, d_A, ctx->tmp.as<double2>());
+            auto kern = alpha == 3.0 && beta == 6.0 ? assemble_loop_kernel<1> : assemble_loop_kernel<0>;
+            const size_t smem = sizeof(LoopSmem) * kLoopWarps;
+            TPE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            kern<<<dim3((unsigned)((ncs + kLoopWarps - 1) / kLoopWarps), (unsigned)nrb), 32 * kLoopWarps, smem,
+                   ctx->stream>>>(ctx->edge_a.as<double4>(), V, R, distExp, eps, d_A, rowslot, colslot);
             TPE_CUDA_TRY(cudaGetLastError());
         }
         KernelScope ks(ctx, TPE_KGROUP_GATHER_A, 1);
-        loop_band_kernel<<<(V + 255) / 256, 256, 0, ctx->stream>>>(ctx->edge_a.as<double4>(), V, nt,
-                                                                 ctx->tmp.as<double2>(), d_A);
+        loop_band_kernel<<<(V + 30) / 31, 256, 0, ctx->stream>>>(ctx->edge_a.as<double4>(), V, R, rowslot,
+                                                                 colslot, d_A);
         TPE_CUDA_TRY(cudaGetLastError());
         return TPE_OK;
     }

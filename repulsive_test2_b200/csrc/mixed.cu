@@ -103,226 +103,8 @@ __global__ void split_copy_kernel(const float* __restrict__ S, int32_t ld, int32
     lo[o] = l;
 }
 
-constexpr int kLd3 = 132;   // row stride of a and z (16-byte aligned rows)
-constexpr int kP3 = 100;    // row stride of plT (the panel, transposed)
-constexpr int kS3 = 36;     // row stride of the 32 x 32 scratch blocks
-constexpr int kTs3 = 36;    // row stride of the off-diagonal T scratch
-constexpr int kPw3 = 32;
-
-// shared-memory offsets (floats)
-constexpr int kOffA = 0;
-constexpr int kOffZ = kOffA + kT * kLd3;
-constexpr int kOffP = kOffZ + kT * kLd3;               // plT: 32 x kP3, also the final T scratch
-constexpr int kPSize = 3 * 32 * kTs3 > 32 * kP3 ? 3 * 32 * kTs3 : 32 * kP3;
-constexpr int kOffTsc = kOffP + kPSize;               // 2 x 32 x kTs3
-constexpr int kOffRd = kOffTsc + 2 * 32 * kTs3;       // 128
-constexpr int kOffZdT = kOffRd + kT;                  // 32 x kS3: Z_dd^T of the current panel
-constexpr int kOffLt = kOffZdT + 32 * kS3;            // 32 x kS3: L_dd^T (wf32 scratch)
-constexpr int kSmem3Floats = kOffLt + 32 * kS3;
-static_assert(kOffZ % 4 == 0 && kOffP % 4 == 0 && kOffTsc % 4 == 0 && kOffZdT % 4 == 0 &&
-              kOffLt % 4 == 0, "float4 alignment");
-
-__device__ __forceinline__ void tri_decode(int e, int& ti, int& tj) {
-    int t = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);
-    while ((t + 1) * (t + 2) / 2 <= e) t++;
-    while (t * (t + 1) / 2 > e) t--;
-    ti = t;
-    tj = e - t * (t + 1) / 2;
-}
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ float f4(const float4& v, int i) {
-    return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
-}
-
-// One warp factors the 32 x 32 diagonal part at (c0, c0) of a (lane = row) and
-// inverts it: one rank-1 update per column by shuffles, with each column's
-// pivot formed ahead on its own lane. The inverse (lane = column of Z) reads L
-// column-wise from a transposed copy. Writes L to a, Z (lower) to z, Z^T to zdt, 1/L_ii to rd.
-__device__ __noinline__ void warp_factor32(float* sm, int c0, int lane, int32_t* bad) {
-    float* a = sm + kOffA;
-    float* z = sm + kOffZ;
-    float* rd = sm + kOffRd;
-    float* zdt = sm + kOffZdT;
-    float* lt = sm + kOffLt;
-    float v[32];
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const float4 x = ld4(a + (c0 + lane) * kLd3 + c0 + 4 * q);
-        v[4 * q] = (4 * q <= lane) ? x.x : 0.0f;
-        v[4 * q + 1] = (4 * q + 1 <= lane) ? x.y : 0.0f;
-        v[4 * q + 2] = (4 * q + 2 <= lane) ? x.z : 0.0f;
-        v[4 * q + 3] = (4 * q + 3 <= lane) ? x.w : 0.0f;
-    }
-    bool brk = false;
-    float myrs = 1.0f;
-    // The pivot of column K + 1 is formed on its own lane right after column K
-    // (dn = v[K+1] - L[K+1][K]^2: the last update of that diagonal entry uses
-    // the lane's own value) and broadcast before column K's other updates, so
-    // the pivot chain holds one shuffle per column; the updates themselves run
-    // in the same order as one rank-1 update per column.
-    float piv = __shfl_sync(0xffffffffu, v[0], 0);
-#pragma unroll
-    for (int K = 0; K < 32; K++) {
-        if (!(piv > 0.0f) || !isfinite(piv)) {
-            brk = true;
-            piv = 1.0f;
-        }
-        const float rs = rsqrtf(piv);
-        const float lk = (lane == K) ? piv * rs : v[K] * rs;  // L[lane][K] (lanes >= K)
-        if (lane >= K) v[K] = lk;
-        if (lane == K) myrs = rs;
-        float pnext = 0.0f;
-        if (K + 1 < 32) pnext = __shfl_sync(0xffffffffu, fmaf(-lk, lk, v[K + 1]), K + 1);
-#pragma unroll
-        for (int m = K + 1; m < 32; m++) {
-            const float lmk = __shfl_sync(0xffffffffu, lk, m);
-            if (lane >= m) v[m] = fmaf(-lk, lmk, v[m]);
-        }
-        piv = pnext;
-    }
-    if (brk && lane == 0) atomicExch(bad, 1);
-    // L back to a (rows, 16-byte stores), L^T to lt (lt[k][lane] = L[lane][k]), 1/L_ii
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-        st4(a + (c0 + lane) * kLd3 + c0 + 4 * q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
-#pragma unroll
-    for (int k = 0; k < 32; k++) lt[k * kS3 + lane] = v[k];
-    rd[c0 + lane] = myrs;
-    __syncwarp();
-    // inverse, lane = column j: x[i] = Z[i][j]
-    float x[32];
-#pragma unroll
-    for (int i = 0; i < 32; i++) x[i] = (i == lane) ? 1.0f : 0.0f;
-    float rdv[32];
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        const float4 r4 = ld4(rd + c0 + 4 * q);
-        rdv[4 * q] = r4.x;
-        rdv[4 * q + 1] = r4.y;
-        rdv[4 * q + 2] = r4.z;
-        rdv[4 * q + 3] = r4.w;
-    }
-#pragma unroll
-    for (int k = 0; k < 32; k++) {
-        x[k] *= rdv[k];
-#pragma unroll
-        for (int q = (k + 1) / 4; q < 8; q++) {
-            const float4 l4 = ld4(lt + k * kS3 + 4 * q);
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int i = 4 * q + u;
-                if (i > k) x[i] = fmaf(-f4(l4, u), x[k], x[i]);
-            }
-        }
-    }
-    // Z rows to z (column lane), Z^T rows to zdt (row lane)
-#pragma unroll
-    for (int i = 0; i < 32; i++) z[(c0 + i) * kLd3 + c0 + lane] = (i >= lane) ? x[i] : 0.0f;
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-        st4(zdt + lane * kS3 + 4 * q,
-            make_float4(4 * q >= lane ? x[4 * q] : 0.0f, 4 * q + 1 >= lane ? x[4 * q + 1] : 0.0f,
-                        4 * q + 2 >= lane ? x[4 * q + 2] : 0.0f, 4 * q + 3 >= lane ? x[4 * q + 3] : 0.0f));
-    __syncwarp();
-}
-
-// a[R..R+3][C..C+3] -= P rows (4ti..) P rows (4tj..)^T over the 32 panel columns
-// (P transposed in plT).
-__device__ __forceinline__ void update_tile(float* a, const float* plt, int ti, int tj, int base) {
-    float acc[4][4];
-#pragma unroll
-    for (int x = 0; x < 4; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) acc[x][y] = 0.0f;
-#pragma unroll 8
-    for (int k = 0; k < kPw3; k++) {
-        const float4 pr = ld4(plt + k * kP3 + 4 * ti);
-        const float4 pc = ld4(plt + k * kP3 + 4 * tj);
-#pragma unroll
-        for (int x = 0; x < 4; x++)
-#pragma unroll
-            for (int y = 0; y < 4; y++) acc[x][y] += f4(pr, x) * f4(pc, y);
-    }
-    const int R = base + 4 * ti, Cc = base + 4 * tj;
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-        float* p = a + (R + x) * kLd3 + Cc;
-        float4 o = ld4(p);
-        o.x -= acc[x][0];
-        o.y -= acc[x][1];
-        o.z -= acc[x][2];
-        o.w -= acc[x][3];
-        st4(p, o);
-    }
-}
-
-__device__ __forceinline__ void group_sync(int bar, int nthr) {
-    asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nthr) : "memory");
-}
-
-// Off-diagonal 32 x 32 blocks of Z inside the block: for each listed pair
-// (bi, bj), bj < bi, T = sum_{c=bj}^{bi-1} L_{bi,c} Z_{c,bj}, then
-// Z_{bi,bj} = -Z_{bi,bi} T. 64 threads per pair (8 x 8 threads of 4 x 4 outputs).
-__device__ void offdiag_blocks(const float* __restrict__ a, float* __restrict__ z,
-                                float* __restrict__ tsc, const int* pa, const int* pb, int npairs,
-                                int t, int nthr, int bar) {
-    const int slot = t >> 6;
-    const bool act = slot < npairs;
-    const int tr = (t >> 3) & 7, tc = t & 7;
-    const int bi = act ? pa[slot] : 0, bj = act ? pb[slot] : 0;
-    float acc[4][4];
-#pragma unroll
-    for (int x = 0; x < 4; x++)
-#pragma unroll
-        for (int y = 0; y < 4; y++) acc[x][y] = 0.0f;
-    if (act) {
-        for (int k4 = bj * kPw3; k4 < bi * kPw3; k4 += 4) {
-            float4 lr[4], zc[4];
-#pragma unroll
-            for (int x = 0; x < 4; x++) lr[x] = ld4(a + (bi * kPw3 + 4 * tr + x) * kLd3 + k4);
-#pragma unroll
-            for (int u = 0; u < 4; u++) zc[u] = ld4(z + (k4 + u) * kLd3 + bj * kPw3 + 4 * tc);
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int x = 0; x < 4; x++)
-#pragma unroll
-                    for (int y = 0; y < 4; y++) acc[x][y] += f4(lr[x], u) * f4(zc[u], y);
-        }
-#pragma unroll
-        for (int x = 0; x < 4; x++)
-            st4(tsc + (slot * kPw3 + 4 * tr + x) * kTs3 + 4 * tc,
-                make_float4(acc[x][0], acc[x][1], acc[x][2], acc[x][3]));
-    }
-    group_sync(bar, nthr);
-    if (act) {
-#pragma unroll
-        for (int x = 0; x < 4; x++)
-#pragma unroll
-            for (int y = 0; y < 4; y++) acc[x][y] = 0.0f;
-        const int qmax = 4 * tr + 4;  // Z_aa is lower: columns q <= row
-        for (int q4 = 0; q4 < qmax; q4 += 4) {
-            float4 zr[4], tq[4];
-#pragma unroll
-            for (int x = 0; x < 4; x++) zr[x] = ld4(z + (bi * kPw3 + 4 * tr + x) * kLd3 + bi * kPw3 + q4);
-#pragma unroll
-            for (int u = 0; u < 4; u++) tq[u] = ld4(tsc + (slot * kPw3 + q4 + u) * kTs3 + 4 * tc);
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-#pragma unroll
-                for (int x = 0; x < 4; x++)
-#pragma unroll
-                    for (int y = 0; y < 4; y++) acc[x][y] += f4(zr[x], u) * f4(tq[u], y);
-        }
-#pragma unroll
-        for (int x = 0; x < 4; x++)
-            st4(z + (bi * kPw3 + 4 * tr + x) * kLd3 + bj * kPw3 + 4 * tc,
-                make_float4(-acc[x][0], -acc[x][1], -acc[x][2], -acc[x][3]));
-    }
-    group_sync(bar, nthr);
-}
+constexpr int kLdZ = 132;       // row stride of the shared vectors (16-byte aligned rows)
+constexpr int kPotrfThr = 512;  // 16 warps of eight columns
 
 // One CTA factors the 128 x 128 diagonal block at (j0, j0) of S (its lower
 // triangle) and writes Z_jj = L_jj^{-1} (split, zero above the diagonal) to Z.
@@ -330,133 +112,129 @@ __device__ void offdiag_blocks(const float* __restrict__ a, float* __restrict__ 
 // uses only the blocks below the diagonal), and W_jj = Z_jj^T is written by
 // diag_transpose_kernel once the whole factorization is done.
 //
-// Blocked right-looking over four 32-column panels with an in-CTA look-ahead:
-// warp 0 factors a panel's 32 x 32 diagonal part in registers and inverts it
-// (warp_factor32); all eight warps solve the rows below against that inverse
-// (warp = 4 columns, lane = row, the panel stored transposed); then warps 0
-// and 1 apply the rank-32 update to the next panel's diagonal part and warp 0
-// factors it, while warps 1-7 update the rest of the trailing triangle (4 x 4
-// register tiles from 16-byte loads) and form the off-diagonal 32 x 32 blocks
-// of the inverse, Z_ab = -Z_aa sum_{b<=c<a} L_ac Z_cb, one block distance at a
-// time. Reciprocal square roots are the fast approximate ones: the factor is a
-// preconditioner, CG restores FP64 accuracy. *bad = 1 when a pivot is not
-// positive and finite. Rows of a and z are 132 floats apart (16-byte aligned),
-// so every shared-memory access of the inner loops is a 16-byte one.
-__global__ void __launch_bounds__(256, 1)
+// Factor and inverse in one sweep over the columns, right-looking on the rows of S
+// and, below them, the rows of the identity, which become L^-T. At column k only
+// the rows of S below k and the identity's rows up to k are alive, 128 in all, so slot
+// r holds S's row r until column r is done and the identity's row r from then on: 32
+// registers a thread (warp w: columns 8w .. 8w + 7; lane: rows lane + 32h). Warp p
+// factors its eight columns (the 8 x 8 block that the pivots come from in every lane)
+// and leaves them unscaled in rows 8p .. of z; each warp after it applies all eight as
+// soon as they are there, and goes on to its own when it has applied the one before: a
+// barrier per panel, which only the warps from p on take part in. The scaling by 1/L_kk
+// happens on the way out. The approximate reciprocals are good enough: the factor is a
+// preconditioner, CG restores FP64 accuracy. *bad = 1 when a pivot is not positive and
+// finite. Bound: the latency of 16 panels on one SM. @@
+__global__ void __launch_bounds__(kPotrfThr, 1)
 potrf128_kernel(const float* __restrict__ S, int32_t ld, int32_t j0, float* __restrict__ Zhi,
-            float* __restrict__ Zlo, int32_t* __restrict__ bad) {
-    extern __shared__ __align__(16) float sm[];
-    float* a = sm + kOffA;
-    float* z = sm + kOffZ;
-    float* plt = sm + kOffP;
-    float* zdt = sm + kOffZdT;
-    float* tsc = sm + kOffTsc;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+                float* __restrict__ Zlo, int32_t* __restrict__ bad) {
+    extern __shared__ __align__(16) float z[];  // kT x kLdZ, then the reciprocal pivots
+    float* inv = z + kT * kLdZ;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int e = 0; e < kT / 16; e++)
+        *reinterpret_cast<float4*>(z + (w + 16 * e) * kLdZ + 4 * lane) =
+            *reinterpret_cast<const float4*>(S + (size_t)(j0 + w + 16 * e) * ld + j0 + 4 * lane);
+    __syncthreads();
+    float v[4][8];
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+        const int r = lane + 32 * h;
+        const float4 x = *reinterpret_cast<const float4*>(z + r * kLdZ + 8 * w);
+        const float4 y = *reinterpret_cast<const float4*>(z + r * kLdZ + 8 * w + 4);
+        const float t[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[h][q] = r >= 8 * w + q ? t[q] : 0.0f;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p < w; p++) {
+        asm volatile("bar.sync %0, %1;" ::"r"(p + 1), "r"(32 * (16 - p)) : "memory");
+        const int i = lane - ((8 * p) & 31), hp = p >> 2;
+        const float* zp = z + 8 * p * kLdZ;
+        float l[8][8];
+        float iv[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            const float4 x = *reinterpret_cast<const float4*>(zp + c * kLdZ + 8 * w);
+            const float4 y = *reinterpret_cast<const float4*>(zp + c * kLdZ + 8 * w + 4);
+            l[c][0] = x.x, l[c][1] = x.y, l[c][2] = x.z, l[c][3] = x.w;
+            l[c][4] = y.x, l[c][5] = y.y, l[c][6] = y.z, l[c][7] = y.w;
+            iv[c] = -inv[8 * p + c];
+        }
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            if (h > hp && 4 * h + 4 <= w) continue;  // rows above these columns that have not turned
+            if (h == hp && i >= 0 && i < 8) {        // the panel's slots turn
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[h][q] = 0.0f;
+            }
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                const float t = zp[c * kLdZ + lane + 32 * h] * iv[c];
+#pragma unroll
+                for (int q = 0; q < 8; q++) v[h][q] = fmaf(t, l[c][q], v[h][q]);
+            }
+        }
+    }
+    // the panel's own 8 x 8 block in every lane, so that its pivots need no shuffle, and
+    // the identity's eight rows that its slots turn into
+    float d[8][8], u[8];
     {
-        float4 buf[16];
+        const int hp = w >> 2, i = lane - ((8 * w) & 31);
+        const bool mine = i >= 0 && i < 8;
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int e = tid + 256 * q;  // float4 index
-            const int r = e >> 5, c = (e & 31) * 4;
-            buf[q] = *reinterpret_cast<const float4*>(S + (size_t)(j0 + r) * ld + j0 + c);
+        for (int c = 0; c < 8; c++) {
+            const float x = hp < 2 ? (hp == 0 ? v[0][c] : v[1][c]) : (hp == 2 ? v[2][c] : v[3][c]);
+            u[c] = i == c ? 1.0f : 0.0f;
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (q >= c) d[q][c] = __shfl_sync(0xffffffffu, x, ((8 * w) & 31) + q);
         }
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
-            const int e = tid + 256 * q;
-            const int r = e >> 5, c = (e & 31) * 4;
-            st4(a + r * kLd3 + c, buf[q]);
-        }
-    }
-    __syncthreads();
-    if (warp == 0) warp_factor32(sm, 0, lane, bad);
-    __syncthreads();
-    for (int p = 0; p < kT / kPw3 - 1; p++) {
-        const int c0 = p * kPw3;
-        const int nr = kT - c0 - kPw3;
-        // panel rows below: plT[m][r] = sum_k A[c0+32+r][c0+k] * Zd[m][k]
-        {
-            const int m0 = 4 * warp;
-            for (int r0 = 0; r0 < nr; r0 += 32) {
-                const int r = r0 + lane;
-                const float* arow = a + (c0 + kPw3 + r) * kLd3 + c0;
-                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int c = 0; c < 8; c++) {
+            const float piv = d[c][c];
+            const float iv = __fdividef(1.0f, piv > 0.0f && isfinite(piv) ? piv : 1.0f);
+            if (lane == 0) inv[8 * w + c] = iv;
+            float* zc = z + (8 * w + c) * kLdZ;
+            if (mine) zc[8 * w + i] = u[c];
 #pragma unroll
-                for (int k4 = 0; k4 < kPw3; k4 += 4) {
-                    const float4 ak = ld4(arow + k4);
+            for (int h = 0; h < 4; h++)
+                if (!(mine && h == hp)) zc[lane + 32 * h] = v[h][c];
 #pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const float4 zk = ld4(zdt + (k4 + u) * kS3 + m0);
-                        const float av = f4(ak, u);
-                        acc[0] += av * zk.x;
-                        acc[1] += av * zk.y;
-                        acc[2] += av * zk.z;
-                        acc[3] += av * zk.w;
-                    }
+            for (int q = 0; q < 8; q++)
+                if (q > c) {
+                    const float m = -d[q][c] * iv;
+#pragma unroll
+                    for (int r = 0; r < 8; r++)
+                        if (r >= q) d[r][q] = fmaf(m, d[r][c], d[r][q]);
+                    u[q] = fmaf(m, u[c], u[q]);
+#pragma unroll
+                    for (int h = 0; h < 4; h++) v[h][q] = fmaf(m, v[h][c], v[h][q]);
                 }
+        }
+        if (w < 15) asm volatile("bar.arrive %0, %1;" ::"r"(w + 1), "r"(32 * (16 - w)) : "memory");
+    }
+    // these rows of z stay as they are: out with them while the warps after this one go on
+    __syncwarp();
+    bool brk = false;
 #pragma unroll
-                for (int t = 0; t < 4; t++) plt[(m0 + t) * kP3 + r] = acc[t];
-            }
+    for (int c = 0; c < 8; c++) {
+        const int k = 8 * w + c;
+        float piv = d[c][c];
+        if (!(piv > 0.0f) || !isfinite(piv)) {
+            brk = true;
+            piv = 1.0f;
         }
-        __syncthreads();
-            const int base = c0 + kPw3;
-        const int nt = nr / 4;
-        const int ntiles = nt * (nt + 1) / 2;
-        constexpr int kNext = 36;  // 4 x 4 tiles of the next 32 x 32 diagonal part (packed first)
-        if (warp < 2) {
-            // warps 0 and 1: the next diagonal part, then warp 0 factors it
-            const int e = warp * 18 + lane;
-            if (lane < 18) {
-                int ti, tj;
-                tri_decode(e, ti, tj);
-                update_tile(a, plt, ti, tj, base);
-            }
-            group_sync(3, 64);
-        }
-        if (warp == 0) {
-            warp_factor32(sm, base, lane, bad);
-        } else {
-            for (int e = kNext + tid - 32; e < ntiles; e += 224) {
-                int ti, tj;
-                tri_decode(e, ti, tj);
-                update_tile(a, plt, ti, tj, base);
-            }
-            // the panel rows become final L
-            for (int e = tid - 32; e < nr * kPw3; e += 224) {
-                const int r = e >> 5, m = e & 31;
-                a[(base + r) * kLd3 + c0 + m] = plt[m * kP3 + r];
-            }
-            // while warp 0 factors the next panel: the off-diagonal Z blocks of
-            // block row p (inputs final: L columns < 32 p, Z blocks of rows <= p)
-            if (p > 0) {
-                int pa[2], pb[2];
-                for (int q = 0; q < p; q++) {
-                    pa[q] = p;
-                    pb[q] = p - 1 - q;
-                }
-                offdiag_blocks(a, z, tsc, pa, pb, p, tid - 32, 224, 1);
-            }
-        }
-        __syncthreads();
-        }
-    // the last block row of Z: its three off-diagonal blocks at once
-    {
-        const int pa[3] = {3, 3, 3}, pb[3] = {2, 1, 0};
-        offdiag_blocks(a, z, plt, pa, pb, 3, tid, 256, 2);
+        const float rs = rsqrtf(piv);
+        const float4 x = *reinterpret_cast<const float4*>(z + k * kLdZ + 4 * lane);
+        float y[4] = {x.x, x.y, x.z, x.w}, hi[4], lo[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) split32(4 * lane + q <= k ? y[q] * rs : 0.0f, hi[q], lo[q]);
+        const size_t o = (size_t)(j0 + k) * ld + j0 + 4 * lane;
+        *reinterpret_cast<float4*>(Zhi + o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<float4*>(Zlo + o) = make_float4(lo[0], lo[1], lo[2], lo[3]);
     }
-    // Z_jj (split), four columns per thread step, zero above the diagonal
-    for (int e = tid; e < kT * kT / 4; e += 256) {
-        const int r = e >> 5, c = (e & 31) * 4;
-        const float4 zz = ld4(z + r * kLd3 + c);
-        float4 h, l;
-        split32(c <= r ? zz.x : 0.0f, h.x, l.x);
-        split32(c + 1 <= r ? zz.y : 0.0f, h.y, l.y);
-        split32(c + 2 <= r ? zz.z : 0.0f, h.z, l.z);
-        split32(c + 3 <= r ? zz.w : 0.0f, h.w, l.w);
-        const size_t o = (size_t)(j0 + r) * ld + j0 + c;
-        *reinterpret_cast<float4*>(Zhi + o) = h;
-        *reinterpret_cast<float4*>(Zlo + o) = l;
-    }
-    __syncthreads();
+    if (brk && lane == 0) atomicExch(bad, 1);
 }
 
 // W_jj = Z_jj^T for the diagonal blocks b0 + blockIdx.z, split.
@@ -1042,7 +820,7 @@ int32_t mixed_factor(tpe_ctx* ctx, const double* d_A, int32_t V, double rho, boo
         }
     }
     const int nb = Vp / kT;
-    const size_t potrf_smem = sizeof(float) * kSmem3Floats;
+    const size_t potrf_smem = sizeof(float) * (kT * kLdZ + kT);
     TPE_CUDA_TRY(cudaFuncSetAttribute(potrf128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)potrf_smem));
     // Critical path on the main stream, per block j: potrf, then one CTA that
@@ -1082,7 +860,7 @@ int32_t mixed_factor(tpe_ctx* ctx, const double* d_A, int32_t V, double rho, boo
         TPE_CUDA_TRY(cudaGetLastError());
         for (int j = 0; j < nb; j++) {
             const int32_t j0 = j * kT;
-            potrf128_kernel<<<1, 256, potrf_smem, st>>>(S, Vp, j0, mf.Z.hi, mf.Z.lo, d_bad);
+            potrf128_kernel<<<1, kPotrfThr, potrf_smem, st>>>(S, Vp, j0, mf.Z.hi, mf.Z.lo, d_bad);
             TPE_CUDA_TRY(cudaGetLastError());
             if (j + 1 == nb) break;
             const int32_t rows = Vp - j0 - kT;

@@ -123,7 +123,9 @@ constexpr int kPotrfThr = 512;  // 16 warps of eight columns
 // barrier per panel, which only the warps from p on take part in. The scaling by 1/L_kk
 // happens on the way out. The approximate reciprocals are good enough: the factor is a
 // preconditioner, CG restores FP64 accuracy. *bad = 1 when a pivot is not positive and
-// finite. Bound: the latency of 16 panels on one SM. @@
+// finite. Bound: the latency of 16 panels on one SM, 1040 clocks for the eight columns
+// and 1000 to 2000 for their way into the next panel: 25 us (40 us as blocks of 32
+// columns with the inverse formed after them).
 __global__ void __launch_bounds__(kPotrfThr, 1)
 potrf128_kernel(const float* __restrict__ S, int32_t ld, int32_t j0, float* __restrict__ Zhi,
                 float* __restrict__ Zlo, int32_t* __restrict__ bad) {

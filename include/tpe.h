@@ -105,14 +105,15 @@ typedef struct {
     double proj_tol_abs, proj_tol_rel;         /* 1e-4, 1e-4 */
     int32_t proj_max_iter;                     /* 8 */
     int32_t precision;             /* TPE_PRECISION_* (extension): MIXED factors in 3xTF32 on the
-                                      tensor cores with an FP64 CG, or, for more than 64
-                                      constraint rows with frozen projection, forms the
-                                      explicit inverses from int8 digit products */
+                                      tensor cores with an FP64 CG (up to 2800 vertices, where
+                                      that is slower, in FP64, held to the same residual), or,
+                                      for more than 64 constraint rows with frozen projection,
+                                      forms the explicit inverses from int8 digit products */
     int32_t trials;                /* frozen projection: step sizes projected together per batch
                                       (extension; default 8, 1 = one at a time; the accepted tau
                                       and vertices do not depend on it) */
     int32_t collect_field;         /* write g~ into descent_field when non-null */
-    int32_t refine_max_iter;       /* mixed path: CG iteration cap, default 60 (extension) */
+    int32_t refine_max_iter;       /* mixed path: cap on its iterations, default 60 (extension) */
     int32_t reserved;
     double refine_tol;             /* mixed path: relative residual target (extension) */
 } tpe_step_opts;
@@ -130,11 +131,12 @@ typedef struct {
     int32_t converged;
     int32_t projection_iterations; /* -1 = null */
     int32_t reason;                /* TPE_REASON_* */
-    int32_t refine_iterations;     /* mixed path: CG iterations of the gradient solve;
-                                      0 = FP64 factorization, or (large constraint sets)
-                                      the int8-tensor-core inverses; -1 = mixed requested but
-                                      the FP32 factor broke down, CG missed refine_tol, or the
-                                      int8 inverses missed the residual gate (FP64 used) */
+    int32_t refine_iterations;     /* mixed path: CG iterations of the gradient solve (with the
+                                      FP64 factor: 1 + its corrections); 0 = FP64 factorization,
+                                      or (large constraint sets) the int8-tensor-core inverses;
+                                      -1 = mixed requested but the FP32 factor broke down,
+                                      refine_tol was missed, or the int8 inverses missed the
+                                      residual gate (FP64 used) */
     int32_t trials_evaluated;      /* tau trials whose energy was evaluated */
 } tpe_step_stats;
 

@@ -189,6 +189,44 @@ struct RowStats {
     double Cabs = 0.0;
 };
 
+// Block c, column c of the right-hand sides (the rows of C, then those of b): the residual
+// b - y - shift (1^T x) 1 to R (which may be Y or the right-hand sides), its squared norm to
+// out[2c] and ||b||^2 to out[2c + 1].
+__global__ void solve_residual_kernel(const double* C, int32_t nc, const double* b,
+                                      const double* __restrict__ X, const double* Y, int32_t V,
+                                      double shift, double* R, double* __restrict__ out) {
+    __shared__ double red[3][8];
+    const int32_t c = blockIdx.x;
+    const double* rhs = c < nc ? C + (int64_t)c * V : b + (int64_t)(c - nc) * V;
+    const double* x = X + (int64_t)c * V;
+    const double* y = Y + (int64_t)c * V;
+    double* res = R + (int64_t)c * V;
+    auto total = [&](int32_t slot, double s) {
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if ((threadIdx.x & 31) == 0) red[slot][threadIdx.x >> 5] = s;
+        __syncthreads();
+        s = 0.0;
+        for (int w = 0; w < 8; w++) s += red[slot][w];
+        return s;
+    };
+    double s = 0.0;
+    for (int32_t i = threadIdx.x; i < V; i += blockDim.x) s += x[i];
+    const double u = shift * total(0, s);
+    double r2 = 0.0, b2 = 0.0;
+    for (int32_t i = threadIdx.x; i < V; i += blockDim.x) {
+        const double bi = rhs[i], r = bi - y[i] - u;
+        res[i] = r;
+        r2 += r * r;
+        b2 += bi * bi;
+    }
+    r2 = total(1, r2);
+    b2 = total(2, b2);
+    if (threadIdx.x == 0) {
+        out[2 * c] = r2;
+        out[2 * c + 1] = b2;
+    }
+}
+
 __global__ void row_stats_kernel(const double* __restrict__ C, int32_t V,
                                  double* __restrict__ out) {
     __shared__ double red[4][8];
@@ -381,8 +419,10 @@ namespace {
 
 // Factor A_rho and the Schur complement from ctx->mat_A (V x V) and ctx->con_C (k x 3V).
 // *singular set when the reference would report a singular system.
+// may_direct: the mixed mode may take the FP64 factor (kMixedDirect).
 int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
-                    const double* b_flat = nullptr, const tpe_step_opts* o = nullptr) {
+                    const double* b_flat = nullptr, const tpe_step_opts* o = nullptr,
+                    bool may_direct = true) {
     SaddleOp& op = ctx->op;
     op.valid = false;
     op.mixed = false;
@@ -461,7 +501,46 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
     };
     const int32_t nrhs = 3 * rows;
     bool flags_unread = false;  // the FP64 factorization's {singular, timed out}
-    if (o && o->precision == TPE_PRECISION_MIXED && nrhs <= kMixedMaxRhs) {
+    const double tol = 32.0 * 2.220446049250313e-16 * (tm[1] + rho / V);
+    auto factor_fp64 = [&]() -> int32_t {
+        TPE_TRY(shift_copy(ctx, op.A, op.L, V, rho / V));
+        // the right-hand sides' forward solves ride along with the factorization
+        TPE_TRY(load_rhs());
+        CholDag f;
+        f.L = op.L;
+        f.Linv = op.Linv;
+        f.n = V;
+        f.tol = tol;
+        f.B = op.Y;
+        f.nr = nrhs;
+        TPE_TRY(chol_dag(ctx, f, nullptr));
+        return chol_solve(ctx, op.L, op.Linv, V, op.Y, nrhs, false);
+    };
+    const bool mixed = o && o->precision == TPE_PRECISION_MIXED && nrhs <= kMixedMaxRhs;
+    // at smaller sizes the FP64 factor is the faster one: its solves, held to the same residual
+    const bool direct = mixed && may_direct && V <= kMixedDirect;
+    const size_t nv = (size_t)nrhs * V;
+    double *R = nullptr, *D = nullptr, *AX = nullptr;  // residuals, corrections, A X
+    // AX = A X, then residuals and norms against the nc rows at C and those at b
+    auto residuals = [&](const double* C, int32_t nc, const double* b, const double* X) -> int32_t {
+        for (int32_t c = 0; c < nrhs; c += 16)
+            TPE_TRY(mrhs_fp64(ctx, op.A, V, X + (size_t)c * V, V, std::min(nrhs - c, 16),
+                              AX + (size_t)c * V));
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+        solve_residual_kernel<<<nrhs, 256, 0, ctx->stream>>>(C, nc, b, X, AX, V, rho / V, R, AX + nv);
+        TPE_CUDA_TRY(cudaGetLastError());
+        return TPE_OK;
+    };
+    if (direct) {
+        TPE_TRY(factor_fp64());
+        flags_unread = true;
+        TPE_TRY(ensure(ctx, ctx->mx_vec, sizeof(double) * (3 * nv + 2 * (size_t)nrhs)));
+        R = ctx->mx_vec.as<double>();
+        D = R + nv;
+        AX = D + nv;
+        if (nrhs > 0) TPE_TRY(residuals(op.C, 3 * k, b_flat, op.Y));
+    }
+    if (mixed && !direct) {
         // FP32 tensor-core factor as the preconditioner of an FP64 CG; the FP64
         // factorization below is the fallback (breakdown or no convergence).
         bool ok = false;
@@ -475,24 +554,19 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
             op.refine_iters = it;
             ok = conv;
         }
-        if (ok) {
-            op.mixed = true;
-        } else {
-            op.mixed_fallback = true;
-        }
+        op.mixed = ok;
+        op.mixed_fallback = !ok;
     }
-    if (!op.mixed) {
-        TPE_TRY(shift_copy(ctx, op.A, op.L, V, rho / V));
-        const double tol = 32.0 * 2.220446049250313e-16 * (tm[1] + rho / V);
-        // mixed precision with a large set: the explicit inverses with their
-        // products on the integer tensor cores (schur.cu), no FP64 factor here
-        op.int8 = o && o->precision == TPE_PRECISION_MIXED && k > kLargeSchur &&
-                  o->projection_mode == TPE_PROJECTION_FROZEN;
+    if (!op.mixed && !direct) {
         op.chol_tol = tol;
         if (k > kLargeSchur) {
-            // explicit inverses, Y by gathers, the Schur complement on the device
+            // explicit inverses, Y by gathers, the Schur complement on the device; in
+            // mixed precision their products on the integer tensor cores (schur.cu)
+            op.int8 = o && o->precision == TPE_PRECISION_MIXED &&
+                      o->projection_mode == TPE_PROJECTION_FROZEN;
             op.large = true;
             op.Scc.clear();
+            TPE_TRY(shift_copy(ctx, op.A, op.L, V, rho / V));
             bool sing = false;
             TPE_TRY(large_schur_build(ctx, op, b_flat, &sing));
             if (sing) {
@@ -500,46 +574,69 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
                 return TPE_OK;
             }
         } else {
-            // the right-hand sides' forward solves ride along with the factorization
-            TPE_TRY(load_rhs());
-            CholDag f;
-            f.L = op.L;
-            f.Linv = op.Linv;
-            f.n = V;
-            f.tol = tol;
-            f.B = op.Y;
-            f.nr = nrhs;
-            TPE_TRY(chol_dag(ctx, f, nullptr));
-            TPE_TRY(chol_solve(ctx, op.L, op.Linv, V, op.Y, nrhs, false));
+            TPE_TRY(factor_fp64());
             flags_unread = true;
         }
     }
-    if (k > 0) {
-        TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double) * ((op.large ? 0 : (size_t)k * k) +
-                                                         4 * (size_t)k + 16)));
-        double* dS = ctx->tmp.as<double>();
-        if (!op.large) TPE_TRY(gram_dots(ctx, op.C, k, op.Y, k, 3 * (int64_t)V, dS));
-        double* dR = op.large ? op.sp.stats : dS + (size_t)k * k;
-        if (!op.large) {
+    TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double) * ((op.large ? 0 : (size_t)k * k) + 4 * (size_t)k + 16)));
+    double* dS = ctx->tmp.as<double>();
+    double* dR = op.large ? op.sp.stats : dS + (size_t)k * k;
+    std::vector<double> rs((size_t)4 * k), rn((size_t)2 * nrhs), bn;
+    double worst = 0.0;  // largest ||r|| / ||b||, squared, of the correction before
+    for (int32_t it = 1;; it++) {
+        if (k > 0 && !op.large) {
+            TPE_TRY(gram_dots(ctx, op.C, k, op.Y, k, 3 * (int64_t)V, dS));
             KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
             row_stats_kernel<<<k, 256, 0, ctx->stream>>>(op.C, V, dR);
             TPE_CUDA_TRY(cudaGetLastError());
         }
-        std::vector<double> rs((size_t)4 * k);
+        if (k == 0 && !flags_unread) break;
         int32_t late = 0;  // a triangular solve's wait ran out
         int32_t ff[2] = {0, 0};
-        const HostCopy cp[4] = {
+        const HostCopy cp[5] = {
             {op.Scc.data(), dS, op.large ? 0 : sizeof(double) * (size_t)k * k},
             {rs.data(), dR, sizeof(double) * 4 * (size_t)k},
             {&late, ctx->dag_err.ptr, ctx->dag_err.ptr ? sizeof(int32_t) : 0},
-            {ff, ctx->dag_flags.ptr, flags_unread ? sizeof(ff) : 0}};
-        TPE_TRY(download_many(ctx, ctx->stream, cp, 4));
+            {ff, ctx->dag_flags.ptr, flags_unread ? sizeof(ff) : 0},
+            {rn.data(), direct ? AX + nv : nullptr, direct ? sizeof(double) * rn.size() : 0}};
+        TPE_TRY(download_many(ctx, ctx->stream, cp, 5));
         TPE_TRY(chol_dag_status(ctx, ff));
         if (late) return chol_timeout(ctx);
         if (ff[0]) {
+            // (the FP32 factor may still manage)
+            if (direct) return op_finalize(ctx, V, k, singular, b_flat, o, false);
             *singular = true;
             return TPE_OK;
         }
+        if (!direct || nrhs == 0) break;
+        if (it == 1) bn = rn;
+        double w = 0.0;
+        bool small = true;
+        for (int32_t c = 0; c < nrhs; c++) {
+            const double b2 = bn[2 * c + 1], r2 = rn[2 * c];
+            small = small && r2 <= o->refine_tol * o->refine_tol * b2;
+            w = std::max(w, b2 > 0.0 ? r2 / b2 : 0.0);
+        }
+        op.refine_iters = it;
+        if (small && it <= o->refine_max_iter) break;
+        if (it >= o->refine_max_iter || (it > 1 && !(w < 0.25 * worst))) {
+            // the FP64 step, whose solves are the first ones
+            if (it > 1) {
+                tpe_step_opts o64 = *o;
+                o64.precision = TPE_PRECISION_FP64;
+                TPE_TRY(op_finalize(ctx, V, k, singular, b_flat, &o64));
+            }
+            op.mixed_fallback = true;
+            if (it > 1) return TPE_OK;
+            break;
+        }
+        worst = w;
+        TPE_CUDA_TRY(cudaMemcpyAsync(D, R, sizeof(double) * nv, cudaMemcpyDeviceToDevice, ctx->stream));
+        TPE_TRY(chol_solve(ctx, op.L, op.Linv, V, D, nrhs, true));
+        TPE_TRY(axpby(ctx, (int64_t)nv, 1.0, D, 1.0, op.Y));
+        TPE_TRY(residuals(R, nrhs, nullptr, D));
+    }
+    if (k > 0) {
         // symmetrise the Gram matrix (two sides of one dot product)
         if (!op.large)
             for (int32_t i = 0; i < k; i++)
@@ -1745,7 +1842,8 @@ int32_t step_impl(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, cons
         // The FP64 factorization of a small constraint set takes the right-hand
         // sides along (their forward solves), so there the gradient runs beside
         // the assembly, on all SMs.
-        ctx->grad_first = o->precision != TPE_PRECISION_MIXED && S.k <= kLargeSchur;
+        ctx->grad_first = S.k <= kLargeSchur && (o->precision != TPE_PRECISION_MIXED || V <= kMixedDirect ||
+                                                 3 * (S.k + 1) > kMixedMaxRhs);
         if (ctx->grad_first) TPE_TRY(launch_gradient(ctx));
     } else {
         // sequential (finite differences, or the per-phase timing ledger)
@@ -1803,7 +1901,7 @@ int32_t step_impl(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, cons
             }
         }
     }
-    st->refine_iterations = ctx->op.mixed ? ctx->op.refine_iters : (ctx->op.mixed_fallback ? -1 : 0);
+    st->refine_iterations = ctx->op.mixed_fallback ? -1 : ctx->op.refine_iters;
     if (singular) {
         double e = o->energy_before;
         if (!o->has_energy_before) TPE_TRY(objective(ctx, P, o, pen, &e, timings));

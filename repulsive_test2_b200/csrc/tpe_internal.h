@@ -45,6 +45,13 @@ constexpr int kNB = 64;
 // Most right-hand sides (3 per constraint row, +3 for b) the mixed solve takes
 // at factor time; larger sets use the FP64 factorization.
 constexpr int kMixedMaxRhs = 48;
+// Up to this many vertices the mixed mode takes the FP64 factor too (op_finalize): one
+// data-flow launch where the FP32 factor and its CG take 150 to 250, and one solve where the
+// CG takes 3 to 8. A step on a jittered trefoil or a random walk, FP32 against FP64 factor:
+// V = 2048 2510 -> 2120 us (walk), 2500 2718 -> 2290 and 2811 -> 2615, 3000 3289 -> 3365 and
+// 3166 -> 3026; from 3000 on a smooth curve's first residual tends to miss 1e-12, and a
+// correction costs 700 us. 64 curves of 256 to 1500 vertices together: 44 -> 16 ms.
+constexpr int32_t kMixedDirect = 2800;
 // Most step sizes one batched line-search launch projects together.
 constexpr int kMaxTrials = 16;
 
@@ -71,7 +78,7 @@ struct SaddleOp {
     bool trans_constrained = false;  // set contains a barycenter or point block
     bool mixed = false;              // solves use the FP32 factor + FP64 CG (mixed.cu)
     bool mixed_fallback = false;     // mixed requested, FP64 factorization used instead
-    int refine_iters = 0;            // CG iterations of the factor-time solve
+    int refine_iters = 0;            // CG iterations (FP64 factor: solves) at factor time
     int refine_max_iter = 60;
     double refine_tol = 1e-12;
     double rho = 0.0;                // A_rho = A + (rho/V) 1 1^T

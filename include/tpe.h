@@ -105,7 +105,7 @@ typedef struct {
     double proj_tol_abs, proj_tol_rel;         /* 1e-4, 1e-4 */
     int32_t proj_max_iter;                     /* 8 */
     int32_t precision;             /* TPE_PRECISION_* (extension): MIXED factors in 3xTF32 on the
-                                      tensor cores with an FP64 CG (up to 2800 vertices, where
+                                      tensor cores with an FP64 CG (up to 5000 vertices, where
                                       that is slower, in FP64, held to the same residual), or,
                                       for more than 64 constraint rows with frozen projection,
                                       forms the explicit inverses from int8 digit products */

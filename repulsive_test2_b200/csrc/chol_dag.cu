@@ -20,11 +20,11 @@
 // (mma.sync m8n8k4), operands staged by 16-byte cp.async, K in ascending order:
 // the result does not depend on which block took which tile.
 //
-// Measured against that (us): factor, order 777: 1380 -> 259, 2048: 3190 -> 812,
-// 4096: 6750 -> 2780, 12288: 40100 -> 29000; with the explicit inverse, 777: 2220
-// -> 327, 2500: 7200 -> 1780, 8192: 38500 -> 22400; two triangular solves of 15
-// right-hand sides, 777: 345 -> 132, 2048: 844 -> 342. Bound: to about 1500 rows
-// the chain (per 64 columns 9.7 us for the diagonal block, 7 for its two products,
+// Measured against that (us): factor, order 777: 1380 -> 242, 2048: 3190 -> 575,
+// 4096: 6750 -> 1330, 8192: 7100; with the explicit inverse, 777: 2220
+// -> 252, 2500: 7200 -> 1010, 8192: 38500 -> 20800; two triangular solves of 15
+// right-hand sides, 777: 345 -> 132, 2048: 844 -> 342. Bound: to about 3500 rows
+// the chain (per 64 columns 9.7 us for the diagonal block, 8 for its two products,
 // loads and flags), above it the workers' products (2.4 us each at the FP64
 // tensor rate of one SM).
 //
@@ -64,7 +64,8 @@ struct Dag {
     int64_t ld;              // row length of L, W and X (n or more); B and Ainv have n
     double tol;
     int32_t* flag;  // [(nb + nrb + nb) x nb] tiles done, then diag, preA, preD [nb each]
-    int32_t* ctl;   // [0] a pivot failed, [1] a wait ran out, [2] role ticket, [3] tile counter
+    // [0] a pivot failed, [1] a wait ran out, [2] role ticket, [3] tile counter, [4] the chain's SM + 1
+    int32_t* ctl;
 };
 
 __device__ __forceinline__ int32_t ld_acquire(const int32_t* p) {
@@ -709,17 +710,26 @@ __global__ void __launch_bounds__(kThr, 2) chol_dag_kernel(const Dag g) {
     Smem& sm = *reinterpret_cast<Smem*>(dyn);
     if (threadIdx.x == 0) sm.item = atomicAdd(g.ctl + 2, 1);
     __syncthreads();
+    uint32_t smid;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
     if (sm.item == 0) {
+        if (threadIdx.x == 0) atomicExch(g.ctl + 4, (int32_t)smid + 1);
         chain<kAl>(g, sm);
+        if (threadIdx.x == 0) atomicExch(g.ctl + 4, 0);
         // (then a worker like the others)
     }
     int32_t j = 0;
     int64_t before = 0;  // tiles in the columns before j
     for (;;) {
         __syncthreads();
-        if (threadIdx.x == 0) sm.item = atomicAdd(g.ctl + 3, 1);
+        if (threadIdx.x == 0) {
+            // the chain has its SM to itself (order 3500: 1230 -> 1030 us)
+            const bool off = ld_acquire(g.ctl + 4) == (int32_t)smid + 1;
+            sm.item = off ? -1 : atomicAdd(g.ctl + 3, 1);
+        }
         __syncthreads();
         const int64_t x = sm.item;
+        if (x < 0) return;
         while (j < g.nb && x >= before + column_count(g, j)) before += column_count(g, j++);
         if (j < g.nb) {
             if (!column_tile<kAl>(g, sm, j, (int32_t)(x - before))) return;
@@ -896,19 +906,25 @@ int32_t chol_dag(tpe_ctx* ctx, const CholDag& c, int32_t* singular) {
     g.nrb = (c.nr + NB - 1) / NB;
     g.tol = c.tol;
     const size_t nflag = (size_t)(2 * g.nb + g.nrb) * g.nb + 3 * (size_t)g.nb;
-    TPE_TRY(ensure(ctx, ctx->dag_flags, sizeof(int32_t) * (nflag + 4)));
+    TPE_TRY(ensure(ctx, ctx->dag_flags, sizeof(int32_t) * (nflag + 5)));
     g.ctl = ctx->dag_flags.as<int32_t>();
-    g.flag = g.ctl + 4;
+    g.flag = g.ctl + 5;
     const cudaStream_t st = ctx->stream;
-    TPE_CUDA_TRY(cudaMemsetAsync(g.ctl, 0, sizeof(int32_t) * (nflag + 4), st));
+    TPE_CUDA_TRY(cudaMemsetAsync(g.ctl, 0, sizeof(int32_t) * (nflag + 5), st));
     auto even = [](const double* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     const bool al = (c.n & 1) == 0 && (g.ld & 1) == 0 && even(c.L) && even(c.B) && even(c.W);
     auto kern = al ? chol_dag_kernel<true> : chol_dag_kernel<false>;
     const size_t smem = (sizeof(Smem) + 15) / 16 * 16 + sizeof(double) * kTile;
     TPE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // tiles in flight: enough for the widest column, at most two blocks per SM
+    // Blocks: a worker holds its tile until the last factor of its sum is done, so the
+    // columns ahead of the chain need blocks of their own; nb / 8 - 1 columns of them (nine
+    // with the inverse), at most two blocks per SM. Against one column's worth (two with
+    // the inverse), us: order 2048 767 -> 575, 3500 1965 -> 1030, 4096 2600 -> 1310; with
+    // the inverse 1200 510 -> 357, 2500 1750 -> 1010. Below 1500 rows the chain is the
+    // bound, and blocks that wait only take room from other contexts' kernels.
     const int64_t widest = g.nb + g.nrb + 1;
-    const unsigned grid = (unsigned)std::min<int64_t>(2 * (int64_t)ctx->num_sms, 1 + (c.Ainv ? 2 : 1) * widest);
+    const unsigned grid = (unsigned)std::min<int64_t>(
+        2 * (int64_t)ctx->num_sms, 1 + (c.Ainv ? 9 : std::max(1, g.nb / 8 - 1)) * widest);
     {
         KernelScope ks(ctx, TPE_KGROUP_CHOLESKY, 1);
         kern<<<grid, kThr, smem, st>>>(g);

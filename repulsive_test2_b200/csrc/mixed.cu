@@ -170,17 +170,21 @@ potrf128_kernel(const float* __restrict__ S, int32_t ld, int32_t j0, float* __re
 #pragma unroll
                 for (int q = 0; q < 8; q++) v[h][q] = 0.0f;
             }
+            // the panel's eight products, then one rounding of what they come off
+            float sum[8];
 #pragma unroll
             for (int c = 0; c < 8; c++) {
                 const float t = zp[c * kLdZ + lane + 32 * h] * iv[c];
 #pragma unroll
-                for (int q = 0; q < 8; q++) v[h][q] = fmaf(t, l[c][q], v[h][q]);
+                for (int q = 0; q < 8; q++) sum[q] = c == 0 ? t * l[c][q] : fmaf(t, l[c][q], sum[q]);
             }
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[h][q] += sum[q];
         }
     }
     // the panel's own 8 x 8 block in every lane, so that its pivots need no shuffle, and
     // the identity's eight rows that its slots turn into
-    float d[8][8], u[8];
+    float d[8][8], u[8], rs[8];
     {
         const int hp = w >> 2, i = lane - ((8 * w) & 31);
         const bool mine = i >= 0 && i < 8;
@@ -195,7 +199,10 @@ potrf128_kernel(const float* __restrict__ S, int32_t ld, int32_t j0, float* __re
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             const float piv = d[c][c];
-            const float iv = __fdividef(1.0f, piv > 0.0f && isfinite(piv) ? piv : 1.0f);
+            // 1/piv as the square of the factor that scales the column: the update is then
+            // that of the L which goes out, whatever the approximation's error
+            rs[c] = rsqrtf(piv > 0.0f && isfinite(piv) ? piv : 1.0f);
+            const float iv = rs[c] * rs[c];
             if (lane == 0) inv[8 * w + c] = iv;
             float* zc = z + (8 * w + c) * kLdZ;
             if (mine) zc[8 * w + i] = u[c];
@@ -222,16 +229,11 @@ potrf128_kernel(const float* __restrict__ S, int32_t ld, int32_t j0, float* __re
 #pragma unroll
     for (int c = 0; c < 8; c++) {
         const int k = 8 * w + c;
-        float piv = d[c][c];
-        if (!(piv > 0.0f) || !isfinite(piv)) {
-            brk = true;
-            piv = 1.0f;
-        }
-        const float rs = rsqrtf(piv);
+        if (!(d[c][c] > 0.0f) || !isfinite(d[c][c])) brk = true;
         const float4 x = *reinterpret_cast<const float4*>(z + k * kLdZ + 4 * lane);
         float y[4] = {x.x, x.y, x.z, x.w}, hi[4], lo[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) split32(4 * lane + q <= k ? y[q] * rs : 0.0f, hi[q], lo[q]);
+        for (int q = 0; q < 4; q++) split32(4 * lane + q <= k ? y[q] * rs[c] : 0.0f, hi[q], lo[q]);
         const size_t o = (size_t)(j0 + k) * ld + j0 + 4 * lane;
         *reinterpret_cast<float4*>(Zhi + o) = make_float4(hi[0], hi[1], hi[2], hi[3]);
         *reinterpret_cast<float4*>(Zlo + o) = make_float4(lo[0], lo[1], lo[2], lo[3]);

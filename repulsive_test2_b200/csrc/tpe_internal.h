@@ -47,11 +47,13 @@ constexpr int kNB = 64;
 constexpr int kMixedMaxRhs = 48;
 // Up to this many vertices the mixed mode takes the FP64 factor too (op_finalize): one
 // data-flow launch where the FP32 factor and its CG take 150 to 250, and one solve where the
-// CG takes 3 to 8. A step on a jittered trefoil or a random walk, FP32 against FP64 factor:
-// V = 2048 2510 -> 2120 us (walk), 2500 2718 -> 2290 and 2811 -> 2615, 3000 3289 -> 3365 and
-// 3166 -> 3026; from 3000 on a smooth curve's first residual tends to miss 1e-12, and a
-// correction costs 700 us. 64 curves of 256 to 1500 vertices together: 44 -> 16 ms.
-constexpr int32_t kMixedDirect = 2800;
+// CG takes 3 to 11. A step on a random walk or a jittered trefoil, FP32 against FP64 factor
+// (us): V = 1024 1910 -> 1330, 2500 2810 -> 2325 and 2720 -> 1910, 4096 4614 -> 3234 and 4636
+// -> 2822, 6000 6866 -> 5668 and 7209 -> 5379, 8192 10610 -> 10956 and 10269 -> 10355. A
+// correction, which rough curves of 3600 and smooth ones of 3000 and more vertices need to
+// reach 1e-12, adds 900 (4096) to 1400 (6000): then 5000 5340 -> 5350 and 6000 -> 5060, 6000
+// 6866 -> 7100 and 7209 -> 6760. 64 curves of 256 to 1500 vertices together: 44 -> 16 ms.
+constexpr int32_t kMixedDirect = 5000;
 // Most step sizes one batched line-search launch projects together.
 constexpr int kMaxTrials = 16;
 

@@ -283,7 +283,8 @@ int32_t tpe_energy_bh(tpe_ctx* ctx, const double* xyz, const tpe_params* p, doub
  * pairs. */
 enum { TPE_BCT_HIGH = 0, TPE_BCT_LOW = 1 };
 /* The edge tree those two calls build (build_edge_bvh, oracle/tpe_stage2_oracle.py:467-502),
- * on the host only (no device, no context), for checking it node by node: per node
+ * on the host only (no device, no context; tpe_energy_bh builds the same tree on the
+ * device), for checking it node by node: per node
  * node_f[9] = center xyz, mean tangent xyz, mass, rx, rT and node_i[4] = first
  * position in perm, edge count, left, right (-1 for a leaf); perm[E] lists the
  * edges so that every node's edges are one contiguous range. *n_nodes receives

@@ -11,8 +11,9 @@
 // center (bh_ordered_cluster_term, :515-529); a leaf that is not admissible is
 // summed exactly. theta = 0 admits nothing and gives the exact energy.
 //
-// The tree is built on the host, in the oracle's order of operations, so that
-// the device traverses the same tree: split on the coordinate of largest
+// The energy's tree is built on the device (up to 2^19 edges and leaves of 512; on the
+// host otherwise, and for the block cluster tree), in the oracle's order of operations,
+// so that it is the same tree: split on the coordinate of largest
 // spread of the 6-D points (midpoint, unit tangent), stable sort, the first
 // half (rounded down) to the left; node centers, tangents and masses summed as
 // numpy sums them (sequential along the rows, pairwise for the mass). Node
@@ -210,16 +211,23 @@ struct Builder {
     }
 };
 
+// |e x d|^alpha / |d|^beta, each with eps added to the length; k36: exponents 3 and 6.
+template <bool k36>
 __device__ __forceinline__ double term(double ex, double ey, double ez, double dx, double dy,
                                        double dz, double alpha, double beta, double eps) {
     const double cx = ey * dz - ez * dy, cy = ez * dx - ex * dz, cz = ex * dy - ey * dx;
     const double dn = sqrt((dx * dx + dy * dy) + dz * dz) + eps;
     const double cn = sqrt((cx * cx + cy * cy) + cz * cz) + eps;
+    if constexpr (k36) {
+        const double d2 = dn * dn;
+        return cn * cn * cn / (d2 * d2 * d2);
+    }
     return pow(cn, alpha) / pow(dn, beta);
 }
 
 // One thread per target edge I: its ordered sum over the tree, and the visit,
 // approximated-edge and direct-pair counts.
+template <bool k36>
 __global__ void __launch_bounds__(128)
 bh_energy_kernel(const double* __restrict__ pos, const int2* __restrict__ edges, int32_t E,
                  const Node* __restrict__ nodes, const int32_t* __restrict__ perm,
@@ -262,8 +270,8 @@ bh_energy_kernel(const double* __restrict__ pos, const int2* __restrict__ edges,
         }
         if (admiss) {
             approx += nd.count;
-            const double s = term(ex, ey, ez, ax - nd.cx, ay - nd.cy, az - nd.cz, alpha, beta, eps) +
-                             term(ex, ey, ez, bx - nd.cx, by - nd.cy, bz - nd.cz, alpha, beta, eps);
+            const double s = term<k36>(ex, ey, ez, ax - nd.cx, ay - nd.cy, az - nd.cz, alpha, beta, eps) +
+                             term<k36>(ex, ey, ez, bx - nd.cx, by - nd.cy, bz - nd.cz, alpha, beta, eps);
             val += 0.5 * pI * nd.mass * s;
         } else if (nd.left < 0) {
             for (int32_t k = nd.begin; k < nd.begin + nd.count; k++) {
@@ -275,10 +283,10 @@ bh_energy_kernel(const double* __restrict__ pos, const int2* __restrict__ edges,
                 const double dx = pos[3 * eJ.y], dy = pos[3 * eJ.y + 1], dz = pos[3 * eJ.y + 2];
                 const double fx = dx - cx, fy = dy - cy, fz = dz - cz;
                 const double ellJ = sqrt((fx * fx + fy * fy) + fz * fz) + eps;
-                const double s = term(ex, ey, ez, ax - cx, ay - cy, az - cz, alpha, beta, eps) +
-                                 term(ex, ey, ez, ax - dx, ay - dy, az - dz, alpha, beta, eps) +
-                                 term(ex, ey, ez, bx - cx, by - cy, bz - cz, alpha, beta, eps) +
-                                 term(ex, ey, ez, bx - dx, by - dy, bz - dz, alpha, beta, eps);
+                const double s = term<k36>(ex, ey, ez, ax - cx, ay - cy, az - cz, alpha, beta, eps) +
+                                 term<k36>(ex, ey, ez, ax - dx, ay - dy, az - dz, alpha, beta, eps) +
+                                 term<k36>(ex, ey, ez, bx - cx, by - cy, bz - cz, alpha, beta, eps) +
+                                 term<k36>(ex, ey, ez, bx - dx, by - dy, bz - dz, alpha, beta, eps);
                 val += 0.25 * pI * ellJ * s;
             }
         } else {
@@ -296,15 +304,18 @@ bh_energy_kernel(const double* __restrict__ pos, const int2* __restrict__ edges,
     counts[3 * (size_t)I + 2] = direct;
 }
 
-// Fixed-order totals: one block sums the per-edge values and counts.
+// Fixed-order totals in two launches: kRedPer edges a block, then the blocks' sums by one
+// (224 us as one block over 131072 edges, 10 as two launches).
+constexpr int kRedPer = 1024;
 __global__ void __launch_bounds__(256)
 bh_reduce_kernel(const double* __restrict__ val, const long long* __restrict__ counts, int32_t E,
-                 double* __restrict__ total, long long* __restrict__ ctot) {
+                 double* __restrict__ total, long long* __restrict__ ctot, double scale, int32_t per) {
     __shared__ double sv[256];
     __shared__ long long sc[3][256];
     double v = 0.0;
     long long c0 = 0, c1 = 0, c2 = 0;
-    for (int32_t i = threadIdx.x; i < E; i += 256) {
+    const int32_t i0 = (int32_t)blockIdx.x * per, i1 = min(E, i0 + per);
+    for (int32_t i = i0 + threadIdx.x; i < i1; i += 256) {
         v += val[i];
         c0 += counts[3 * (size_t)i];
         c1 += counts[3 * (size_t)i + 1];
@@ -323,9 +334,569 @@ bh_reduce_kernel(const double* __restrict__ val, const long long* __restrict__ c
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        total[0] = 0.5 * sv[0];
-        for (int q = 0; q < 3; q++) ctot[q] = sc[q][0];
+        total[blockIdx.x] = scale * sv[0];
+        for (int q = 0; q < 3; q++) ctot[3 * (size_t)blockIdx.x + q] = sc[q][0];
     }
+}
+
+// ---- the same tree, built on the device ------------------------------------------------
+//
+// A node's halves depend on its count alone, so the tree's shape is known in advance: node
+// `idx` of level l is entry 2^l - 1 + idx, its children 2i + 1 and 2i + 2. Every value is
+// rounded as the host builder rounds it (no contraction, sums in the same order), so both
+// give the same nodes.
+//   top levels (nodes of more than kSubtree edges): per level the dimension of largest
+//     spread, and a bitonic sort of (coordinate, position), which is the stable order;
+//     then one launch for the statistics of all their nodes;
+//   below: one block per subtree, its edges in shared memory, all levels in one launch.
+// 131072 edges: a call takes 2.4 ms (23.6 with the host's tree, 19 of them its build and
+// copies): 1.6 the tree, 0.7 the traversal, whose powers are products at exponents 3
+// and 6 (2.35 with pow). Bound: the sort's 90 small launches, 0.9 ms, beside which the
+// root's sums run, one addition after the other (0.6 ms, 9 clocks each).
+constexpr int kSubtree = 1024;
+constexpr int kSubThr = 512;
+constexpr int kTile = 2048;  // elements sorted in shared memory at the top levels
+constexpr int kSeq = 992;    // a chunk of the sequential sums (31 warps fetch, one adds)
+constexpr int32_t kDeviceTreeEdges = 1 << 19;
+constexpr int kDeviceTreeLeaf = 512;
+constexpr int kPairDepth = 13;  // halvings until 2^19 terms are at most 128
+
+struct DevTree {
+    const double* pos;
+    const int2* edges;
+    int32_t E, leaf, top;  // `top` levels above the subtrees
+    double eps;
+    double *X, *m;   // 6 x E (midpoint, unit tangent) and E, by edge
+    int32_t* perm;   // (top + 1) x E: the edges in order at each level
+    unsigned long long* key;
+    int32_t* ord;    // positions, sorted with their keys
+    double* sums;    // 7 per top node: the six weighted sums and the mass
+    unsigned long long* spread;  // 12 per top node (tree_spread_kernel)
+    Node* nodes;
+    int32_t *final_perm, *where;
+};
+
+// Edges [begin, begin + count) of node idx of a level (count = 0: its parent is a leaf).
+__device__ __forceinline__ int2 span_of(int32_t begin, int32_t count, int32_t leaf, int level, int32_t idx) {
+    for (int q = level - 1; q >= 0; q--) {
+        if (count <= leaf) return make_int2(begin, 0);
+        const int32_t l = count / 2;
+        if ((idx >> q) & 1) {
+            begin += l;
+            count -= l;
+        } else {
+            count = l;
+        }
+    }
+    return make_int2(begin, count);
+}
+
+// x's place in the order of doubles (-0 as +0).
+__device__ __forceinline__ unsigned long long order_key(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(__dadd_rn(x, 0.0));
+    return b >> 63 ? ~b : b | (1ull << 63);
+}
+
+__device__ __forceinline__ double norm3_sq(double x, double y, double z) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+}
+
+__global__ void tree_edges_kernel(const DevTree t) {
+    const int32_t I = blockIdx.x * blockDim.x + threadIdx.x;
+    if (I >= t.E) return;
+    const int2 e = t.edges[I];
+    double d[3];
+    for (int q = 0; q < 3; q++) {
+        const double a = t.pos[3 * (size_t)e.x + q], b = t.pos[3 * (size_t)e.y + q];
+        d[q] = __dsub_rn(b, a);
+        t.X[(size_t)q * t.E + I] = __dmul_rn(0.5, __dadd_rn(a, b));
+    }
+    const double ell = __dsqrt_rn(norm3_sq(d[0], d[1], d[2]));
+    for (int q = 0; q < 3; q++)
+        t.X[(size_t)(3 + q) * t.E + I] = ell >= kTangentTol ? __ddiv_rn(d[q], ell) : 0.0;
+    t.m[I] = __dadd_rn(ell, t.eps);
+    t.perm[I] = I;
+}
+
+__device__ __forceinline__ double key_value(unsigned long long k) {
+    return __longlong_as_double((long long)(k >> 63 ? k & ~(1ull << 63) : ~k));
+}
+
+// Spreads of a top level's nodes: per node and coordinate the largest key and the largest
+// complement (of the smallest), from zeros. kKeysPer edges a block.
+constexpr int kKeysPer = 2048;
+__global__ void __launch_bounds__(256) tree_spread_kernel(const DevTree t, int level) {
+    const int2 s = span_of(0, t.E, t.leaf, level, blockIdx.y);
+    const int32_t* perm = t.perm + (size_t)level * t.E;
+    __shared__ double red[12][8];
+    double lo[6], hi[6];
+    for (int d = 0; d < 6; d++) {
+        lo[d] = INFINITY;
+        hi[d] = -INFINITY;
+    }
+    const int32_t k0 = s.x + blockIdx.x * kKeysPer, k1 = min(s.x + s.y, k0 + kKeysPer);
+    for (int32_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+        const int32_t J = perm[k];
+        for (int d = 0; d < 6; d++) {
+            const double x = t.X[(size_t)d * t.E + J];
+            lo[d] = fmin(lo[d], x);
+            hi[d] = fmax(hi[d], x);
+        }
+    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int d = 0; d < 6; d++) {
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        }
+        if (lane == 0) {
+            red[d][w] = lo[d];
+            red[6 + d][w] = hi[d];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x >= 12 || k0 >= k1) return;
+    double x = red[threadIdx.x][0];
+    for (int q = 1; q < 8; q++) x = threadIdx.x < 6 ? fmin(x, red[threadIdx.x][q]) : fmax(x, red[threadIdx.x][q]);
+    const unsigned long long k = order_key(x);
+    atomicMax(t.spread + 12 * ((size_t)(1 << level) - 1 + blockIdx.y) + threadIdx.x, threadIdx.x < 6 ? ~k : k);
+}
+// The sort keys of a top level: the coordinate of largest spread, the first on ties.
+__global__ void __launch_bounds__(256) tree_keys_kernel(const DevTree t, int level) {
+    const int2 s = span_of(0, t.E, t.leaf, level, blockIdx.y);
+    const int32_t* perm = t.perm + (size_t)level * t.E;
+    const unsigned long long* sp = t.spread + 12 * ((size_t)(1 << level) - 1 + blockIdx.y);
+    int dim = 0;
+    double best = 0.0;
+    for (int d = 0; d < 6; d++) {
+        const double width = __dsub_rn(key_value(sp[6 + d]), key_value(~sp[d]));
+        if (d == 0 || width > best) {
+            best = width;
+            dim = d;
+        }
+    }
+    const double* x = t.X + (size_t)dim * t.E;
+    const int32_t k0 = s.x + blockIdx.x * kKeysPer, k1 = min(s.x + s.y, k0 + kKeysPer);
+    for (int32_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+        t.key[k] = order_key(x[perm[k]]);
+        t.ord[k] = k;
+    }
+}
+
+__device__ __forceinline__ bool after(unsigned long long ka, int32_t oa, unsigned long long kb, int32_t ob) {
+    return ka > kb || (ka == kb && oa > ob);
+}
+// Pair p of a bitonic step (every comparison ascending, so that places beyond the end are
+// as good as filled with the largest key): the mirror step of blocks of k, or distance h.
+__device__ __forceinline__ int2 mirror_pair(int32_t p, int32_t k) {
+    const int32_t b = p / (k / 2) * k, o = p % (k / 2);
+    return make_int2(b + o, b + k - 1 - o);
+}
+__device__ __forceinline__ int2 distance_pair(int32_t p, int32_t h) {
+    const int32_t i = p / h * 2 * h + p % h;
+    return make_int2(i, i + h);
+}
+
+// One step of all nodes of a level: block k's mirror step (h = 0) or distance h.
+__global__ void tree_step_kernel(const DevTree t, int level, int32_t k, int32_t h) {
+    const int2 s = span_of(0, t.E, t.leaf, level, blockIdx.y);
+    const int2 p = h ? distance_pair(blockIdx.x * blockDim.x + threadIdx.x, h)
+                     : mirror_pair(blockIdx.x * blockDim.x + threadIdx.x, k);
+    if (p.y >= s.y) return;
+    const int32_t a = s.x + p.x, b = s.x + p.y;
+    const unsigned long long ka = t.key[a], kb = t.key[b];
+    const int32_t oa = t.ord[a], ob = t.ord[b];
+    if (!after(ka, oa, kb, ob)) return;
+    t.key[a] = kb, t.key[b] = ka;
+    t.ord[a] = ob, t.ord[b] = oa;
+}
+
+// The steps within tiles of kTile: from nothing (k0 = 2), or the rest of merge k0.
+__global__ void __launch_bounds__(kTile / 2) tree_tile_kernel(const DevTree t, int level, int32_t k0) {
+    __shared__ unsigned long long key[kTile];
+    __shared__ int32_t ord[kTile];
+    const int2 s = span_of(0, t.E, t.leaf, level, blockIdx.y);
+    const int32_t t0 = s.x + blockIdx.x * kTile, n = min(kTile, s.y - (int32_t)blockIdx.x * kTile);
+    if (n <= 0) return;
+    for (int32_t e = threadIdx.x; e < n; e += blockDim.x) {
+        key[e] = t.key[t0 + e];
+        ord[e] = t.ord[t0 + e];
+    }
+    auto exchange = [&](int2 p) {
+        __syncthreads();
+        if (p.y < n && after(key[p.x], ord[p.x], key[p.y], ord[p.y])) {
+            const unsigned long long k = key[p.x];
+            const int32_t o = ord[p.x];
+            key[p.x] = key[p.y], key[p.y] = k;
+            ord[p.x] = ord[p.y], ord[p.y] = o;
+        }
+    };
+    if (k0 > kTile) {
+        for (int32_t h = kTile / 2; h > 0; h /= 2) exchange(distance_pair(threadIdx.x, h));
+    } else {
+        for (int32_t k = 2; k <= kTile; k *= 2) {
+            exchange(mirror_pair(threadIdx.x, k));
+            for (int32_t h = k / 4; h > 0; h /= 2) exchange(distance_pair(threadIdx.x, h));
+        }
+    }
+    __syncthreads();
+    for (int32_t e = threadIdx.x; e < n; e += blockDim.x) {
+        t.key[t0 + e] = key[e];
+        t.ord[t0 + e] = ord[e];
+    }
+}
+
+__global__ void tree_order_kernel(const DevTree t, int level) {
+    const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < t.E) t.perm[(size_t)(level + 1) * t.E + k] = t.perm[(size_t)level * t.E + t.ord[k]];
+}
+
+// np_pairwise_sum of at most 128 terms get(0 .. n - 1).
+template <class F>
+__device__ __forceinline__ double pairwise_base(F&& get, int32_t n) {
+    if (n < 8) {
+        double s = 0.0;
+        for (int32_t i = 0; i < n; i++) s = __dadd_rn(s, get(i));
+        return s;
+    }
+    double r[8];
+    for (int j = 0; j < 8; j++) r[j] = get(j);
+    int32_t i = 8;
+    for (; i < n - n % 8; i += 8)
+        for (int j = 0; j < 8; j++) r[j] = __dadd_rn(r[j], get(i + j));
+    double s = __dadd_rn(__dadd_rn(__dadd_rn(r[0], r[1]), __dadd_rn(r[2], r[3])),
+                         __dadd_rn(__dadd_rn(r[4], r[5]), __dadd_rn(r[6], r[7])));
+    for (; i < n; i++) s = __dadd_rn(s, get(i));
+    return s;
+}
+// The piece at `path` (its first `depth` halvings, first one in the top bit) of np_pairwise_sum's
+// recursion over n terms: (first, count), count 0 where the recursion ended before.
+__device__ __forceinline__ int2 pairwise_piece(int32_t n, int32_t path, int depth) {
+    int32_t at = 0;
+    for (int q = depth - 1; q >= 0; q--) {
+        const bool right = (path >> q) & 1;
+        if (n <= 128) {
+            if (right) return make_int2(at, 0);
+            continue;
+        }
+        int32_t l = n / 2;
+        l -= l % 8;
+        if (right) {
+            at += l;
+            n -= l;
+        } else {
+            n = l;
+        }
+    }
+    return make_int2(at, n);
+}
+
+// The sequential sums (y = 0) and the pairwise mass (y = 1) of each top node.
+__global__ void __launch_bounds__(1024) tree_sums_kernel(const DevTree t, int32_t first) {
+    extern __shared__ __align__(16) double buf[];
+    const int32_t node = first + (int32_t)blockIdx.x;
+    const int level = 31 - __clz(node + 1);
+    const int2 s = span_of(0, t.E, t.leaf, level, node + 1 - (1 << level));
+    const int32_t* perm = t.perm + (size_t)level * t.E + s.x;
+    double* out = t.sums + 7 * (size_t)node;
+    if (blockIdx.y == 0) {
+        constexpr int kRow = kSeq + 1;
+        auto fetch = [&](int32_t c) {
+            const int32_t e = (int32_t)threadIdx.x - 32, k = c * kSeq + e;
+            if (e < 0 || k >= s.y) return;
+            const int32_t J = perm[k];
+            const double mass = t.m[J];
+            for (int d = 0; d < 6; d++)
+                buf[((c & 1) * 6 + d) * kRow + e] = __dmul_rn(mass, t.X[(size_t)d * t.E + J]);
+        };
+        double sum = 0.0;
+        fetch(0);
+        for (int32_t c = 0; c * kSeq < s.y; c++) {
+            __syncthreads();
+            fetch(c + 1);
+            if (threadIdx.x < 6) {
+                const double* row = buf + ((c & 1) * 6 + threadIdx.x) * kRow;
+                const int32_t n = min(kSeq, s.y - c * kSeq);
+                int32_t k = 0;
+                for (; k + 16 <= n; k += 16) {
+                    double x[16];
+#pragma unroll
+                    for (int q = 0; q < 16; q++) x[q] = row[k + q];
+#pragma unroll
+                    for (int q = 0; q < 16; q++) sum = __dadd_rn(sum, x[q]);
+                }
+                for (; k < n; k++) sum = __dadd_rn(sum, row[k]);
+            }
+        }
+        if (threadIdx.x < 6) out[threadIdx.x] = sum;
+        return;
+    }
+    for (int32_t p = threadIdx.x; p < 1 << kPairDepth; p += blockDim.x) {
+        const int2 r = pairwise_piece(s.y, p, kPairDepth);
+        if (r.y > 0) buf[p] = pairwise_base([&](int32_t i) { return t.m[perm[r.x + i]]; }, r.y);
+    }
+    for (int depth = kPairDepth - 1; depth >= 0; depth--) {
+        __syncthreads();
+        for (int32_t p = threadIdx.x; p < 1 << depth; p += blockDim.x) {
+            const int2 r = pairwise_piece(s.y, p, depth);
+            if (r.y > 128) {
+                const int w = 1 << (kPairDepth - depth);
+                buf[p * w] = __dadd_rn(buf[p * w], buf[p * w + w / 2]);
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) out[6] = buf[0];
+}
+
+__device__ __forceinline__ Node make_node(const double (&c)[6], double mass, double rx2, double rT2, int2 s,
+                                          int32_t leaf, int32_t i) {
+    Node nd;
+    nd.cx = c[0], nd.cy = c[1], nd.cz = c[2];
+    nd.tx = c[3], nd.ty = c[4], nd.tz = c[5];
+    nd.mass = mass;
+    nd.rx = __dsqrt_rn(rx2);  // (of the largest square: the root is monotonic)
+    nd.rT = __dsqrt_rn(rT2);
+    nd.begin = s.x, nd.count = s.y;
+    nd.left = s.y > leaf ? 2 * i + 1 : -1;
+    nd.right = s.y > leaf ? 2 * i + 2 : -1;
+    nd.parent = i > 0 ? (i - 1) / 2 : -1;
+    nd.pad = 0;
+    return nd;
+}
+
+// Centers and radii of each top node.
+__global__ void __launch_bounds__(1024) tree_top_kernel(const DevTree t) {
+    const int level = 31 - __clz(blockIdx.x + 1);
+    const int2 s = span_of(0, t.E, t.leaf, level, (int32_t)blockIdx.x + 1 - (1 << level));
+    const int32_t* perm = t.perm + (size_t)level * t.E;
+    const double* in = t.sums + 7 * (size_t)blockIdx.x;
+    double c[6];
+    for (int d = 0; d < 6; d++) c[d] = __ddiv_rn(in[d], in[6]);
+    double r[2] = {0.0, 0.0};
+    for (int32_t k = s.x + threadIdx.x; k < s.x + s.y; k += blockDim.x) {
+        const int32_t J = perm[k];
+        double x[6];
+        for (int d = 0; d < 6; d++) x[d] = __dsub_rn(t.X[(size_t)d * t.E + J], c[d]);
+        r[0] = fmax(r[0], norm3_sq(x[0], x[1], x[2]));
+        r[1] = fmax(r[1], norm3_sq(x[3], x[4], x[5]));
+    }
+    __shared__ double red[2][32];
+    for (int q = 0; q < 2; q++) {
+        for (int o = 16; o > 0; o >>= 1) r[q] = fmax(r[q], __shfl_xor_sync(0xffffffffu, r[q], o));
+        if ((threadIdx.x & 31) == 0) red[q][threadIdx.x >> 5] = r[q];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 2; q++)
+            for (int w = 0; w < 32; w++) r[q] = fmax(r[q], red[q][w]);
+        t.nodes[blockIdx.x] = make_node(c, in[6], r[0], r[1], s, t.leaf, blockIdx.x);
+    }
+}
+
+// One block per subtree of at most kSubtree edges: its nodes, level by level, and the final
+// order. Shared memory: the edges' coordinates and masses, the sort's keys and positions, the
+// order, and per node of a level its sums (and spreads), mass and squared radii.
+struct SubSmem {
+    double X[6][kSubtree], m[kSubtree];
+    unsigned long long key[kSubtree];
+    int32_t pos[kSubtree];         // sorted with key
+    int32_t ord[2][kSubtree];      // element at each place
+    double c[kSubtree][6];         // per node
+    double width[kSubtree / 2][6];
+    double mass[kSubtree];
+    unsigned long long r2[kSubtree][2];
+    int32_t dim[kSubtree / 2];
+};
+
+template <int D, class F>
+__device__ double pairwise_small(F&& get, int32_t at, int32_t n) {
+    if constexpr (D > 0) {
+        if (n > 128) {
+            int32_t l = n / 2;
+            l -= l % 8;
+            const double a = pairwise_small<D - 1>(get, at, l);
+            return __dadd_rn(a, pairwise_small<D - 1>(get, at + l, n - l));
+        }
+    }
+    return pairwise_base([&](int32_t i) { return get(at + i); }, n);
+}
+
+__global__ void __launch_bounds__(kSubThr) tree_sub_kernel(const DevTree t) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    SubSmem& sm = *reinterpret_cast<SubSmem*>(raw);
+    const int tid = threadIdx.x;
+    const int2 root = span_of(0, t.E, t.leaf, t.top, blockIdx.x);
+    const int32_t n = root.y;
+    const int32_t* perm = t.perm + (size_t)t.top * t.E + root.x;
+    for (int32_t e = tid; e < n; e += kSubThr) {
+        const int32_t J = perm[e];
+        for (int d = 0; d < 6; d++) sm.X[d][e] = t.X[(size_t)d * t.E + J];
+        sm.m[e] = t.m[J];
+        sm.ord[0][e] = e;
+    }
+    int cur = 0;
+    for (int depth = 0;; depth++) {
+        const int32_t nn = 1 << depth;  // nodes of this level (some may not exist)
+        const int32_t* ord = sm.ord[cur];
+        auto span = [&](int32_t idx) { return span_of(0, n, t.leaf, depth, idx); };
+        __syncthreads();
+        // sums and spreads, a thread per node and coordinate; masses, a thread per node
+        // (in the upper half of the block, beside them)
+        for (int32_t q = tid; tid < kSubThr / 2 && q < 6 * nn; q += kSubThr / 2) {
+            const int32_t idx = q / 6, d = q % 6;
+            const int2 s = span(idx);
+            double sum = 0.0, lo = INFINITY, hi = -INFINITY;
+#pragma unroll 4
+            for (int32_t k = s.x; k < s.x + s.y; k++) {
+                const int32_t e = ord[k];
+                const double x = sm.X[d][e];
+                sum = __dadd_rn(sum, __dmul_rn(sm.m[e], x));
+                lo = fmin(lo, x);
+                hi = fmax(hi, x);
+            }
+            sm.c[idx][d] = sum;
+            if (s.y > t.leaf) sm.width[idx][d] = __dsub_rn(hi, lo);
+        }
+        for (int32_t idx = tid - kSubThr / 2; tid >= kSubThr / 2 && idx < nn; idx += kSubThr / 2) {
+            const int2 s = span(idx);
+            sm.mass[idx] = pairwise_small<5>([&](int32_t k) { return sm.m[ord[k]]; }, s.x, s.y);
+            sm.r2[idx][0] = sm.r2[idx][1] = 0;
+        }
+        __syncthreads();
+        int32_t more = 0;  // does a node of this level split
+        for (int32_t q = tid; q < 6 * nn; q += kSubThr) sm.c[q / 6][q % 6] = __ddiv_rn(sm.c[q / 6][q % 6], sm.mass[q / 6]);
+        for (int32_t idx = tid; idx < nn; idx += kSubThr) {
+            if (span(idx).y <= t.leaf) continue;
+            more = 1;
+            int dim = 0;
+            for (int d = 1; d < 6; d++)
+                if (sm.width[idx][d] > sm.width[idx][dim]) dim = d;
+            sm.dim[idx] = dim;
+        }
+        more = __syncthreads_or(more);
+        // radii and sort keys, a thread per place
+        for (int32_t k = tid; k < n; k += kSubThr) {
+            int32_t idx = 0, b = 0, c = n;
+            bool in = true;
+            for (int q = 0; q < depth && in; q++) {
+                in = c > t.leaf;
+                if (!in) break;
+                const int32_t l = c / 2;
+                const bool right = k >= b + l;
+                idx = 2 * idx + right;
+                if (right) {
+                    b += l;
+                    c -= l;
+                } else {
+                    c = l;
+                }
+            }
+            const int32_t e = ord[k];
+            sm.pos[k] = k;
+            if (!in) continue;
+            double x[6];
+            for (int d = 0; d < 6; d++) x[d] = __dsub_rn(sm.X[d][e], sm.c[idx][d]);
+            const double a = norm3_sq(x[0], x[1], x[2]), g = norm3_sq(x[3], x[4], x[5]);
+            if (a > 0.0) atomicMax(&sm.r2[idx][0], (unsigned long long)__double_as_longlong(a));
+            if (g > 0.0) atomicMax(&sm.r2[idx][1], (unsigned long long)__double_as_longlong(g));
+            if (c > t.leaf) sm.key[k] = order_key(sm.X[sm.dim[idx]][e]);
+        }
+        __syncthreads();
+        for (int32_t idx = tid; idx < nn; idx += kSubThr) {
+            const int2 s = span(idx);
+            if (s.y == 0) continue;
+            double c[6];
+            for (int d = 0; d < 6; d++) c[d] = sm.c[idx][d];
+            const int32_t i = (1 << (t.top + depth)) - 1 + ((int32_t)blockIdx.x << depth) + idx;
+            t.nodes[i] = make_node(c, sm.mass[idx], __longlong_as_double((long long)sm.r2[idx][0]),
+                                   __longlong_as_double((long long)sm.r2[idx][1]),
+                                   make_int2(root.x + s.x, s.y), t.leaf, i);
+        }
+        if (!more) break;
+        // sort every node that splits
+        int32_t P = 2;
+        while (P < (n + nn - 1) / nn) P *= 2;
+        auto step = [&](int32_t k, int32_t h) {
+            __syncthreads();
+            for (int32_t p = tid; p < nn * (P / 2); p += kSubThr) {
+                const int32_t idx = p / (P / 2);
+                const int2 s = span(idx);
+                if (s.y <= t.leaf) continue;
+                const int2 r = h ? distance_pair(p % (P / 2), h) : mirror_pair(p % (P / 2), k);
+                if (r.y >= s.y) continue;
+                const int32_t a = s.x + r.x, b = s.x + r.y;
+                const unsigned long long ka = sm.key[a], kb = sm.key[b];
+                const int32_t pa = sm.pos[a], pb = sm.pos[b];
+                if (!after(ka, pa, kb, pb)) continue;
+                sm.key[a] = kb, sm.key[b] = ka;
+                sm.pos[a] = pb, sm.pos[b] = pa;
+            }
+        };
+        for (int32_t k = 2; k <= P; k *= 2) {
+            step(k, 0);
+            for (int32_t h = k / 4; h > 0; h /= 2) step(0, h);
+        }
+        __syncthreads();
+        for (int32_t k = tid; k < n; k += kSubThr) sm.ord[cur ^ 1][k] = ord[sm.pos[k]];
+        cur ^= 1;
+    }
+    for (int32_t k = tid; k < n; k += kSubThr) {
+        const int32_t J = perm[sm.ord[cur][k]];
+        t.final_perm[root.x + k] = J;
+        t.where[J] = root.x + k;
+    }
+}
+
+// Queues the build of the tree over ctx's edges at d_xyz into t (buffers set).
+int32_t build_tree_device(tpe_ctx* ctx, const DevTree& t) {
+    const cudaStream_t st = ctx->stream;
+    const int32_t E = t.E;
+    const unsigned flat = (unsigned)((E + 255) / 256);
+    KernelScope ks(ctx, TPE_KGROUP_ENERGY, 4 + 4 * t.top);
+    const size_t smem = sizeof(double) * std::max<size_t>(12 * (kSeq + 1), (size_t)1 << kPairDepth);
+    TPE_CUDA_TRY(cudaFuncSetAttribute(tree_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    TPE_CUDA_TRY(cudaFuncSetAttribute(tree_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(SubSmem)));
+    TPE_CUDA_TRY(cudaMemsetAsync(t.spread, 0, sizeof(double) * 12 * ((size_t)1 << t.top), st));
+    tree_edges_kernel<<<flat, 256, 0, st>>>(t);
+    // the sums of the first levels, the longest, beside the sorting
+    cudaEvent_t ev[2] = {ctx->ev_prep, ctx->ev_grad};
+    const cudaStream_t side[2] = {ctx->stream2, ctx->stream3};
+    const int early = std::min(t.top, 2);
+    for (int l = 0; l < t.top; l++) {
+        if (l < early) {
+            TPE_CUDA_TRY(cudaEventRecord(ev[l], st));
+            TPE_CUDA_TRY(cudaStreamWaitEvent(side[l], ev[l], 0));
+            tree_sums_kernel<<<dim3(1u << l, 2), 1024, smem, side[l]>>>(t, (1 << l) - 1);
+            TPE_CUDA_TRY(cudaEventRecord(ev[l], side[l]));
+        }
+        const unsigned nn = 1u << l;
+        const int32_t n = (E + (int32_t)nn - 1) / (int32_t)nn;
+        const unsigned tiles = (unsigned)((n + kTile - 1) / kTile);
+        int32_t P = kTile;
+        while (P < n) P *= 2;
+        const dim3 per((unsigned)((n + kKeysPer - 1) / kKeysPer), nn);
+        tree_spread_kernel<<<per, 256, 0, st>>>(t, l);
+        tree_keys_kernel<<<per, 256, 0, st>>>(t, l);
+        tree_tile_kernel<<<dim3(tiles, nn), kTile / 2, 0, st>>>(t, l, 2);
+        for (int32_t k = 2 * kTile; k <= P; k *= 2) {
+            const dim3 grid((unsigned)(P / 2 / 256), nn);
+            tree_step_kernel<<<grid, 256, 0, st>>>(t, l, k, 0);
+            for (int32_t h = k / 4; h >= kTile; h /= 2) tree_step_kernel<<<grid, 256, 0, st>>>(t, l, k, h);
+            tree_tile_kernel<<<dim3(tiles, nn), kTile / 2, 0, st>>>(t, l, k);
+        }
+        tree_order_kernel<<<flat, 256, 0, st>>>(t, l);
+    }
+    tree_sub_kernel<<<1u << t.top, kSubThr, sizeof(SubSmem), st>>>(t);
+    if (t.top > early) {
+        const int32_t first = (1 << early) - 1, nn = (1 << t.top) - 1 - first;
+        tree_sums_kernel<<<dim3((unsigned)nn, 2), 1024, smem, st>>>(t, first);
+    }
+    for (int l = 0; l < early; l++) TPE_CUDA_TRY(cudaStreamWaitEvent(st, ev[l], 0));
+    if (t.top > 0) tree_top_kernel<<<(1u << t.top) - 1, 1024, 0, st>>>(t);
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
 }
 
 // Edge geometry as edge_geometry computes it (tpe_stage2_oracle.py:72-82) and
@@ -421,36 +992,78 @@ int32_t bh_energy(tpe_ctx* ctx, const double* h_xyz, const double* d_xyz, double
         if (stats) stats[0] = stats[1] = stats[2] = 0;
         return TPE_OK;
     }
+    // the device builds the tree where its scratch and the shape of a subtree allow
+    const bool device = E <= kDeviceTreeEdges && leaf <= kDeviceTreeLeaf;
     Tree tr;
-    build_tree(ctx->h_edges.data(), ctx->E, h_xyz, eps, leaf, tr);
-    const size_t nn = tr.nodes.size();
+    size_t nn = 1;
+    DevTree t{};
+    if (device) {
+        while ((E + (1 << t.top) - 1) >> t.top > kSubtree) t.top++;
+        while (((int64_t)E + (int64_t)nn - 1) / (int64_t)nn > leaf) nn *= 2;
+        nn = 2 * nn - 1;
+    } else {
+        build_tree(ctx->h_edges.data(), ctx->E, h_xyz, eps, leaf, tr);
+        nn = tr.nodes.size();
+    }
     const size_t bytes_nodes = sizeof(Node) * nn, bytes_idx = sizeof(int32_t) * (size_t)E;
-    const size_t off_perm = (bytes_nodes + 255) / 256 * 256;
-    const size_t off_where = off_perm + (bytes_idx + 255) / 256 * 256;
-    const size_t off_val = off_where + (bytes_idx + 255) / 256 * 256;
-    const size_t off_cnt = off_val + (sizeof(double) * (size_t)E + 255) / 256 * 256;
-    const size_t off_tot = off_cnt + (sizeof(long long) * 3 * (size_t)E + 255) / 256 * 256;
-    TPE_TRY(ensure(ctx, ctx->bh_buf, off_tot + 256));
+    size_t end = 0;
+    auto place = [&](size_t bytes) {
+        const size_t at = end;
+        end += (bytes + 255) / 256 * 256;
+        return at;
+    };
+    const size_t off_nodes = place(bytes_nodes), off_perm = place(bytes_idx), off_where = place(bytes_idx);
+    const size_t off_val = place(sizeof(double) * (size_t)E), off_cnt = place(sizeof(long long) * 3 * (size_t)E);
+    const int32_t parts = (E + kRedPer - 1) / kRedPer;
+    const size_t off_tot = place(256), off_part = place(sizeof(double) * 4 * (size_t)parts);
+    const size_t off_x = place(device ? sizeof(double) * 7 * (size_t)E : 0);
+    const size_t off_ord = place(device ? bytes_idx * (size_t)(t.top + 2) : 0);
+    const size_t off_key = place(device ? sizeof(double) * (size_t)E : 0);
+    const size_t off_sums = place(device ? sizeof(double) * 7 * ((size_t)1 << t.top) : 0);
+    const size_t off_spread = place(device ? sizeof(double) * 12 * ((size_t)1 << t.top) : 0);
+    TPE_TRY(ensure(ctx, ctx->bh_buf, end));
     uint8_t* base = ctx->bh_buf.as<uint8_t>();
     const cudaStream_t st = ctx->stream;
-    TPE_CUDA_TRY(cudaMemcpyAsync(base, tr.nodes.data(), bytes_nodes, cudaMemcpyHostToDevice, st));
-    TPE_CUDA_TRY(cudaMemcpyAsync(base + off_perm, tr.perm.data(), bytes_idx, cudaMemcpyHostToDevice, st));
-    TPE_CUDA_TRY(cudaMemcpyAsync(base + off_where, tr.where.data(), bytes_idx, cudaMemcpyHostToDevice, st));
+    if (device) {
+        t.pos = d_xyz;
+        t.edges = ctx->d_edges.as<int2>();
+        t.E = E;
+        t.leaf = leaf;
+        t.eps = eps;
+        t.X = reinterpret_cast<double*>(base + off_x);
+        t.m = t.X + 6 * (size_t)E;
+        t.ord = reinterpret_cast<int32_t*>(base + off_ord);
+        t.perm = t.ord + E;
+        t.key = reinterpret_cast<unsigned long long*>(base + off_key);
+        t.sums = reinterpret_cast<double*>(base + off_sums);
+        t.spread = reinterpret_cast<unsigned long long*>(base + off_spread);
+        t.nodes = reinterpret_cast<Node*>(base + off_nodes);
+        t.final_perm = reinterpret_cast<int32_t*>(base + off_perm);
+        t.where = reinterpret_cast<int32_t*>(base + off_where);
+        TPE_TRY(build_tree_device(ctx, t));
+    } else {
+        TPE_CUDA_TRY(cudaMemcpyAsync(base + off_nodes, tr.nodes.data(), bytes_nodes, cudaMemcpyHostToDevice, st));
+        TPE_CUDA_TRY(cudaMemcpyAsync(base + off_perm, tr.perm.data(), bytes_idx, cudaMemcpyHostToDevice, st));
+        TPE_CUDA_TRY(cudaMemcpyAsync(base + off_where, tr.where.data(), bytes_idx, cudaMemcpyHostToDevice, st));
+    }
     int32_t* err = reinterpret_cast<int32_t*>(base + off_tot + 32);
     TPE_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int32_t), st));
     {
-        KernelScope ks(ctx, TPE_KGROUP_ENERGY, 2);
-        bh_energy_kernel<<<(E + 127) / 128, 128, 0, st>>>(
-            d_xyz, ctx->d_edges.as<int2>(), E, reinterpret_cast<const Node*>(base),
+        KernelScope ks(ctx, TPE_KGROUP_ENERGY, 3);
+        (alpha == 3.0 && beta == 6.0 ? bh_energy_kernel<true> : bh_energy_kernel<false>)<<<(E + 127) / 128, 128, 0, st>>>(
+            d_xyz, ctx->d_edges.as<int2>(), E, reinterpret_cast<const Node*>(base + off_nodes),
             reinterpret_cast<const int32_t*>(base + off_perm),
             reinterpret_cast<const int32_t*>(base + off_where), ctx->d_inc_off.as<int32_t>(),
             ctx->d_inc.as<int32_t>(), alpha, beta, eps, theta, theta_t,
             reinterpret_cast<double*>(base + off_val), reinterpret_cast<long long*>(base + off_cnt), err);
         TPE_CUDA_TRY(cudaGetLastError());
-        bh_reduce_kernel<<<1, 256, 0, st>>>(reinterpret_cast<const double*>(base + off_val),
-                                            reinterpret_cast<const long long*>(base + off_cnt), E,
-                                            reinterpret_cast<double*>(base + off_tot),
-                                            reinterpret_cast<long long*>(base + off_tot + 8));
+        double* part = reinterpret_cast<double*>(base + off_part);
+        long long* cpart = reinterpret_cast<long long*>(part + parts);
+        bh_reduce_kernel<<<(unsigned)parts, 256, 0, st>>>(reinterpret_cast<const double*>(base + off_val),
+                                                          reinterpret_cast<const long long*>(base + off_cnt), E,
+                                                          part, cpart, 1.0, kRedPer);
+        bh_reduce_kernel<<<1, 256, 0, st>>>(part, cpart, parts, reinterpret_cast<double*>(base + off_tot),
+                                            reinterpret_cast<long long*>(base + off_tot + 8), 0.5, parts);
         TPE_CUDA_TRY(cudaGetLastError());
     }
     // total (8 bytes), three counts (24 bytes), the stack flag (4 bytes)

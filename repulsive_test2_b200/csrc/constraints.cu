@@ -79,9 +79,10 @@ __global__ void __launch_bounds__(kBS)
 phi_part_kernel(const double* __restrict__ pos, const int2* __restrict__ edges, int32_t E,
                 int32_t V, const DevBlock* __restrict__ blocks, double* __restrict__ phi,
                 int64_t pos_stride, const int32_t* __restrict__ idx, int32_t k,
-                double* __restrict__ part) {
+                double* __restrict__ part, const int32_t* __restrict__ done) {
     const DevBlock B = blocks[blockIdx.x];
     const int32_t y = blockIdx.y, sp = blockIdx.z;
+    if (done && done[y]) return;
     pos += (idx ? idx[y] : y) * pos_stride;
     phi += (size_t)y * k;
     double* out = part + ((size_t)(y * gridDim.x + blockIdx.x) * kPhiSplit + sp) * 5;
@@ -141,20 +142,13 @@ phi_part_kernel(const double* __restrict__ pos, const int2* __restrict__ edges, 
     }
 }
 
-// One thread per (block, position set): the partials of phi_part_kernel in
-// order, then the block's rows, squared norm and scale.
-__global__ void phi_final_kernel(const double* __restrict__ pos, int32_t V,
-                                 const DevBlock* __restrict__ blocks, int32_t nblocks,
-                                 double* __restrict__ phi, double* __restrict__ ns,
-                                 int64_t pos_stride, const int32_t* __restrict__ idx, int32_t k,
-                                 int32_t n, const double* __restrict__ part) {
-    const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * nblocks) return;
-    const int32_t y = t / nblocks, b = t % nblocks;
+// Block b of position set y: the partials of phi_part_kernel in order, then the
+// block's rows, squared norm and scale.
+__device__ __forceinline__ void phi_final_block(const double* pos, int32_t V,
+                                                const DevBlock* __restrict__ blocks, int32_t nblocks,
+                                                double* phi, double* ns, int32_t y, int32_t b,
+                                                const double* __restrict__ part) {
     const DevBlock B = blocks[b];
-    pos += (idx ? idx[y] : y) * pos_stride;
-    phi += (size_t)y * k;
-    ns += (size_t)y * 2 * nblocks;
     const double* in = part + (size_t)(y * nblocks + b) * kPhiSplit * 5;
     if (B.kind == TPE_BLOCK_BARYCENTER) {
         double v[5] = {in[0], in[1], in[2], in[3], in[4]};
@@ -191,6 +185,112 @@ __global__ void phi_final_kernel(const double* __restrict__ pos, int32_t V,
         ns[2 * b] = s2;
         ns[2 * b + 1] = js_max(1.0, v);
     }
+}
+__global__ void phi_final_kernel(const double* __restrict__ pos, int32_t V,
+                                 const DevBlock* __restrict__ blocks, int32_t nblocks,
+                                 double* __restrict__ phi, double* __restrict__ ns,
+                                 int64_t pos_stride, const int32_t* __restrict__ idx, int32_t k,
+                                 int32_t n, const double* __restrict__ part) {
+    const int32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n * nblocks) return;
+    const int32_t y = t / nblocks, b = t % nblocks;
+    phi_final_block(pos + (idx ? idx[y] : y) * pos_stride, V, blocks, nblocks, phi + (size_t)y * k,
+                    ns + (size_t)y * 2 * nblocks, y, b, part);
+}
+
+// x = (L L^T)^{-1} x for n <= kProjRows, rounded as the host's solver rounds it.
+__device__ __forceinline__ void small_chol_solve(const double* L, int32_t n, double* x) {
+    for (int32_t i = 0; i < n; i++) {
+        double s = x[i];
+        for (int32_t m = 0; m < i; m++) s = __dsub_rn(s, __dmul_rn(L[i * n + m], x[m]));
+        x[i] = __ddiv_rn(s, L[i * n + i]);
+    }
+    for (int32_t i = n - 1; i >= 0; i--) {
+        double s = x[i];
+        for (int32_t m = i + 1; m < n; m++) s = __dsub_rn(s, __dmul_rn(L[m * n + i], x[m]));
+        x[i] = __ddiv_rn(s, L[i * n + i]);
+    }
+}
+
+// One warp per trial: its Phi from phi_part_kernel's partials, what the projection does next
+// (project_batch_dev's decisions, in its order and roundings) and the multipliers of the next
+// correction. state: done, ok, iters, bad, `trials` entries each.
+__global__ void proj_decide_kernel(const double* __restrict__ cur, int64_t stride, int32_t V,
+                                   const DevBlock* __restrict__ blocks, const ProjSolve p, int32_t it,
+                                   double* __restrict__ phi, double* __restrict__ ns,
+                                   double* __restrict__ coef, double* __restrict__ norm,
+                                   int32_t* __restrict__ state, int32_t trials,
+                                   const double* __restrict__ part) {
+    const int32_t a = threadIdx.x >> 5, lane = threadIdx.x & 31, k = p.k, nb = p.nblocks;
+    int32_t *done = state, *ok = state + trials, *iters = state + 2 * trials;
+    const int32_t* bad = state + 3 * trials;
+    if (done[a]) return;
+    double* ph = phi + (size_t)a * k;
+    double* nsq = ns + (size_t)a * 2 * nb;
+    if (lane < nb) phi_final_block(cur + a * stride, V, blocks, nb, ph, nsq, a, lane, part);
+    __syncwarp();
+    if (lane != 0) return;
+    if (it > 0 && bad[a]) {  // the last correction was not finite
+        iters[a] = it - 1;
+        done[a] = 1;
+        return;
+    }
+    double sq = 0.0;
+    bool finite = true, converged = true;
+    for (int32_t r = 0; r < k; r++) {
+        sq = __dadd_rn(sq, __dmul_rn(ph[r], ph[r]));
+        finite = finite && isfinite(ph[r]);
+    }
+    norm[a] = __dsqrt_rn(sq);
+    for (int32_t b = 0; b < nb; b++)
+        if (__dsqrt_rn(nsq[2 * b]) > js_max(p.tol_abs, __dmul_rn(p.tol_rel, nsq[2 * b + 1]))) {
+            converged = false;
+            break;
+        }
+    if (converged || it == p.max_iter || !finite) {
+        if (converged) ok[a] = 1;
+        iters[a] = it;  // (the cap's own count where it is reached)
+        done[a] = 1;
+        return;
+    }
+    double x[kProjRows], mu[3] = {0.0, 0.0, 0.0};
+    for (int32_t r = 0; r < k; r++) x[r] = __dadd_rn(0.0, ph[r]);
+    small_chol_solve(p.Scc, k, x);
+    if (p.trans) {
+        for (int c = 0; c < 3; c++) {
+            double s = 0.0;
+            for (int32_t r = 0; r < k; r++) s = __dadd_rn(s, __dmul_rn(p.Scu[3 * r + c], x[r]));
+            mu[c] = s;
+        }
+        small_chol_solve(p.M, 3, mu);
+        for (int32_t r = 0; r < k; r++) {
+            x[r] = __dadd_rn(0.0, ph[r]);
+            for (int c = 0; c < 3; c++) x[r] = __dsub_rn(x[r], __dmul_rn(p.Scu[3 * r + c], mu[c]));
+        }
+        small_chol_solve(p.Scc, k, x);
+    }
+    double* out = coef + (size_t)a * (k + 3);
+    for (int32_t r = 0; r < k; r++) out[r] = x[r];
+    for (int c = 0; c < 3; c++) out[k + c] = __dmul_rn(mu[c], p.su);
+}
+
+// cur[a] (interleaved V x 3) += -Y^T coef[a] - mu term for the trials that go on (the sums of
+// ycomb_part_kernel and proj_final_kernel), flagging a non-finite correction.
+__global__ void __launch_bounds__(128)
+proj_apply_kernel(const double* __restrict__ Y, int32_t k, int32_t V, const double* __restrict__ coef,
+                  double* __restrict__ cur, int32_t* __restrict__ state, int32_t trials) {
+    const int64_t m = 3 * (int64_t)V, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int32_t a = blockIdx.y;
+    if (t >= m || state[a]) return;
+    const double* cf = coef + (size_t)a * (k + 3);
+    double part = 0.0;
+    for (int32_t s = 0; s < k; s++) part -= Y[(int64_t)s * m + t] * cf[s];
+    const int c = (int)(t / V);
+    double v = 0.0 + part;
+    v -= cf[k + c];
+    if (!isfinite(v)) state[3 * trials + a] = 1;
+    double* x = cur + (int64_t)a * m + 3 * (t % V) + c;
+    *x = *x + v;
 }
 
 // Dense C (k x 3V): one thread per vertex, all blocks.
@@ -406,10 +506,31 @@ int32_t eval_constraints_batch(tpe_ctx* ctx, const double* d_pos, int64_t stride
     KernelScope ks(ctx, TPE_KGROUP_OTHER, 2);
     phi_part_kernel<<<dim3((unsigned)nblocks, (unsigned)n, kPhiSplit), kBS, 0, ctx->stream>>>(
         d_pos, ctx->d_edges.as<int2>(), ctx->E, ctx->V, ctx->con_blocks.as<DevBlock>(), d_phi,
-        stride, d_idx, k, ctx->con_part.as<double>());
+        stride, d_idx, k, ctx->con_part.as<double>(), nullptr);
     phi_final_kernel<<<(unsigned)((n * nblocks + 127) / 128), 128, 0, ctx->stream>>>(
         d_pos, ctx->V, ctx->con_blocks.as<DevBlock>(), nblocks, d_phi, d_ns, stride, d_idx, k, n,
         ctx->con_part.as<double>());
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
+}
+
+int32_t project_iterations(tpe_ctx* ctx, const ProjSolve& p, const double* d_Y, int32_t it0, int32_t it1,
+                           int32_t trials, double* d_cur, double* d_phi, double* d_ns, double* d_coef,
+                           double* d_norm, int32_t* d_state) {
+    const int64_t m = 3 * (int64_t)ctx->V;
+    TPE_TRY(ensure(ctx, ctx->con_part, sizeof(double) * (size_t)trials * p.nblocks * kPhiSplit * 5));
+    for (int32_t it = it0; it < it1; it++) {
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, it < p.max_iter ? 3 : 2);
+        phi_part_kernel<<<dim3((unsigned)p.nblocks, (unsigned)trials, kPhiSplit), kBS, 0, ctx->stream>>>(
+            d_cur, ctx->d_edges.as<int2>(), ctx->E, ctx->V, ctx->con_blocks.as<DevBlock>(), d_phi, m,
+            nullptr, p.k, ctx->con_part.as<double>(), d_state);
+        proj_decide_kernel<<<1, 32 * (unsigned)trials, 0, ctx->stream>>>(
+            d_cur, m, ctx->V, ctx->con_blocks.as<DevBlock>(), p, it, d_phi, d_ns, d_coef, d_norm, d_state,
+            trials, ctx->con_part.as<double>());
+        if (it < p.max_iter)
+            proj_apply_kernel<<<dim3((unsigned)((m + 127) / 128), (unsigned)trials), 128, 0, ctx->stream>>>(
+                d_Y, p.k, ctx->V, d_coef, d_cur, d_state, trials);
+    }
     TPE_CUDA_TRY(cudaGetLastError());
     return TPE_OK;
 }
@@ -427,7 +548,7 @@ int32_t eval_constraints(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int
     { KernelScope ks(ctx, TPE_KGROUP_OTHER, 2);
     phi_part_kernel<<<dim3((unsigned)nblocks, 1, kPhiSplit), kBS, 0, ctx->stream>>>(
         d_pos, ctx->d_edges.as<int2>(), E, V, ctx->con_blocks.as<DevBlock>(), dphi, 0, nullptr, k,
-        ctx->con_part.as<double>());
+        ctx->con_part.as<double>(), nullptr);
     phi_final_kernel<<<(unsigned)((nblocks + 127) / 128), 128, 0, ctx->stream>>>(
         d_pos, V, ctx->con_blocks.as<DevBlock>(), nblocks, dphi, dns, 0, nullptr, k, 1,
         ctx->con_part.as<double>()); }

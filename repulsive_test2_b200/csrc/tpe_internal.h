@@ -484,6 +484,18 @@ int32_t eval_constraints(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int
 int32_t eval_constraints_batch(tpe_ctx* ctx, const double* d_pos, int64_t stride,
                                const int32_t* d_idx, int32_t n, int32_t nblocks, int32_t k,
                                double* d_phi, double* d_ns);
+// The frozen projection of a small set on the device, iterations it0 .. it1 - 1 of `trials`
+// (<= kMaxTrials) trials at d_cur, nothing read back: state = {done, ok, iters, bad}[trials],
+// norm the last ||Phi||. (The Schur factors travel as a kernel argument.)
+constexpr int32_t kProjRows = 16;
+struct ProjSolve {
+    int32_t k, nblocks, max_iter, trans;
+    double tol_abs, tol_rel, su;  // su = 1 / (rho sqrt(V))
+    double Scc[kProjRows * kProjRows], Scu[kProjRows * 3], M[9];
+};
+int32_t project_iterations(tpe_ctx* ctx, const ProjSolve& p, const double* d_Y, int32_t it0, int32_t it1,
+                           int32_t trials, double* d_cur, double* d_phi, double* d_ns, double* d_coef,
+                           double* d_norm, int32_t* d_state);
 
 // ---- small device helpers (dense.cu) --------------------------------------
 int32_t interleaved_to_block(tpe_ctx* ctx, const double* d_v3, double* d_flat, int32_t V);

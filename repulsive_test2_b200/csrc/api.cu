@@ -316,9 +316,16 @@ __global__ void trace_max_kernel(const double* __restrict__ A, int32_t n, double
     }
 }
 
-__global__ void add_flat_kernel(double* __restrict__ v3, const double* __restrict__ f, int32_t V) {
+__global__ void nonfinite_flag_kernel(const double* __restrict__ x, int64_t n, int32_t* __restrict__ flag) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n && !isfinite(x[t])) *flag = 1;
+}
+
+// v3 (interleaved) += f (blocks), unless *skip.
+__global__ void add_flat_kernel(double* __restrict__ v3, const double* __restrict__ f, int32_t V,
+                                const int32_t* __restrict__ skip) {
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= V) return;
+    if (i >= V || *skip) return;
     v3[3 * i] = v3[3 * i] + f[i];
     v3[3 * i + 1] = v3[3 * i + 1] + f[V + i];
     v3[3 * i + 2] = v3[3 * i + 2] + f[2 * V + i];
@@ -697,15 +704,6 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
             if (op.large) TPE_TRY(large_set_mu(ctx, op, op.Scu.data(), op.M.data()));
         }
     }
-    if (k == 0 && flags_unread) {
-        int32_t ff[2] = {0, 0};
-        TPE_TRY(download(ctx, ff, ctx->dag_flags.ptr, sizeof(ff)));
-        TPE_TRY(chol_dag_status(ctx, ff));
-        if (ff[0]) {
-            *singular = true;
-            return TPE_OK;
-        }
-    }
     op.valid = true;
     return TPE_OK;
 }
@@ -727,8 +725,7 @@ int32_t op_build(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int32_t k, 
         TPE_TRY(launch_gradient(ctx));
     }
     TPE_TRY(ensure(ctx, ctx->con_C, sizeof(double) * (size_t)(k > 0 ? k : 1) * 3 * V));
-    std::vector<double> phi, ns;
-    TPE_TRY(eval_constraints(ctx, d_pos, nblocks, k, ctx->con_C.as<double>(), phi, ns));
+    TPE_TRY(eval_jacobian(ctx, d_pos, nblocks, k, ctx->con_C.as<double>()));
     Timer t(ctx, timings, TPE_PHASE_FACTOR);
     return op_finalize(ctx, V, k, singular, b_flat, o);
 }
@@ -798,20 +795,19 @@ int32_t op_solve_once(tpe_ctx* ctx, const double* b_flat, const double* d, doubl
             }
         }
         if (k > 0) {
+            // C w and the coordinates' sums U^T w, read together
             TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double) * ((size_t)k + 16)));
+            double* cw = ctx->tmp.as<double>();
             if (op.large)
-                TPE_TRY(large_cx(ctx, op, w, ctx->tmp.as<double>()));
+                TPE_TRY(large_cx(ctx, op, w, cw));
             else
-                TPE_TRY(gram_dots(ctx, op.C, k, w, 1, m, ctx->tmp.as<double>()));
-            TPE_TRY(download(ctx, rc.data(), ctx->tmp.as<double>(), sizeof(double) * k));
-        }
-        if (op.trans_constrained) {
+                TPE_TRY(gram_dots(ctx, op.C, k, w, 1, m, cw));
+            if (op.trans_constrained) TPE_TRY(row_sums(ctx, w, 3, V, cw + k));
+            const HostCopy cp[2] = {{rc.data(), cw, sizeof(double) * k},
+                                    {ru.data(), cw + k, op.trans_constrained ? sizeof(double) * 3 : 0}};
+            TPE_TRY(download_many(ctx, ctx->stream, cp, 2));
             const double su = 1.0 / sqrt((double)V);
-            for (int c = 0; c < 3; c++) {
-                double s = 0.0;
-                TPE_TRY(dot(ctx, V, w + (size_t)c * V, nullptr, &s));
-                ru[c] = s * su;
-            }
+            for (int c = 0; c < 3; c++) ru[c] *= su;
         }
     }
     if (d)
@@ -887,8 +883,10 @@ int32_t op_solve(tpe_ctx* ctx, const double* b_flat, const double* d, double* x_
 
 // ---- energies -------------------------------------------------------------------
 
+// (extra: a device double to read along with the energy, or null)
 int32_t energy_of(tpe_ctx* ctx, const double* d_pos, double alpha, double beta, double eps,
-                  double* out, int32_t precision = TPE_PRECISION_FP64) {
+                  double* out, int32_t precision = TPE_PRECISION_FP64, const double* d_extra = nullptr,
+                  double* extra = nullptr) {
     TPE_TRY(ensure(ctx, ctx->scalars, sizeof(double) * 600));
     double* de = ctx->scalars.as<double>() + 520;
     if (precision == TPE_PRECISION_MIXED) {
@@ -898,15 +896,16 @@ int32_t energy_of(tpe_ctx* ctx, const double* d_pos, double alpha, double beta, 
         TPE_TRY(edge_prep(ctx, d_pos, 1, eps, alpha));
         TPE_TRY(energy_fp64(ctx, 1, alpha, beta, eps, de));
     }
-    return download(ctx, out, de, sizeof(double));
+    const HostCopy cp[2] = {{out, de, sizeof(double)}, {extra, d_extra, d_extra ? sizeof(double) : 0}};
+    return download_many(ctx, ctx->stream, cp, 2);
 }
 
 int32_t objective(tpe_ctx* ctx, const double* d_pos, const tpe_step_opts* o, bool pen,
-                  double* out, double* timings) {
+                  double* out, double* timings, const double* d_extra = nullptr, double* extra = nullptr) {
     double e = 0.0;
     {
         Timer t(ctx, timings, TPE_PHASE_ENERGY);
-        TPE_TRY(energy_of(ctx, d_pos, o->alpha, o->beta, o->epsilon, &e));
+        TPE_TRY(energy_of(ctx, d_pos, o->alpha, o->beta, o->epsilon, &e, TPE_PRECISION_FP64, d_extra, extra));
     }
     if (pen) {
         double pe = 0.0;
@@ -973,8 +972,16 @@ int32_t project_dev(tpe_ctx* ctx, const double* d_start, const SetInfo& S, const
     *ok = 0;
     *iters = o->proj_max_iter;
     std::vector<double> phi, ns, lam;
+    TPE_TRY(ensure(ctx, ctx->status, sizeof(int32_t) * 4));
+    int32_t* d_bad = ctx->status.as<int32_t>();
+    TPE_CUDA_TRY(cudaMemsetAsync(d_bad, 0, sizeof(int32_t), ctx->stream));
     for (int32_t it = 0; it <= o->proj_max_iter; it++) {
-        TPE_TRY(eval_constraints(ctx, d_cur, S.nblocks, S.k, nullptr, phi, ns));
+        int32_t bad = 0;  // the last correction was not finite (and was not applied)
+        TPE_TRY(eval_constraints(ctx, d_cur, S.nblocks, S.k, nullptr, phi, ns, d_bad, &bad));
+        if (bad) {
+            *iters = it - 1;
+            break;
+        }
         double sq = 0.0;
         for (double v : phi) sq += v * v;
         finalPhiNorm = sqrt(sq);
@@ -1012,14 +1019,9 @@ int32_t project_dev(tpe_ctx* ctx, const double* d_start, const SetInfo& S, const
             Timer t(ctx, timings, TPE_PHASE_SADDLE);
             TPE_TRY(op_solve(ctx, nullptr, negphi.data(), x, lam, nullptr));
         }
-        int64_t bad = 0;
-        TPE_TRY(count_nonfinite(ctx, m, x, &bad));
-        if (bad) {
-            *iters = it;
-            break;
-        }
-        { KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
-        add_flat_kernel<<<(V + 255) / 256, 256, 0, ctx->stream>>>(d_cur, x, V); }
+        { KernelScope ks(ctx, TPE_KGROUP_OTHER, 2);
+        nonfinite_flag_kernel<<<(unsigned)((m + 255) / 256), 256, 0, ctx->stream>>>(x, m, d_bad);
+        add_flat_kernel<<<(V + 255) / 256, 256, 0, ctx->stream>>>(d_cur, x, V, d_bad); }
         TPE_CUDA_TRY(cudaGetLastError());
     }
     *phi_norm = finalPhiNorm;
@@ -1204,7 +1206,7 @@ void stats_reset(tpe_step_stats* st) {
 // The accepted (or echoed) vertices end in d_out.
 int32_t line_search_dev(tpe_ctx* ctx, const double* d_pos, const double* d_dE, const double* d_g,
                         const SetInfo& S, const tpe_step_opts* o, bool frozen, double* d_out,
-                        tpe_step_stats* st, double* timings) {
+                        tpe_step_stats* st, double* timings, const double* norm = nullptr) {
     Timer tls(ctx, timings, TPE_PHASE_LINESEARCH);
     const int32_t V = ctx->V;
     const int64_t m = 3 * (int64_t)V;
@@ -1221,7 +1223,10 @@ int32_t line_search_dev(tpe_ctx* ctx, const double* d_pos, const double* d_dE, c
     TPE_CUDA_TRY(cudaMemcpyAsync(d_out, d_pos, sizeof(double) * m, cudaMemcpyDeviceToDevice,
                                  ctx->stream));
     double gradNorm = 0.0;
-    TPE_TRY(l2_curve_norm(ctx, d_g, d_pos, &gradNorm));
+    if (norm)
+        gradNorm = *norm;  // d_g's, already known
+    else
+        TPE_TRY(l2_curve_norm(ctx, d_g, d_pos, &gradNorm));
     if (!isfinite(gradNorm) || gradNorm <= 0) {
         st->reason = TPE_REASON_ZERO_OR_NONFINITE_GRADIENT_NORM;
         st->projection_iterations = 0;
@@ -1278,11 +1283,13 @@ int32_t line_search_dev(tpe_ctx* ctx, const double* d_pos, const double* d_dE, c
             }
             for (int32_t a = 0; a < nk; a++) {
                 double* ca = bcur + (size_t)a * m;
-                int64_t bad = 0;
-                if (okv[a]) TPE_TRY(count_nonfinite(ctx, m, ca, &bad));
-                if (okv[a] && !bad) {
-                    double e1 = 0.0;
-                    TPE_TRY(objective(ctx, ca, o, pen, &e1, timings));
+                double e1 = 0.0, bad = 0.0;  // (bad: non-finite coordinates)
+                if (okv[a]) {
+                    const double* d_bad = nullptr;
+                    TPE_TRY(count_nonfinite(ctx, m, ca, &d_bad));
+                    TPE_TRY(objective(ctx, ca, o, pen, &e1, timings, d_bad, &bad));
+                }
+                if (okv[a] && bad == 0.0) {
                     trials++;
                     if (isfinite(e1) && e1 <= e0 - o->c1 * taus[a] * slope) {
                         st->accepted = 1;
@@ -1317,11 +1324,13 @@ int32_t line_search_dev(tpe_ctx* ctx, const double* d_pos, const double* d_dE, c
             Timer tp(ctx, timings, TPE_PHASE_PROJECTION);
             TPE_TRY(project_dev(ctx, raw, S, o, frozen, cur, &ok, &iters, &phiNorm, timings));
         }
-        int64_t bad = 0;
-        TPE_TRY(count_nonfinite(ctx, m, cur, &bad));
-        if (ok && !bad) {
-            double e1 = 0.0;
-            TPE_TRY(objective(ctx, cur, o, pen, &e1, timings));
+        double e1 = 0.0, bad = 0.0;  // (bad: non-finite coordinates)
+        if (ok) {
+            const double* d_bad = nullptr;
+            TPE_TRY(count_nonfinite(ctx, m, cur, &d_bad));
+            TPE_TRY(objective(ctx, cur, o, pen, &e1, timings, d_bad, &bad));
+        }
+        if (ok && bad == 0.0) {
             trials++;
             if (isfinite(e1) && e1 <= e0 - o->c1 * tau * slope) {
                 st->accepted = 1;
@@ -1966,7 +1975,7 @@ int32_t step_impl(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, cons
     tpe_step_stats ls;
     stats_reset(&ls);
     TPE_TRY(line_search_dev(ctx, P, dE, g, S, o, o->projection_mode == TPE_PROJECTION_FROZEN, out,
-                            &ls, timings));
+                            &ls, timings, &gn));
     st->energy = ls.energy;
     st->energy_before = ls.energy_before;
     st->accepted = ls.accepted;

@@ -535,8 +535,21 @@ int32_t project_iterations(tpe_ctx* ctx, const ProjSolve& p, const double* d_Y, 
     return TPE_OK;
 }
 
+int32_t eval_jacobian(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int32_t k, double* d_C) {
+    if (nblocks == 0) return TPE_OK;
+    const int32_t V = ctx->V;
+    TPE_CUDA_TRY(cudaMemsetAsync(d_C, 0, sizeof(double) * (size_t)k * 3 * V, ctx->stream));
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    jacobian_kernel<<<(V + 127) / 128, 128, 0, ctx->stream>>>(
+        d_pos, ctx->d_edges.as<int2>(), ctx->d_inc_off.as<int32_t>(), ctx->d_inc.as<int32_t>(),
+        V, ctx->con_blocks.as<DevBlock>(), nblocks, d_C);
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
+}
+
 int32_t eval_constraints(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int32_t k,
-                         double* d_C, std::vector<double>& phi, std::vector<double>& ns) {
+                         double* d_C, std::vector<double>& phi, std::vector<double>& ns,
+                         const int32_t* d_flag, int32_t* flag) {
     const int32_t V = ctx->V, E = ctx->E;
     phi.assign((size_t)k, 0.0);
     ns.assign((size_t)2 * nblocks, 0.0);
@@ -553,17 +566,11 @@ int32_t eval_constraints(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int
         d_pos, V, ctx->con_blocks.as<DevBlock>(), nblocks, dphi, dns, 0, nullptr, k, 1,
         ctx->con_part.as<double>()); }
     TPE_CUDA_TRY(cudaGetLastError());
-    if (d_C) {
-        TPE_CUDA_TRY(cudaMemsetAsync(d_C, 0, sizeof(double) * (size_t)k * 3 * V, ctx->stream));
-        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
-        jacobian_kernel<<<(V + 127) / 128, 128, 0, ctx->stream>>>(
-            d_pos, ctx->d_edges.as<int2>(), ctx->d_inc_off.as<int32_t>(), ctx->d_inc.as<int32_t>(),
-            V, ctx->con_blocks.as<DevBlock>(), nblocks, d_C);
-        TPE_CUDA_TRY(cudaGetLastError());
-    }
-    const HostCopy cp[2] = {{phi.data(), dphi, k > 0 ? sizeof(double) * k : 0},
-                            {ns.data(), dns, sizeof(double) * 2 * nblocks}};
-    return download_many(ctx, ctx->stream, cp, 2);
+    if (d_C) TPE_TRY(eval_jacobian(ctx, d_pos, nblocks, k, d_C));
+    const HostCopy cp[3] = {{phi.data(), dphi, k > 0 ? sizeof(double) * k : 0},
+                            {ns.data(), dns, sizeof(double) * 2 * nblocks},
+                            {flag, d_flag, flag ? sizeof(int32_t) : 0}};
+    return download_many(ctx, ctx->stream, cp, 3);
 }
 
 static PenW resolve(const tpe_penalties* p, bool* active) {

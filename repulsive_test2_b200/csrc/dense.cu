@@ -266,6 +266,16 @@ sum_kernel(const double* __restrict__ part, int32_t n, double* __restrict__ out)
     if (threadIdx.x == 0) *out = s;
 }
 
+// out[r] = the sum of row r (n entries), one block a row.
+__global__ void __launch_bounds__(256)
+row_sums_kernel(const double* __restrict__ x, int32_t n, double* __restrict__ out) {
+    const double* row = x + (size_t)blockIdx.x * n;
+    double s = 0.0;
+    for (int32_t t = threadIdx.x; t < n; t += blockDim.x) s += row[t];
+    s = block_sum<256>(s);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
+}
+
 // Per-edge l2CurveNorm terms (lineSearch.ts:53-75).
 __global__ void l2_terms_kernel(const double* __restrict__ vals, const double* __restrict__ pos,
                                 const int2* __restrict__ edges, int32_t E,
@@ -421,6 +431,13 @@ int32_t gram_dots(tpe_ctx* ctx, const double* X, int32_t nx, const double* Y, in
     return TPE_OK;
 }
 
+int32_t row_sums(tpe_ctx* ctx, const double* x, int32_t rows, int32_t n, double* d_out) {
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+    row_sums_kernel<<<rows, 256, 0, ctx->stream>>>(x, n, d_out);
+    TPE_CUDA_TRY(cudaGetLastError());
+    return TPE_OK;
+}
+
 int32_t shift_copy(tpe_ctx* ctx, const double* d_A, double* d_L, int32_t n, double shift) {
     const int64_t nn = (int64_t)n * n;
     KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
@@ -474,15 +491,15 @@ int32_t dot(tpe_ctx* ctx, int64_t n, const double* x, const double* y, double* o
     return reduce_to_host(ctx, ctx->scalars.as<double>(), g, out);
 }
 
-int32_t count_nonfinite(tpe_ctx* ctx, int64_t n, const double* x, int64_t* out) {
+int32_t count_nonfinite(tpe_ctx* ctx, int64_t n, const double* x, const double** d_out) {
     const int32_t g = 256;
-    TPE_TRY(ensure(ctx, ctx->scalars, sizeof(double) * (g + 8)));
-    { KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
-    nonfinite_partial_kernel<<<g, 256, 0, ctx->stream>>>(n, x, ctx->scalars.as<double>()); }
+    TPE_TRY(ensure(ctx, ctx->scalars, sizeof(double) * 600));
+    double* part = ctx->scalars.as<double>();
+    KernelScope ks(ctx, TPE_KGROUP_OTHER, 2);
+    nonfinite_partial_kernel<<<g, 256, 0, ctx->stream>>>(n, x, part);
+    sum_kernel<<<1, 256, 0, ctx->stream>>>(part, g, part + g);
     TPE_CUDA_TRY(cudaGetLastError());
-    double d = 0.0;
-    TPE_TRY(reduce_to_host(ctx, ctx->scalars.as<double>(), g, &d));
-    *out = (int64_t)d;
+    *d_out = part + g;
     return TPE_OK;
 }
 
@@ -519,8 +536,7 @@ int32_t combine_solution(tpe_ctx* ctx, const double* d_w, const double* d_Y, int
     ycomb_part_kernel<<<dim3(grid_for(m, 256), nks), 256, 0, ctx->stream>>>(d_Y, k, m, dc, 1, part);
     combine_final_kernel<<<grid_for(m, 256), 256, 0, ctx->stream>>>(d_w, part, nks, k, dc, V, d_x);
     TPE_CUDA_TRY(cudaGetLastError());
-    TPE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return TPE_OK;
+    return TPE_OK;  // (a copy from pageable memory returns once the data is staged)
 }
 
 int32_t project_update(tpe_ctx* ctx, const double* d_Y, int32_t k, int32_t V, const double* d_coef,
@@ -567,26 +583,30 @@ int32_t saddle_residual(tpe_ctx* ctx, const double* d_A, int32_t V, const double
                                                         rr, rb, d_res_top);
     }
     TPE_CUDA_TRY(cudaGetLastError());
-    double top_r = 0.0, top_b = 0.0;
-    TPE_TRY(dot(ctx, V, rr, nullptr, &top_r));
-    TPE_TRY(dot(ctx, V, rb, nullptr, &top_b));
-    // bottom rows C x - rhs_bottom
-    double bot_r = 0.0, bot_b = 0.0;
+    // the two norms and the bottom rows C x - rhs_bottom, read together
+    double* cx = ctx->tmp.as<double>() + 2 * V;
+    double* tops = cx + k;
+    {
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+        row_sums_kernel<<<2, 256, 0, ctx->stream>>>(rr, V, tops);
+        TPE_CUDA_TRY(cudaGetLastError());
+    }
     if (k > 0) {
-        double* cx = ctx->tmp.as<double>() + 2 * V;
         if (large)
             TPE_TRY(large_cx(ctx, *large, d_x, cx));
         else
             TPE_TRY(gram_dots(ctx, d_C, k, d_x, 1, 3 * (int64_t)V, cx));
-        std::vector<double> h((size_t)k);
-        TPE_TRY(download_on(ctx, ctx->stream, h.data(), cx, sizeof(double) * k));
-        for (int32_t r = 0; r < k; r++) {
-            const double b = rhs_bottom ? rhs_bottom[r] : 0.0;
-            const double d = h[r] - b;
-            if (res_bottom) res_bottom[r] = -d;
-            bot_r += d * d;
-            bot_b += b * b;
-        }
+    }
+    std::vector<double> h((size_t)k + 2);
+    TPE_TRY(download_on(ctx, ctx->stream, h.data(), cx, sizeof(double) * ((size_t)k + 2)));
+    const double top_r = h[(size_t)k], top_b = h[(size_t)k + 1];
+    double bot_r = 0.0, bot_b = 0.0;
+    for (int32_t r = 0; r < k; r++) {
+        const double b = rhs_bottom ? rhs_bottom[r] : 0.0;
+        const double d = h[r] - b;
+        if (res_bottom) res_bottom[r] = -d;
+        bot_r += d * d;
+        bot_b += b * b;
     }
     const double rn = sqrt(top_r + bot_r), bn = sqrt(top_b + bot_b);
     *out = rn / (bn > 1.0 ? bn : 1.0);

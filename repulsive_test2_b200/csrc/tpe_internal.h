@@ -477,7 +477,10 @@ int32_t upload_set(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, int
 // Phi (k) and per-block {norm^2, scale} (2*nblocks) into host arrays; dense C
 // (k x 3V, device) when d_C != nullptr.
 int32_t eval_constraints(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int32_t k,
-                         double* d_C, std::vector<double>& phi, std::vector<double>& norm_scale);
+                         double* d_C, std::vector<double>& phi, std::vector<double>& norm_scale,
+                         const int32_t* d_flag = nullptr, int32_t* flag = nullptr);
+// The Jacobian alone (nothing read back).
+int32_t eval_jacobian(tpe_ctx* ctx, const double* d_pos, int32_t nblocks, int32_t k, double* d_C);
 
 // Phi (d_phi: n x k) and per-block {norm^2, scale} (d_ns: n x 2 nblocks), on the
 // device, for the position sets pos + idx[q] * stride, q < n (idx on the device).
@@ -504,8 +507,10 @@ int32_t block_to_interleaved(tpe_ctx* ctx, const double* d_flat, double* d_v3, i
 int32_t axpby(tpe_ctx* ctx, int64_t n, double a, const double* x, double b, double* y);
 // host result: sum(x*y) over n (deterministic)
 int32_t dot(tpe_ctx* ctx, int64_t n, const double* x, const double* y, double* out);
-// host result: number of non-finite entries in x[n]
-int32_t count_nonfinite(tpe_ctx* ctx, int64_t n, const double* x, int64_t* out);
+// *d_out: the number (device, in ctx->scalars) of non-finite entries in x[n]
+int32_t count_nonfinite(tpe_ctx* ctx, int64_t n, const double* x, const double** d_out);
+// d_out[r] = the sum of row r of x (n entries each)
+int32_t row_sums(tpe_ctx* ctx, const double* x, int32_t rows, int32_t n, double* d_out);
 // l2CurveNorm of interleaved values at interleaved positions (host result)
 int32_t l2_curve_norm(tpe_ctx* ctx, const double* d_vals, const double* d_pos, double* out);
 // x_flat(3V) = w - sum_s Y[s] * lam[s] - U mu / rho ; lam/mu are host arrays

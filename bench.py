@@ -35,12 +35,11 @@ sys.path.insert(0, HERE)
 METRIC = "descent steps/s at V=8192: mixed+batched vs plain FP64 GPU, at <=1e-8 rel energy err"
 
 
-# Algorithmic flops per unordered disjoint edge pair (both orders), counted from
-# the kernels' arithmetic with +, -, *, /, sqrt and rsqrt as one flop each and
-# integer powers as their multiplies: the energy (4 endpoint pairs x 60 + 9),
-# the adjoint gradient with its energy (4 x 163 + 141) and the Gram pair
-# weights with their stencil (4 x 63 + 26).
-FLOP_PER_UNORDERED_PAIR = {"energy": 249, "gradient": 793, "pair_weights": 278}
+# FP64 instructions per unordered disjoint edge pair (both orders), two flops each as the
+# pipe's rate counts them: an (edge, vertex) pair takes 52 for the energy and 104 for the
+# gradient with its energy (two such pairs per pair of edges), the Gram pair weights with
+# their stencil 100.
+FLOP_PER_UNORDERED_PAIR = {"energy": 208, "gradient": 416, "pair_weights": 200}
 
 
 def max_over_ranks(ms, dist, device):
@@ -204,8 +203,8 @@ def extras(args):
     # Barnes-Hut energy (the hierarchical path) against the exact GPU energy on a
     # smooth curve far larger than the step's V
     bh = {"workload": "closed trefoil (the stage-2 oracle's check curve), theta 0.5, theta_t 0.75, leaf 8; "
-                      "wall time of the public calls (tree and block lists built on the host, traversal and "
-                      "products on the device); bct_high: the high-order kernel product against theta = 0"}
+                      "wall time of the public calls (the energy's tree built on the device, the products' tree "
+                      "and block lists on the host); bct_high: the high-order kernel product against theta = 0"}
     for n in (32768, 131072):
         tt = np.linspace(0.0, 2.0 * np.pi, n, endpoint=False)
         tv = np.stack([np.sin(tt) + 2.0 * np.sin(2.0 * tt), np.cos(tt) - 2.0 * np.cos(2.0 * tt),
@@ -610,7 +609,7 @@ def run_repulsive(args):
     groups = abi.KGROUPS
     ms_g = {g: kms[i] for i, g in enumerate(groups)}
     nl = {g: kl[i] for i, g in enumerate(groups)}
-    # The gradient runs beside the factorization on two fifths of the SMs (its group
+    # The gradient runs beside the factorization on a quarter of the SMs (its group
     # time is the stream3 span, not a full-GPU kernel time): the roofline is taken
     # for the dominant group on the main stream, the gradient reported apart.
     dom = max((g for g in ms_g if g != "gradient" or args.precision != "mixed"), key=lambda g: ms_g[g])
@@ -621,7 +620,7 @@ def run_repulsive(args):
     if dom in ("gradient", "energy", "pair_weights"):
         fl = FLOP_PER_UNORDERED_PAIR[dom]
         per_launch_flop = P / 2 * fl
-        n_launch = max(1, nl[dom] // {"gradient": 2, "energy": 2, "pair_weights": 1}[dom])
+        n_launch = max(1, nl[dom] // {"gradient": 3, "energy": 2, "pair_weights": 1}[dom])
         roof = {"bound": "tensor", "unit": "TFLOP/s", "peak": fp64_peak,
                 "peak_source": "cuBLAS FP64 GEMM measured in this run (the FP64 pipe; MEASURED_PEAKS.json "
                                "lists HBM and bf16 only)",
@@ -656,8 +655,8 @@ def run_repulsive(args):
     roof["group_ms"] = {g: round(ms_g[g], 3) for g in groups}
     if args.precision == "mixed" and nl["gradient"] > 0:
         nsm = torch.cuda.get_device_properties(dev).multi_processor_count
-        gsm = int(os.environ.get("TPE_GRAD_SMS", nsm * 2 // 5))
-        g_ach = P / 2 * FLOP_PER_UNORDERED_PAIR["gradient"] * max(1, nl["gradient"] // 2) / (ms_g["gradient"] * 1e-3) / 1e12
+        gsm = int(os.environ.get("TPE_GRAD_SMS", nsm // 4))
+        g_ach = P / 2 * FLOP_PER_UNORDERED_PAIR["gradient"] * max(1, nl["gradient"] // 3) / (ms_g["gradient"] * 1e-3) / 1e12
         roof["concurrent_gradient"] = {
             "sms": gsm, "achieved": g_ach, "peak_on_its_sms": fp64_peak * gsm / nsm,
             "frac": g_ach / (fp64_peak * gsm / nsm) if fp64_peak else None, "unit": "TFLOP/s",

@@ -18,11 +18,12 @@
 //      S y = D b in FP64, x = D y. Z and W are copied once to plain FP32
 //      (hi + lo is exact in FP32) and every product of the CG -- S p with the
 //      FP64 A, Z r and W u with the FP32 copies -- runs in FP64 arithmetic on
-//      the FP64 tensor cores (mrhs_dmma_kernel).
+//      the FP64 tensor cores (mrhs_t_kernel).
 // At V=8192 (kappa(A_rho) ~ 1e10, kappa(S) ~ 1e8) plain iterative refinement
 // with an FP32 factor diverges (kappa(S) * u32 > 1); CG with it reaches a 1e-13
 // relative residual in about 7 iterations. The FP64 path remains the fallback
-// whenever the FP32 factorization breaks down or CG does not converge.
+// whenever the FP32 factorization breaks down or CG does not converge, and the
+// first choice up to kMixedDirect vertices.
 #include <math.h>
 
 #include <algorithm>

@@ -22,8 +22,8 @@
 //
 // Measured against that (us): factor, order 777: 1380 -> 242, 2048: 3190 -> 575,
 // 4096: 6750 -> 1330, 8192: 7100; with the explicit inverse, 777: 2220
-// -> 252, 2500: 7200 -> 1010, 8192: 38500 -> 20800; two triangular solves of 15
-// right-hand sides, 777: 345 -> 132, 2048: 844 -> 342. Bound: to about 3500 rows
+// -> 252, 2500: 7200 -> 1010, 8192: 38500 -> 20800; one triangular solve of 15
+// right-hand sides, 777: 172 -> 69, 2048: 422 -> 154. Bound: to about 3500 rows
 // the chain (per 64 columns 9.7 us for the diagonal block, 8 for its two products,
 // loads and flags), above it the workers' products (2.4 us each at the FP64
 // tensor rate of one SM).
@@ -754,7 +754,9 @@ __global__ void __launch_bounds__(kThr, 2) chol_dag_kernel(const Dag g) {
 // take their columns from a ticket in solving order, so each waits only for
 // blocks that run; the tile of L for the next step is in shared memory before the
 // step's vectors are ready. Bound: the chain of columns (flag, vectors, two small
-// products, store). A wait that runs out sets *err and leaves NaN.
+// products, store): 4.7 us each. What does not hang on it is read before the waits (the
+// inverse, the block's own right-hand sides): order 2048 175 -> 154 us, 8192 790 -> 594.
+// A wait that runs out sets *err and leaves NaN.
 constexpr int kMaxG = 4;  // groups of 16 right-hand sides
 
 template <bool NT>  // C[r][c] += sum_m A[r][m] B[c][m] (NT) or A[r][m] B[m][c]; warp = 8 columns
@@ -794,13 +796,20 @@ tri_dag_kernel(const double* __restrict__ L, const double* __restrict__ Linv, in
         else  // rows of block k, columns of block j; rows past n meet zero vectors
             load_tile<kAl>(tile[q & 1], Rows{L + (int64_t)k * NB * n, n, min(NB, n - k * NB)}, j * NB, n);
     };
-    for (int e = threadIdx.x; e < NB * NB; e += kThr)
-        z[(e >> 6) * kTP + (e & 63)] = Linv[(int64_t)j * NB * NB + e];
+    load_tile<true>(z, Rows{Linv + (int64_t)j * NB * NB, NB, NB}, 0, NB);
     if (t > 0) fetch(0);
     cp_commit();
-    double acc[2 * kMaxG][2];
+    // (the block's own right-hand sides are read before the waits, too)
+    double acc[2 * kMaxG][2], own[2 * kMaxG][2];
 #pragma unroll
-    for (int q = 0; q < 2 * kMaxG; q++) acc[q][0] = acc[q][1] = 0.0;
+    for (int q = 0; q < 2 * kMaxG; q++) {
+        acc[q][0] = acc[q][1] = 0.0;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int r = 8 * q + (lane >> 2), c = 8 * w + 2 * (lane & 3) + e;
+            own[q][e] = q < 2 * ng && r < nr && c < s ? B[(int64_t)r * n + j * NB + c] : 0.0;
+        }
+    }
     bool bad = false;
     for (int32_t q = 0; q < t; q++) {
         if (q + 1 < t) fetch(q + 1);
@@ -835,7 +844,7 @@ tri_dag_kernel(const double* __restrict__ L, const double* __restrict__ Linv, in
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const int r = 8 * q + (lane >> 2), c = 8 * w + 2 * (lane & 3) + e;
-                v[r * kTP + c] = r < nr && c < s ? B[(int64_t)r * n + j * NB + c] - acc[q][e] : 0.0;
+                v[r * kTP + c] = r < nr && c < s ? own[q][e] - acc[q][e] : 0.0;
                 acc[q][e] = 0.0;
             }
     __syncthreads();

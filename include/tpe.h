@@ -163,6 +163,13 @@ void tpe_destroy(tpe_ctx* ctx);
 /* Message for the last non-OK status returned on this context. */
 const char* tpe_last_error(const tpe_ctx* ctx);
 
+/* Settings of one context for checks of the library itself (a program needs none of
+ * them); a negative value restores the default.
+ * TPE_TUNE_FAIL_ALLOC: the value-th growth of a device buffer from here on fails, as if
+ *   the device were out of memory (0: none, the default). */
+enum { TPE_TUNE_FAIL_ALLOC = 0 };
+int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value);
+
 /* ---- topology ------------------------------------------------------------- */
 /* Replaces calculateDisjointPairs (src/core/tangentPointEnergy.ts:33-47): the
  * ordered disjoint-pair lists are never materialised; disjointness is tested

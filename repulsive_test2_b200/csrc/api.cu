@@ -102,7 +102,9 @@ int32_t ensure(tpe_ctx* ctx, DevBuf& b, size_t bytes) {
         b.bytes = 0;
     }
     const size_t want = bytes + bytes / 8;
-    cudaError_t e = cudaMalloc(&b.ptr, want);
+    // (fail_alloc: tpe_tune's stand-in for an allocation that fails)
+    const bool fail = ctx->fail_alloc > 0 && --ctx->fail_alloc == 0;
+    cudaError_t e = fail ? cudaErrorMemoryAllocation : cudaMalloc(&b.ptr, want);
     if (e != cudaSuccess) {
         b.ptr = nullptr;
         set_error(ctx, TPE_ERR_OUT_OF_MEMORY,
@@ -1511,6 +1513,16 @@ void tpe_destroy(tpe_ctx* ctx) {
 
 const char* tpe_last_error(const tpe_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 
+int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value) {
+    return guarded(ctx, [&]() -> int32_t {
+        if (!ctx) return TPE_ERR_BAD_ARG;
+        switch (what) {
+            case TPE_TUNE_FAIL_ALLOC: ctx->fail_alloc = std::max<int64_t>(value, 0); return TPE_OK;
+            default: set_error(ctx, TPE_ERR_BAD_ARG, "tpe_tune: unknown setting"); return TPE_ERR_BAD_ARG;
+        }
+    });
+}
+
 int32_t tpe_set_topology(tpe_ctx* ctx, const int32_t* edges, int32_t E, int32_t V) {
     return guarded(ctx, [&]() -> int32_t {
         if (!ctx) return TPE_ERR_BAD_ARG;
@@ -1855,10 +1867,22 @@ int32_t tpe_line_search_step(tpe_ctx* ctx, const double* xyz, const double* dE,
 namespace tpe {
 namespace {
 
+// However the step ends, no gradient stays pending: a later build would take its edge
+// records for those of its own positions (op_build) and read penalties that are gone.
+struct GradientGuard {
+    tpe_ctx* ctx;
+    ~GradientGuard() {
+        if (!ctx->grad_pending) return;
+        ctx->grad_pending = ctx->grad_unlaunched = false;
+        cudaStreamSynchronize(ctx->stream3);
+    }
+};
+
 // sobolevStepSet with the input vertices already in ctx->pos; the result is
 // left in *d_result (device, V x 3).
 int32_t step_impl(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, const tpe_step_opts* o,
                   tpe_step_stats* st, double* timings, double* descent_field, const double** d_result) {
+    const GradientGuard guard{ctx};
     const int32_t V = ctx->V;
     const size_t m = 3 * (size_t)V;
     SetInfo S;

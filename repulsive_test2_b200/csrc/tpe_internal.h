@@ -209,6 +209,9 @@ struct tpe_ctx {
     size_t h_stage_bytes = 0;
     std::vector<double> h_tmp;
 
+    // settings of tpe_tune
+    int64_t fail_alloc = 0;  // the growth of a device buffer that fails (1: the next one)
+
     // instrumentation: kernel launch count and per-group CUDA-event timing
     int64_t launches = 0;
     bool profiling = false;

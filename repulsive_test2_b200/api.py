@@ -73,6 +73,7 @@ class Context:
         V = int(np.asarray(vertices).reshape(-1, 3).shape[0])
         key = e.tobytes() + V.to_bytes(8, "little")
         if key != self._edges_key:
+            self._edges_key = None  # (a call that fails leaves the context without one)
             self.check(self.lib.tpe_set_topology(self.ptr, e.ctypes.data_as(abi.ip), len(e), V),
                        "tpe_set_topology")
             self._edges_key = key

@@ -1536,6 +1536,10 @@ int32_t tpe_set_topology(tpe_ctx* ctx, const int32_t* edges, int32_t E, int32_t 
                 return TPE_ERR_BAD_ARG;
             }
         TPE_CUDA_TRY(cudaSetDevice(ctx->device));
+        // (none until every list of the new one is in place)
+        ctx->has_topology = false;
+        ctx->ev_state = 0;
+        ctx->op.valid = false;
         ctx->V = V;
         ctx->E = E;
         ctx->h_edges.assign(edges, edges + 2 * (size_t)E);
@@ -1557,8 +1561,6 @@ int32_t tpe_set_topology(tpe_ctx* ctx, const int32_t* edges, int32_t E, int32_t 
         TPE_TRY(upload(ctx, ctx->d_inc, ctx->h_inc.data(), sizeof(int32_t) * 2 * (size_t)(E > 0 ? E : 1)));
         TPE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
         ctx->has_topology = true;
-        ctx->ev_state = 0;
-        ctx->op.valid = false;
         return TPE_OK;
     });
 }

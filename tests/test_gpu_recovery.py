@@ -47,23 +47,17 @@ def test_a_topology_that_failed_is_none(monkeypatch):
     """No call runs on the sizes of a topology whose lists are not in place."""
     v, e = F.trefoil(40, jitter=0.01, seed=1)
     w, f = F.trefoil(700, jitter=0.01, seed=2)
-    ctx = T.Context()
-    monkeypatch.setattr(T, "_CTX", ctx)
-    small, large = T.calculateEnergy(v, e), None
-    for n in range(1, 12):
+    small, large = T.calculateEnergy(v, e), T.calculateEnergy(w, f)
+    for n in range(1, 4):  # the topology's three lists
+        ctx = T.Context()
+        monkeypatch.setattr(T, "_CTX", ctx)
         assert T.calculateEnergy(v, e) == small
         ctx.lib.tpe_tune(ctx.ptr, abi.TUNE_FAIL_ALLOC, n)
-        try:
-            large = T.calculateEnergy(w, f)
-            break
-        except T.TpeError:
-            if n <= 3:  # one of the topology's own lists
-                en, p = np.zeros(1), abi.tpe_params(3.0, 6.0, 1e-10)
-                rc = ctx.lib.tpe_energy(ctx.ptr, T._dp(np.zeros((700, 3))), p, T._dp(en))
-                assert rc == abi.TPE_ERR_NO_TOPOLOGY
-        finally:
-            ctx.lib.tpe_tune(ctx.ptr, abi.TUNE_FAIL_ALLOC, 0)
-    assert n > 3 and large is not None
-    ctx.close()
-    monkeypatch.setattr(T, "_CTX", None)
-    assert T.calculateEnergy(w, f) == large
+        with pytest.raises(T.TpeError):
+            T.calculateEnergy(w, f)
+        en = np.zeros(1)
+        rc = ctx.lib.tpe_energy(ctx.ptr, T._dp(np.zeros((700, 3))), abi.tpe_params(3.0, 6.0, 1e-10), T._dp(en))
+        assert rc == abi.TPE_ERR_NO_TOPOLOGY
+        assert T.calculateEnergy(v, e) == small
+        assert T.calculateEnergy(w, f) == large
+        ctx.close()

@@ -37,6 +37,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "pair_math.cuh"
 #include "tpe_internal.h"
@@ -47,6 +48,7 @@ namespace {
 constexpr int kW = 128;      // threads of a worker
 constexpr int kTile = 128;   // vertices staged at a time
 constexpr int kWorkers = 3;  // workers per block of the SM-bounded form
+constexpr int kGroup = kTile / 8;  // most chunks of one energy item (ev_split)
 constexpr int kAcc = 7;      // per (chunk, edge): force on both endpoints, sum of M N (G1 + G2)
 
 // The curve's records and the topology lists every kernel here reads.
@@ -146,7 +148,7 @@ __device__ __forceinline__ void sub_cross(V3& f, const V3& a, const V3& b) {
 struct EvSmem {
     double4 sv[kTile];                 // x, y, z, m
     double acc[kW / 32][kTile][4];     // per warp: force on the swept vertex, sum of l_I^(1-a) N (G1 + G2)
-    double red[kW / 32];
+    double red[kGroup][kW / 32];       // per chunk of the group and warp
     int next;
 };
 
@@ -190,11 +192,11 @@ __device__ __forceinline__ double near_length(const EvTopo& t, const double4* __
     return m;
 }
 
-// Sweeps the vertices [vb, vb + n) (n <= kTile, staged in sm.sv) for the
+// Sweeps the vertices [vb, vb + n) (n <= kTile, staged from sm.sv[s0] on) for the
 // thread's R edges. CHAIN: the edges run head to tail (R + 1 vertices), else
 // every edge has its own two. near_lo / near_hi bound the thread's near slots.
 template <int MODE, int R, bool GRAD, bool CHAIN>
-__device__ __forceinline__ void sweep(EvSmem& sm, int32_t vb, int32_t n, const EvTopo& t, int32_t I0,
+__device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_t n, const EvTopo& t, int32_t I0,
                                       const V3 (&P)[CHAIN ? R + 1 : 2 * R],
                                       const int32_t (&ip)[CHAIN ? R + 1 : 2 * R], const double (&pw)[R],
                                       int32_t near_lo, int32_t near_hi, double alpha, double beta,
@@ -219,7 +221,7 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t vb, int32_t n, const E
         const bool careful = __any_sync(0xffffffffu, any != 0u);
         const int32_t gn = min(32, n - g0);
         for (int32_t j = 0; j < gn; j++) {
-            const double4 q4 = sm.sv[g0 + j];
+            const double4 q4 = sm.sv[s0 + g0 + j];
             const V3 q{q4.x, q4.y, q4.z};
             V3 d[NV], c[R];
             double x[NV], G[NV], gD[NV], h[NV], c2[R], N[R], kN[R];
@@ -306,12 +308,13 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t vb, int32_t n, const E
     }
 }
 
-// Work item (edge block ib, vertex chunk ch) of one curve. GRAD: edge_acc
-// [ch][kAcc][E] and vert_acc [ib][VA][4]; else the item's energy (near pairs
-// included by chunk 0) to *part.
+// Work item (edge block ib, vertex chunks from ch0, `group` of them) of one curve. GRAD:
+// one chunk, edge_acc [ch][kAcc][E] and vert_acc [ib][VA][4]; else each chunk's energy
+// (near pairs included by chunk 0) to part[chunk]. Several chunks have at most kTile
+// vertices together, staged at once.
 template <int MODE, int R, bool GRAD>
-__device__ __forceinline__ void ev_item(int ib, int ch, int32_t chunk, int tid, int bar, EvSmem& sm,
-                                        const EvTopo& t, const double4* __restrict__ ea,
+__device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chunk, int32_t nch, int tid, int bar,
+                                        EvSmem& sm, const EvTopo& t, const double4* __restrict__ ea,
                                         const double4* __restrict__ eb,
                                         const double4* __restrict__ vr, double alpha, double beta,
                                         double eps, double* __restrict__ edge_acc,
@@ -329,7 +332,6 @@ __device__ __forceinline__ void ev_item(int ib, int ch, int32_t chunk, int tid, 
         p2[r] = {eb[I].x, eb[I].y, eb[I].z};
         pw[r] = eb[I].w;
         ei[r] = t.ev[I];
-        S[r] = 0.0;
         if (r > 0) chain = chain && ei[r - 1].y == ei[r].x;
         if (I0 + r < t.E) {
             near_lo = min(near_lo, t.near[t.near_off[I]]);
@@ -337,26 +339,22 @@ __device__ __forceinline__ void ev_item(int ib, int ch, int32_t chunk, int tid, 
         }
     }
     const bool run = __all_sync(0xffffffffu, chain);
-    const int32_t v0 = ch * chunk, v1 = min(t.VA, v0 + chunk);
+    const int32_t ch1 = min(ch0 + group, nch), last = min(t.VA, ch1 * chunk);
+    int32_t s0 = 0, s1 = 0;  // the vertices in sm.sv
     V3 f1[R], f2[R];
-#pragma unroll
-    for (int r = 0; r < R; r++) f1[r] = f2[r] = {0.0, 0.0, 0.0};
-    if (R > 1 && run) {
-        V3 P[R + 1], F[R + 1];
-        int32_t ip[R + 1];
-#pragma unroll
-        for (int a = 0; a <= R; a++) {
-            P[a] = a < R ? p1[a < R ? a : 0] : p2[R - 1];
-            ip[a] = a < R ? ei[a < R ? a : 0].x : ei[R - 1].y;
-            F[a] = {0.0, 0.0, 0.0};
-        }
+    // the vertices [v0, v1) for the edges' points P
+    auto march = [&](auto chained, const auto& P, const auto& ip, auto& F, int32_t v0, int32_t v1) {
         for (int32_t vb = v0; vb < v1; vb += kTile) {
             const int32_t n = min(kTile, v1 - vb);
-            worker_sync(bar);
-            if (tid < n) sm.sv[tid] = vr[vb + tid];
-            worker_sync(bar);
-            sweep<MODE, R, GRAD, true>(sm, vb, n, t, I0, P, ip, pw, near_lo, near_hi, alpha, beta, eps,
-                                       S, F);
+            if (vb >= s1) {
+                s0 = vb;
+                s1 = min(vb + kTile, last);
+                worker_sync(bar);
+                if (tid < s1 - s0) sm.sv[tid] = vr[s0 + tid];
+                worker_sync(bar);
+            }
+            sweep<MODE, R, GRAD, decltype(chained)::value>(sm, vb - s0, vb, n, t, I0, P, ip, pw, near_lo, near_hi,
+                                                           alpha, beta, eps, S, F);
             if (GRAD) {
                 worker_sync(bar);
                 for (int k = tid; k < 4 * n; k += kW) {
@@ -367,46 +365,71 @@ __device__ __forceinline__ void ev_item(int ib, int ch, int32_t chunk, int tid, 
                 }
             }
         }
-        // a shared vertex's force goes to the edge it begins
+    };
+    for (int32_t ch = ch0; ch < ch1; ch++) {
+        const int32_t v0 = ch * chunk, v1 = min(t.VA, v0 + chunk);
 #pragma unroll
-        for (int r = 0; r < R; r++) f1[r] = F[r];
-        f2[R - 1] = F[R];
-    } else {
-        V3 P[2 * R], F[2 * R];
-        int32_t ip[2 * R];
+        for (int r = 0; r < R; r++) S[r] = 0.0;
+        if (R > 1 && run) {
+            V3 P[R + 1], F[R + 1];
+            int32_t ip[R + 1];
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-            P[2 * r] = p1[r];
-            P[2 * r + 1] = p2[r];
-            ip[2 * r] = ei[r].x;
-            ip[2 * r + 1] = ei[r].y;
-            F[2 * r] = F[2 * r + 1] = {0.0, 0.0, 0.0};
-        }
-        for (int32_t vb = v0; vb < v1; vb += kTile) {
-            const int32_t n = min(kTile, v1 - vb);
-            worker_sync(bar);
-            if (tid < n) sm.sv[tid] = vr[vb + tid];
-            worker_sync(bar);
-            sweep<MODE, R, GRAD, false>(sm, vb, n, t, I0, P, ip, pw, near_lo, near_hi, alpha, beta, eps,
-                                        S, F);
-            if (GRAD) {
-                worker_sync(bar);
-                for (int k = tid; k < 4 * n; k += kW) {
-                    double s = 0.0;
+            for (int a = 0; a <= R; a++) {
+                P[a] = a < R ? p1[a < R ? a : 0] : p2[R - 1];
+                ip[a] = a < R ? ei[a < R ? a : 0].x : ei[R - 1].y;
+                F[a] = {0.0, 0.0, 0.0};
+            }
+            march(std::true_type{}, P, ip, F, v0, v1);
+            // a shared vertex's force goes to the edge it begins
 #pragma unroll
-                    for (int w = 0; w < kW / 32; w++) s += (&sm.acc[w][0][0])[k];
-                    vert_acc[((int64_t)ib * t.VA + vb) * 4 + k] = s;
-                }
+            for (int r = 0; r < R; r++) {
+                f1[r] = F[r];
+                f2[r] = {0.0, 0.0, 0.0};
+            }
+            f2[R - 1] = F[R];
+        } else {
+            V3 P[2 * R], F[2 * R];
+            int32_t ip[2 * R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                P[2 * r] = p1[r];
+                P[2 * r + 1] = p2[r];
+                ip[2 * r] = ei[r].x;
+                ip[2 * r + 1] = ei[r].y;
+                F[2 * r] = F[2 * r + 1] = {0.0, 0.0, 0.0};
+            }
+            march(std::false_type{}, P, ip, F, v0, v1);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                f1[r] = F[2 * r];
+                f2[r] = F[2 * r + 1];
             }
         }
+        if (GRAD) break;  // (one chunk)
+        double en = 0.0;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            f1[r] = F[2 * r];
-            f2[r] = F[2 * r + 1];
+            const int32_t I = I0 + r;
+            if (I >= t.E) break;
+            if (ch == 0) {
+                const int2 edge = t.edges[I];
+                for (int32_t k = t.near_off[I]; k < t.near_off[I + 1]; k++) {
+                    const int32_t v = t.near[k];
+                    if (v == ei[r].x || v == ei[r].y) continue;
+                    const double m = near_length(t, ea, edge, v);
+                    if (m == 0.0) continue;
+                    const double4 q = vr[v];
+                    const PairTerms<MODE> pt(p1[r], p2[r], {q.x, q.y, q.z}, alpha, beta, eps);
+                    S[r] += m * (pt.N * pt.GS);
+                }
+            }
+            en += pw[r] * S[r];
         }
+        for (int o = 16; o > 0; o >>= 1) en += __shfl_down_sync(0xffffffffu, en, o);
+        if ((tid & 31) == 0) sm.red[ch - ch0][tid >> 5] = en;
     }
     if (GRAD) {
-        double* o = edge_acc + (int64_t)ch * kAcc * t.E;
+        double* o = edge_acc + (int64_t)ch0 * kAcc * t.E;
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int32_t I = I0 + r;
@@ -421,47 +444,26 @@ __device__ __forceinline__ void ev_item(int ib, int ch, int32_t chunk, int tid, 
         }
         return;
     }
-    double en = 0.0;
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-        const int32_t I = I0 + r;
-        if (I >= t.E) break;
-        if (ch == 0) {
-            const int2 edge = t.edges[I];
-            for (int32_t k = t.near_off[I]; k < t.near_off[I + 1]; k++) {
-                const int32_t v = t.near[k];
-                if (v == ei[r].x || v == ei[r].y) continue;
-                const double m = near_length(t, ea, edge, v);
-                if (m == 0.0) continue;
-                const double4 q = vr[v];
-                const PairTerms<MODE> pt(p1[r], p2[r], {q.x, q.y, q.z}, alpha, beta, eps);
-                S[r] += m * (pt.N * pt.GS);
-            }
-        }
-        en += pw[r] * S[r];
-    }
-    for (int o = 16; o > 0; o >>= 1) en += __shfl_down_sync(0xffffffffu, en, o);
-    if ((tid & 31) == 0) sm.red[tid >> 5] = en;
     worker_sync(bar);
-    if (tid == 0) {
+    if (tid < ch1 - ch0) {
         double s = 0.0;
-        for (int w = 0; w < kW / 32; w++) s += sm.red[w];
-        *part = s;
+        for (int w = 0; w < kW / 32; w++) s += sm.red[tid][w];
+        part[ch0 + tid] = s;
     }
 }
 
-// One item per block; blockIdx = (chunk, edge block, curve).
+// One item per block; blockIdx = (group of chunks, edge block, curve).
 template <int MODE, int R, bool GRAD>
 __global__ void __launch_bounds__(kW, GRAD && R == 2 ? 3 : 4)
 ev_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
-          const double4* __restrict__ vr, EvTopo t, int32_t chunk, double alpha, double beta,
-          double eps, double* __restrict__ edge_acc, double* __restrict__ vert_acc,
+          const double4* __restrict__ vr, EvTopo t, int32_t chunk, int32_t nch, int32_t group, double alpha,
+          double beta, double eps, double* __restrict__ edge_acc, double* __restrict__ vert_acc,
           double* __restrict__ part) {
     __shared__ EvSmem sm;
     const int64_t c = blockIdx.z;
-    ev_item<MODE, R, GRAD>(blockIdx.y, blockIdx.x, chunk, threadIdx.x, 0, sm, t, ea + c * t.E,
+    ev_item<MODE, R, GRAD>(blockIdx.y, blockIdx.x * group, group, chunk, nch, threadIdx.x, 0, sm, t, ea + c * t.E,
                            eb + c * t.E, vr + c * t.VA, alpha, beta, eps, edge_acc, vert_acc,
-                           part + (c * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x);
+                           part + (c * gridDim.y + blockIdx.y) * nch);
 }
 
 // The gradient's items on a bounded number of SMs: kWorkers independent workers
@@ -483,7 +485,7 @@ ev_persist_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb
         const int x = sm.next;
         worker_sync(1 + w);
         if (x >= items) break;
-        ev_item<MODE, R, true>(x / nch, x % nch, chunk, tid, 1 + w, sm, t, ea, eb, vr, alpha, beta, eps,
+        ev_item<MODE, R, true>(x / nch, x % nch, 1, chunk, nch, tid, 1 + w, sm, t, ea, eb, vr, alpha, beta, eps,
                                edge_acc, vert_acc, nullptr);
     }
 }
@@ -665,9 +667,13 @@ EvTopo topo_of(const tpe_ctx* ctx) {
 // 276 against 320 us for the energy, 608 against 680 for the gradient; equal at
 // 2048; four edges per thread spill). Below, one: more items, shorter chains
 // (1024 edges: 21 against 23 us). Items of 8 to 128 vertices, about six per SM.
+// Neither depends on how many curves a launch has: the order of an energy's sum, and with
+// it its last bits, are those of the curve alone (differences of energies from launches of
+// different sizes are taken). With more curves a block takes `group` chunks of one edge
+// block, up to kTile vertices, one after the other.
 struct EvSplit {
     int R;
-    int32_t nib, chunk, nch;
+    int32_t nib, chunk, nch, group;
 };
 EvSplit ev_split(const tpe_ctx* ctx, int32_t ncurves) {
     EvSplit s;
@@ -675,12 +681,14 @@ EvSplit ev_split(const tpe_ctx* ctx, int32_t ncurves) {
     s.R = E >= 2048 ? 2 : 1;
     s.nib = (E + kW * s.R - 1) / (kW * s.R);
     const int64_t want = 6 * (int64_t)ctx->num_sms;  // items
-    int64_t c = ((int64_t)VA * s.nib * ncurves + want - 1) / want;
+    int64_t c = ((int64_t)VA * s.nib + want - 1) / want;
     c = (c + 7) / 8 * 8;
     // at most 96 chunks (partials per edge), or items of 128 vertices where that is more
     const int64_t most = std::max<int64_t>(kTile, ((VA + 95) / 96 + kTile - 1) / kTile * kTile);
     s.chunk = (int32_t)std::min<int64_t>(std::max<int64_t>(c, 8), most);
     s.nch = (VA + s.chunk - 1) / s.chunk;
+    const int64_t g = ((int64_t)s.nch * s.nib * ncurves + want - 1) / want;
+    s.group = (int32_t)std::max<int64_t>(1, std::min<int64_t>(g, kTile / s.chunk));
     return s;
 }
 
@@ -773,11 +781,11 @@ namespace {
 template <int MODE>
 int32_t energy_launch(tpe_ctx* ctx, int32_t ncurves, const EvSplit& s, double alpha, double beta,
                       double eps) {
-    const dim3 grid((unsigned)s.nch, (unsigned)s.nib, (unsigned)ncurves);
+    const dim3 grid((unsigned)((s.nch + s.group - 1) / s.group), (unsigned)s.nib, (unsigned)ncurves);
     auto kern = s.R == 2 ? ev_kernel<MODE, 2, false> : ev_kernel<MODE, 1, false>;
     kern<<<grid, kW, 0, ctx->stream>>>(ctx->edge_a.as<double4>(), ctx->edge_b.as<double4>(),
-                                       ctx->ev_vert.as<double4>(), topo_of(ctx), s.chunk, alpha, beta,
-                                       eps, nullptr, nullptr, ctx->partial.as<double>());
+                                       ctx->ev_vert.as<double4>(), topo_of(ctx), s.chunk, s.nch, s.group,
+                                       alpha, beta, eps, nullptr, nullptr, ctx->partial.as<double>());
     TPE_CUDA_TRY(cudaGetLastError());
     return TPE_OK;
 }
@@ -805,7 +813,7 @@ int32_t grad_launch(tpe_ctx* ctx, const EvSplit& s, double alpha, double beta, d
     } else {
         const dim3 grid((unsigned)s.nch, (unsigned)s.nib, 1);
         auto kern = s.R == 2 ? ev_kernel<MODE, 2, true> : ev_kernel<MODE, 1, true>;
-        kern<<<grid, kW, 0, ctx->stream>>>(ea, eb, vr, t, s.chunk, alpha, beta, eps, acc, vacc, nullptr);
+        kern<<<grid, kW, 0, ctx->stream>>>(ea, eb, vr, t, s.chunk, s.nch, 1, alpha, beta, eps, acc, vacc, nullptr);
     }
     TPE_CUDA_TRY(cudaGetLastError());
     ev_edge_kernel<MODE><<<(unsigned)((t.E + 31) / 32), 256, 0, ctx->stream>>>(

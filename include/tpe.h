@@ -169,6 +169,11 @@ const char* tpe_last_error(const tpe_ctx* ctx);
  *   the device were out of memory (0: none, the default). */
 enum { TPE_TUNE_FAIL_ALLOC = 0 };
 int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value);
+/* The roots of the pair kernels at x[0..n) (device arrays): out[2 i] as those kernels form
+ * them, out[2 i + 1] CUDA's own function. TPE_ROOT_RSQRT: x^(-1/2), TPE_ROOT_INV_CBRT:
+ * x^(-1/3). */
+enum { TPE_ROOT_RSQRT = 0, TPE_ROOT_INV_CBRT = 1 };
+int32_t tpe_root_check(tpe_ctx* ctx, int32_t which, const double* x, int32_t n, double* out);
 
 /* ---- topology ------------------------------------------------------------- */
 /* Replaces calculateDisjointPairs (src/core/tangentPointEnergy.ts:33-47): the

@@ -45,6 +45,7 @@ PRECISION_FP64, PRECISION_MIXED = 0, 1
 GEMM_FP64, GEMM_INT8_EMULATED = 0, 1
 BCT_HIGH, BCT_LOW = 0, 1
 TUNE_FAIL_ALLOC = 0
+ROOT_RSQRT, ROOT_INV_CBRT = 0, 1
 
 PHASE_KEYS = ["dE", "energy", "bHigh", "bLow", "assembleA", "expand", "saddle", "factor",
               "projection", "lineSearch", "step", "refine"]
@@ -136,6 +137,7 @@ SIGNATURES = {
     "tpe_destroy": (None, [vp]),
     "tpe_last_error": (C.c_char_p, [vp]),
     "tpe_tune": (C.c_int32, [vp, C.c_int32, C.c_int64]),
+    "tpe_root_check": (C.c_int32, [vp, C.c_int32, vp, C.c_int32, vp]),
     "tpe_set_topology": (C.c_int32, [vp, ip, C.c_int32, C.c_int32]),
     "tpe_disjoint_pairs": (C.c_int32, [vp, ip, ip, C.c_int64]),
     "tpe_energy": (C.c_int32, [vp, dp, C.POINTER(tpe_params), dp]),

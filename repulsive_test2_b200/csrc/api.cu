@@ -25,6 +25,7 @@
 #include <chrono>
 #include <vector>
 
+#include "pair_math.cuh"
 #include "tpe_internal.h"
 #include <cstring>
 
@@ -366,6 +367,15 @@ __global__ void fd_positions_kernel(const double* __restrict__ p, int64_t m, int
     double v = p[i];
     if (i == base + c) v += h;
     out[t] = v;
+}
+
+__global__ void root_check_kernel(int32_t which, const double* __restrict__ x, int32_t n,
+                                  double* __restrict__ out) {
+    const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const bool cbrt = which == TPE_ROOT_INV_CBRT;
+    out[2 * (int64_t)i] = cbrt ? inv_cbrt(x[i]) : rsqrt_normal(x[i]);
+    out[2 * (int64_t)i + 1] = cbrt ? rcbrt(x[i]) : rsqrt(x[i]);
 }
 
 int32_t check_topology(tpe_ctx* ctx) {
@@ -1520,6 +1530,22 @@ int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value) {
             case TPE_TUNE_FAIL_ALLOC: ctx->fail_alloc = std::max<int64_t>(value, 0); return TPE_OK;
             default: set_error(ctx, TPE_ERR_BAD_ARG, "tpe_tune: unknown setting"); return TPE_ERR_BAD_ARG;
         }
+    });
+}
+
+int32_t tpe_root_check(tpe_ctx* ctx, int32_t which, const double* x, int32_t n, double* out) {
+    return guarded(ctx, [&]() -> int32_t {
+        if (!ctx) return TPE_ERR_BAD_ARG;
+        if (which < TPE_ROOT_RSQRT || which > TPE_ROOT_INV_CBRT || !x || !out || n < 1) {
+            set_error(ctx, TPE_ERR_BAD_ARG, "tpe_root_check: bad arguments");
+            return TPE_ERR_BAD_ARG;
+        }
+        TPE_CUDA_TRY(cudaSetDevice(ctx->device));
+        KernelScope ks(ctx, TPE_KGROUP_OTHER, 1);
+        root_check_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(which, x, n, out);
+        TPE_CUDA_TRY(cudaGetLastError());
+        TPE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        return TPE_OK;
     });
 }
 

@@ -26,16 +26,6 @@ namespace tpe {
 namespace {
 
 
-// x^(-1/3) for x > 0: an FP32 estimate y (exp2 of log2) times the binomial series
-// of (1 - e)^(-1/3), e = 1 - x y^3, through e^2 (the e^3 left out is below 2^-60).
-// Beyond the range where FP32 holds y and y^3, CUDA's own.
-__device__ __forceinline__ double inv_cbrt(double x) {
-    if (!(x > 1e-30 && x < 1e30)) return rcbrt(x);
-    const double y = (double)exp2f(-0.33333334f * __log2f((float)x));
-    const double e = fma(-x * y, y * y, 1.0);
-    return fma(y * e, fma(2.0 / 9.0, e, 1.0 / 3.0), y);
-}
-
 // (|d|+eps)^(-(2 sigma + 1)) from dn = |d|+eps and its reciprocal idn;
 // MODE 1: alpha = 3, beta = 6 -> exponent 7/3.
 template <int MODE>
@@ -389,19 +379,14 @@ assemble_loop_kernel(const double4* __restrict__ ea, int32_t V, int32_t R, doubl
         dz = z - me.z;
         x2 = dx * dx + dy * dy + dz * dz;
         if (MODE == 1) {
-            const double ir = rsqrt_normal(x2);
-            const double t = eps * ir;
-            const double idn = fma(-ir, t * (1.0 - t), ir);
-            const double dn = fma(x2, ir, eps);
-            const float y0 = exp2f(-0.33333334f * __log2f((float)dn));
-            const double yd = (double)y0;
-            const double e = fma(-dn * yd, yd * yd, 1.0);
-            const double ic = fma(yd * e, fma(2.0 / 9.0, e, 1.0 / 3.0), yd);
+            // without a branch but for the rare case
+            double ir, idn, ic;
+            const bool far = inv_dist_fast(x2, eps, ir, idn);
+            const bool mid = inv_cbrt_fast(fma(x2, ir, eps), ic);
             const double i2 = idn * idn;
             kd = ic * i2;
             kq = kd * (i2 * i2);
-            // near zero, or beyond what FP32 holds: the general form
-            if (!(t < 9.5367431640625e-07 && dn > 1e-30 && dn < 1e30)) dist_weights<MODE>(x2, distExp, eps, kd, kq);
+            if (!(far && mid)) dist_weights<MODE>(x2, distExp, eps, kd, kq);
         } else {
             dist_weights<MODE>(x2, distExp, eps, kd, kq);
         }

@@ -102,13 +102,12 @@ __device__ __forceinline__ void area_power(double c2, double alpha, double eps, 
 // The same for a = 3, b = 6 where the distance is beyond 1e6 eps and the area
 // above 1e-14 (and finite), without a branch; false elsewhere.
 __device__ __forceinline__ bool dist_power_fast(double x, double eps, double& G, double& gD) {
-    const double r = rsqrt_normal(x);
-    const double t = eps * r;
-    const double inve = fma(-r, t * (1.0 - t), r);
+    double r, inve;
+    const bool ok = inv_dist_fast(x, eps, r, inve);
     const double i2 = inve * inve;
     G = i2 * i2 * i2;
     gD = G * inve * r;
-    return t < 9.5367431640625e-07;
+    return ok;
 }
 __device__ __forceinline__ bool area_power_fast(double c2, double eps, double& N, double& kN) {
     const double inv = rsqrt_normal(c2);

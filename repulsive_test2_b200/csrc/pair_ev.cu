@@ -65,8 +65,11 @@ struct EvTopo {
     int32_t E, VA;
 };
 
+// G = (|d| + eps)^-b and gI = 1 / (|d| (|d| + eps)) (0 below |d| = 1e-14) of x = |d|^2: G and
+// gI on their own, since their product, -dG/d|d| / (b |d|), falls out of the double range at
+// 1e38 (b = 6), well before the gradient's terms do.
 template <int MODE>
-__device__ __forceinline__ void dist_power(double x, double beta, double eps, double& G, double& gD) {
+__device__ __forceinline__ void dist_power(double x, double beta, double eps, double& G, double& gI) {
     double s, inv, inve;
     dist_terms(x, eps, s, inv, inve);
     if (MODE == 1) {
@@ -75,7 +78,7 @@ __device__ __forceinline__ void dist_power(double x, double beta, double eps, do
     } else {
         G = 1.0 / pow(s + eps, beta);
     }
-    gD = G * inve * inv;  // -dG/d|d| / (b |d|)
+    gI = inve * inv;
 }
 
 // N = (|c| + eps)^a and kN = (|c| + eps)^(a-1) / |c| (0 below |c| = 1e-14).
@@ -101,12 +104,12 @@ __device__ __forceinline__ void area_power(double c2, double alpha, double eps, 
 
 // The same for a = 3, b = 6 where the distance is beyond 1e6 eps and the area
 // above 1e-14 (and finite), without a branch; false elsewhere.
-__device__ __forceinline__ bool dist_power_fast(double x, double eps, double& G, double& gD) {
+__device__ __forceinline__ bool dist_power_fast(double x, double eps, double& G, double& gI) {
     double r, inve;
     const bool ok = inv_dist_fast(x, eps, r, inve);
     const double i2 = inve * inve;
     G = i2 * i2 * i2;
-    gD = G * inve * r;
+    gI = inve * r;
     return ok;
 }
 __device__ __forceinline__ bool area_power_fast(double c2, double eps, double& N, double& kN) {
@@ -156,18 +159,18 @@ __device__ __forceinline__ void worker_sync(int bar) {
 }
 
 // One edge against one vertex outside the sweep: N, G1 + G2 and the derivative
-// terms (f1, f2: d|d| coefficients, kc = K c with K = a (G1 + G2) kN).
+// terms (G1 g1, G2 g2: dist_power's; kc = K c with K = a (G1 + G2) kN).
 template <int MODE>
 struct PairTerms {
     double GS, N;
     V3 d1, d2, kc;
-    double g1, g2;
+    double G1, G2, g1, g2;
     __device__ __forceinline__ PairTerms(const V3& p1, const V3& p2, const V3& q, double alpha,
                                          double beta, double eps) {
         d1 = sub(p1, q);
         d2 = sub(p2, q);
         const double x1 = dot3(d1, d1), x2 = dot3(d2, d2);
-        double G1, G2, kN;
+        double kN;
         dist_power<MODE>(x1, beta, eps, G1, g1);
         dist_power<MODE>(x2, beta, eps, G2, g2);
         const V3 e = sub(p2, p1);
@@ -223,7 +226,7 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
             const double4 q4 = sm.sv[s0 + g0 + j];
             const V3 q{q4.x, q4.y, q4.z};
             V3 d[NV], c[R];
-            double x[NV], G[NV], gD[NV], h[NV], c2[R], N[R], kN[R];
+            double x[NV], G[NV], gI[NV], h[NV], c2[R], N[R], kN[R];
             // the common case without a branch, so that the runs of all R edges
             // interleave; a distance near zero or a flat triangle redoes the lane's
             bool rare = false;
@@ -234,9 +237,9 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
                 // an endpoint against itself: any finite distance, its edges are masked
                 if (careful && ip[a] == base + j) x[a] = 1.0;
                 if (MODE == 1)
-                    rare |= !dist_power_fast(x[a], eps, G[a], gD[a]);
+                    rare |= !dist_power_fast(x[a], eps, G[a], gI[a]);
                 else
-                    dist_power<MODE>(x[a], beta, eps, G[a], gD[a]);
+                    dist_power<MODE>(x[a], beta, eps, G[a], gI[a]);
                 h[a] = 0.0;
             }
 #pragma unroll
@@ -254,7 +257,7 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
             }
             if (rare) {
 #pragma unroll
-                for (int a = 0; a < NV; a++) dist_power<MODE>(x[a], beta, eps, G[a], gD[a]);
+                for (int a = 0; a < NV; a++) dist_power<MODE>(x[a], beta, eps, G[a], gI[a]);
 #pragma unroll
                 for (int r = 0; r < R; r++) area_power<MODE>(c2[r], alpha, eps, N[r], kN[r]);
             }
@@ -284,7 +287,7 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
             if (GRAD) {
 #pragma unroll
                 for (int a = 0; a < NV; a++) {
-                    const double f = -beta * (h[a] * gD[a]);
+                    const double f = -beta * ((h[a] * G[a]) * gI[a]);
                     axpy3(F[a], f, d[a]);
                     axpy3(Q, -f, d[a]);
                 }
@@ -535,8 +538,8 @@ ev_edge_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
         sub_cross(f1, pt.d2, kc);
         add_cross(f2, pt.d1, kc);
         const double tn = -beta * (mp * pt.N);
-        axpy3(f1, tn * pt.g1, pt.d1);
-        axpy3(f2, tn * pt.g2, pt.d2);
+        axpy3(f1, (tn * pt.G1) * pt.g1, pt.d1);
+        axpy3(f2, (tn * pt.G2) * pt.g2, pt.d2);
     }
     // dE/dl_I through M: the edges K disjoint from I, at both of I's vertices
 #pragma unroll
@@ -599,8 +602,8 @@ ev_vertex_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
             const V3 kc{mp * pt.kc.x, mp * pt.kc.y, mp * pt.kc.z};
             add_cross(g, sub(p2, p1), kc);
             const double tn = beta * (mp * pt.N);
-            axpy3(g, tn * pt.g1, pt.d1);
-            axpy3(g, tn * pt.g2, pt.d2);
+            axpy3(g, (tn * pt.G1) * pt.g1, pt.d1);
+            axpy3(g, (tn * pt.G2) * pt.g2, pt.d2);
         }
         for (int32_t k = t.inc_off[w]; k < t.inc_off[w + 1]; k++) {
             const int32_t I = t.inc[k] >> 1, c = 3 * (t.inc[k] & 1);

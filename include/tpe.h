@@ -166,8 +166,17 @@ const char* tpe_last_error(const tpe_ctx* ctx);
 /* Settings of one context for checks of the library itself (a program needs none of
  * them); a negative value restores the default.
  * TPE_TUNE_FAIL_ALLOC: the value-th growth of a device buffer from here on fails, as if
- *   the device were out of memory (0: none, the default). */
-enum { TPE_TUNE_FAIL_ALLOC = 0 };
+ *   the device were out of memory (0: none, the default).
+ * TPE_TUNE_FACTOR_POLLS, TPE_TUNE_SOLVE_POLLS: polls after which a wait inside the FP64
+ *   factorization or its triangular solves gives up (0: some seconds' worth, the default).
+ * TPE_TUNE_FACTOR_BLOCKS: thread blocks of the FP64 factorization (0: by its order, the
+ *   default; 1: as where other kernels hold the rest of the device). */
+enum {
+    TPE_TUNE_FAIL_ALLOC = 0,
+    TPE_TUNE_FACTOR_POLLS = 1,
+    TPE_TUNE_SOLVE_POLLS = 2,
+    TPE_TUNE_FACTOR_BLOCKS = 3
+};
 int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value);
 /* The roots of the pair kernels at x[0..n) (device arrays): out[2 i] as those kernels form
  * them, out[2 i + 1] CUDA's own function. TPE_ROOT_RSQRT: x^(-1/2), TPE_ROOT_INV_CBRT:

@@ -44,7 +44,7 @@ FACTOR_LDLT, FACTOR_LU = 0, 1
 PRECISION_FP64, PRECISION_MIXED = 0, 1
 GEMM_FP64, GEMM_INT8_EMULATED = 0, 1
 BCT_HIGH, BCT_LOW = 0, 1
-TUNE_FAIL_ALLOC = 0
+TUNE_FAIL_ALLOC, TUNE_FACTOR_POLLS, TUNE_SOLVE_POLLS, TUNE_FACTOR_BLOCKS = range(4)
 ROOT_RSQRT, ROOT_INV_CBRT = 0, 1
 
 PHASE_KEYS = ["dE", "energy", "bHigh", "bLow", "assembleA", "expand", "saddle", "factor",

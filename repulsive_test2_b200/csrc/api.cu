@@ -1526,8 +1526,12 @@ const char* tpe_last_error(const tpe_ctx* ctx) { return ctx ? ctx->err.c_str() :
 int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value) {
     return guarded(ctx, [&]() -> int32_t {
         if (!ctx) return TPE_ERR_BAD_ARG;
+        auto bounded = [&](int64_t most) { return (int32_t)std::min(std::max<int64_t>(value, 0), most); };
         switch (what) {
             case TPE_TUNE_FAIL_ALLOC: ctx->fail_alloc = std::max<int64_t>(value, 0); return TPE_OK;
+            case TPE_TUNE_FACTOR_POLLS: ctx->factor_polls = bounded(1 << 22); return TPE_OK;
+            case TPE_TUNE_SOLVE_POLLS: ctx->solve_polls = bounded(1 << 22); return TPE_OK;
+            case TPE_TUNE_FACTOR_BLOCKS: ctx->factor_blocks = bounded(2 * ctx->num_sms); return TPE_OK;
             default: set_error(ctx, TPE_ERR_BAD_ARG, "tpe_tune: unknown setting"); return TPE_ERR_BAD_ARG;
         }
     });

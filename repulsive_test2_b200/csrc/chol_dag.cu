@@ -51,7 +51,7 @@ constexpr int kPad = kKC + 4;  // row stride of a staged chunk (doubles)
 constexpr int kTP = NB + 4;    // row stride of a whole tile
 constexpr int kStage = NB * kPad;
 constexpr int kTile = NB * kTP;
-constexpr int64_t kSpin = 1 << 22;  // polls before a wait gives up (seconds)
+constexpr int32_t kSpin = 1 << 22;  // polls before a wait gives up (seconds)
 
 struct Dag {
     double* L;     // n x n (rows ld apart): A on entry (lower), L on return
@@ -63,6 +63,7 @@ struct Dag {
     int32_t n, nb, nr, nrb;  // nrb row blocks of right-hand sides
     int64_t ld;              // row length of L, W and X (n or more); B and Ainv have n
     double tol;
+    int32_t limit;  // polls before a wait gives up
     int32_t* flag;  // [(nb + nrb + nb) x nb] tiles done, then diag, preA, preD [nb each]
     // [0] a pivot failed, [1] a wait ran out, [2] role ticket, [3] tile counter, [4] the chain's SM + 1
     int32_t* ctl;
@@ -346,10 +347,9 @@ __device__ __forceinline__ void each_row(const RowAcc& acc, F&& f) {
 // Thread 0 waits until *f is set; false when the wait ran out or another did.
 __device__ __forceinline__ bool wait_one(const Dag& g, const int32_t* f, int32_t* ok) {
     if (threadIdx.x == 0) {
-        int64_t it = 0;
-        int32_t good = 1;
+        int32_t it = 0, good = 1;
         while (ld_acquire(f) == 0) {
-            if (++it > kSpin || ((it & 63) == 0 && ld_acquire(g.ctl + 1))) {
+            if (++it > g.limit || ((it & 63) == 0 && ld_acquire(g.ctl + 1))) {
                 atomicExch(g.ctl + 1, 1);
                 good = 0;
                 break;
@@ -370,8 +370,7 @@ __device__ __forceinline__ bool wait_more(const Dag& g, const int32_t* fa, const
                                           int32_t end, int32_t* ready) {
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
-        int64_t it = 0;
-        int32_t got;
+        int32_t it = 0, got;
         for (;;) {
             const bool in = k + lane < end;
             const int32_t s = !in || (ld_acquire(fa + k + lane) && ld_acquire(fb + k + lane));
@@ -379,7 +378,7 @@ __device__ __forceinline__ bool wait_more(const Dag& g, const int32_t* fa, const
             got = m == 0xffffffffu ? 32 : __ffs(~m) - 1;
             if (got > 0) break;
             int32_t stop = 0;
-            if (lane == 0) stop = ++it > kSpin || ((it & 63) == 0 && ld_acquire(g.ctl + 1));
+            if (lane == 0) stop = ++it > g.limit || ((it & 63) == 0 && ld_acquire(g.ctl + 1));
             if (__shfl_sync(0xffffffffu, stop, 0)) break;
             __nanosleep(20);
         }
@@ -566,18 +565,28 @@ __device__ __forceinline__ bool column_tile(const Dag& g, Smem& sm, int32_t j, i
     return true;
 }
 
-// The chain's wait at column j: polls for a while, then works on the tiles of the
-// columns up to j itself (none of them needs the chain any further), so that one
-// running block is enough to finish. *helped: sm.buf was used.
+// The chain's wait at column j for fa and fb: polls for a while, then works on the tiles
+// of the columns up to j itself (none of them needs the chain any further), one after the
+// other until both flags are up, so that one running block is enough to finish. The limit counts
+// the polls since the last tile. *helped: sm.buf was used.
+constexpr int32_t kPatience = 8192;
 template <bool kAl>
-__device__ __forceinline__ bool chain_wait(const Dag& g, Smem& sm, const int32_t* f, int32_t j, bool* helped) {
+__device__ __forceinline__ bool chain_wait(const Dag& g, Smem& sm, const int32_t* fa, const int32_t* fb, int32_t j,
+                                           bool* helped) {
     *helped = false;
-    for (int64_t round = 0; round < kSpin / 8192; round++) {
+    bool took = false;
+    for (int32_t polls = 0; polls <= g.limit; polls += kPatience) {
         if (threadIdx.x == 0) {
             sm.item = -1;
-            int32_t it = 0;
-            while (ld_acquire(f) == 0 && ++it < 8192 && !((it & 63) == 0 && ld_acquire(g.ctl + 1))) __nanosleep(20);
-            if (ld_acquire(f)) {
+            int32_t it = took ? kPatience - 1 : 0;
+            auto up = [&](const int32_t* f) {
+                while (ld_acquire(f) == 0) {
+                    if (++it >= kPatience || ((it & 63) == 0 && ld_acquire(g.ctl + 1))) return false;
+                    __nanosleep(20);
+                }
+                return true;
+            };
+            if (up(fa) && up(fb)) {
                 sm.ok = 1;
             } else if (ld_acquire(g.ctl + 1)) {
                 sm.ok = 0;
@@ -585,21 +594,28 @@ __device__ __forceinline__ bool chain_wait(const Dag& g, Smem& sm, const int32_t
                 sm.ok = 2;
                 int64_t end = 0;
                 for (int32_t c = 0; c <= j; c++) end += column_count(g, c);
-                const int32_t x = ld_acquire(g.ctl + 3);
-                if (x < end && atomicCAS(g.ctl + 3, x, x + 1) == x) sm.item = x;
+                for (int32_t x = ld_acquire(g.ctl + 3), now; x < end; x = now) {
+                    now = atomicCAS(g.ctl + 3, x, x + 1);
+                    if (now == x) {
+                        sm.item = x;
+                        break;
+                    }
+                }
             }
         }
         __syncthreads();
         const int32_t ok = sm.ok, x = sm.item;
         __syncthreads();
         if (ok < 2) return ok == 1;
-        if (x >= 0) {
+        took = x >= 0;
+        if (took) {
             int64_t y = x;
             int32_t c = 0;
             while (y >= column_count(g, c)) y -= column_count(g, c++);
             *helped = true;
             if (!column_tile<kAl>(g, sm, c, (int32_t)y)) return false;
             __syncthreads();
+            polls = -kPatience;
         }
     }
     if (threadIdx.x == 0) atomicExch(g.ctl + 1, 1);
@@ -650,11 +666,10 @@ __device__ __forceinline__ void chain(const Dag& g, Smem& sm) {
         }
         if (j + 1 == g.nb) break;
         const int32_t r1 = r0 + NB, rows = min(NB, g.n - r1);
-        bool helped[2] = {false, false};
-        if (j > 0 && !(chain_wait<kAl>(g, sm, preA + j, j, helped) && chain_wait<kAl>(g, sm, preD + j, j, helped + 1)))
-            return;
+        bool helped = false;
+        if (j > 0 && !chain_wait<kAl>(g, sm, preA + j, preD + j, j, &helped)) return;
         __syncthreads();  // L_jj is stored: a may be overwritten
-        if (helped[0] || helped[1]) load_tile<true>(z, Rows{g.Linv + (int64_t)j * NB * NB, NB, NB}, 0, NB);
+        if (helped) load_tile<true>(z, Rows{g.Linv + (int64_t)j * NB * NB, NB, NB}, 0, NB);
         load_tile<kAl>(t, Rows{g.L + (int64_t)r1 * g.ld, g.ld, rows}, r0, g.n);
         cp_commit();
         fetch_diag(j + 1);
@@ -775,7 +790,7 @@ __device__ __forceinline__ void mma_rhs(double (&acc)[2 * kMaxG][2], int ng, con
 template <bool kAl, bool FWD>
 __global__ void __launch_bounds__(kThr)
 tri_dag_kernel(const double* __restrict__ L, const double* __restrict__ Linv, int32_t n, int32_t nb, double* B,
-               int32_t nr, int32_t* flag, int32_t* ticket, int32_t* err) {
+               int32_t nr, int32_t limit, int32_t* flag, int32_t* ticket, int32_t* err) {
     extern __shared__ __align__(16) double dyn[];
     double* tile[2] = {dyn, dyn + kTile};
     double* z = dyn + 2 * kTile;
@@ -815,10 +830,10 @@ tri_dag_kernel(const double* __restrict__ L, const double* __restrict__ Linv, in
         if (q + 1 < t) fetch(q + 1);
         cp_commit();
         if (threadIdx.x == 0) {
-            int64_t it = 0;
+            int32_t it = 0;
             sh = 1;
             while (ld_acquire(flag + q) == 0)
-                if (++it > kSpin) {
+                if (++it > limit) {
                     atomicExch(err, 1);
                     sh = 0;
                     break;
@@ -886,8 +901,9 @@ int32_t chol_solve(tpe_ctx* ctx, const double* L, const double* Linv, int32_t n,
         double* b = B + (size_t)r0 * n;
         TPE_CUDA_TRY(cudaMemsetAsync(ctl, 0, sizeof(int32_t) * (2 * (size_t)nb + 2), st));
         KernelScope ks(ctx, TPE_KGROUP_TRSV, down ? 2 : 1);
-        if (down) kdown<<<(unsigned)nb, kThr, smem, st>>>(L, Linv, n, nb, b, q, ctl + 2, ctl, err);
-        kup<<<(unsigned)nb, kThr, smem, st>>>(L, Linv, n, nb, b, q, ctl + 2 + nb, ctl + 1, err);
+        const int32_t limit = ctx->solve_polls > 0 ? ctx->solve_polls : kSpin;
+        if (down) kdown<<<(unsigned)nb, kThr, smem, st>>>(L, Linv, n, nb, b, q, limit, ctl + 2, ctl, err);
+        kup<<<(unsigned)nb, kThr, smem, st>>>(L, Linv, n, nb, b, q, limit, ctl + 2 + nb, ctl + 1, err);
         TPE_CUDA_TRY(cudaGetLastError());
     }
     return TPE_OK;
@@ -914,6 +930,7 @@ int32_t chol_dag(tpe_ctx* ctx, const CholDag& c, int32_t* singular) {
     g.nr = c.nr;
     g.nrb = (c.nr + NB - 1) / NB;
     g.tol = c.tol;
+    g.limit = ctx->factor_polls > 0 ? ctx->factor_polls : kSpin;
     const size_t nflag = (size_t)(2 * g.nb + g.nrb) * g.nb + 3 * (size_t)g.nb;
     TPE_TRY(ensure(ctx, ctx->dag_flags, sizeof(int32_t) * (nflag + 5)));
     g.ctl = ctx->dag_flags.as<int32_t>();
@@ -932,7 +949,7 @@ int32_t chol_dag(tpe_ctx* ctx, const CholDag& c, int32_t* singular) {
     // the inverse 1200 510 -> 357, 2500 1750 -> 1010. Below 1500 rows the chain is the
     // bound, and blocks that wait only take room from other contexts' kernels.
     const int64_t widest = g.nb + g.nrb + 1;
-    const unsigned grid = (unsigned)std::min<int64_t>(
+    const unsigned grid = ctx->factor_blocks > 0 ? (unsigned)ctx->factor_blocks : (unsigned)std::min<int64_t>(
         2 * (int64_t)ctx->num_sms, 1 + (c.Ainv ? 9 : std::max(1, g.nb / 8 - 1)) * widest);
     {
         KernelScope ks(ctx, TPE_KGROUP_CHOLESKY, 1);

@@ -88,8 +88,9 @@ __device__ __forceinline__ void area_power(double c2, double alpha, double eps, 
     if (c2 >= 1e-28 && c2 <= 1e300) {
         inv = rsqrt_normal(c2);
         rc = c2 * inv;
-    } else {
+    } else {  // flat, or beyond rsqrt_normal's range
         rc = sqrt(c2);
+        inv = rc < 1e-14 ? 0.0 : 1.0 / rc;
     }
     const double cn = rc + eps;
     if (MODE == 1) {

@@ -12,8 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n", [33, 700, 2050])
-@pytest.mark.parametrize("alpha,beta,power", [(2.0, 4.0, 100), (2.0, 4.0, 200), (2.0, 4.0, 240), (3.0, 6.0, 100),
-                                              (3.0, 6.0, 130), (3.0, 6.0, 155), (3.0, 6.0, 162)])
+@pytest.mark.parametrize("alpha,beta,power", [(2.0, 4.0, 100), (2.0, 4.0, 200), (2.0, 4.0, 240), (2.0, 4.0, 250),
+                                              (2.0, 4.0, 252), (3.0, 6.0, 100), (3.0, 6.0, 130), (3.0, 6.0, 155), (3.0, 6.0, 162)])
 def test_large_curves(n, alpha, beta, power):
     v, e = F.trefoil(n, jitter=0.01, seed=2)
     s = 2.0 ** power

@@ -421,7 +421,10 @@ template <bool kAl>
 __device__ __forceinline__ bool sum_tiles(const Dag& g, Smem& sm, Acc& acc, const Rows& A, const int32_t* fa,
                                           const Rows& B, const int32_t* fb, int32_t k0, int32_t k1) {
     if (k0 >= k1) return true;
-    if (!wait_more(g, fa, fb, k0, k1, &sm.ready)) return false;
+    if (!wait_more(g, fa, fb, k0, k1, &sm.ready)) {
+        cp_wait<0>();  // (the caller's own fetch)
+        return false;
+    }
     int32_t ready = sm.ready;
     auto load = [&](int st, int32_t c) {
         load_chunk<kAl>(sm.buf + (2 * st) * kStage, A, c, g.n);

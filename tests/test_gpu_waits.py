@@ -48,3 +48,26 @@ def test_one_block_finishes(ctx, n, kind):
     for blocks in (1, 2, 7):
         _tune(ctx, blocks=blocks, polls=4 * 8192)
         assert np.array_equal(call(), want), blocks
+
+
+@pytest.mark.parametrize("n,kind,precision", [(777, "length", "fp64"), (300, "length", "mixed"), (300, "edges", "fp64"),
+                                              (300, "edges", "mixed")])
+def test_factorization_timeout(ctx, n, kind, precision):
+    call = _call(n, kind, precision)
+    want = call()
+    _tune(ctx, polls=1)
+    with pytest.raises(T.TpeError, match="factorization kernel ran out"):
+        call()
+    _tune(ctx, polls=0)
+    assert np.array_equal(call(), want)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_solve_timeout(ctx, precision):
+    call = _call(777, "length", precision)
+    want = call()
+    _tune(ctx, solve=1)
+    with pytest.raises(T.TpeError, match="triangular solve ran out"):
+        call()
+    _tune(ctx, solve=0)
+    assert np.array_equal(call(), want)

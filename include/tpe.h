@@ -180,8 +180,8 @@ enum {
 int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value);
 /* The roots of the pair kernels at x[0..n) (device arrays): out[2 i] as those kernels form
  * them, out[2 i + 1] CUDA's own function. TPE_ROOT_RSQRT: x^(-1/2), TPE_ROOT_INV_CBRT:
- * x^(-1/3). */
-enum { TPE_ROOT_RSQRT = 0, TPE_ROOT_INV_CBRT = 1 };
+ * x^(-1/3), TPE_ROOT_RECIP: 1/x (of the factorization's pivots). */
+enum { TPE_ROOT_RSQRT = 0, TPE_ROOT_INV_CBRT = 1, TPE_ROOT_RECIP = 2 };
 int32_t tpe_root_check(tpe_ctx* ctx, int32_t which, const double* x, int32_t n, double* out);
 
 /* ---- topology ------------------------------------------------------------- */

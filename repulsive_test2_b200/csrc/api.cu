@@ -373,9 +373,14 @@ __global__ void root_check_kernel(int32_t which, const double* __restrict__ x, i
                                   double* __restrict__ out) {
     const int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const bool cbrt = which == TPE_ROOT_INV_CBRT;
-    out[2 * (int64_t)i] = cbrt ? inv_cbrt(x[i]) : rsqrt_normal(x[i]);
-    out[2 * (int64_t)i + 1] = cbrt ? rcbrt(x[i]) : rsqrt(x[i]);
+    double* o = out + 2 * (int64_t)i;
+    const double v = x[i];
+    if (which == TPE_ROOT_RSQRT)
+        o[0] = rsqrt_normal(v), o[1] = rsqrt(v);
+    else if (which == TPE_ROOT_INV_CBRT)
+        o[0] = inv_cbrt(v), o[1] = rcbrt(v);
+    else
+        o[0] = recip_normal(v), o[1] = 1.0 / v;
 }
 
 int32_t check_topology(tpe_ctx* ctx) {
@@ -1540,7 +1545,7 @@ int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value) {
 int32_t tpe_root_check(tpe_ctx* ctx, int32_t which, const double* x, int32_t n, double* out) {
     return guarded(ctx, [&]() -> int32_t {
         if (!ctx) return TPE_ERR_BAD_ARG;
-        if (which < TPE_ROOT_RSQRT || which > TPE_ROOT_INV_CBRT || !x || !out || n < 1) {
+        if (which < TPE_ROOT_RSQRT || which > TPE_ROOT_RECIP || !x || !out || n < 1) {
             set_error(ctx, TPE_ERR_BAD_ARG, "tpe_root_check: bad arguments");
             return TPE_ERR_BAD_ARG;
         }

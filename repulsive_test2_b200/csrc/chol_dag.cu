@@ -39,6 +39,7 @@
 
 #include <algorithm>
 
+#include "pair_math.cuh"
 #include "tpe_internal.h"
 
 namespace tpe {
@@ -172,15 +173,6 @@ __device__ __forceinline__ void each(const Acc& acc, F&& f) {
 
 // ---- the chain's diagonal block ----------------------------------------------
 
-// 1/x for normal x: the hardware's approximation y (20 bits) times the geometric
-// series of 1/(1 - e), e = 1 - x y, through e^2.
-__device__ __forceinline__ double recip(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-
 // a (64 x 64, lower) -> L in a, L^-1 in z (whole tile, zero above the diagonal).
 // Factor and inverse in one sweep over the columns: right-looking on the 64 rows
 // of A and, below them, the rows of the identity, which become L^-T. At column
@@ -218,7 +210,7 @@ __device__ __forceinline__ void potrf64(double* a, double* z, double* inv, doubl
 #pragma unroll
                 for (int q = c + 1; q < 8; q++) l[q] = __shfl_sync(0xffffffffu, xs, own + q);
                 if (!(piv > tol)) piv = 1.0;
-                const double iv = recip(piv);
+                const double iv = recip_normal(piv);
                 if (lane == 0) inv[8 * p + c] = iv;
                 const double t0 = r0 == c ? iv : x0 * iv, t1 = r1 == c ? iv : x1 * iv;
 #pragma unroll

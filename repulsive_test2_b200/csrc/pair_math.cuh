@@ -1,4 +1,4 @@
-// Distance and power helpers shared by the pair kernels.
+// Roots and distances shared by the pair kernels, and the factorization's reciprocal.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -6,15 +6,27 @@
 
 namespace tpe {
 
-// 1/sqrt(x) for normal x > 0, to about one unit in the last place: the hardware's
-// approximation y (20 bits) corrected by the binomial series of (1 - e)^(-1/2),
-// e = 1 - x y^2, through e^2 (the e^3 left out is below 2^-60). Zero, subnormal,
-// infinite and NaN x give infinity or NaN: the callers test for what they accept.
+// 1/sqrt(x) for normal x > 0: the hardware's approximation y (20 bits) corrected by the
+// binomial series of (1 - e)^(-1/2), e = 1 - x y^2, through e^2 (|e| is below 2^-19, the
+// 5/16 e^3 left out below 2^-58). Zero, subnormal, infinite and NaN x give infinity or
+// NaN: the callers test for what they accept. Largest error in a million samples 1.24
+// units of 2^-53, root mean square 0.48 (CUDA's rsqrt, which branches: 1.00 and 0.43).
 __device__ __forceinline__ double rsqrt_normal(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-(x * y), y, 1.0);
     return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// 1/x for normal x whose reciprocal is normal: the hardware's approximation y (20 bits)
+// times the geometric series of 1/(1 - e), e = 1 - x y, through e^2 (the e^3 left out is
+// below 2^-57). Largest error 1.002 units of 2^-53; the division's is 1, and takes 2.3 us
+// more per 64 columns of the factorization.
+__device__ __forceinline__ double recip_normal(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 
 // x^(-1/3): an FP32 estimate y (exp2 of log2) times the binomial series of

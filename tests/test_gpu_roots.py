@@ -42,3 +42,21 @@ def test_inverse_cube_root(lo, hi):
     exact = 1.0 / np.cbrt(np.longdouble(x))
     assert _err(own, exact) <= (1.34 if -30 <= lo and hi <= 30 else 2.0) * U
     assert _err(cuda, exact) <= 2.0 * U
+
+
+# x^(-1/2): the last sum rounds (1), the product x y rounds and half of it counts, the e^3 left out is
+# 5/16 2^-57 (0.02). 1/x: the last sum, and e^3 of 2^-57 (0.07). Every normal number whose result is one.
+@pytest.mark.parametrize("which,bound", [(abi.ROOT_RSQRT, 1.53), (abi.ROOT_RECIP, 1.08)])
+@pytest.mark.parametrize("lo,hi", [(-307.6, 307.6), (-307.6, -300), (300, 307.6), (-1, 1)])
+def test_hardware_estimates(which, bound, lo, hi):
+    x = _samples(lo, hi)
+    own, cuda = _roots(which, x)
+    exact = 1.0 / (np.sqrt(np.longdouble(x)) if which == abi.ROOT_RSQRT else np.longdouble(x))
+    assert _err(own, exact) <= bound * U
+    assert _err(cuda, exact) <= (2.0 if which == abi.ROOT_RSQRT else 1.0) * U
+
+
+def test_beyond_normal_numbers():
+    """What rsqrt_normal's callers rely on: no finite result there."""
+    own, _ = _roots(abi.ROOT_RSQRT, np.array([0.0, 5e-324, 2e-308, np.inf, np.nan, -1.0]))
+    assert not np.isfinite(own).any()

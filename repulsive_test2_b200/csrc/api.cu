@@ -41,11 +41,15 @@ void set_error(tpe_ctx* ctx, int32_t code, const std::string& msg) {
     if (ctx) ctx->err = msg;
 }
 
-KernelScope::KernelScope(tpe_ctx* c, int g, int64_t n) : ctx(c), group(g) {
+void KernelScope::count(int64_t n) {
     ctx->launches += n;
     ctx->prof_launches[TPE_KGROUP_COUNT] += n;
+    if (ctx->profiling) ctx->prof_launches[group] += n;
+}
+
+KernelScope::KernelScope(tpe_ctx* c, int g, int64_t n) : ctx(c), group(g) {
+    count(n);
     if (!ctx->profiling) return;
-    ctx->prof_launches[g] += n;
     cudaEvent_t a;
     if (ctx->prof_pool.size() >= 2) {
         a = ctx->prof_pool.back();

@@ -853,7 +853,7 @@ int32_t build_tree_device(tpe_ctx* ctx, const DevTree& t) {
     const cudaStream_t st = ctx->stream;
     const int32_t E = t.E;
     const unsigned flat = (unsigned)((E + 255) / 256);
-    KernelScope ks(ctx, TPE_KGROUP_ENERGY, 4 + 4 * t.top);
+    KernelScope ks(ctx, TPE_KGROUP_ENERGY, 2);
     const size_t smem = sizeof(double) * std::max<size_t>(12 * (kSeq + 1), (size_t)1 << kPairDepth);
     TPE_CUDA_TRY(cudaFuncSetAttribute(tree_sums_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     TPE_CUDA_TRY(cudaFuncSetAttribute(tree_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -870,6 +870,7 @@ int32_t build_tree_device(tpe_ctx* ctx, const DevTree& t) {
             TPE_CUDA_TRY(cudaStreamWaitEvent(side[l], ev[l], 0));
             tree_sums_kernel<<<dim3(1u << l, 2), 1024, smem, side[l]>>>(t, (1 << l) - 1);
             TPE_CUDA_TRY(cudaEventRecord(ev[l], side[l]));
+            ks.count(1);
         }
         const unsigned nn = 1u << l;
         const int32_t n = (E + (int32_t)nn - 1) / (int32_t)nn;
@@ -880,10 +881,15 @@ int32_t build_tree_device(tpe_ctx* ctx, const DevTree& t) {
         tree_spread_kernel<<<per, 256, 0, st>>>(t, l);
         tree_keys_kernel<<<per, 256, 0, st>>>(t, l);
         tree_tile_kernel<<<dim3(tiles, nn), kTile / 2, 0, st>>>(t, l, 2);
+        ks.count(4);  // (with the order)
         for (int32_t k = 2 * kTile; k <= P; k *= 2) {
             const dim3 grid((unsigned)(P / 2 / 256), nn);
             tree_step_kernel<<<grid, 256, 0, st>>>(t, l, k, 0);
-            for (int32_t h = k / 4; h >= kTile; h /= 2) tree_step_kernel<<<grid, 256, 0, st>>>(t, l, k, h);
+            ks.count(2);
+            for (int32_t h = k / 4; h >= kTile; h /= 2) {
+                tree_step_kernel<<<grid, 256, 0, st>>>(t, l, k, h);
+                ks.count(1);
+            }
             tree_tile_kernel<<<dim3(tiles, nn), kTile / 2, 0, st>>>(t, l, k);
         }
         tree_order_kernel<<<flat, 256, 0, st>>>(t, l);
@@ -892,9 +898,13 @@ int32_t build_tree_device(tpe_ctx* ctx, const DevTree& t) {
     if (t.top > early) {
         const int32_t first = (1 << early) - 1, nn = (1 << t.top) - 1 - first;
         tree_sums_kernel<<<dim3((unsigned)nn, 2), 1024, smem, st>>>(t, first);
+        ks.count(1);
     }
     for (int l = 0; l < early; l++) TPE_CUDA_TRY(cudaStreamWaitEvent(st, ev[l], 0));
-    if (t.top > 0) tree_top_kernel<<<(1u << t.top) - 1, 1024, 0, st>>>(t);
+    if (t.top > 0) {
+        tree_top_kernel<<<(1u << t.top) - 1, 1024, 0, st>>>(t);
+        ks.count(1);
+    }
     TPE_CUDA_TRY(cudaGetLastError());
     return TPE_OK;
 }

@@ -236,6 +236,7 @@ struct KernelScope {
     cudaEvent_t b = nullptr;
     KernelScope(tpe_ctx* c, int g, int64_t n);
     ~KernelScope();
+    void count(int64_t n);  // n more launches
 };
 
 void set_error(tpe_ctx* ctx, int32_t code, const std::string& msg);

@@ -170,12 +170,15 @@ const char* tpe_last_error(const tpe_ctx* ctx);
  * TPE_TUNE_FACTOR_POLLS, TPE_TUNE_SOLVE_POLLS: polls after which a wait inside the FP64
  *   factorization or its triangular solves gives up (0: some seconds' worth, the default).
  * TPE_TUNE_FACTOR_BLOCKS: thread blocks of the FP64 factorization (0: by its order, the
- *   default; 1: as where other kernels hold the rest of the device). */
+ *   default; 1: as where other kernels hold the rest of the device).
+ * TPE_TUNE_MIXED_DIRECT: most vertices for which the mixed mode takes the FP64 factor (0:
+ *   the FP32 factor at any size; -1: 5000, the default). */
 enum {
     TPE_TUNE_FAIL_ALLOC = 0,
     TPE_TUNE_FACTOR_POLLS = 1,
     TPE_TUNE_SOLVE_POLLS = 2,
-    TPE_TUNE_FACTOR_BLOCKS = 3
+    TPE_TUNE_FACTOR_BLOCKS = 3,
+    TPE_TUNE_MIXED_DIRECT = 4
 };
 int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value);
 /* The roots of the pair kernels at x[0..n) (device arrays): out[2 i] as those kernels form

@@ -44,7 +44,7 @@ FACTOR_LDLT, FACTOR_LU = 0, 1
 PRECISION_FP64, PRECISION_MIXED = 0, 1
 GEMM_FP64, GEMM_INT8_EMULATED = 0, 1
 BCT_HIGH, BCT_LOW = 0, 1
-TUNE_FAIL_ALLOC, TUNE_FACTOR_POLLS, TUNE_SOLVE_POLLS, TUNE_FACTOR_BLOCKS = range(4)
+TUNE_FAIL_ALLOC, TUNE_FACTOR_POLLS, TUNE_SOLVE_POLLS, TUNE_FACTOR_BLOCKS, TUNE_MIXED_DIRECT = range(5)
 ROOT_RSQRT, ROOT_INV_CBRT, ROOT_RECIP = range(3)
 
 PHASE_KEYS = ["dE", "energy", "bHigh", "bLow", "assembleA", "expand", "saddle", "factor",

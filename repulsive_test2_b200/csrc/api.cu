@@ -546,7 +546,7 @@ int32_t op_finalize(tpe_ctx* ctx, int32_t V, int32_t k, bool* singular,
     };
     const bool mixed = o && o->precision == TPE_PRECISION_MIXED && nrhs <= kMixedMaxRhs;
     // at smaller sizes the FP64 factor is the faster one: its solves, held to the same residual
-    const bool direct = mixed && may_direct && V <= kMixedDirect;
+    const bool direct = mixed && may_direct && V <= ctx->mixed_direct;
     const size_t nv = (size_t)nrhs * V;
     double *R = nullptr, *D = nullptr, *AX = nullptr;  // residuals, corrections, A X
     // AX = A X, then residuals and norms against the nc rows at C and those at b
@@ -1540,6 +1540,7 @@ int32_t tpe_tune(tpe_ctx* ctx, int32_t what, int64_t value) {
             case TPE_TUNE_FAIL_ALLOC: ctx->fail_alloc = std::max<int64_t>(value, 0); return TPE_OK;
             case TPE_TUNE_FACTOR_POLLS: ctx->factor_polls = bounded(1 << 22); return TPE_OK;
             case TPE_TUNE_SOLVE_POLLS: ctx->solve_polls = bounded(1 << 22); return TPE_OK;
+            case TPE_TUNE_MIXED_DIRECT: ctx->mixed_direct = value < 0 ? kMixedDirect : bounded(INT32_MAX); return TPE_OK;
             case TPE_TUNE_FACTOR_BLOCKS: ctx->factor_blocks = bounded(2 * ctx->num_sms); return TPE_OK;
             default: set_error(ctx, TPE_ERR_BAD_ARG, "tpe_tune: unknown setting"); return TPE_ERR_BAD_ARG;
         }
@@ -1954,7 +1955,7 @@ int32_t step_impl(tpe_ctx* ctx, const tpe_constraint* set, int32_t nblocks, cons
         // The FP64 factorization of a small constraint set takes the right-hand
         // sides along (their forward solves), so there the gradient runs beside
         // the assembly, on all SMs.
-        ctx->grad_first = S.k <= kLargeSchur && (o->precision != TPE_PRECISION_MIXED || V <= kMixedDirect ||
+        ctx->grad_first = S.k <= kLargeSchur && (o->precision != TPE_PRECISION_MIXED || V <= ctx->mixed_direct ||
                                                  3 * (S.k + 1) > kMixedMaxRhs);
         if (ctx->grad_first) TPE_TRY(launch_gradient(ctx));
     } else {

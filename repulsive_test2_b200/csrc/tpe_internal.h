@@ -211,6 +211,7 @@ struct tpe_ctx {
 
     // settings of tpe_tune
     int64_t fail_alloc = 0;  // the growth of a device buffer that fails (1: the next one)
+    int32_t mixed_direct = tpe::kMixedDirect;
     int32_t factor_polls = 0, solve_polls = 0, factor_blocks = 0;  // chol_dag.cu (0: its own)
 
     // instrumentation: kernel launch count and per-group CUDA-event timing

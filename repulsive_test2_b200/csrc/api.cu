@@ -348,7 +348,7 @@ __global__ void step_batch_kernel(const double* __restrict__ p, const double* __
 
 // One projection correction for each active trial a = idx[y]: the Newton step
 // x = -sum_s Y[s] lam_a[s] - mu_a[c] / (rho sqrt V) (the same operations, in the
-// same order, as combine_kernel) added to the positions cur[a]; bad[a] = 1 when
+// same order, as combine_final_kernel) added to the positions cur[a]; bad[a] = 1 when
 // x has a non-finite entry (the trial is then abandoned).
 __global__ void step_kernel(const double* __restrict__ p, const double* __restrict__ dir,
                             double tau, int64_t n, double* __restrict__ out) {
@@ -1501,7 +1501,7 @@ void tpe_destroy(tpe_ctx* ctx) {
                       &ctx->flat3, &ctx->dir, &ctx->pairM, &ctx->edge_m, &ctx->mat_A, &ctx->mat_L,
                       &ctx->mat_Linv, &ctx->mat_B, &ctx->mat_B0, &ctx->con_C, &ctx->con_Y,
                       &ctx->con_phi, &ctx->con_blocks, &ctx->con_ell0, &ctx->con_red, &ctx->con_part, &ctx->oz_planes, &ctx->oz_err, &ctx->oz_base, &ctx->bh_buf, &ctx->rhs,
-                      &ctx->sol, &ctx->tmp, &ctx->solve_scratch, &ctx->status,
+                      &ctx->sol, &ctx->tmp, &ctx->status,
                       &ctx->trial_raw, &ctx->trial_cur, &ctx->mx_d, &ctx->mx_dinv, &ctx->mx_S,
                       &ctx->mx_Lhi, &ctx->mx_Llo, &ctx->mx_Zhi, &ctx->mx_Zlo, &ctx->mx_Whi,
                       &ctx->mx_Wlo, &ctx->mx_Thi, &ctx->mx_Tlo, &ctx->mx_T2hi, &ctx->mx_T2lo, &ctx->mx_vec, &ctx->mx_part,

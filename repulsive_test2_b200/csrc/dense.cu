@@ -12,6 +12,9 @@ namespace {
 
 // ---- C = alpha A B^T + beta C on the FP64 tensor cores ------------------------
 //
+// For the public product (tpe_gemm_nt_device) alone: the step's own products are chol_dag.cu's
+// and ozaki.cu's.
+//
 // mma.sync m8n8k4 f64: 128x128 output tiles, 8 warps as 2 (rows) x 4 (cols), each
 // warp 64x32 = 8x4 MMA tiles. K runs in chunks of 32 staged by 16-byte cp.async
 // into two shared-memory buffers; rows are padded to 36 doubles (72 words = 8

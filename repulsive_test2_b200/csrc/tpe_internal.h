@@ -196,7 +196,7 @@ struct tpe_ctx {
     tpe::DevBuf mat_A, mat_L, mat_Linv, mat_B, mat_B0;
     tpe::DevBuf con_C, con_Y, con_phi, con_blocks, con_ell0, con_red;
     tpe::DevBuf con_part;  // split partial reductions of the constraint rows
-    tpe::DevBuf rhs, sol, tmp, solve_scratch;
+    tpe::DevBuf rhs, sol, tmp;
     tpe::DevBuf status;                     // device-side int flags
     tpe::DevBuf trial_raw, trial_cur;       // batched line-search trials (K x 3V each)
     tpe::SaddleOp op;
@@ -207,7 +207,6 @@ struct tpe_ctx {
     tpe::MixedFactor mf;
     void* h_stage = nullptr;  // pinned staging of small device-to-host copies (download_many)
     size_t h_stage_bytes = 0;
-    std::vector<double> h_tmp;
 
     // settings of tpe_tune
     int64_t fail_alloc = 0;  // the growth of a device buffer that fails (1: the next one)

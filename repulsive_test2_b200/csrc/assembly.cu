@@ -564,9 +564,11 @@ int32_t assemble_fp64(tpe_ctx* ctx, double alpha, double beta, double eps, doubl
         const double s = (beta - 1.0) / alpha;
         const double distExp = 2.0 * (s - 1.0) + 1.0;
         // rows per warp: short marches where there are few warps, few first rows on large
-        // curves (with the band, us: V = 128 24 / 28 / 35 at 4 / 8 / 16 rows, 777 37 / 31 / 39,
-        // 2048 75 / 70 / 67 / 97 at 8 / 16 / 32 / 64, 8192 599 / 559 / 545 at 16 / 32 / 64)
-        const int32_t R = V >= 3072 ? 64 : (V >= 1400 ? 32 : (V >= 400 ? 8 : 4));
+        // curves (with the band, us: at 4 / 8 rows V = 400 25 / 28, 500 29.2 / 29.4, 777 35 / 32;
+        // at 8 / 16 1000 34 / 42, 1200 43.6 / 43.5, 1400 48 / 44; at 16 / 32 1700 57 / 65, 2048
+        // 68 / 66, 2600 93 / 93, 3600 148 / 139; at 32 / 64 4096 171 / 169, 6000 320 / 328, 8192
+        // 564 / 551)
+        const int32_t R = V >= 7000 ? 64 : V >= 1900 ? 32 : V >= 1200 ? 16 : V >= 550 ? 8 : 4;
         const int32_t ncs = (V + kStrip - 1) / kStrip, nrb = (V + R - 1) / R;
         TPE_TRY(ensure(ctx, ctx->tmp, sizeof(double2) * (size_t)(ncs + nrb) * V));
         double2* rowslot = ctx->tmp.as<double2>();

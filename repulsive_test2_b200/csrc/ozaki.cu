@@ -522,8 +522,9 @@ int32_t ozaki_status(tpe_ctx* ctx, cudaStream_t stream) {
 namespace {
 
 // Largest block factored and inverted by the FP64 data-flow kernel (per-edge step
-// with blocks of 512 / 1024 / 2048 / 4096, ms: V = 2500 10.6 / 9.0 / 8.6 / 9.4, 4096
-// 18.7 / 17.5 / 17.8 / 19.1, 8192 62.3 / 60.0 / 61.0 / 64.5).
+// with blocks of 512 / 1024 / 2048, ms: V = 1500 5.9 / 5.1 / 4.6, 2500 10.1 / 8.5 / 8.2, 4096
+// 18.0 / 16.9 / 15.1, 8192 61.2 / 59.1 / 55.1). The plain FP64 step takes 4.0, 6.3, 14.4
+// and 68.8 of them: below some 6000 vertices the int8 inverses do not pay.
 constexpr int32_t kBase = 2048;
 
 // The base block size: kBase, or TPE_INT8_BASE (128..kBase) to test the

@@ -12,16 +12,18 @@
 // ordered (I, v) where the edge-pair form needs 4 of each. For a vertex that no
 // edge joins to I, M(I, v) is m_v, the length of all edges at v. The few near
 // vertices of I (its endpoints and their neighbours, a sorted list per edge)
-// are masked out of the sweep; the near ones that are not endpoints are summed
-// over their disjoint edges one by one afterwards.
+// are masked out of the sweep, in a copy of its inner loop for the groups of 32
+// vertices that hold one; the near ones that are not endpoints are summed over
+// their disjoint edges one by one afterwards.
 //
 // Bound: the FP64 pipe and its latency. 52 FP64 instructions per ordered (I, v)
 // for the energy, 104 for the gradient; at 8192 edges the pipe is active 65 and
 // 70 % of the time (three to four warps per scheduler: 128 and 168 registers). The sweep's common
 // case has no branch, so that the runs of a thread's edges interleave: with the
-// rare cases tested one by one the same sums took 343 and 685 us. Measured, 8192
-// edges of a closed curve: energy 699 -> 276 us, gradient 2239 -> 608 us against
-// the edge-pair kernels; 128 edges: 160 -> 13 and 239 -> 31 us.
+// rare cases tested one by one the same sums took 343 and 685 us, with the masks in
+// the one loop 276 and 608. Measured, 8192 edges of a closed curve: energy 699 -> 264
+// us, gradient 2239 -> 583 us against the edge-pair kernels; 128 edges: 160 -> 14 and
+// 239 -> 31 us.
 //
 // Work split: a worker of 128 threads owns 128 R consecutive edges (R per
 // thread, so that a run of edges shares its vertices' distances) and sweeps a
@@ -195,13 +197,25 @@ __device__ __forceinline__ double near_length(const EvTopo& t, const double4* __
     return m;
 }
 
+// No edge is disjoint from this one: it has no terms, whatever its coordinates.
+__device__ __forceinline__ bool lonely(const EvTopo& t, int2 ei) {
+    int32_t n = 0;  // edges at its vertices
+    for (int s = 0; s < (ei.x == ei.y ? 1 : 2); s++) {
+        const int32_t w = s ? ei.y : ei.x;
+        for (int32_t k = t.inc_off[w]; k < t.inc_off[w + 1]; k++) {
+            const int2 e = t.edges[t.inc[k] >> 1];
+            if (e.x == e.y ? (t.inc[k] & 1) == 0 : !(s && (e.x == ei.x || e.y == ei.x))) n++;
+        }
+    }
+    return n == t.E;
+}
+
 // Sweeps the vertices [vb, vb + n) (n <= kTile, staged from sm.sv[s0] on) for the
 // thread's R edges. CHAIN: the edges run head to tail (R + 1 vertices), else
 // every edge has its own two. near_lo / near_hi bound the thread's near slots.
 template <int MODE, int R, bool GRAD, bool CHAIN>
 __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_t n, const EvTopo& t, int32_t I0,
-                                      const V3 (&P)[CHAIN ? R + 1 : 2 * R],
-                                      const int32_t (&ip)[CHAIN ? R + 1 : 2 * R], const double (&pw)[R],
+                                      const V3 (&P)[CHAIN ? R + 1 : 2 * R], const double (&pw)[R],
                                       int32_t near_lo, int32_t near_hi, double alpha, double beta,
                                       double eps, double (&S)[R], V3 (&F)[CHAIN ? R + 1 : 2 * R]) {
     constexpr int NV = CHAIN ? R + 1 : 2 * R;
@@ -223,7 +237,11 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
         }
         const bool careful = __any_sync(0xffffffffu, any != 0u);
         const int32_t gn = min(32, n - g0);
-        for (int32_t j = 0; j < gn; j++) {
+        // MASKED: near pairs are left out, whatever their values (a distance of zero, a
+        // coordinate that is no number)
+        auto vertex = [&](auto masked, int32_t j) {
+            constexpr bool MASKED = decltype(masked)::value;
+            auto off = [&](int r) { return MASKED && (mask[r] >> j & 1u); };
             const double4 q4 = sm.sv[s0 + g0 + j];
             const V3 q{q4.x, q4.y, q4.z};
             V3 d[NV], c[R];
@@ -235,8 +253,10 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
             for (int a = 0; a < NV; a++) {
                 d[a] = sub(P[a], q);
                 x[a] = dot3(d[a], d[a]);
-                // an endpoint against itself: any finite distance, its edges are masked
-                if (careful && ip[a] == base + j) x[a] = 1.0;
+                if (MASKED && (CHAIN ? (a == 0 || off(a - 1)) && (a == R || off(a)) : off(a / 2))) {
+                    d[a] = {0.0, 0.0, 0.0};  // (no edge of this point counts)
+                    x[a] = 1.0;
+                }
                 if (MODE == 1)
                     rare |= !dist_power_fast(x[a], eps, G[a], gI[a]);
                 else
@@ -250,7 +270,7 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
                 const bool first = x[a] <= x[b];
                 const V3 dn{first ? d[a].x : d[b].x, first ? d[a].y : d[b].y, first ? d[a].z : d[b].z};
                 c[r] = cross3(e, dn);
-                c2[r] = dot3(c[r], c[r]);
+                c2[r] = off(r) ? 1.0 : dot3(c[r], c[r]);
                 if (MODE == 1)
                     rare |= !area_power_fast(c2[r], eps, N[r], kN[r]);
                 else
@@ -268,7 +288,7 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
             for (int r = 0; r < R; r++) {
                 const int a = CHAIN ? r : 2 * r, b = a + 1;
                 const V3 e = sub(P[b], P[a]);
-                if (careful && (mask[r] >> j & 1u)) N[r] = kN[r] = 0.0;
+                if (off(r)) continue;
                 const double GS = G[a] + G[b];
                 const double NG = N[r] * GS;
                 S[r] += q4.w * NG;
@@ -307,7 +327,11 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
                 k0 += __shfl_xor_sync(0xffffffffu, k0, 1);
                 if ((lane & 7) == 0) sm.acc[warp][g0 + j][lane >> 3] = k0;
             }
-        }
+        };
+        if (careful)
+            for (int32_t j = 0; j < gn; j++) vertex(std::true_type{}, j);
+        else
+            for (int32_t j = 0; j < gn; j++) vertex(std::false_type{}, j);
     }
 }
 
@@ -346,7 +370,7 @@ __device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chun
     int32_t s0 = 0, s1 = 0;  // the vertices in sm.sv
     V3 f1[R], f2[R];
     // the vertices [v0, v1) for the edges' points P
-    auto march = [&](auto chained, const auto& P, const auto& ip, auto& F, int32_t v0, int32_t v1) {
+    auto march = [&](auto chained, const auto& P, auto& F, int32_t v0, int32_t v1) {
         for (int32_t vb = v0; vb < v1; vb += kTile) {
             const int32_t n = min(kTile, v1 - vb);
             if (vb >= s1) {
@@ -356,7 +380,7 @@ __device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chun
                 if (tid < s1 - s0) sm.sv[tid] = vr[s0 + tid];
                 worker_sync(bar);
             }
-            sweep<MODE, R, GRAD, decltype(chained)::value>(sm, vb - s0, vb, n, t, I0, P, ip, pw, near_lo, near_hi,
+            sweep<MODE, R, GRAD, decltype(chained)::value>(sm, vb - s0, vb, n, t, I0, P, pw, near_lo, near_hi,
                                                            alpha, beta, eps, S, F);
             if (GRAD) {
                 worker_sync(bar);
@@ -375,14 +399,12 @@ __device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chun
         for (int r = 0; r < R; r++) S[r] = 0.0;
         if (R > 1 && run) {
             V3 P[R + 1], F[R + 1];
-            int32_t ip[R + 1];
 #pragma unroll
             for (int a = 0; a <= R; a++) {
                 P[a] = a < R ? p1[a < R ? a : 0] : p2[R - 1];
-                ip[a] = a < R ? ei[a < R ? a : 0].x : ei[R - 1].y;
                 F[a] = {0.0, 0.0, 0.0};
             }
-            march(std::true_type{}, P, ip, F, v0, v1);
+            march(std::true_type{}, P, F, v0, v1);
             // a shared vertex's force goes to the edge it begins
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -392,16 +414,13 @@ __device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chun
             f2[R - 1] = F[R];
         } else {
             V3 P[2 * R], F[2 * R];
-            int32_t ip[2 * R];
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 P[2 * r] = p1[r];
                 P[2 * r + 1] = p2[r];
-                ip[2 * r] = ei[r].x;
-                ip[2 * r + 1] = ei[r].y;
                 F[2 * r] = F[2 * r + 1] = {0.0, 0.0, 0.0};
             }
-            march(std::false_type{}, P, ip, F, v0, v1);
+            march(std::false_type{}, P, F, v0, v1);
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 f1[r] = F[2 * r];
@@ -426,7 +445,7 @@ __device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chun
                     S[r] += m * (pt.N * pt.GS);
                 }
             }
-            en += pw[r] * S[r];
+            if (isfinite(pw[r]) || !lonely(t, t.edges[I])) en += pw[r] * S[r];
         }
         for (int o = 16; o > 0; o >>= 1) en += __shfl_down_sync(0xffffffffu, en, o);
         if ((tid & 31) == 0) sm.red[ch - ch0][tid >> 5] = en;
@@ -558,7 +577,10 @@ ev_edge_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
     }
     const V3 e = sub(p2, p1);
     const double raw = sqrt(dot3(e, e));
-    if (!(raw < 1e-14)) {
+    if (!(isfinite(raw) && isfinite(pw)) && lonely(t, edge)) {
+        f1 = f2 = {0.0, 0.0, 0.0};
+        S = 0.0;
+    } else if (!(raw < 1e-14)) {
         const double dl = (Rl + (1.0 - alpha) * pow(a4.w, -alpha) * S) / raw;
         axpy3(f1, -dl, e);
         axpy3(f2, dl, e);
@@ -569,7 +591,7 @@ ev_edge_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
     edge_f[3 * (int64_t)t.E + I] = f2.x;
     edge_f[4 * (int64_t)t.E + I] = f2.y;
     edge_f[5 * (int64_t)t.E + I] = f2.z;
-    edge_e[I] = pw * S;
+    edge_e[I] = !isfinite(pw) && lonely(t, edge) ? 0.0 : pw * S;
 }
 
 // grad[v] = 1/8 (its edges' forces + its own sweep partials + the edges it is near to).
@@ -667,8 +689,8 @@ EvTopo topo_of(const tpe_ctx* ctx) {
 
 // Edges per thread and vertices per item. Two edges per thread from 2048 edges
 // on (1.5 distances per area and one warp reduction per two edges: 8192 edges
-// 276 against 320 us for the energy, 608 against 680 for the gradient; equal at
-// 2048; four edges per thread spill). Below, one: more items, shorter chains
+// 264 against 306 us for the energy, 583 against 657 for the gradient, 2048 edges 37
+// against 37 and 74 against 81; four edges per thread spill). Below, one: more items, shorter chains
 // (1024 edges: 21 against 23 us). Items of 8 to 128 vertices, about six per SM.
 // Neither depends on how many curves a launch has: the order of an energy's sum, and with
 // it its last bits, are those of the curve alone (differences of energies from launches of

@@ -191,7 +191,9 @@ int32_t tpe_root_check(tpe_ctx* ctx, int32_t which, const double* x, int32_t n, 
 /* Replaces calculateDisjointPairs (src/core/tangentPointEnergy.ts:33-47): the
  * ordered disjoint-pair lists are never materialised; disjointness is tested
  * in-kernel from endpoint indices. Uploads edges and the vertex->edge
- * incidence used by the gather kernels. */
+ * incidence used by the gather kernels. The first energy or gradient on the new
+ * topology also lists each edge's neighbours on the host (8192 edges: 0.4 ms), so a
+ * program with several curves keeps a context for each. */
 int32_t tpe_set_topology(tpe_ctx* ctx, const int32_t* edges, int32_t E, int32_t V);
 /* Optional: materialise the ordered lists exactly as calculateDisjointPairs
  * (offsets[E+1], partners[cap]); for callers that still want them. */

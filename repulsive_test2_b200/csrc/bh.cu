@@ -351,7 +351,7 @@ bh_reduce_kernel(const double* __restrict__ val, const long long* __restrict__ c
 //   below: one block per subtree, its edges in shared memory, all levels in one launch.
 // 131072 edges: a call takes 2.4 ms (23.6 with the host's tree, 19 of them its build and
 // copies): 1.6 the tree, 0.7 the traversal, whose powers are products at exponents 3
-// and 6 (2.35 with pow). Bound: the sort's 90 small launches, 0.9 ms, beside which the
+// and 6 (2.35 with pow). Bound: the sort's 84 small launches, 0.9 ms, beside which the
 // root's sums run, one addition after the other (0.6 ms, 9 clocks each).
 constexpr int kSubtree = 1024;
 constexpr int kSubThr = 512;

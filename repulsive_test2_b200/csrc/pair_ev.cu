@@ -17,8 +17,8 @@
 // their disjoint edges one by one afterwards.
 //
 // Bound: the FP64 pipe and its latency. 52 FP64 instructions per ordered (I, v)
-// for the energy, 104 for the gradient; at 8192 edges the pipe is active 65 and
-// 70 % of the time (three to four warps per scheduler: 128 and 168 registers). The sweep's common
+// for the energy, 104 for the gradient; at 8192 edges the pipe is active 82 and
+// 78 % of the time (three to four warps per scheduler: 120 and 168 registers). The sweep's common
 // case has no branch, so that the runs of a thread's edges interleave: with the
 // rare cases tested one by one the same sums took 343 and 685 us, with the masks in
 // the one loop 276 and 608. Measured, 8192 edges of a closed curve: energy 699 -> 264

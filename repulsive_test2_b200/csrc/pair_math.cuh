@@ -20,7 +20,7 @@ __device__ __forceinline__ double rsqrt_normal(double x) {
 
 // 1/x for normal x whose reciprocal is normal: the hardware's approximation y (20 bits)
 // times the geometric series of 1/(1 - e), e = 1 - x y, through e^2 (the e^3 left out is
-// below 2^-57). Largest error 1.002 units of 2^-53; the division's is 1, and takes 2.3 us
+// below 2^-57). Largest error 1.002 units of 2^-53; the division's is 1, and takes 2.5 us
 // more per 64 columns of the factorization.
 __device__ __forceinline__ double recip_normal(double x) {
     double y;

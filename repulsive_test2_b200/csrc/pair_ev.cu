@@ -185,12 +185,25 @@ struct PairTerms {
     }
 };
 
-// M(I, v) of a near vertex slot v: the edges at v that are disjoint from I.
-__device__ __forceinline__ double near_length(const EvTopo& t, const double4* __restrict__ ea, int2 ei,
-                                              int32_t v) {
+// M(I, v) of a near vertex slot v that is not an endpoint: the edges at v that are disjoint
+// from I, m_v of them in all. One by one; at a vertex of many edges as m_v without those that
+// lead to I's endpoints, where they are the smaller part (nothing cancels then).
+__device__ __forceinline__ double near_length(const EvTopo& t, const double4* __restrict__ ea, int2 ei, int32_t v,
+                                              double m_v) {
+    const int32_t w = t.vid[v], k0 = t.inc_off[w], k1 = t.inc_off[w + 1];
+    if (k1 - k0 > 8) {
+        double off = 0.0;
+        for (int s = 0; s < (ei.x == ei.y ? 1 : 2); s++) {
+            const int32_t u = s ? ei.y : ei.x;
+            for (int32_t k = t.inc_off[u]; k < t.inc_off[u + 1]; k++) {
+                const int2 e = t.edges[t.inc[k] >> 1];
+                if (e.x == w || e.y == w) off += ea[t.inc[k] >> 1].w;
+            }
+        }
+        if (off < 0.5 * m_v) return m_v - off;
+    }
     double m = 0.0;
-    const int32_t w = t.vid[v];
-    for (int32_t k = t.inc_off[w]; k < t.inc_off[w + 1]; k++) {
+    for (int32_t k = k0; k < k1; k++) {
         const int32_t J = t.inc[k] >> 1;
         if (disjoint(ei, t.edges[J])) m += ea[J].w;
     }
@@ -228,11 +241,22 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
 #pragma unroll
         for (int r = 0; r < R; r++) {
             mask[r] = I0 + r < t.E ? 0u : 0xffffffffu;
-            if (I0 + r < t.E && near_hi >= base && near_lo < base + 32)
-                for (int32_t k = t.near_off[I0 + r]; k < t.near_off[I0 + r + 1]; k++) {
-                    const int32_t d = t.near[k] - base;
-                    if (d >= 0 && d < 32) mask[r] |= 1u << d;
+            if (I0 + r < t.E && near_hi >= base && near_lo < base + 32) {
+                int32_t k = t.near_off[I0 + r];
+                const int32_t end = t.near_off[I0 + r + 1];
+                for (int32_t h = end; h - k > 16;) {  // (a long list: to its part from base on)
+                    const int32_t mid = (k + h) >> 1;
+                    if (t.near[mid] < base)
+                        k = mid;
+                    else
+                        h = mid;
                 }
+                for (; k < end; k++) {
+                    const int32_t d = t.near[k] - base;
+                    if (d >= 32) break;
+                    if (d >= 0) mask[r] |= 1u << d;
+                }
+            }
             any |= mask[r];
         }
         const bool careful = __any_sync(0xffffffffu, any != 0u);
@@ -337,7 +361,7 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
 
 // Work item (edge block ib, vertex chunks from ch0, `group` of them) of one curve. GRAD:
 // one chunk, edge_acc [ch][kAcc][E] and vert_acc [ib][VA][4]; else each chunk's energy
-// (near pairs included by chunk 0) to part[chunk]. Several chunks have at most kTile
+// (the near pairs dealt over the chunks) to part[chunk]. Several chunks have at most kTile
 // vertices together, staged at once.
 template <int MODE, int R, bool GRAD>
 __device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chunk, int32_t nch, int tid, int bar,
@@ -433,17 +457,14 @@ __device__ __forceinline__ void ev_item(int ib, int ch0, int group, int32_t chun
         for (int r = 0; r < R; r++) {
             const int32_t I = I0 + r;
             if (I >= t.E) break;
-            if (ch == 0) {
-                const int2 edge = t.edges[I];
-                for (int32_t k = t.near_off[I]; k < t.near_off[I + 1]; k++) {
-                    const int32_t v = t.near[k];
-                    if (v == ei[r].x || v == ei[r].y) continue;
-                    const double m = near_length(t, ea, edge, v);
-                    if (m == 0.0) continue;
-                    const double4 q = vr[v];
-                    const PairTerms<MODE> pt(p1[r], p2[r], {q.x, q.y, q.z}, alpha, beta, eps);
-                    S[r] += m * (pt.N * pt.GS);
-                }
+            for (int32_t k = t.near_off[I] + ch; k < t.near_off[I + 1]; k += nch) {
+                const int32_t v = t.near[k];
+                if (v == ei[r].x || v == ei[r].y) continue;
+                const double4 q = vr[v];
+                const double m = near_length(t, ea, t.edges[I], v, q.w);
+                if (m == 0.0) continue;
+                const PairTerms<MODE> pt(p1[r], p2[r], {q.x, q.y, q.z}, alpha, beta, eps);
+                S[r] += m * (pt.N * pt.GS);
             }
             if (isfinite(pw[r]) || !lonely(t, t.edges[I])) en += pw[r] * S[r];
         }
@@ -522,59 +543,73 @@ ev_edge_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
                double beta, double eps, const double* __restrict__ edge_acc,
                const double* __restrict__ vert_acc, double* __restrict__ edge_f,
                double* __restrict__ edge_e) {
-    __shared__ double red[8][kAcc][32];
+    __shared__ double red[8][kAcc + 1][32];
     const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
     const int32_t I = blockIdx.x * 32 + x;
-    double s[kAcc];
-#pragma unroll
-    for (int q = 0; q < kAcc; q++) s[q] = 0.0;
-    if (I < t.E)
-        for (int32_t c = y; c < nch; c += 8)
-#pragma unroll
-            for (int q = 0; q < kAcc; q++) s[q] += edge_acc[((int64_t)c * kAcc + q) * t.E + I];
-#pragma unroll
-    for (int q = 0; q < kAcc; q++) red[y][q][x] = s[q];
-    __syncthreads();
-    if (y != 0 || I >= t.E) return;
-#pragma unroll
-    for (int q = 0; q < kAcc; q++)
-        for (int g = 1; g < 8; g++) s[q] += red[g][q][x];
-    const double4 a4 = ea[I], b4 = eb[I];
+    const bool in = I < t.E;
+    const double4 a4 = ea[in ? I : 0], b4 = eb[in ? I : 0];
     const V3 p1{a4.x, a4.y, a4.z}, p2{b4.x, b4.y, b4.z};
     const double pw = b4.w;
-    const int2 edge = t.edges[I], slot = t.ev[I];
-    V3 f1{s[0], s[1], s[2]}, f2{s[3], s[4], s[5]};
-    double S = s[6], Rl = 0.0;
-    for (int32_t k = t.near_off[I]; k < t.near_off[I + 1]; k++) {
-        const int32_t v = t.near[k];
-        if (v == slot.x || v == slot.y) continue;
-        const double m = near_length(t, ea, edge, v);
-        if (m == 0.0) continue;
-        const double4 q = vr[v];
-        const PairTerms<MODE> pt(p1, p2, {q.x, q.y, q.z}, alpha, beta, eps);
-        S += m * (pt.N * pt.GS);
-        const double mp = m * pw;
-        const V3 kc{mp * pt.kc.x, mp * pt.kc.y, mp * pt.kc.z};
-        sub_cross(f1, pt.d2, kc);
-        add_cross(f2, pt.d1, kc);
-        const double tn = -beta * (mp * pt.N);
-        axpy3(f1, (tn * pt.G1) * pt.g1, pt.d1);
-        axpy3(f2, (tn * pt.G2) * pt.g2, pt.d2);
-    }
-    // dE/dl_I through M: the edges K disjoint from I, at both of I's vertices
+    const int2 edge = t.edges[in ? I : 0], slot = t.ev[in ? I : 0];
+    V3 f1{0.0, 0.0, 0.0}, f2 = f1;
+    double S = 0.0, Rl = 0.0;
+    if (in) {
+        for (int32_t c = y; c < nch; c += 8) {
+            const double* o = edge_acc + (int64_t)c * kAcc * t.E + I;
+            f1.x += o[0];
+            f1.y += o[t.E];
+            f1.z += o[2 * (int64_t)t.E];
+            f2.x += o[3 * (int64_t)t.E];
+            f2.y += o[4 * (int64_t)t.E];
+            f2.z += o[5 * (int64_t)t.E];
+            S += o[6 * (int64_t)t.E];
+        }
+        for (int32_t k = t.near_off[I] + y; k < t.near_off[I + 1]; k += 8) {
+            const int32_t v = t.near[k];
+            if (v == slot.x || v == slot.y) continue;
+            const double4 q = vr[v];
+            const double m = near_length(t, ea, edge, v, q.w);
+            if (m == 0.0) continue;
+            const PairTerms<MODE> pt(p1, p2, {q.x, q.y, q.z}, alpha, beta, eps);
+            S += m * (pt.N * pt.GS);
+            const double mp = m * pw;
+            const V3 kc{mp * pt.kc.x, mp * pt.kc.y, mp * pt.kc.z};
+            sub_cross(f1, pt.d2, kc);
+            add_cross(f2, pt.d1, kc);
+            const double tn = -beta * (mp * pt.N);
+            axpy3(f1, (tn * pt.G1) * pt.g1, pt.d1);
+            axpy3(f2, (tn * pt.G2) * pt.g2, pt.d2);
+        }
+        // dE/dl_I through M: the edges K disjoint from I, at both of I's vertices
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-        const int32_t v = e ? slot.y : slot.x;
-        const V3 q = e ? p2 : p1;
-        for (int32_t b = 0; b < nib; b++) Rl += vert_acc[((int64_t)b * t.VA + v) * 4 + 3];
-        for (int32_t k = t.rev_off[v]; k < t.rev_off[v + 1]; k++) {
-            const int32_t K = t.rev[k];
-            if (!disjoint(edge, t.edges[K])) continue;
-            const double4 ka = ea[K], kb = eb[K];
-            const PairTerms<MODE> pt({ka.x, ka.y, ka.z}, {kb.x, kb.y, kb.z}, q, alpha, beta, eps);
-            Rl += kb.w * (pt.N * pt.GS);
+        for (int e = 0; e < 2; e++) {
+            const int32_t v = e ? slot.y : slot.x;
+            const V3 q = e ? p2 : p1;
+            for (int32_t b = y; b < nib; b += 8) Rl += vert_acc[((int64_t)b * t.VA + v) * 4 + 3];
+            for (int32_t k = t.rev_off[v] + y; k < t.rev_off[v + 1]; k += 8) {
+                const int32_t K = t.rev[k];
+                if (!disjoint(edge, t.edges[K])) continue;
+                const double4 ka = ea[K], kb = eb[K];
+                const PairTerms<MODE> pt({ka.x, ka.y, ka.z}, {kb.x, kb.y, kb.z}, q, alpha, beta, eps);
+                Rl += kb.w * (pt.N * pt.GS);
+            }
         }
     }
+    const double mine[kAcc + 1] = {f1.x, f1.y, f1.z, f2.x, f2.y, f2.z, S, Rl};
+#pragma unroll
+    for (int q = 0; q <= kAcc; q++) red[y][q][x] = mine[q];
+    __syncthreads();
+    if (y != 0 || !in) return;
+    double s[kAcc + 1];
+#pragma unroll
+    for (int q = 0; q <= kAcc; q++) {
+        s[q] = mine[q];
+        for (int g = 1; g < 8; g++) s[q] += red[g][q][x];
+    }
+    f1 = {s[0], s[1], s[2]};
+    f2 = {s[3], s[4], s[5]};
+    S = s[6];
+    Rl = s[7];
     const V3 e = sub(p2, p1);
     const double raw = sqrt(dot3(e, e));
     if (!(isfinite(raw) && isfinite(pw)) && lonely(t, edge)) {
@@ -595,18 +630,19 @@ ev_edge_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
 }
 
 // grad[v] = 1/8 (its edges' forces + its own sweep partials + the edges it is near to).
+// 32 vertices x 8 lanes, as the edges.
 template <int MODE>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 ev_vertex_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb, EvTopo t,
                  int32_t nib, int32_t V, const int32_t* __restrict__ slot_of, const double4* __restrict__ vr,
                  double alpha, double beta, double eps, const double* __restrict__ vert_acc,
                  const double* __restrict__ edge_f, double* __restrict__ grad) {
-    const int32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= V) return;
-    const int32_t v = slot_of[w];
+    __shared__ double red[8][3][32];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int32_t w = blockIdx.x * 32 + x, v = w < V ? slot_of[w] : -1;
     V3 g{0.0, 0.0, 0.0};
     if (v >= 0) {
-        for (int32_t b = 0; b < nib; b++) {
+        for (int32_t b = y; b < nib; b += 8) {
             const double* o = vert_acc + ((int64_t)b * t.VA + v) * 4;
             const double2 xy = *reinterpret_cast<const double2*>(o);
             g.x += xy.x;
@@ -614,9 +650,9 @@ ev_vertex_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
             g.z += o[2];
         }
         const double4 q = vr[v];
-        for (int32_t k = t.rev_off[v]; k < t.rev_off[v + 1]; k++) {
+        for (int32_t k = t.rev_off[v] + y; k < t.rev_off[v + 1]; k += 8) {
             const int32_t I = t.rev[k];
-            const double m = near_length(t, ea, t.edges[I], v);
+            const double m = near_length(t, ea, t.edges[I], v, q.w);
             if (m == 0.0) continue;
             const double4 a = ea[I], b = eb[I];
             const V3 p1{a.x, a.y, a.z}, p2{b.x, b.y, b.z};
@@ -628,16 +664,23 @@ ev_vertex_kernel(const double4* __restrict__ ea, const double4* __restrict__ eb,
             axpy3(g, (tn * pt.G1) * pt.g1, pt.d1);
             axpy3(g, (tn * pt.G2) * pt.g2, pt.d2);
         }
-        for (int32_t k = t.inc_off[w]; k < t.inc_off[w + 1]; k++) {
+        for (int32_t k = t.inc_off[w] + y; k < t.inc_off[w + 1]; k += 8) {
             const int32_t I = t.inc[k] >> 1, c = 3 * (t.inc[k] & 1);
             g.x += edge_f[(int64_t)c * t.E + I];
             g.y += edge_f[(int64_t)(c + 1) * t.E + I];
             g.z += edge_f[(int64_t)(c + 2) * t.E + I];
         }
     }
-    grad[3 * w] = 0.125 * g.x;
-    grad[3 * w + 1] = 0.125 * g.y;
-    grad[3 * w + 2] = 0.125 * g.z;
+    red[y][0][x] = g.x;
+    red[y][1][x] = g.y;
+    red[y][2][x] = g.z;
+    __syncthreads();
+    if (y != 0 || w >= V) return;
+    for (int q = 0; q < 3; q++) {
+        double s = red[0][q][x];
+        for (int h = 1; h < 8; h++) s += red[h][q][x];
+        grad[3 * (int64_t)w + q] = 0.125 * s;
+    }
 }
 
 // Edge records (as edge_prep_kernel) and vertex records (x, y, z, m) of the
@@ -845,7 +888,7 @@ int32_t grad_launch(tpe_ctx* ctx, const EvSplit& s, double alpha, double beta, d
         ea, eb, vr, t, s.nch, s.nib, alpha, beta, eps, acc, vacc, ef, ctx->partial.as<double>());
     TPE_CUDA_TRY(cudaGetLastError());
     if (d_grad) {
-        ev_vertex_kernel<MODE><<<(unsigned)((ctx->V + 127) / 128), 128, 0, ctx->stream>>>(
+        ev_vertex_kernel<MODE><<<(unsigned)((ctx->V + 31) / 32), 256, 0, ctx->stream>>>(
             ea, eb, t, s.nib, ctx->V, ctx->ev_lists.as<int32_t>() + ctx->ev_at[5], vr, alpha, beta, eps,
             vacc, ef, d_grad);
         TPE_CUDA_TRY(cudaGetLastError());

@@ -11,7 +11,7 @@
 // center (bh_ordered_cluster_term, :515-529); a leaf that is not admissible is
 // summed exactly. theta = 0 admits nothing and gives the exact energy.
 //
-// The energy's tree is built on the device (up to 2^19 edges and leaves of 512; on the
+// The energy's tree is built on the device (1300 to 2^19 edges, leaves up to 512; on the
 // host otherwise, and for the block cluster tree), in the oracle's order of operations,
 // so that it is the same tree: split on the coordinate of largest
 // spread of the 6-D points (midpoint, unit tangent), stable sort, the first
@@ -357,6 +357,10 @@ constexpr int kSubtree = 1024;
 constexpr int kSubThr = 512;
 constexpr int kTile = 2048;  // elements sorted in shared memory at the top levels
 constexpr int kSeq = 992;    // a chunk of the sequential sums (31 warps fetch, one adds)
+// Below 1300 edges the host's tree with its copies is the sooner one (a call, us, device / host:
+// smooth curves of 500 edges 408 / 352, 1000 568 / 484, 1500 564 / 531, 2000 587 / 598; random
+// walks 814 / 792, 1459 / 1498, 2224 / 2398, 2808 / 3134).
+constexpr int32_t kDeviceTreeFrom = 1300;
 constexpr int32_t kDeviceTreeEdges = 1 << 19;
 constexpr int kDeviceTreeLeaf = 512;
 constexpr int kPairDepth = 13;  // halvings until 2^19 terms are at most 128
@@ -1003,7 +1007,7 @@ int32_t bh_energy(tpe_ctx* ctx, const double* h_xyz, const double* d_xyz, double
         return TPE_OK;
     }
     // the device builds the tree where its scratch and the shape of a subtree allow
-    const bool device = E <= kDeviceTreeEdges && leaf <= kDeviceTreeLeaf;
+    const bool device = E >= kDeviceTreeFrom && E <= kDeviceTreeEdges && leaf <= kDeviceTreeLeaf;
     Tree tr;
     size_t nn = 1;
     DevTree t{};

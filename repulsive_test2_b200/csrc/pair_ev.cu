@@ -22,8 +22,9 @@
 // case has no branch, so that the runs of a thread's edges interleave: with the
 // rare cases tested one by one the same sums took 343 and 685 us, with the masks in
 // the one loop 276 and 608. Measured, 8192 edges of a closed curve: energy 699 -> 264
-// us, gradient 2239 -> 583 us against the edge-pair kernels; 128 edges: 160 -> 14 and
-// 239 -> 31 us.
+// us, gradient 2239 -> 575 us against the edge-pair kernels; 128 edges: 160 -> 12 and
+// 239 -> 26 us. A hub's lists are dealt over the energy's chunks and over eight rows of
+// the reductions (four hubs of 40 spokes, 964 edges: gradient 274 -> 126 us).
 //
 // Work split: a worker of 128 threads owns 128 R consecutive edges (R per
 // thread, so that a run of edges shares its vertices' distances) and sweeps a
@@ -237,11 +238,11 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
         // bit j of mask[r]: vertex vb + g0 + j is near edge r (or the edge does not exist)
         uint32_t mask[R];
         uint32_t any = 0;
-        const int32_t base = vb + g0;
+        const int32_t base = vb + g0, gn = min(32, n - g0);
 #pragma unroll
         for (int r = 0; r < R; r++) {
             mask[r] = I0 + r < t.E ? 0u : 0xffffffffu;
-            if (I0 + r < t.E && near_hi >= base && near_lo < base + 32) {
+            if (I0 + r < t.E && near_hi >= base && near_lo < base + gn) {
                 int32_t k = t.near_off[I0 + r];
                 const int32_t end = t.near_off[I0 + r + 1];
                 for (int32_t h = end; h - k > 16;) {  // (a long list: to its part from base on)
@@ -253,14 +254,13 @@ __device__ __forceinline__ void sweep(EvSmem& sm, int32_t s0, int32_t vb, int32_
                 }
                 for (; k < end; k++) {
                     const int32_t d = t.near[k] - base;
-                    if (d >= 32) break;
+                    if (d >= gn) break;
                     if (d >= 0) mask[r] |= 1u << d;
                 }
             }
             any |= mask[r];
         }
         const bool careful = __any_sync(0xffffffffu, any != 0u);
-        const int32_t gn = min(32, n - g0);
         // MASKED: near pairs are left out, whatever their values (a distance of zero, a
         // coordinate that is no number)
         auto vertex = [&](auto masked, int32_t j) {
